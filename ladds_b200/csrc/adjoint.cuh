@@ -21,8 +21,8 @@
 //       lr += (da/dr)^T g,  lv += (da/dv)^T g,  lbc += (da/dbc)^T g.
 // Every term but drag is the gradient of a potential (central, zonal J2/J3,
 // tesseral C22/S22 in the rotating frame, third body, cannonball SRP), so its
-// Jacobian is symmetric and (da/dr)^T g = (da/dr) g: a forward-mode
-// directional derivative (dual numbers) of those terms along g.  The SRP
+// Jacobian is symmetric and (da/dr)^T g = (da/dr) g: the directional
+// derivative of those terms along g.  The SRP
 // shadow switch and the atmosphere band are piecewise constant and contribute
 // nothing.  Drag, a = K(|r|) |w| w with w = v + Omega r (co-rotating
 // atmosphere) and K = -0.5e3 rho(h) bcInv, has its transposed Jacobian
@@ -38,95 +38,77 @@
 
 namespace ladds {
 
-struct Dual {
-  double v, d;
-};
-__device__ __forceinline__ Dual operator+(Dual a, Dual b) { return {a.v + b.v, a.d + b.d}; }
-__device__ __forceinline__ Dual operator-(Dual a, Dual b) { return {a.v - b.v, a.d - b.d}; }
-__device__ __forceinline__ Dual operator*(Dual a, Dual b) { return {a.v * b.v, a.d * b.v + a.v * b.d}; }
-__device__ __forceinline__ Dual operator*(double s, Dual a) { return {s * a.v, s * a.d}; }
-__device__ __forceinline__ Dual operator-(double s, Dual a) { return {s - a.v, -a.d}; }
-__device__ __forceinline__ Dual drsqrt(Dual a) {
-  const double r = rsqrt(a.v);
-  return {r, -0.5 * r * r * r * a.d};
-}
-
-// Directional derivative along dr of the potential-derived terms of the FP64
-// acceleration set (everything in accel<false> except drag).
-__device__ __forceinline__ void accelConservativeJvp(uint32_t mask, const double r[3], const double dr[3], double aom,
+// Directional derivative along g of the potential-derived terms of the FP64
+// acceleration set (everything in accel except drag), term by term of
+// earthGravity and accel: with m = r.g and n = -m / |r|^2 (the relative change
+// of 1 / |r| along g), d(1 / |r|^k) = k n / |r|^k.
+__device__ __forceinline__ void accelConservativeJvp(uint32_t mask, const double r[3], const double g[3], double aom,
                                                      const EphEntry &e, double da[3]) {
-  const Dual x{r[0], dr[0]}, y{r[1], dr[1]}, z{r[2], dr[2]};
-  const Dual r2 = x * x + y * y + z * z;
-  const Dual rinv = drsqrt(r2);
-  const Dual rinv2 = rinv * rinv;
-  Dual ax{0, 0}, ay{0, 0}, az{0, 0};
-  if (mask & kPropKEP) {
-    const Dual k = -kMuEarth * (rinv2 * rinv);
-    ax = ax + k * x;
-    ay = ay + k * y;
-    az = az + k * z;
+  const double x = r[0], y = r[1], z = r[2];
+  double c[3] = {0.0, 0.0, 0.0};
+  if (mask & (kPropSOL | kPropSRP)) {
+    // k d / |d|^3, d = s - r (the indirect term and the shadow are constant)
+    const double dx = e.sun[0] - x, dy = e.sun[1] - y, dz = e.sun[2] - z;
+    const double di = rsqrt(dx * dx + dy * dy + dz * dz), di2 = di * di;
+    double k = (mask & kPropSOL) ? kMuSun : 0.0;
+    if ((mask & kPropSRP) && !inShadow(x, y, z, x * x + y * y + z * z, e.sunHat)) k -= kSrpCoef * aom;
+    k *= di2 * di;
+    const double t = 3.0 * di2 * (dx * g[0] + dy * g[1] + dz * g[2]);
+    c[0] += k * (t * dx - g[0]);
+    c[1] += k * (t * dy - g[1]);
+    c[2] += k * (t * dz - g[2]);
   }
-  if (mask & kPropJ2) {
-    const Dual k = (-1.5 * kJ2 * kMuEarth * kREarth * kREarth) * (rinv2 * rinv2 * rinv);
-    const Dual zr2 = z * z * rinv2;
-    ax = ax + k * x * (1.0 - 5.0 * zr2);
-    ay = ay + k * y * (1.0 - 5.0 * zr2);
-    az = az + k * z * (3.0 - 5.0 * zr2);
+  if (mask & kPropLUN) {
+    const double dx = e.moon[0] - x, dy = e.moon[1] - y, dz = e.moon[2] - z;
+    const double di = rsqrt(dx * dx + dy * dy + dz * dz), di2 = di * di;
+    const double k = kMuMoon * (di2 * di);
+    const double t = 3.0 * di2 * (dx * g[0] + dy * g[1] + dz * g[2]);
+    c[0] += k * (t * dx - g[0]);
+    c[1] += k * (t * dy - g[1]);
+    c[2] += k * (t * dz - g[2]);
   }
-  if (mask & kPropJ3) {
-    const Dual k = (-2.5 * kJ3 * kMuEarth * kREarth * kREarth * kREarth) * (rinv2 * rinv2 * rinv2 * rinv);
-    const Dual z2 = z * z;
-    const Dual f = 3.0 * z - 7.0 * (z2 * z * rinv2);
-    ax = ax + k * x * f;
-    ay = ay + k * y * f;
-    az = az + k * (6.0 * z2 - 7.0 * (z2 * z2 * rinv2) - 0.6 * r2);
-  }
-  if (mask & (kPropC22 | kPropS22)) {
-    const double C = (mask & kPropC22) ? kC22 : 0.0;
-    const double S = (mask & kPropS22) ? kS22 : 0.0;
-    const double c = e.cosT, s = e.sinT;
-    const Dual xf = c * x + s * y, ye = (-s) * x + c * y;
-    const Dual g = C * (xf * xf - ye * ye) + (2.0 * S) * (xf * ye);
-    const Dual k = (3.0 * kMuEarth * kREarth * kREarth) * (rinv2 * rinv2 * rinv);
-    const Dual axf = k * (2.0 * (C * xf + S * ye) - 5.0 * (g * xf * rinv2));
-    const Dual ayf = k * (2.0 * (S * xf - C * ye) - 5.0 * (g * ye * rinv2));
-    ax = ax + (c * axf - s * ayf);
-    ay = ay + (s * axf + c * ayf);
-    az = az + k * (-5.0 * (g * z * rinv2));
-  }
-#pragma unroll
-  for (int body = 0; body < 2; ++body) {
-    const uint32_t bit = body == 0 ? kPropSOL : kPropLUN;
-    if (!(mask & bit)) continue;
-    const double *sp = body == 0 ? e.sun : e.moon;
-    const double mu = body == 0 ? kMuSun : kMuMoon;
-    const Dual dx = sp[0] - x, dy = sp[1] - y, dz = sp[2] - z;
-    const Dual di = drsqrt(dx * dx + dy * dy + dz * dz);
-    const Dual kd = mu * (di * di * di);
-    ax = ax + kd * dx;  // the indirect term is constant in r
-    ay = ay + kd * dy;
-    az = az + kd * dz;
-  }
-  if (mask & kPropSRP) {
-    const double proj = r[0] * e.sunHat[0] + r[1] * e.sunHat[1] + r[2] * e.sunHat[2];
-    const bool shadow = proj < 0.0 && (r2.v - proj * proj) < kREarth * kREarth;
-    if (!shadow) {
-      const Dual ux = x - Dual{e.sun[0], 0}, uy = y - Dual{e.sun[1], 0}, uz = z - Dual{e.sun[2], 0};
-      const Dual ui = drsqrt(ux * ux + uy * uy + uz * uz);
-      const Dual k = ((kCR * kPSrp * kAU * kAU * 1.0e3) * aom) * (ui * ui * ui);
-      ax = ax + k * ux;
-      ay = ay + k * uy;
-      az = az + k * uz;
+  if (mask & (kPropKEP | kPropJ2 | kPropJ3 | kPropTesseral)) {
+    const double rinv = rsqrt(x * x + y * y + z * z);
+    const double i2 = rinv * rinv, i3 = i2 * rinv;
+    const double n = -i2 * (x * g[0] + y * g[1] + z * g[2]);
+    double s = (mask & kPropKEP) ? -kMuEarth * i3 : 0.0, ds = 3.0 * n * s;
+    if (mask & (kPropJ2 | kPropJ3 | kPropTesseral)) {
+      const double i5 = i3 * i2, n5 = 5.0 * n;
+      const double q = z * z * i2, dq = 2.0 * (z * g[2] * i2 + n * q);
+      const double c2 = (mask & kPropJ2) ? kJ2Coef : 0.0;
+      double b = c2 * (1.0 - 5.0 * q), db = -5.0 * c2 * dq;
+      double t = 2.0 * c2 * z, dt = 2.0 * c2 * g[2];
+      if (mask & (kPropJ3 | kPropTesseral)) {
+        const double c3 = (mask & kPropJ3) ? kJ3Coef : 0.0;
+        const double p = (mask & kPropTesseral) ? e.p : 0.0, h = (mask & kPropTesseral) ? e.q : 0.0;
+        const double u = p * x + h * y, w = h * x - p * y;
+        const double du = p * g[0] + h * g[1], dw = h * g[0] - p * g[1];
+        const double f = 3.0 - 7.0 * q;
+        const double in = c3 * z * f - 2.5 * (x * u + y * w);
+        const double din = c3 * (g[2] * f - 7.0 * z * dq) - 5.0 * (g[0] * u + g[1] * w);
+        b += i2 * in;
+        db += i2 * (2.0 * n * in + din);
+        t += c3 * (3.0 * q - 0.6);
+        dt += 3.0 * c3 * dq;
+        c[0] += i5 * (n5 * u + du);
+        c[1] += i5 * (n5 * w + dw);
+      }
+      s += i5 * b;
+      ds += i5 * (n5 * b + db);
+      c[2] += i5 * (n5 * t + dt);
     }
+    c[0] += ds * x + s * g[0];
+    c[1] += ds * y + s * g[1];
+    c[2] += ds * z + s * g[2];
   }
-  da[0] = ax.d;
-  da[1] = ay.d;
-  da[2] = az.d;
+  da[0] = c[0];
+  da[1] = c[1];
+  da[2] = c[2];
 }
 
 // g^T (da/dr, da/dv, da/dbc) of the full FP64 set at (r, v), accumulated into lr, lv, lbc
 __device__ __forceinline__ void accelVjp(uint32_t mask, const double r[3], const double v[3], double aom,
-                                         double bcInv, const EphEntry &e, const AtmShared &atm, const double g[3],
+                                         double bcInv, const EphEntry &e, const AtmShared<false> &atm, const double g[3],
                                          double lr[3], double lv[3], double &lbc) {
   if (mask & ~kPropDRAG) {
     double dc[3];
@@ -137,17 +119,16 @@ __device__ __forceinline__ void accelVjp(uint32_t mask, const double r[3], const
   }
   if (mask & kPropDRAG) {
     const double x = r[0], y = r[1], z = r[2];
-    const double rn = sqrt(x * x + y * y + z * z);
+    const double r2 = x * x + y * y + z * z, rinv = rsqrt(r2);
     const double wx = v[0] + kOmegaEarth * y, wy = v[1] - kOmegaEarth * x, wz = v[2];
-    const double wn = sqrt(wx * wx + wy * wy + wz * wz);
-    const double h = rn - kREarth;
+    const double w2 = wx * wx + wy * wy + wz * wz, winv = w2 > 0.0 ? rsqrt(w2) : 0.0, wn = w2 * winv;
+    const double h = r2 * rinv - kREarth;
     const int b = atmBand(atm, h);
-    const double rho = atm.rho0[b] * exp(-(h - atm.h0[b]) / atm.H[b]);
+    const double rho = atm.rho0[b] * exp((atm.h0[b] - h) * atm.invH[b]);
     const double K = -0.5e3 * rho * bcInv;
     const double wg = wx * g[0] + wy * g[1] + wz * g[2];
-    // the quotients do not depend on the density: they are formed beside its
-    // exponential instead of after it
-    const double wgw = wn > 0.0 ? wg / wn : 0.0, kq = wn * wg / (atm.H[b] * rn);
+    // formed beside the density's exponential, which they do not depend on
+    const double wgw = wg * winv, kq = wn * wg * (atm.invH[b] * rinv);
     const double c1 = K * wn, c2 = K * wgw;
     const double qx = c1 * g[0] + c2 * wx, qy = c1 * g[1] + c2 * wy, qz = c1 * g[2] + c2 * wz;
     lv[0] += qx;
@@ -165,12 +146,12 @@ __device__ __forceinline__ void accelVjp(uint32_t mask, const double r[3], const
 // One FP64 Yoshida step (the expression forms of k_propagate); the three stage
 // accelerations go to acc if non-null.  e3 = the step's three stage entries.
 __device__ __forceinline__ void adjStep(uint32_t mask, double r[3], double v[3], double aom, double bc,
-                                        const EphEntry *e3, const AtmShared &atm, const PropConsts &pc,
+                                        const EphEntry *e3, const AtmShared<false> &atm, const PropConsts &pc,
                                         double acc[3][3]) {
   double a[3];
 #pragma unroll
   for (int k = 0; k < 3; ++k) r[k] += pc.hc1 * v[k];
-  accel<false>(mask, r, v, aom, bc, e3[0], atm, a);
+  accel(mask, r, v, aom, bc, e3[0], atm, a);
 #pragma unroll
   for (int k = 0; k < 3; ++k) {
     acc[0][k] = a[k];
@@ -178,7 +159,7 @@ __device__ __forceinline__ void adjStep(uint32_t mask, double r[3], double v[3],
   }
 #pragma unroll
   for (int k = 0; k < 3; ++k) r[k] += pc.hc2 * v[k];
-  accel<false>(mask, r, v, aom, bc, e3[1], atm, a);
+  accel(mask, r, v, aom, bc, e3[1], atm, a);
 #pragma unroll
   for (int k = 0; k < 3; ++k) {
     acc[1][k] = a[k];
@@ -186,7 +167,7 @@ __device__ __forceinline__ void adjStep(uint32_t mask, double r[3], double v[3],
   }
 #pragma unroll
   for (int k = 0; k < 3; ++k) r[k] += pc.hc2 * v[k];
-  accel<false>(mask, r, v, aom, bc, e3[2], atm, a);
+  accel(mask, r, v, aom, bc, e3[2], atm, a);
 #pragma unroll
   for (int k = 0; k < 3; ++k) {
     acc[2][k] = a[k];
@@ -291,7 +272,7 @@ struct EphStage {
 template <int N>
 __device__ __forceinline__ void adjStepWarps(AdjExchange<N> &ex, int &half, uint32_t mask, double r[3],
                                              double v[3], double aom, double bc, const EphEntry *e3,
-                                             const AtmShared &atm, const PropConsts &pc, double acc[3][3]) {
+                                             const AtmShared<false> &atm, const PropConsts &pc, double acc[3][3]) {
   const uint32_t mine = mask & adjWarpTerms(threadIdx.x >> 5);
   const double hc[3] = {pc.hc1, pc.hc2, pc.hc2}, hd[3] = {pc.hd1, pc.hd2, pc.hd1};
 #pragma unroll
@@ -299,7 +280,7 @@ __device__ __forceinline__ void adjStepWarps(AdjExchange<N> &ex, int &half, uint
     double a[3];
 #pragma unroll
     for (int k = 0; k < 3; ++k) r[k] += hc[st] * v[k];
-    accel<false>(mine, r, v, aom, bc, e3[st], atm, a);
+    accel(mine, r, v, aom, bc, e3[st], atm, a);
     warpTermSum(ex, half, a);
 #pragma unroll
     for (int k = 0; k < 3; ++k) {
@@ -314,7 +295,7 @@ __device__ __forceinline__ void adjStepWarps(AdjExchange<N> &ex, int &half, uint
 // accelVjp with the terms shared out over the block's warps, summed into lr, lv, lbc
 __device__ __forceinline__ void accelVjpWarps(AdjExchange<7> &ex, int &half, uint32_t mask, const double r[3],
                                               const double v[3], double aom, double bc, const EphEntry &e,
-                                              const AtmShared &atm, const double g[3], double lr[3],
+                                              const AtmShared<false> &atm, const double g[3], double lr[3],
                                               double lv[3], double &lbc) {
   double t[7] = {0.0, 0.0, 0.0, 0.0, 0.0, 0.0, 0.0};
   accelVjp(mask & adjWarpTerms(threadIdx.x >> 5), r, v, aom, bc, e, atm, g, t, t + 3, t[6]);
@@ -332,7 +313,7 @@ __device__ __forceinline__ void accelVjpWarps(AdjExchange<7> &ex, int &half, uin
 __device__ __forceinline__ void adjReverseStepWarps(AdjExchange<7> &ex, int &half, uint32_t mask,
                                                     const double r0[3], const double v0[3],
                                                     const double acc[3][3], double aom, double bc,
-                                                    const EphEntry *e3, const AtmShared &atm,
+                                                    const EphEntry *e3, const AtmShared<false> &atm,
                                                     const PropConsts &pc, double lr[3], double lv[3],
                                                     double &lbc) {
   double r1[3], v1[3], r2[3], v2[3], r3[3];
@@ -381,7 +362,7 @@ __device__ __forceinline__ double pairMiss(const double ri[3], const double vi[3
   return dot3rn(dr, dr);
 }
 
-__device__ __forceinline__ void loadAtm(AtmShared &atm) { loadAtmTable(atm, c_atm); }
+__device__ __forceinline__ void loadAtm(AtmShared<false> &atm) { loadAtmTable(atm, c_atm); }
 
 __device__ __forceinline__ double shflPartner(unsigned m, double x) { return __shfl_xor_sync(m, x, 1); }
 
@@ -395,7 +376,7 @@ __global__ void __launch_bounds__(kAdjWarps * 32) k_adj_forward(
     const double *__restrict__ st, const double *__restrict__ bc, const double *__restrict__ aom, int nObj,
     int steps, int ck, const EphEntry *__restrict__ eph, PropConsts pc, double dt, double *__restrict__ ckpt,
     double *__restrict__ miss, int *__restrict__ argStep) {
-  __shared__ AtmShared atm;
+  __shared__ AtmShared<false> atm;
   __shared__ AdjExchange<3> ex;
   __shared__ uint4 ephBuf[kEphChunkWords];
   loadAtm(atm);
@@ -452,7 +433,7 @@ __global__ void __launch_bounds__(kAdjWarps * 32) k_adj_backward(
     const double *__restrict__ bc, const double *__restrict__ aom, int nObj, int steps, int ck,
     const EphEntry *__restrict__ eph, PropConsts pc, double dt, const double *__restrict__ ckpt,
     const int *__restrict__ argStep, double *__restrict__ rec, double *__restrict__ grad) {
-  __shared__ AtmShared atm;
+  __shared__ AtmShared<false> atm;
   __shared__ AdjExchange<7> ex;
   __shared__ uint4 ephBuf[kEphChunkWords];
   loadAtm(atm);
@@ -586,7 +567,7 @@ __global__ void __launch_bounds__(128) k_adj_make_pairs(double *__restrict__ st,
                                                         const int *__restrict__ tca, const double *__restrict__ off,
                                                         const EphEntry *__restrict__ eph, PropConsts pc,
                                                         PropConsts back) {
-  __shared__ AtmShared atm;
+  __shared__ AtmShared<false> atm;
   loadAtm(atm);
   __syncthreads();
   const int p = blockIdx.x * blockDim.x + threadIdx.x;

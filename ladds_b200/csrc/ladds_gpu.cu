@@ -42,9 +42,10 @@ __global__ void k_advance(int64_t *iter, int by) {
   if (threadIdx.x == 0 && blockIdx.x == 0) *iter += by;
 }
 // also stores the chunk's first iteration in *iterBase (the scans' step index)
-__global__ void k_ephemeris_dev(EphEntry *__restrict__ out, int nSteps, const int64_t *__restrict__ iterPtr,
+template <typename Entry>
+__global__ void k_ephemeris_dev(Entry *__restrict__ out, int nSteps, const int64_t *__restrict__ iterPtr,
                                 int64_t *__restrict__ iterBase, double t0, double dt, double hc1, double hc2,
-                                double jdEpoch, double theta0) {
+                                double jdEpoch, double theta0, uint32_t mask) {
   const int i = blockIdx.x * blockDim.x + threadIdx.x;
   if (i == 0) *iterBase = *iterPtr;
   if (i >= 3 * nSteps) return;
@@ -53,7 +54,7 @@ __global__ void k_ephemeris_dev(EphEntry *__restrict__ out, int nSteps, const in
   double tau = tn + hc1;
   if (stage >= 1) tau += hc2;
   if (stage >= 2) tau += hc2;
-  ephemeris(jdEpoch, theta0, tau, out[i]);
+  ephemerisEntry(jdEpoch, theta0, tau, mask, out[i]);
 }
 
 inline int blocksFor(size_t n, int b) { return (int)((n + (size_t)b - 1) / (size_t)b); }
@@ -452,12 +453,17 @@ void collectTimes(ladds_gpu_ctx *c) {
 // ----- pipeline pieces (all enqueue on c->st; no synchronisation) -----
 
 cudaError_t enqueueEphemeris(ladds_gpu_ctx *c, int nSteps) {
-  const int threads = 3 * nSteps;
-  k_ephemeris_dev<<<blocksFor(threads, 128), 128, 0, c->st>>>(c->dEph, nSteps, c->dIter, c->dIterBase,
-                                                                c->cfg.startTime, c->cfg.deltaT, c->pc.hc1,
-                                                                c->pc.hc2, c->cfg.epochJD, c->theta0);
-  return cudaMemcpyToSymbolAsync(c_eph, c->dEph, (size_t)threads * sizeof(EphEntry), 0, cudaMemcpyDeviceToDevice,
-                                 c->st);
+  const int threads = 3 * nSteps, g = blocksFor(threads, 128);
+  const bool split = c->cfg.precision == LADDS_PRECISION_SPLIT;
+  if (split)
+    k_ephemeris_dev<<<g, 128, 0, c->st>>>(reinterpret_cast<EphEntryF *>(c->dEph), nSteps, c->dIter, c->dIterBase,
+                                          c->cfg.startTime, c->cfg.deltaT, c->pc.hc1, c->pc.hc2, c->cfg.epochJD,
+                                          c->theta0, c->pc.mask);
+  else
+    k_ephemeris_dev<<<g, 128, 0, c->st>>>(c->dEph, nSteps, c->dIter, c->dIterBase, c->cfg.startTime, c->cfg.deltaT,
+                                          c->pc.hc1, c->pc.hc2, c->cfg.epochJD, c->theta0, c->pc.mask);
+  return cudaMemcpyToSymbolAsync(c_eph, c->dEph, (size_t)threads * (split ? sizeof(EphEntryF) : sizeof(EphEntry)), 0,
+                                 cudaMemcpyDeviceToDevice, c->st);
 }
 
 // the bulk copies of k_propagate_staged need 16-byte aligned arrays
@@ -2461,7 +2467,7 @@ int adjPrepare(ladds_gpu_ctx *c, size_t nPairs, int steps, int ck, bool backward
 int adjEphemeris(ladds_gpu_ctx *c, int steps) {
   k_ephemeris<<<blocksFor((size_t)3 * steps, 128), 128, 0, c->st>>>(c->adj.eph, steps, 0, c->cfg.startTime,
                                                                      c->cfg.deltaT, c->pc.hc1, c->pc.hc2,
-                                                                     c->cfg.epochJD, c->theta0);
+                                                                     c->cfg.epochJD, c->theta0, c->pc.mask);
   CK(cudaGetLastError());
   return LADDS_OK;
 }

@@ -71,15 +71,23 @@ struct AtmRow {
    {400, 3.725e-12, 58.515}, {450, 1.585e-12, 60.828}, {500, 6.967e-13, 63.822}, {600, 1.454e-13, 71.835},    \
    {700, 3.614e-14, 88.667}, {800, 1.170e-14, 124.64}, {900, 5.245e-15, 181.05}, {1000, 3.019e-15, 268.00}}
 
-// Ephemeris of one force-evaluation time, shared by every particle.
+// What every particle shares of one force-evaluation time, in the form the
+// force terms use (forces.cuh); terms that the component mask switches off are
+// zero in it.
+//   p, q      C22/S22 potential in inertial axes: the tesseral coefficients
+//             turned by twice the Earth rotation angle, times 6 mu R^2
+//   indirect  indirect third-body acceleration, sum of mu s / |s|^3
+// Binary64 form (every term in binary64):
 struct EphEntry {
-  double sun[3], moon[3];
-  double sunHat[3];        // sun / |sun|
-  double cosT, sinT;       // Earth rotation angle
-  double sunK, moonK;      // mu / |s|^3 of the indirect term
-  float sunf[3], moonf[3];
-  float sunInvS2f, moonInvS2f;  // 1 / |s|^2
-  float cosTf, sinTf;
+  double sun[3], moon[3], sunHat[3], indirect[3];
+  double p, q;
+};
+// Split form (binary32 perturbations; the shadow axis in binary64).
+struct EphEntryF {
+  double sunHat[3];
+  float sun[3], moon[3];
+  float sunInvS2, moonInvS2;  // 1 / |s|^2
+  float cosT, sinT;           // Earth rotation angle
 };
 
 // IAU-1982 Greenwich mean sidereal time [rad] at Julian date jd (UT1 ~ UTC).
@@ -93,7 +101,10 @@ LADDS_HD inline double gmstIAU1982(double jd) {
 
 // Sun and Moon (Montenbruck & Gill sec. 3.3.2, mean equator/equinox J2000) at
 // tau seconds after the epoch, plus the Earth rotation angle theta0 + w tau.
-LADDS_HD inline void ephemeris(double jdEpoch, double theta0, double tau, EphEntry &e) {
+struct EphPositions {
+  double sun[3], moon[3], theta;
+};
+LADDS_HD inline void ephemeris(double jdEpoch, double theta0, double tau, EphPositions &e) {
   constexpr double deg = kPi / 180.0, arcsec = kPi / (180.0 * 3600.0);
   const double T = (jdEpoch + tau / 86400.0 - kJDJ2000) / 36525.0;
   const double eps = kObliquityDeg * deg;
@@ -131,24 +142,51 @@ LADDS_HD inline void ephemeris(double jdEpoch, double theta0, double tau, EphEnt
     e.moon[1] = ye * ce - ze * se;
     e.moon[2] = ye * se + ze * ce;
   }
-  const double th = theta0 + kOmegaEarth * tau;
-  e.cosT = cos(th);
-  e.sinT = sin(th);
-  const double s2 = e.sun[0] * e.sun[0] + e.sun[1] * e.sun[1] + e.sun[2] * e.sun[2];
-  const double sn = sqrt(s2);
-  const double m2 = e.moon[0] * e.moon[0] + e.moon[1] * e.moon[1] + e.moon[2] * e.moon[2];
-  const double mn = sqrt(m2);
+  e.theta = theta0 + kOmegaEarth * tau;
+}
+
+// C22/S22 in inertial axes: with xf, yf the Earth-fixed coordinates,
+//   C (xf^2 - yf^2) + 2 S xf yf = P (x^2 - y^2) + 2 Q x y,
+//   P = C cos 2t - S sin 2t,  Q = C sin 2t + S cos 2t,
+// so the rotation into the Earth-fixed frame and back drops out of the force
+// evaluation.
+LADDS_HD inline void tesseral(uint32_t mask, double theta, double &p, double &q) {
+  const double C = (mask & kPropC22) ? kC22 : 0.0, S = (mask & kPropS22) ? kS22 : 0.0;
+  const double c2 = cos(2.0 * theta), s2 = sin(2.0 * theta), k = 6.0 * kMuEarth * kREarth * kREarth;
+  p = k * (C * c2 - S * s2);
+  q = k * (C * s2 + S * c2);
+}
+
+LADDS_HD inline void ephemerisEntry(double jdEpoch, double theta0, double tau, uint32_t mask, EphEntry &e) {
+  EphPositions b;
+  ephemeris(jdEpoch, theta0, tau, b);
+  const double s2 = b.sun[0] * b.sun[0] + b.sun[1] * b.sun[1] + b.sun[2] * b.sun[2], sn = sqrt(s2);
+  const double m2 = b.moon[0] * b.moon[0] + b.moon[1] * b.moon[1] + b.moon[2] * b.moon[2];
+  const double kS = (mask & kPropSOL) ? kMuSun / (s2 * sn) : 0.0;
+  const double kM = (mask & kPropLUN) ? kMuMoon / (m2 * sqrt(m2)) : 0.0;
   for (int k = 0; k < 3; ++k) {
-    e.sunHat[k] = e.sun[k] / sn;
-    e.sunf[k] = (float)e.sun[k];
-    e.moonf[k] = (float)e.moon[k];
+    e.sun[k] = b.sun[k];
+    e.moon[k] = b.moon[k];
+    e.sunHat[k] = b.sun[k] / sn;
+    e.indirect[k] = kS * b.sun[k] + kM * b.moon[k];
   }
-  e.sunK = kMuSun / (s2 * sn);
-  e.moonK = kMuMoon / (m2 * mn);
-  e.sunInvS2f = (float)(1.0 / s2);
-  e.moonInvS2f = (float)(1.0 / m2);
-  e.cosTf = (float)e.cosT;
-  e.sinTf = (float)e.sinT;
+  tesseral(mask, b.theta, e.p, e.q);
+}
+
+LADDS_HD inline void ephemerisEntry(double jdEpoch, double theta0, double tau, uint32_t, EphEntryF &e) {
+  EphPositions b;
+  ephemeris(jdEpoch, theta0, tau, b);
+  const double s2 = b.sun[0] * b.sun[0] + b.sun[1] * b.sun[1] + b.sun[2] * b.sun[2], sn = sqrt(s2);
+  const double m2 = b.moon[0] * b.moon[0] + b.moon[1] * b.moon[1] + b.moon[2] * b.moon[2];
+  for (int k = 0; k < 3; ++k) {
+    e.sunHat[k] = b.sun[k] / sn;
+    e.sun[k] = (float)b.sun[k];
+    e.moon[k] = (float)b.moon[k];
+  }
+  e.sunInvS2 = (float)(1.0 / s2);
+  e.moonInvS2 = (float)(1.0 / m2);
+  e.cosT = (float)cos(b.theta);
+  e.sinT = (float)sin(b.theta);
 }
 
 }  // namespace ladds

@@ -17,10 +17,19 @@
 #include "forces.cuh"
 #include "state.cuh"
 
+#include <type_traits>
+
 namespace ladds {
 
-constexpr int kMaxEphSteps = 128;  // 3 * 128 entries * 160 B = 61 KB of constant memory
-__constant__ EphEntry c_eph[3 * kMaxEphSteps];
+constexpr int kMaxEphSteps = 128;  // 3 * 128 entries * 112 B (FP64) or 88 B (split): up to 43 KB of constant memory
+template <bool SPLIT>
+using EphOf = typename std::conditional<SPLIT, EphEntryF, EphEntry>::type;
+static_assert(sizeof(EphEntryF) <= sizeof(EphEntry), "the stage table holds entries of either form");
+__constant__ __align__(16) unsigned char c_eph[3 * kMaxEphSteps * sizeof(EphEntry)];
+template <bool SPLIT>
+__device__ __forceinline__ const EphOf<SPLIT> *stageTable() {
+  return reinterpret_cast<const EphOf<SPLIT> *>(c_eph);
+}
 __constant__ AtmRow c_atm[kAtmBands] = LADDS_ATM_TABLE;
 
 struct PropConsts {
@@ -43,35 +52,46 @@ __device__ __forceinline__ uint32_t cellKey(double x, double y, double z, const 
   return (iz * (uint32_t)g.n[1] + iy) * (uint32_t)g.n[0] + ix;
 }
 
-// nSteps Yoshida-4 steps of one object (stage ephemerides c_eph[ephBase ...]);
-// a non-finite end state sets bit 1 of *status
+// nSteps Yoshida-4 steps of one object (stage ephemerides ephBase ... of the
+// stage table); a non-finite end state sets bit 1 of *status.  evasive-preserving
+// objects (Keplerian forces only, Particle.h:48-52) take a loop of their own, so
+// that in the other one the mask is the launch's and its branches are uniform.
 template <bool SPLIT>
-__device__ __forceinline__ void yoshidaSteps(double r[3], double v[3], double aom, double bc, uint32_t tag,
-                                             int nSteps, int ephBase, const PropConsts &pc, const AtmShared &atm,
-                                             unsigned *__restrict__ status) {
-  uint32_t mask = pc.mask;
-  if (tagAct(tag) == kEvasivePreserving) mask &= kPropKEP;  // Particle.h:48-52: Keplerian forces only
+__device__ __forceinline__ void yoshidaLoop(uint32_t mask, double r[3], double v[3], double aom, double bc,
+                                            int nSteps, int ephBase, const PropConsts &pc,
+                                            const AtmShared<SPLIT> &atm) {
+  using C = typename std::conditional<SPLIT, float, double>::type;
+  const C aomC = (C)aom, bcC = (C)bc;
+  const EphOf<SPLIT> *e = stageTable<SPLIT>() + ephBase;
   double a[3];
-  for (int st = 0; st < nSteps; ++st) {
-    const EphEntry *e = &c_eph[ephBase + 3 * st];
+  for (int st = 0; st < nSteps; ++st, e += 3) {
 #pragma unroll
     for (int k = 0; k < 3; ++k) r[k] += pc.hc1 * v[k];
-    accel<SPLIT>(mask, r, v, aom, bc, e[0], atm, a);
+    accel(mask, r, v, aomC, bcC, e[0], atm, a);
 #pragma unroll
     for (int k = 0; k < 3; ++k) v[k] += pc.hd1 * a[k];
 #pragma unroll
     for (int k = 0; k < 3; ++k) r[k] += pc.hc2 * v[k];
-    accel<SPLIT>(mask, r, v, aom, bc, e[1], atm, a);
+    accel(mask, r, v, aomC, bcC, e[1], atm, a);
 #pragma unroll
     for (int k = 0; k < 3; ++k) v[k] += pc.hd2 * a[k];
 #pragma unroll
     for (int k = 0; k < 3; ++k) r[k] += pc.hc2 * v[k];
-    accel<SPLIT>(mask, r, v, aom, bc, e[2], atm, a);
+    accel(mask, r, v, aomC, bcC, e[2], atm, a);
 #pragma unroll
     for (int k = 0; k < 3; ++k) v[k] += pc.hd1 * a[k];
 #pragma unroll
     for (int k = 0; k < 3; ++k) r[k] += pc.hc1 * v[k];
   }
+}
+template <bool SPLIT>
+__device__ __forceinline__ void yoshidaSteps(double r[3], double v[3], double aom, double bc, uint32_t tag,
+                                             int nSteps, int ephBase, const PropConsts &pc,
+                                             const AtmShared<SPLIT> &atm, unsigned *__restrict__ status) {
+  if (tagAct(tag) == kEvasivePreserving)
+    yoshidaLoop<SPLIT>(pc.mask & kPropKEP, r, v, aom, bc, nSteps, ephBase, pc, atm);
+  else
+    yoshidaLoop<SPLIT>(pc.mask, r, v, aom, bc, nSteps, ephBase, pc, atm);
   if (!(isfinite(r[0]) && isfinite(r[1]) && isfinite(r[2]) && isfinite(v[0]) && isfinite(v[1]) && isfinite(v[2])))
     atomicOr(status, 1u);
 }
@@ -83,7 +103,7 @@ __global__ void __launch_bounds__(256, 4) k_propagate(DevState s, int n, int nSt
                                                    GridDesc g, uint32_t *__restrict__ keys,
                                                    uint32_t *__restrict__ rowCount, uint32_t *__restrict__ arrival,
                                                    unsigned *__restrict__ status) {
-  __shared__ AtmShared atm;
+  __shared__ AtmShared<SPLIT> atm;
   loadAtmTable(atm, c_atm);
   __syncthreads();
   const int j = blockIdx.x * blockDim.x + threadIdx.x;
@@ -139,7 +159,7 @@ __global__ void __launch_bounds__(kStageObjects, 4) k_propagate_staged(DevState 
                                                                       uint32_t *__restrict__ rowCount,
                                                                       uint32_t *__restrict__ arrival,
                                                                       unsigned *__restrict__ status) {
-  __shared__ AtmShared atm;
+  __shared__ AtmShared<SPLIT> atm;
   __shared__ __align__(16) double sv[kStageArrays][kStageObjects];
   __shared__ __align__(16) uint32_t stag[kStageObjects];
   __shared__ __align__(8) unsigned long long sbar;
@@ -237,7 +257,7 @@ __global__ void k_layer_histogram(const double *__restrict__ z, const uint32_t *
 // (one thread per stage), written to a global staging table that the host then
 // copies into c_eph.
 __global__ void k_ephemeris(EphEntry *__restrict__ out, int nSteps, int64_t iter, double t0, double dt, double hc1,
-                            double hc2, double jdEpoch, double theta0) {
+                            double hc2, double jdEpoch, double theta0, uint32_t mask) {
   const int i = blockIdx.x * blockDim.x + threadIdx.x;
   if (i >= 3 * nSteps) return;
   const int st = i / 3, stage = i % 3;
@@ -245,7 +265,7 @@ __global__ void k_ephemeris(EphEntry *__restrict__ out, int nSteps, int64_t iter
   double tau = tn + hc1;
   if (stage >= 1) tau += hc2;
   if (stage >= 2) tau += hc2;
-  ephemeris(jdEpoch, theta0, tau, out[i]);
+  ephemerisEntry(jdEpoch, theta0, tau, mask, out[i]);
 }
 
 // cell keys of the current positions + their row counts (as k_propagate<*, true>)
