@@ -7,11 +7,11 @@
 // slot order, and independent of the order the arrays are in before the call.
 //
 //   1. countRowArrival (inside the kernel that computes the keys): objects per
-//      cell row (row = key / nx; warp-aggregated atomics) and each object's
-//      arrival index inside its row; the exclusive scan of the counts is the
-//      row-start table that the pair scan uses.
+//      cell row (row = key / nx) and each object's arrival index inside its
+//      row; the exclusive scan of the counts is the row-start table that the
+//      pair scan uses.
 //   2. k_bucket_place: each object to its row bucket at rowStart + arrival,
-//      with its sort record (ix << 32 | slot) and source index.
+//      as its sort record (ix << 32 | slot).
 //   3. k_bucket_sort_rows (nx <= kRowCountMaxNx): one warp per row of <= 256
 //      objects, counting sort by cell index in shared memory, ties by slot;
 //      k_bucket_sort_small otherwise: warp bitonic sort of the records in
@@ -24,11 +24,12 @@
 #pragma once
 #include <cstdint>
 
+#include "conjunction.cuh"
 #include "state.cuh"
 
 namespace ladds {
 
-constexpr int kLargeRow = 4096;  // objects sorted in shared memory by one CTA (48 KB)
+constexpr int kLargeRow = 4096;  // objects sorted in shared memory by one CTA (32 KB)
 constexpr int kBucketThreads = 256;
 
 // Occupancy bin of the pair scan: cells holding at least minCount objects are
@@ -81,31 +82,38 @@ __device__ __forceinline__ uint32_t laneMaskLt() {
   return m;
 }
 
-// Row count of a key inside the producing kernel: warp-aggregated atomicAdd on
-// rowCount[key / nx]; returns the object's arrival index inside its row (its
+// Row count of an object inside the kernel that computes its cell: atomicAdd
+// on rowCount[row]; returns the object's arrival index inside its row (its
 // place among the row's objects in the scatter).  Every lane of the warp must
-// call it (valid = false for lanes without an object).
-__device__ __forceinline__ uint32_t countRowArrival(uint32_t key, bool valid, uint32_t nx,
-                                                   uint32_t *__restrict__ rowCount) {
-  const int lane = threadIdx.x & 31;
-  const uint32_t row = valid ? key / nx : 0xffffffffu;
-  const uint32_t peers = __match_any_sync(0xffffffffu, row);
-  const int leader = __ffs(peers) - 1;
-  uint32_t base = 0;
-  if (valid && lane == leader) base = atomicAdd(&rowCount[row], (uint32_t)__popc(peers));
-  base = __shfl_sync(0xffffffffu, base, leader);
-  return base + (uint32_t)__popc(peers & laneMaskLt());
+// call it (valid = false for lanes without an object).  Objects come in slot
+// order, so the lanes' rows are as good as random and each has its own atomic;
+// a warp whose objects all lie in one row -- a fragment cloud's -- makes one.
+__device__ __forceinline__ uint32_t countRowArrival(uint32_t row, bool valid, uint32_t *__restrict__ rowCount) {
+  const uint32_t first = __shfl_sync(0xffffffffu, row, 0);
+  if (__all_sync(0xffffffffu, valid && row == first)) {
+    const int lane = threadIdx.x & 31;
+    uint32_t base = 0;
+    if (lane == 0) base = atomicAdd(&rowCount[row], 32u);
+    return __shfl_sync(0xffffffffu, base, 0) + (uint32_t)lane;
+  }
+  return valid ? atomicAdd(&rowCount[row], 1u) : 0u;
 }
 
-// Scatter with the arrival indices of countRowArrival: no atomics.
-__global__ void __launch_bounds__(kBucketThreads) k_bucket_place(const uint32_t *__restrict__ keys,
-                                                                 const uint32_t *__restrict__ arrival,
-                                                                 const uint32_t *__restrict__ tags, int n,
-                                                                 uint32_t nx, const uint32_t *__restrict__ rowStart,
-                                                                 unsigned long long *__restrict__ rec,
-                                                                 uint32_t *__restrict__ src,
-                                                                 unsigned *__restrict__ status) {
+// Scatter with the arrival indices of countRowArrival: no atomics.  Also
+// clears what is counted next: the row counts (nCounts of them), the lengths
+// of the long-row and dense-cell lists, the scan's three list counters.
+__global__ void __launch_bounds__(kBucketThreads) k_bucket_place(
+    const uint32_t *__restrict__ keys, const uint32_t *__restrict__ arrival, int n, uint32_t nx,
+    const uint32_t *__restrict__ rowStart, unsigned long long *__restrict__ rec, uint32_t *__restrict__ rowCounts,
+    uint32_t nCounts, uint32_t *__restrict__ longCount, uint32_t *__restrict__ denseCount,
+    unsigned long long *__restrict__ candCount, unsigned *__restrict__ status) {
   const int j = blockIdx.x * blockDim.x + threadIdx.x;
+  for (uint32_t q = (uint32_t)j; q < nCounts; q += gridDim.x * blockDim.x) rowCounts[q] = 0u;
+  if (j == 0) {
+    *longCount = 0u;
+    *denseCount = 0u;
+    candCount[0] = candCount[1] = candCount[2] = 0ull;
+  }
   if (j >= n) return;
   const uint32_t key = keys[j], row = key / nx;
   const uint32_t pos = rowStart[row] + arrival[j];
@@ -113,8 +121,29 @@ __global__ void __launch_bounds__(kBucketThreads) k_bucket_place(const uint32_t 
     atomicOr(status, 4u);
     return;
   }
-  rec[pos] = ((unsigned long long)(key - row * nx) << 32) | tagSlot(tags[j]);
-  src[pos] = (uint32_t)j;
+  rec[pos] = ((unsigned long long)(key - row * nx) << 32) | (uint32_t)j;
+}
+
+// Where the row sorts put their result: the cell key and the slot of every
+// position of the cell order, and (in != nullptr) what the pair scan reads
+// there, gathered from the slot-ordered records while the order is at hand --
+// one 32-byte sector per object -- instead of by a pass of its own over the
+// population.
+struct CellOrderOut {
+  uint32_t *keys, *perm;
+  const ScanRec *in;
+  float4 *posf, *velf;
+  const uint64_t *parent;  // null: no object has a parent (grp is not written)
+  uint32_t *grp;
+};
+__device__ __forceinline__ void emitCellOrder(const CellOrderOut &o, uint32_t pos, uint32_t key, uint32_t slot) {
+  o.keys[pos] = key;
+  o.perm[pos] = slot;
+  if (!o.in) return;
+  const float4 *r = reinterpret_cast<const float4 *>(o.in + slot);
+  o.posf[pos] = __ldg(r);
+  o.velf[pos] = __ldg(r + 1);
+  if (o.parent) o.grp[pos] = groupOf(__ldg(&o.parent[slot]));
 }
 
 // comparator i of stage (k, jj) of the all-ascending bitonic network
@@ -134,7 +163,7 @@ __device__ __forceinline__ void bitonicPair(uint32_t i, uint32_t k, uint32_t jj,
 // Comparator partners at distance < 32 are other lanes (shuffles), at distance
 // >= 32 other slots of the same lane; the flip stages pair e with e ^ (k-1).
 template <int S>
-__device__ __forceinline__ void warpBitonic(unsigned long long (&v)[S], uint32_t (&p)[S], int lane) {
+__device__ __forceinline__ void warpBitonic(unsigned long long (&v)[S], int lane) {
 #pragma unroll
   for (int k = 2; k <= 32 * S; k <<= 1) {
 #pragma unroll
@@ -146,12 +175,8 @@ __device__ __forceinline__ void warpBitonic(unsigned long long (&v)[S], uint32_t
 #pragma unroll
         for (int s = 0; s < S; ++s) {
           const unsigned long long ov = __shfl_sync(0xffffffffu, v[s], pl);
-          const uint32_t op = __shfl_sync(0xffffffffu, p[s], pl);
           const bool lower = lane < pl;
-          if (lower ? (ov < v[s]) : (ov > v[s])) {
-            v[s] = ov;
-            p[s] = op;
-          }
+          if (lower ? (ov < v[s]) : (ov > v[s])) v[s] = ov;
         }
       } else if (!flip) {  // partner in the same lane: slot ^ (jj / 32)
         const int sm = jj / 32;
@@ -162,29 +187,21 @@ __device__ __forceinline__ void warpBitonic(unsigned long long (&v)[S], uint32_t
             const unsigned long long tv = v[s];
             v[s] = v[t];
             v[t] = tv;
-            const uint32_t tp = p[s];
-            p[s] = p[t];
-            p[t] = tp;
           }
         }
       } else {  // flip across lanes and slots: lane ^ 31, slot ^ (k/32 - 1)
         const int pl = lane ^ 31, sm = k / 32 - 1;
         unsigned long long nv[S];
-        uint32_t np[S];
 #pragma unroll
         for (int s = 0; s < S; ++s) {
           const int t = s ^ sm;
           nv[s] = __shfl_sync(0xffffffffu, v[t], pl);
-          np[s] = __shfl_sync(0xffffffffu, p[t], pl);
         }
 #pragma unroll
         for (int s = 0; s < S; ++s) {
           const int t = s ^ sm;
           const bool lower = (s * 32 + lane) < (t * 32 + pl);
-          if (lower ? (nv[s] < v[s]) : (nv[s] > v[s])) {
-            v[s] = nv[s];
-            p[s] = np[s];
-          }
+          if (lower ? (nv[s] < v[s]) : (nv[s] > v[s])) v[s] = nv[s];
         }
       }
     }
@@ -193,24 +210,20 @@ __device__ __forceinline__ void warpBitonic(unsigned long long (&v)[S], uint32_t
 
 template <int S>
 __device__ __forceinline__ void warpSortRow(uint32_t s0, uint32_t L, uint32_t r, uint32_t nx, int lane,
-                                            const unsigned long long *__restrict__ rec,
-                                            const uint32_t *__restrict__ src, uint32_t *__restrict__ sortedKeys,
-                                            uint32_t *__restrict__ perm, uint16_t *__restrict__ sIx) {
+                                            const unsigned long long *__restrict__ rec, const CellOrderOut &out,
+                                            uint16_t *__restrict__ sIx) {
   unsigned long long v[S];
-  uint32_t p[S];
 #pragma unroll
   for (int s = 0; s < S; ++s) {
     const uint32_t e = (uint32_t)(s * 32 + lane);
     v[s] = e < L ? rec[s0 + e] : ~0ull;
-    p[s] = e < L ? src[s0 + e] : 0u;
   }
-  warpBitonic<S>(v, p, lane);
+  warpBitonic<S>(v, lane);
 #pragma unroll
   for (int s = 0; s < S; ++s) {
     const uint32_t e = (uint32_t)(s * 32 + lane);
     if (e < L) {
-      sortedKeys[s0 + e] = r * nx + (uint32_t)(v[s] >> 32);
-      perm[s0 + e] = p[s];
+      emitCellOrder(out, s0 + e, r * nx + (uint32_t)(v[s] >> 32), (uint32_t)v[s]);
       sIx[e] = (uint16_t)(v[s] >> 32);
     }
   }
@@ -254,8 +267,8 @@ __device__ __forceinline__ void fillCellOffsets(uint16_t *__restrict__ t, uint32
 // may be null) receives the offset of every cell of the row inside the row.
 __global__ void __launch_bounds__(kBucketThreads) k_bucket_sort_small(
     const uint32_t *__restrict__ rowStart, uint32_t nRows, uint32_t nx, const unsigned long long *__restrict__ rec,
-    const uint32_t *__restrict__ src, uint32_t *__restrict__ sortedKeys, uint32_t *__restrict__ perm,
-    uint32_t *__restrict__ longRows, uint32_t *__restrict__ longCount, uint16_t *__restrict__ cellOff) {
+    const CellOrderOut out, uint32_t *__restrict__ longRows, uint32_t *__restrict__ longCount,
+    uint16_t *__restrict__ cellOff) {
   __shared__ uint16_t sIxAll[kBucketThreads / 32][256];
   const int lane = threadIdx.x & 31;
   uint16_t *sIx = sIxAll[threadIdx.x >> 5];
@@ -272,16 +285,15 @@ __global__ void __launch_bounds__(kBucketThreads) k_bucket_sort_small(
 #pragma unroll
       for (int q = 0; q < 32; ++q) rank += __shfl_sync(0xffffffffu, v, q) < v ? 1u : 0u;
       if (lane < (int)L) {
-        sortedKeys[s + rank] = r * nx + (uint32_t)(v >> 32);
-        perm[s + rank] = src[s + lane];
+        emitCellOrder(out, s + rank, r * nx + (uint32_t)(v >> 32), (uint32_t)v);
         sIx[rank] = (uint16_t)(v >> 32);
       }
     } else if (L <= 64) {
-      warpSortRow<2>(s, L, r, nx, lane, rec, src, sortedKeys, perm, sIx);
+      warpSortRow<2>(s, L, r, nx, lane, rec, out, sIx);
     } else if (L <= 128) {
-      warpSortRow<4>(s, L, r, nx, lane, rec, src, sortedKeys, perm, sIx);
+      warpSortRow<4>(s, L, r, nx, lane, rec, out, sIx);
     } else if (L <= 256) {
-      warpSortRow<8>(s, L, r, nx, lane, rec, src, sortedKeys, perm, sIx);
+      warpSortRow<8>(s, L, r, nx, lane, rec, out, sIx);
     } else {
       if (lane == 0) longRows[atomicAdd(longCount, 1u)] = r;
       continue;
@@ -299,8 +311,7 @@ __global__ void __launch_bounds__(kBucketThreads) k_bucket_sort_small(
 // shared memory; their exclusive scan is the row's cell-offset table (written
 // to cellOff as is) and places every object in its cell; objects sharing a
 // cell are ranked by slot.  Longer rows go to the list of k_bucket_sort_large.
-// Shared memory per warp: countWords u32 counters (nx + 1 rounded up to 32),
-// then 256 slots, 256 sources and 256 cell indices.
+// The scan records are gathered as the rows are put in order (emitCellOrder).
 constexpr int kRowCountMaxNx = 1023;
 constexpr int kRowSortThreads = 128;
 // counters of a row: nx + 1 rounded up to 32 x a power of two, so that each lane
@@ -316,25 +327,22 @@ __host__ __device__ __forceinline__ uint32_t rowCountWords(uint32_t nx) { return
 __host__ __device__ __forceinline__ uint32_t rowCountStored(uint32_t nx) {
   return rowCountWords(nx) + 32u;
 }
-// per warp: counters, then 256 entries of (ix | arrival << 16), slot and source
-// in load order, then 256 slots, sources and cell indices in cell order
+// per warp: counters, then 256 entries of (ix | arrival << 16) and slot in load
+// order, then 256 slots and cell indices in cell order
 __host__ __device__ __forceinline__ uint32_t rowSortWarpWords(uint32_t nx) {
-  return rowCountStored(nx) + 256u * 5u + 128u;
+  return rowCountStored(nx) + 256u * 3u + 128u;
 }
 __host__ __device__ __forceinline__ size_t rowSortSmem(uint32_t nx) {
   return (size_t)(kRowSortThreads / 32) * rowSortWarpWords(nx) * 4u;
 }
 
 // one row of <= 256 objects by one warp (see k_bucket_sort_rows); element
-// `lane` of the row is passed in (firstRec, firstSrc)
-__device__ __forceinline__ void sortOneRow(uint32_t r, uint32_t s0, uint32_t L, unsigned long long firstRec,
-                                           uint32_t firstSrc, int lane, uint32_t nx, uint32_t H, uint32_t sh,
-                                           uint32_t pitch, const unsigned long long *__restrict__ rec,
-                                           const uint32_t *__restrict__ src, uint32_t *__restrict__ sortedKeys,
-                                           uint32_t *__restrict__ perm, uint16_t *__restrict__ cellOff,
-                                           const DenseBin &dense, uint32_t *hist, uint32_t *inIxArr,
-                                           uint32_t *inSlot, uint32_t *inSrc, uint32_t *tSlot, uint32_t *tSrc,
-                                           uint16_t *tIx) {
+// `lane` of the row is passed in (firstRec)
+__device__ __forceinline__ void sortOneRow(uint32_t r, uint32_t s0, uint32_t L, unsigned long long firstRec, int lane,
+                                           uint32_t nx, uint32_t H, uint32_t sh, uint32_t pitch,
+                                           const unsigned long long *__restrict__ rec, const CellOrderOut &out,
+                                           uint16_t *__restrict__ cellOff, const DenseBin &dense, uint32_t *hist,
+                                           uint32_t *inIxArr, uint32_t *inSlot, uint32_t *tSlot, uint16_t *tIx) {
     const uint32_t per = 1u << sh;
     auto at = [sh](uint32_t c) { return c + (c >> sh); };  // padded counter index
     for (uint32_t c = lane; c < H + 32u; c += 32) hist[c] = 0u;
@@ -345,7 +353,6 @@ __device__ __forceinline__ void sortOneRow(uint32_t r, uint32_t s0, uint32_t L, 
       const uint32_t ix = (uint32_t)(v >> 32);
       inIxArr[e] = ix | (atomicAdd(&hist[at(ix)], 1u) << 16);
       inSlot[e] = (uint32_t)v;
-      inSrc[e] = e < 32u ? firstSrc : src[s0 + e];
     }
     __syncwarp();
     // exclusive scan of the counts: lane l owns counters [l * per, (l + 1) * per)
@@ -393,7 +400,6 @@ __device__ __forceinline__ void sortOneRow(uint32_t r, uint32_t s0, uint32_t L, 
       const uint32_t ia = inIxArr[e], ix = ia & 0xffffu;
       const uint32_t p = hist[at(ix)] + (ia >> 16);
       tSlot[p] = inSlot[e];
-      tSrc[p] = inSrc[e];
       tIx[p] = (uint16_t)ix;
     }
     __syncwarp();
@@ -401,39 +407,32 @@ __device__ __forceinline__ void sortOneRow(uint32_t r, uint32_t s0, uint32_t L, 
       const uint32_t ix = tIx[p], c0 = hist[at(ix)], c1 = hist[at(ix + 1)], sl = tSlot[p];
       uint32_t rank = 0;
       for (uint32_t q = c0; q < c1; ++q) rank += tSlot[q] < sl ? 1u : 0u;
-      const uint32_t out = s0 + c0 + rank;
-      sortedKeys[out] = r * nx + ix;
-      perm[out] = tSrc[p];
+      emitCellOrder(out, s0 + c0 + rank, r * nx + ix, sl);
     }
     __syncwarp();
 }
 
 __global__ void __launch_bounds__(kRowSortThreads) k_bucket_sort_rows(
     const uint32_t *__restrict__ rowStart, uint32_t nRows, uint32_t nx, const unsigned long long *__restrict__ rec,
-    const uint32_t *__restrict__ src, uint32_t *__restrict__ sortedKeys, uint32_t *__restrict__ perm,
-    uint32_t *__restrict__ longRows, uint32_t *__restrict__ longCount, uint16_t *__restrict__ cellOff,
-    DenseBin dense) {
+    const CellOrderOut out, uint32_t *__restrict__ longRows, uint32_t *__restrict__ longCount,
+    uint16_t *__restrict__ cellOff, DenseBin dense) {
   extern __shared__ uint32_t smemRows[];
   const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
   const uint32_t sh = rowCountShift(nx), H = rowCountWords(nx);
   uint32_t *hist = smemRows + (size_t)warp * rowSortWarpWords(nx);
-  uint32_t *inIxArr = hist + rowCountStored(nx), *inSlot = inIxArr + 256, *inSrc = inSlot + 256;
-  uint32_t *tSlot = inSrc + 256, *tSrc = tSlot + 256;
-  uint16_t *tIx = reinterpret_cast<uint16_t *>(tSrc + 256);
+  uint32_t *inIxArr = hist + rowCountStored(nx), *inSlot = inIxArr + 256, *tSlot = inSlot + 256;
+  uint16_t *tIx = reinterpret_cast<uint16_t *>(tSlot + 256);
   const uint32_t pitch = cellOffPitch(nx);
   const uint32_t warpId = (blockIdx.x * blockDim.x + threadIdx.x) >> 5;
   const uint32_t nWarps = (gridDim.x * blockDim.x) >> 5;
   // software pipeline over the warp's rows: the row starts two rows ahead and
   // the first 32 records one row ahead are in flight while a row is sorted
-  uint32_t r = warpId, s0 = 0, L = 0, firstSrc = 0;
+  uint32_t r = warpId, s0 = 0, L = 0;
   unsigned long long firstRec = 0;
   if (r < nRows) {
     s0 = rowStart[r];
     L = rowStart[r + 1] - s0;
-    if ((uint32_t)lane < L && L <= 256u) {
-      firstRec = rec[s0 + lane];
-      firstSrc = src[s0 + lane];
-    }
+    if ((uint32_t)lane < L && L <= 256u) firstRec = rec[s0 + lane];
   }
   uint32_t rN = r + nWarps, sN = 0, eN = 0;
   if (rN < nRows) {
@@ -443,11 +442,7 @@ __global__ void __launch_bounds__(kRowSortThreads) k_bucket_sort_rows(
   for (; r < nRows; r = rN, rN += nWarps) {
     const uint32_t lN = eN - sN;
     unsigned long long nextRec = 0;
-    uint32_t nextSrc = 0;
-    if (rN < nRows && (uint32_t)lane < lN && lN <= 256u) {
-      nextRec = rec[sN + lane];
-      nextSrc = src[sN + lane];
-    }
+    if (rN < nRows && (uint32_t)lane < lN && lN <= 256u) nextRec = rec[sN + lane];
     const uint32_t rNN = rN + nWarps;
     uint32_t sNN = 0, eNN = 0;
     if (rNN < nRows) {
@@ -456,11 +451,9 @@ __global__ void __launch_bounds__(kRowSortThreads) k_bucket_sort_rows(
     }
     const uint32_t rowS0 = s0, rowL = L;
     const unsigned long long rowFirstRec = firstRec;
-    const uint32_t rowFirstSrc = firstSrc;
     s0 = sN;
     L = lN;
     firstRec = nextRec;
-    firstSrc = nextSrc;
     sN = sNN;
     eN = eNN;
     if (rowL == 0) continue;
@@ -468,20 +461,18 @@ __global__ void __launch_bounds__(kRowSortThreads) k_bucket_sort_rows(
       if (lane == 0) longRows[atomicAdd(longCount, 1u)] = r;
       continue;
     }
-    sortOneRow(r, rowS0, rowL, rowFirstRec, rowFirstSrc, lane, nx, H, sh, pitch, rec, src, sortedKeys, perm,
-               cellOff, dense, hist, inIxArr, inSlot, inSrc, tSlot, tSrc, tIx);
+    sortOneRow(r, rowS0, rowL, rowFirstRec, lane, nx, H, sh, pitch, rec, out, cellOff, dense, hist, inIxArr, inSlot,
+               tSlot, tIx);
   }
 }
 
 
 __global__ void __launch_bounds__(kBucketThreads) k_bucket_sort_large(
-    const uint32_t *__restrict__ rowStart, uint32_t nx, unsigned long long *__restrict__ rec,
-    uint32_t *__restrict__ src, uint32_t *__restrict__ sortedKeys, uint32_t *__restrict__ perm,
+    const uint32_t *__restrict__ rowStart, uint32_t nx, unsigned long long *__restrict__ rec, const CellOrderOut out,
     const uint32_t *__restrict__ longRows, const uint32_t *__restrict__ longCount,
     uint16_t *__restrict__ cellOff, DenseBin dense) {
   extern __shared__ unsigned long long smem[];
   unsigned long long *sv = smem;
-  uint32_t *sp = reinterpret_cast<uint32_t *>(smem + kLargeRow);
   const uint32_t count = *longCount;
   for (uint32_t q = blockIdx.x; q < count; q += gridDim.x) {
     const uint32_t r = longRows[q];
@@ -490,12 +481,8 @@ __global__ void __launch_bounds__(kBucketThreads) k_bucket_sort_large(
     while (P < L) P <<= 1;
     const bool inShared = L <= (uint32_t)kLargeRow;
     unsigned long long *V = inShared ? sv : rec + s;
-    uint32_t *I = inShared ? sp : src + s;
     if (inShared) {
-      for (uint32_t i = threadIdx.x; i < L; i += blockDim.x) {
-        sv[i] = rec[s + i];
-        sp[i] = src[s + i];
-      }
+      for (uint32_t i = threadIdx.x; i < L; i += blockDim.x) sv[i] = rec[s + i];
     }
     __syncthreads();
     if (inShared) {
@@ -509,9 +496,6 @@ __global__ void __launch_bounds__(kBucketThreads) k_bucket_sort_large(
               if (b < a) {
                 V[lo] = b;
                 V[hi] = a;
-                const uint32_t t = I[lo];
-                I[lo] = I[hi];
-                I[hi] = t;
               }
             }
           }
@@ -533,10 +517,7 @@ __global__ void __launch_bounds__(kBucketThreads) k_bucket_sort_large(
           const uint32_t base = bl * (uint32_t)kLargeRow;
           if (base >= L) break;  // blocks of padding only: nothing to compare
           const uint32_t n = min((uint32_t)kLargeRow, L - base);
-          for (uint32_t i = threadIdx.x; i < n; i += blockDim.x) {
-            sv[i] = V[base + i];
-            sp[i] = I[base + i];
-          }
+          for (uint32_t i = threadIdx.x; i < n; i += blockDim.x) sv[i] = V[base + i];
           __syncthreads();
           for (uint32_t kk = kFirst; kk <= kLast; kk <<= 1) {
             for (uint32_t jj = kk == kFirst ? jjFirst : kk / 2; jj > 0; jj >>= 1) {
@@ -548,19 +529,13 @@ __global__ void __launch_bounds__(kBucketThreads) k_bucket_sort_large(
                   if (y < x) {
                     sv[lo] = y;
                     sv[hi] = x;
-                    const uint32_t t = sp[lo];
-                    sp[lo] = sp[hi];
-                    sp[hi] = t;
                   }
                 }
               }
               __syncthreads();
             }
           }
-          for (uint32_t i = threadIdx.x; i < n; i += blockDim.x) {
-            V[base + i] = sv[i];
-            I[base + i] = sp[i];
-          }
+          for (uint32_t i = threadIdx.x; i < n; i += blockDim.x) V[base + i] = sv[i];
           __syncthreads();
         }
       };
@@ -591,9 +566,6 @@ __global__ void __launch_bounds__(kBucketThreads) k_bucket_sort_large(
               if (ok[u] && b[u] < a[u]) {
                 V[lo[u]] = b[u];
                 V[hi[u]] = a[u];
-                const uint32_t t = I[lo[u]];
-                I[lo[u]] = I[hi[u]];
-                I[hi[u]] = t;
               }
             }
           }
@@ -602,10 +574,8 @@ __global__ void __launch_bounds__(kBucketThreads) k_bucket_sort_large(
         blockStages(k, k, (uint32_t)kLargeRow / 2);
       }
     }
-    for (uint32_t i = threadIdx.x; i < L; i += blockDim.x) {
-      sortedKeys[s + i] = r * nx + (uint32_t)(V[i] >> 32);
-      perm[s + i] = I[i];
-    }
+    for (uint32_t i = threadIdx.x; i < L; i += blockDim.x)
+      emitCellOrder(out, s + i, r * nx + (uint32_t)(V[i] >> 32), (uint32_t)V[i]);
     if (cellOff && L <= 65535u) {  // offsets are 16-bit; longer rows are searched by the scan
       uint16_t *t = cellOff + (size_t)r * cellOffPitch(nx);
       fillCellOffsets(t, nx, L, [&](uint32_t i) { return (uint32_t)(V[i] >> 32); }, threadIdx.x, blockDim.x);

@@ -30,12 +30,19 @@ __device__ __forceinline__ float4 floatPosition(double x, double y, double z) {
   const double m = fmax(fabs(x), fmax(fabs(y), fabs(z)));
   return make_float4((float)x, (float)y, (float)z, (float)(m * 0x1p-22) + 1e-12f);
 }
+__device__ __forceinline__ ScanRec scanRec(const double r[3], const double v[3], double radius, bool deleted) {
+  ScanRec o;
+  o.pos = floatPosition(r[0], r[1], r[2]);
+  if (deleted) o.pos.w = -o.pos.w;
+  o.vel = make_float4((float)v[0], (float)v[1], (float)v[2], __double2float_ru(radius));
+  return o;
+}
+__device__ __forceinline__ bool recDeleted(float4 pos) { return __float_as_int(pos.w) < 0; }
 
-// What the pair scan reads of the cell-ordered population: binary32 copies
-// (positions with their rounding bound, velocities with the radius rounded up)
-// in cell order, and, for the few pairs that reach the binary64 functor, the
-// state as it was before the gather (src, indexed through perm) -- the next
-// propagation, which runs beside the scan, writes only the gathered copy.
+// What the pair scan reads: the scan records in cell order (positions and
+// velocities as separate arrays), and, for the few pairs that reach the
+// binary64 functor, the scanned state itself (src, indexed through perm) -- the
+// next propagation, which runs beside the scan, writes the other buffer.
 // Breakup group of an object in the scan: its parent id when that fits 32
 // bits, else kNoGroup (no parent, or an id too large to compare here: such
 // pairs are left to the functor's own parent test).  Two objects of one group
@@ -47,41 +54,11 @@ __device__ __forceinline__ uint32_t groupOf(uint64_t parent) {
 }
 
 struct ScanPack {
-  float4 *posf;          // binary32 x, y, z + rounding bound
-  float4 *velf;          // binary32 vx, vy, vz + radius rounded up
-  DevState src;          // state before the gather
-  const uint32_t *perm;  // cell-order position -> index in src
-  uint32_t *grp;         // breakup group per cell-order position (null: no object has a parent)
+  const float4 *posf;    // binary32 x, y, z + rounding bound
+  const float4 *velf;    // binary32 vx, vy, vz + radius rounded up
+  DevState src;          // the scanned state
+  const uint32_t *perm;  // cell-order position -> slot
 };
-
-__global__ void k_permute(DevState src, DevState dst, const uint32_t *__restrict__ perm, int n, ScanPack pk,
-                          unsigned *__restrict__ status) {
-  const int j = blockIdx.x * blockDim.x + threadIdx.x;
-  if (j >= n) return;
-  uint32_t p = perm[j];
-  if (p >= (uint32_t)n) {  // a sort defect: record it and keep the access in bounds
-    atomicOr(status, 4u);
-    p = (uint32_t)j;
-  }
-  // read-only loads; the gathered state is written with streaming stores (it
-  // is read once, by the next propagation), the scan copies with plain ones
-  const double x = __ldg(&src.x[p]), y = __ldg(&src.y[p]), z = __ldg(&src.z[p]);
-  const double vx = __ldg(&src.vx[p]), vy = __ldg(&src.vy[p]), vz = __ldg(&src.vz[p]);
-  const uint32_t tag = __ldg(&src.tag[p]);
-  const double radius = tagSlot(tag) < (uint32_t)n ? __ldg(&src.radius[tagSlot(tag)]) : 0.0;  // slot-indexed
-  if (pk.grp) pk.grp[j] = tagSlot(tag) < (uint32_t)n ? groupOf(src.parent[tagSlot(tag)]) : kNoGroup;
-  __stcs(&dst.x[j], x);
-  __stcs(&dst.y[j], y);
-  __stcs(&dst.z[j], z);
-  __stcs(&dst.vx[j], vx);
-  __stcs(&dst.vy[j], vy);
-  __stcs(&dst.vz[j], vz);
-  __stcs(&dst.aom[j], __ldg(&src.aom[p]));
-  __stcs(&dst.bc[j], __ldg(&src.bc[p]));
-  __stcs(&dst.tag[j], tag);
-  pk.posf[j] = floatPosition(x, y, z);
-  pk.velf[j] = make_float4((float)vx, (float)vy, (float)vz, __double2float_ru(radius));
-}
 
 __device__ __forceinline__ double dot3rn(const double a[3], const double b[3]) {
   double r = __dadd_rn(0.0, __dmul_rn(a[0], b[0]));
@@ -124,7 +101,6 @@ struct Obj {
   uint32_t tag;
 };
 
-// (positions by the pre-gather position perm[k], radius / id / parent by slot)
 __device__ __forceinline__ void loadObjPacked(const ScanPack &pk, uint32_t k, Obj &o) {
   const uint32_t p = pk.perm[k];
   o.r[0] = pk.src.x[p];
@@ -134,10 +110,9 @@ __device__ __forceinline__ void loadObjPacked(const ScanPack &pk, uint32_t k, Ob
   o.v[1] = pk.src.vy[p];
   o.v[2] = pk.src.vz[p];
   o.tag = pk.src.tag[p];
-  const uint32_t s = tagSlot(o.tag);
-  o.radius = pk.src.radius[s];
-  o.id = pk.src.id[s];
-  o.parent = pk.src.parent[s];
+  o.radius = pk.src.radius[p];
+  o.id = pk.src.id[p];
+  o.parent = pk.src.parent[p];
 }
 
 // CollisionFunctor::AoSFunctor on (i, j) with the gate already evaluated.
@@ -260,26 +235,10 @@ __device__ __forceinline__ void emitPair(const Obj &I, const Obj &J, double dl2,
   }
 }
 
-// Scatter the sorted population back to slot order (download path).
-// (slots are dense in [0, n); the guards only keep a corrupted tag in bounds)
-__global__ void k_unpermute_f64(const double *__restrict__ src, const uint32_t *__restrict__ tag, int n,
-                                double *__restrict__ dst) {
+// activity states of the population (download path)
+__global__ void k_activity(const uint32_t *__restrict__ tag, int n, int8_t *__restrict__ dst) {
   const int j = blockIdx.x * blockDim.x + threadIdx.x;
-  if (j < n && tagSlot(tag[j]) < (uint32_t)n) dst[tagSlot(tag[j])] = src[j];
-}
-__global__ void k_unpermute_act(const uint32_t *__restrict__ tag, int n, int8_t *__restrict__ dst) {
-  const int j = blockIdx.x * blockDim.x + threadIdx.x;
-  if (j < n && tagSlot(tag[j]) < (uint32_t)n) dst[tagSlot(tag[j])] = (int8_t)tagAct(tag[j]);
-}
-__global__ void k_unpermute_tag(const uint32_t *__restrict__ tag, int n, uint32_t *__restrict__ dst) {
-  const int j = blockIdx.x * blockDim.x + threadIdx.x;
-  if (j < n && tagSlot(tag[j]) < (uint32_t)n) dst[tagSlot(tag[j])] = tag[j];
-}
-// Gather slot-ordered values into the current (sorted) order (state upload).
-__global__ void k_permute_from_slots_f64(const double *__restrict__ src, const uint32_t *__restrict__ tag, int n,
-                                         double *__restrict__ dst) {
-  const int j = blockIdx.x * blockDim.x + threadIdx.x;
-  if (j < n && tagSlot(tag[j]) < (uint32_t)n) dst[j] = src[tagSlot(tag[j])];
+  if (j < n) dst[j] = (int8_t)tagAct(tag[j]);
 }
 
 __global__ void k_clear_parents(uint64_t *__restrict__ parent, int n) {
@@ -290,15 +249,14 @@ __global__ void k_clear_parents(uint64_t *__restrict__ parent, int n) {
 // slotMark[slot] = 1 for slots to delete
 __global__ void k_mark_deleted(uint32_t *__restrict__ tag, const uint8_t *__restrict__ slotMark, int n) {
   const int j = blockIdx.x * blockDim.x + threadIdx.x;
-  if (j < n && tagSlot(tag[j]) < (uint32_t)n && slotMark[tagSlot(tag[j])]) tag[j] |= kTagDummy;
+  if (j < n && slotMark[j]) tag[j] |= kTagDummy;
 }
 
 // keep[j] = 1 if the object survives the burn-up test |r|^2 >= crit^2
-// (Simulation.cpp:581-590); aliveBySlot[slot] mirrors it in slot order;
-// *burnt counts the objects that fail it (one atomic per warp that has any).
+// (Simulation.cpp:581-590); *burnt counts the objects that fail it (one atomic
+// per warp that has any).
 __global__ void k_burnup_flags(const double *__restrict__ x, const double *__restrict__ y,
-                               const double *__restrict__ z, const uint32_t *__restrict__ tag, int n,
-                               double critSq, uint32_t *__restrict__ keep, uint32_t *__restrict__ aliveBySlot,
+                               const double *__restrict__ z, int n, double critSq, uint32_t *__restrict__ keep,
                                unsigned *__restrict__ burnt) {
   const int j = blockIdx.x * blockDim.x + threadIdx.x;
   uint32_t k = 1u;
@@ -306,7 +264,6 @@ __global__ void k_burnup_flags(const double *__restrict__ x, const double *__res
     const double a2 = x[j] * x[j] + y[j] * y[j] + z[j] * z[j];
     k = (a2 < critSq) ? 0u : 1u;
     keep[j] = k;
-    if (tagSlot(tag[j]) < (uint32_t)n) aliveBySlot[tagSlot(tag[j])] = k;
   }
   const unsigned below = __ballot_sync(0xffffffffu, k == 0u);
   if (below && (threadIdx.x & 31) == 0) atomicAdd(burnt, (unsigned)__popc(below));
@@ -315,16 +272,14 @@ __global__ void k_burnup_flags(const double *__restrict__ x, const double *__res
 // (slot, id) of every object with keep[j] == 0, appended in any order to
 // outSlot / outIdLo / outIdHi (count[0] = their number): the ids of a removal
 // go to the host without copying population-sized arrays.
-__global__ void k_removed_ids(const uint32_t *__restrict__ keep, const uint32_t *__restrict__ tag,
-                              const uint64_t *__restrict__ idBySlot, int n, uint32_t *__restrict__ outSlot,
-                              uint32_t *__restrict__ outIdLo, uint32_t *__restrict__ outIdHi,
-                              unsigned *__restrict__ count) {
+__global__ void k_removed_ids(const uint32_t *__restrict__ keep, const uint64_t *__restrict__ ids, int n,
+                              uint32_t *__restrict__ outSlot, uint32_t *__restrict__ outIdLo,
+                              uint32_t *__restrict__ outIdHi, unsigned *__restrict__ count) {
   const int j = blockIdx.x * blockDim.x + threadIdx.x;
   if (j >= n || keep[j]) return;
-  const uint32_t slot = tagSlot(tag[j]);
   const uint32_t q = atomicAdd(count, 1u);
-  const uint64_t id = slot < (uint32_t)n ? idBySlot[slot] : 0ull;
-  outSlot[q] = slot;
+  const uint64_t id = ids[j];
+  outSlot[q] = (uint32_t)j;
   outIdLo[q] = (uint32_t)id;
   outIdHi[q] = (uint32_t)(id >> 32);
 }
@@ -332,9 +287,9 @@ __global__ void k_removed_ids(const uint32_t *__restrict__ keep, const uint32_t 
 // keep[j] = 0 for the objects that leave the container: a position or
 // velocity that is not finite, or a position outside [boxMin, boxMax]
 // (AutoPas::updateContainer's leaving particles, Simulation.cpp:314; a NaN
-// position is inside no box); aliveBySlot mirrors keep in slot order.
+// position is inside no box).
 __global__ void k_escape_flags(DevState s, int n, double3 lo, double3 hi, uint32_t *__restrict__ keep,
-                               uint32_t *__restrict__ aliveBySlot, unsigned *__restrict__ escaped) {
+                               unsigned *__restrict__ escaped) {
   const int j = blockIdx.x * blockDim.x + threadIdx.x;
   uint32_t k = 1u;
   if (j < n) {
@@ -343,30 +298,21 @@ __global__ void k_escape_flags(DevState s, int n, double3 lo, double3 hi, uint32
     const bool finiteV = isfinite(s.vx[j]) && isfinite(s.vy[j]) && isfinite(s.vz[j]);
     k = (inside && finiteV) ? 1u : 0u;
     keep[j] = k;
-    if (tagSlot(s.tag[j]) < (uint32_t)n) aliveBySlot[tagSlot(s.tag[j])] = k;
   }
   const unsigned out = __ballot_sync(0xffffffffu, k == 0u);
   if (out && (threadIdx.x & 31) == 0) atomicAdd(escaped, (unsigned)__popc(out));
 }
 
-// keep[j] = 0 for the objects whose slot is marked (slotMark[slot] = 1);
-// aliveBySlot mirrors it in slot order.
-__global__ void k_slot_mark_flags(const uint32_t *__restrict__ tag, int n, const uint8_t *__restrict__ slotMark,
-                                  uint32_t *__restrict__ keep, uint32_t *__restrict__ aliveBySlot) {
+// keep[j] = 0 for the objects whose slot is marked
+__global__ void k_slot_mark_flags(int n, const uint8_t *__restrict__ slotMark, uint32_t *__restrict__ keep) {
   const int j = blockIdx.x * blockDim.x + threadIdx.x;
-  if (j >= n) return;
-  const uint32_t s = tagSlot(tag[j]);
-  const uint32_t k = (s < (uint32_t)n && slotMark[s]) ? 0u : 1u;
-  keep[j] = k;
-  if (s < (uint32_t)n) aliveBySlot[s] = k;
+  if (j < n) keep[j] = slotMark[j] ? 0u : 1u;
 }
 
-// compaction: dst[pos[j]] = src[j] for kept j, slots renumbered via newSlot;
-// the slot-indexed arrays go to the new slots of separate arrays (tRadius,
-// tId, tParent), as the state buffers share theirs
+// compaction: dst[pos[j]] = src[j] for kept j, slots renumbered to pos[j]; the
+// arrays that the state buffers share go to separate ones (tmp)
 __global__ void k_compact(DevState src, DevState dst, const uint32_t *__restrict__ keep,
-                          const uint32_t *__restrict__ pos, const uint32_t *__restrict__ newSlot, int n,
-                          double *__restrict__ tRadius, uint64_t *__restrict__ tId, uint64_t *__restrict__ tParent) {
+                          const uint32_t *__restrict__ pos, int n, DevState tmp) {
   const int j = blockIdx.x * blockDim.x + threadIdx.x;
   if (j >= n || !keep[j]) return;
   const uint32_t p = pos[j];
@@ -376,15 +322,12 @@ __global__ void k_compact(DevState src, DevState dst, const uint32_t *__restrict
   dst.vx[p] = src.vx[j];
   dst.vy[p] = src.vy[j];
   dst.vz[p] = src.vz[j];
-  dst.aom[p] = src.aom[j];
-  dst.bc[p] = src.bc[j];
-  const uint32_t t = src.tag[j], s = tagSlot(t);
-  if (s >= (uint32_t)n) return;  // only with a corrupted tag
-  const uint32_t ns = newSlot[s];
-  dst.tag[p] = (t & ~kTagSlotMask) | (ns & kTagSlotMask);
-  tRadius[ns] = src.radius[s];
-  tId[ns] = src.id[s];
-  tParent[ns] = src.parent[s];
+  tmp.aom[p] = src.aom[j];
+  tmp.bc[p] = src.bc[j];
+  tmp.tag[p] = (src.tag[j] & ~kTagSlotMask) | (p & kTagSlotMask);
+  tmp.radius[p] = src.radius[j];
+  tmp.id[p] = src.id[j];
+  tmp.parent[p] = src.parent[j];
 }
 
 // exclusive scan of u32 flags, three phases (block sums, scan of sums, apply)
@@ -417,6 +360,36 @@ __global__ void __launch_bounds__(kScanBlock) k_scan_blocks(const uint32_t *__re
   const uint32_t off = warp ? ws[warp - 1] : 0u;
   if (i < n) out[i] = off + incl - v;
   if (threadIdx.x == kScanBlock - 1) blockSums[blockIdx.x] = off + incl;
+}
+
+// exclusive scan in one launch, for few blocks: block b sums the values before
+// its own itself (all of them in L2) instead of waiting for a second launch to
+// bring the other blocks' sums.  62,501 rows (250^3 cells): 62 blocks.
+constexpr int kRowScanBlocks = 128;
+__global__ void __launch_bounds__(kScanBlock) k_row_scan(const uint32_t *__restrict__ in, int n,
+                                                         uint32_t *__restrict__ out) {
+  __shared__ uint32_t ws[32], wp[32];
+  const int b = blockIdx.x, t = threadIdx.x, lane = t & 31, warp = t >> 5, i = b * kScanBlock + t;
+  const uint32_t v = i < n ? in[i] : 0u;
+  uint32_t before = 0;  // values of the blocks before this one, 16 bytes at a time
+  const uint4 *in4 = reinterpret_cast<const uint4 *>(in);
+#pragma unroll 4
+  for (int q = t; q < b * (kScanBlock / 4); q += kScanBlock) {
+    const uint4 w = __ldg(&in4[q]);
+    before += (w.x + w.y) + (w.z + w.w);
+  }
+  uint32_t incl = v;
+#pragma unroll
+  for (int o = 1; o < 32; o <<= 1) {
+    const uint32_t u = __shfl_up_sync(0xffffffffu, incl, o);
+    if (lane >= o) incl += u;
+  }
+  before = __reduce_add_sync(0xffffffffu, before);
+  if (lane == 31) ws[warp] = incl;
+  if (lane == 0) wp[warp] = before;
+  __syncthreads();
+  const uint32_t off = __reduce_add_sync(0xffffffffu, wp[lane] + (lane < warp ? ws[lane] : 0u));
+  if (i < n) out[i] = off + incl - v;
 }
 
 // second pass of a two-pass exclusive scan (at most kScanBlock blocks): block b

@@ -59,29 +59,12 @@ __global__ void k_insert_blocked(DevState s, int n, const double *__restrict__ n
   if (lane == 0) blocked[w] = hit ? 1 : 0;
 }
 
-// pos[q] = position in the state arrays of wanted slot q (wanted sorted ascending)
-__global__ void k_find_slots(const uint32_t *__restrict__ tags, int n, const uint32_t *__restrict__ wanted, int m,
-                             int32_t *__restrict__ pos) {
-  const int j = blockIdx.x * blockDim.x + threadIdx.x;
-  if (j >= n) return;
-  const uint32_t slot = tagSlot(tags[j]);
-  int lo = 0, hi = m;
-  while (lo < hi) {
-    const int mid = (lo + hi) >> 1;
-    if (wanted[mid] < slot)
-      lo = mid + 1;
-    else
-      hi = mid;
-  }
-  if (lo < m && wanted[lo] == slot) pos[lo] = j;
-}
-
-__global__ void k_gather_records(DevState s, const int32_t *__restrict__ pos, int m,
+// records of the objects slots[0..m)
+__global__ void k_gather_records(DevState s, const uint32_t *__restrict__ slots, int m,
                                  ladds_state_record *__restrict__ out) {
   const int q = blockIdx.x * blockDim.x + threadIdx.x;
   if (q >= m) return;
-  const int32_t j = pos[q];
-  if (j < 0) return;
+  const uint32_t j = slots[q];
   ladds_state_record r;
   r.r[0] = s.x[j];
   r.r[1] = s.y[j];
@@ -89,42 +72,61 @@ __global__ void k_gather_records(DevState s, const int32_t *__restrict__ pos, in
   r.v[0] = s.vx[j];
   r.v[1] = s.vy[j];
   r.v[2] = s.vz[j];
-  const uint32_t slot = tagSlot(s.tag[j]);  // radius, id and parent are indexed by slot
-  r.radius = s.radius[slot];
+  r.radius = s.radius[j];
   r.aom = s.aom[j];
   r.bcInv = s.bc[j];
-  r.id = s.id[slot];
-  r.parentId = s.parent[slot];
+  r.id = s.id[j];
+  r.parentId = s.parent[j];
   r.activity = tagAct(s.tag[j]);
   r.deleted = tagDummy(s.tag[j]) ? 1u : 0u;
   out[q] = r;
 }
 
 // Layer selection of the device-resident exchange (ladds_gpu_pack_layers):
-// sel[j] = 1 for the live objects whose cell layer lies in [lo, hi), keep[j]
-// = !sel[j] and aliveBySlot its slot-order mirror (for the removal).
-__global__ void k_layer_flags(const double *__restrict__ z, const uint32_t *__restrict__ tag, int n, GridDesc g,
-                              int32_t lo, int32_t hi, uint32_t *__restrict__ sel, uint32_t *__restrict__ keep,
-                              uint32_t *__restrict__ aliveBySlot) {
-  const int j = blockIdx.x * blockDim.x + threadIdx.x;
-  if (j >= n) return;
-  const uint32_t t = tag[j];
+// sel[i] = 1 if the i-th object of the population's order -- perm for the
+// first m, then slot order -- is live and its cell layer lies in [lo, hi);
+// keep[slot] = !sel (for the removal).
+__global__ void k_layer_flags(const double *__restrict__ z, const uint32_t *__restrict__ tag, int n,
+                              const uint32_t *__restrict__ perm, int m, GridDesc g, int32_t lo, int32_t hi,
+                              uint32_t *__restrict__ sel, uint32_t *__restrict__ keep) {
+  const int i = blockIdx.x * blockDim.x + threadIdx.x;
+  if (i >= n) return;
+  const uint32_t j = i < m ? perm[i] : (uint32_t)i;
   const int32_t iz = (int32_t)cellCoord(z[j], g.boxMin[2], g.invCell, g.n[2]);
-  const uint32_t s = (!tagDummy(t) && iz >= lo && iz < hi) ? 1u : 0u;
-  sel[j] = s;
+  const uint32_t s = (!tagDummy(tag[j]) && iz >= lo && iz < hi) ? 1u : 0u;
+  sel[i] = s;
   keep[j] = 1u - s;
-  if (tagSlot(t) < (uint32_t)n) aliveBySlot[tagSlot(t)] = 1u - s;
 }
 
-// positions of the selected objects in their (current) order: idx[pos[j]] = j
-__global__ void k_selected_positions(const uint32_t *__restrict__ sel, const uint32_t *__restrict__ pos, int n,
-                                     int32_t *__restrict__ idx) {
+// slots of the selected objects in that order
+__global__ void k_selected_slots(const uint32_t *__restrict__ sel, const uint32_t *__restrict__ pos,
+                                 const uint32_t *__restrict__ perm, int m, int n, uint32_t *__restrict__ slots) {
+  const int i = blockIdx.x * blockDim.x + threadIdx.x;
+  if (i < n && sel[i]) slots[pos[i]] = i < m ? perm[i] : (uint32_t)i;
+}
+
+// compaction of an order: flag[i] = keep[perm[i]]; then moved[at[i]] = the new slot of a kept one
+__global__ void k_order_flags(const uint32_t *__restrict__ perm, const uint32_t *__restrict__ keep, int m,
+                              uint32_t *__restrict__ flag) {
+  const int i = blockIdx.x * blockDim.x + threadIdx.x;
+  if (i < m) flag[i] = keep[perm[i]];
+}
+__global__ void k_order_compact(const uint32_t *__restrict__ perm, const uint32_t *__restrict__ flag,
+                                const uint32_t *__restrict__ at, const uint32_t *__restrict__ pos, int m,
+                                uint32_t *__restrict__ moved) {
+  const int i = blockIdx.x * blockDim.x + threadIdx.x;
+  if (i < m && flag[i]) moved[at[i]] = pos[perm[i]];
+}
+// a truncation's flags and slots
+__global__ void k_below_flags(int n, uint32_t n0, uint32_t *__restrict__ keep, uint32_t *__restrict__ pos) {
   const int j = blockIdx.x * blockDim.x + threadIdx.x;
-  if (j < n && sel[j]) idx[pos[j]] = j;
+  if (j < n) {
+    keep[j] = (uint32_t)j < n0 ? 1u : 0u;
+    pos[j] = (uint32_t)j;
+  }
 }
 
-// State records (device memory) appended at positions / slots offset..offset+m
-// (slot-indexed radius, id and parent at the same index); bad[0] counts
+// State records (device memory) appended at slots offset..offset+m; bad[0] counts
 // records with a non-finite value or an activity state out of range, bad[1]
 // is set when a record has a parent id.
 __global__ void k_append_records(const ladds_state_record *__restrict__ in, int m, DevState s, uint32_t offset,
@@ -150,17 +152,6 @@ __global__ void k_append_records(const ladds_state_record *__restrict__ in, int 
   s.id[at] = r.id;
   s.parent[at] = r.parentId;
   s.tag[at] = makeTag(at, ok ? r.activity : 0, r.deleted != 0u);
-}
-
-// keep[j] = slot < n0 (the removal of a truncation), aliveBySlot its mirror
-__global__ void k_truncate_flags(const uint32_t *__restrict__ tag, int n, uint32_t n0, uint32_t *__restrict__ keep,
-                                 uint32_t *__restrict__ aliveBySlot) {
-  const int j = blockIdx.x * blockDim.x + threadIdx.x;
-  if (j >= n) return;
-  const uint32_t sl = tagSlot(tag[j]);
-  const uint32_t k = sl < n0 ? 1u : 0u;
-  keep[j] = k;
-  if (sl < (uint32_t)n) aliveBySlot[sl] = k;
 }
 
 }  // namespace ladds

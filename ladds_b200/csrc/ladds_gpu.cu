@@ -1,15 +1,18 @@
 // ladds_gpu.cu -- C ABI of the B200 hot path (see include/ladds_gpu.h).
 //
-// One context = one device, one stream, the device-resident population in two
-// SoA copies (current + alternate; a conjunction scan gathers the current copy
-// into cell order in the alternate one and swaps them) plus a third copy used
-// to roll a ladds_gpu_step call back when it has to be re-run.
+// One context = one device, one stream, the device-resident population: one
+// array per attribute in slot order, positions and velocities in two copies
+// (the propagation that ends at a scan reads the current one and writes the
+// other, and they change places) and a third that rolls a ladds_gpu_step call
+// of several iterations back when it has to be re-run.
 //
-// A scan iteration is: ephemeris of the three stage times -> constant memory,
-// Yoshida step with the cell key of the end position (one kernel), radix
-// sort of (key, index), gather into cell order, row-start table, pair scan.
+// A scan iteration is: ephemeris of the stage times -> constant memory,
+// Yoshida steps with the cell key, row count and scan record of the end state
+// (one kernel), row-start scan, scatter to the cell rows, sort inside the rows
+// with the gather of the scan records, pair scan.  The population itself is
+// never moved.
 // Multi-iteration calls are captured once into a CUDA graph per (iterations,
-// iteration % k, current buffer) and replayed.
+// iteration % k, current buffers) and replayed.
 #include <cuda_runtime.h>
 
 #include <algorithm>
@@ -38,19 +41,25 @@ namespace {
 // c_eph is per device: calls on one device are serialised.
 std::mutex g_deviceMutex[64];
 
-__global__ void k_advance(int64_t *iter, int by) {
-  if (threadIdx.x == 0 && blockIdx.x == 0) *iter += by;
-}
-// also stores the chunk's first iteration in *iterBase (the scans' step index)
+// Ephemeris entries of the stage times of the next nSteps iterations
+// (<= kMaxEphSteps, one block): also stores the first of them in *iterBase (the
+// scans' step index) and advances the iteration counter past them.
 template <typename Entry>
-__global__ void k_ephemeris_dev(Entry *__restrict__ out, int nSteps, const int64_t *__restrict__ iterPtr,
-                                int64_t *__restrict__ iterBase, double t0, double dt, double hc1, double hc2,
-                                double jdEpoch, double theta0, uint32_t mask) {
-  const int i = blockIdx.x * blockDim.x + threadIdx.x;
-  if (i == 0) *iterBase = *iterPtr;
+__global__ void __launch_bounds__(3 * kMaxEphSteps) k_ephemeris_dev(Entry *__restrict__ out, int nSteps,
+                                                                    int64_t *__restrict__ iterPtr,
+                                                                    int64_t *__restrict__ iterBase, double t0,
+                                                                    double dt, double hc1, double hc2, double jdEpoch,
+                                                                    double theta0, uint32_t mask) {
+  const int i = threadIdx.x;
+  const int64_t iter = *iterPtr;
+  __syncthreads();
+  if (i == 0) {
+    *iterBase = iter;
+    *iterPtr = iter + nSteps;
+  }
   if (i >= 3 * nSteps) return;
   const int st = i / 3, stage = i % 3;
-  const double tn = t0 + (double)(*iterPtr + st) * dt;
+  const double tn = t0 + (double)(iter + st) * dt;
   double tau = tn + hc1;
   if (stage >= 1) tau += hc2;
   if (stage >= 2) tau += hc2;
@@ -77,42 +86,45 @@ struct ladds_gpu_ctx {
   int dev = 0;
   cudaStream_t st = nullptr;   // main stream
   cudaStream_t st2 = nullptr;  // pair scans, overlapped with the next propagation
-  cudaStream_t st3 = nullptr;  // device-to-host copies of ladds_gpu_step_host
-  cudaEvent_t evCells = nullptr, evScan = nullptr;
-  cudaEvent_t evXfer[7] = {};  // per-array hand-offs between copies and (un)permutes of set/get_state
+  cudaStream_t st3 = nullptr;  // sorts between a propagation and its scan; device-to-host copies of ladds_gpu_step_host
+  cudaEvent_t evProp = nullptr, evSort[2] = {}, evScan[3] = {};  // hand-offs between the streams (evSort, evScan: the last ones)
   cudaEvent_t evPipe[3 * kHostChunks + 1] = {};  // chunk hand-offs of ladds_gpu_step_host
   double *pinStage = nullptr;  // pinned staging of ladds_gpu_step_host for pageable arrays (12 x pinCap)
   size_t pinCap = 0;
   std::vector<ladds_pair> pending;  // records of a ladds_gpu_step_host call whose buffer was too small
   int64_t *dIterBase = nullptr;  // first iteration of the chunk being run (device)
   size_t n = 0, cap = 0;
-  DevState cur{}, alt{}, snap{};
-  uint32_t *keys0 = nullptr, *keys1 = nullptr, *vals0 = nullptr, *vals1 = nullptr;
-  uint32_t *sortedKeys = nullptr, *perm = nullptr;  // results of the last sort
+  DevState cur{}, alt{}, alt2{}, snap{};  // the current state, the next two buffers of its ring, the roll-back copy
+  uint32_t *keys = nullptr, *arrival = nullptr;     // cell keys and row arrivals of the state to be scanned, slot order
+  ScanRec *scanRecs = nullptr;                      // its scan records, slot order
   unsigned long long *sortRec = nullptr;  // (ix << 32 | slot) sort records of the bucket sort
-  uint32_t *rowCounts = nullptr;          // objects per row (nRows + 1 used of 2 x (nRows + 1))
+  uint32_t *rowCounts = nullptr;          // objects per row; all zero but between a propagation and its sort
   uint32_t *longRows = nullptr, *longCount = nullptr;  // rows with more than 256 objects
   uint16_t *cellOff = nullptr;            // per row: offset of every cell inside the row (cellOffPitch entries)
   uint32_t *scanWs = nullptr;             // block sums of the exclusive scans
+  uint32_t *sortedKeys = nullptr, *perm = nullptr;  // result of the last sort: cell keys, slots
   float4 *posf = nullptr;                 // binary32 positions + rounding bound, cell order
   float4 *velf = nullptr;                 // binary32 velocities + radius of the cell order
   uint32_t *grp = nullptr;                // breakup group of the cell order (parent id, or kNoGroup)
   bool anyParent = false;                 // some object has a parent id: the scan writes and reads grp
   uint32_t *rowStart = nullptr;
   uint32_t nRows = 0;
-  uint32_t *scratchA = nullptr, *scratchB = nullptr, *scratchC = nullptr, *blockSums = nullptr;
+  uint32_t *scratchA = nullptr, *scratchB = nullptr, *scratchC = nullptr;
   ladds_pair *dPairs = nullptr;
   size_t pairCap = 0;
   unsigned long long *dCount = nullptr;
   uint2 *dCand = nullptr;  // candidate pairs (sorted indices) of the pair scan
   size_t candCap = 0;  // entries of each of the two candidate lists
-  unsigned long long *dCandCount = nullptr;  // lengths of the candidate lists of the current scan
+  unsigned long long *dCandCount = nullptr;  // lengths of the candidate lists of the current scan, dense-bin cursor
   unsigned long long *dCandNeed = nullptr;   // largest candidate count of the call
   unsigned *dStatus = nullptr;
   EphEntry *dEph = nullptr;
   int64_t *dIter = nullptr;
   int64_t hostIter = 0;
   bool orderValid = false;
+  // objects that perm has in the order of the last scan (later ones follow in
+  // slot order); 0 from before a sort is enqueued until it is known to have run
+  size_t orderN = 0;
   bool profiling = false;
   std::vector<std::tuple<int, cudaEvent_t, cudaEvent_t, int>> events;  // phase, start, end, kernels
   std::vector<cudaEvent_t> eventPool;
@@ -120,7 +132,7 @@ struct ladds_gpu_ctx {
   cudaEvent_t callStart = nullptr, callEnd = nullptr;
   std::map<std::tuple<int, int, int, size_t, size_t>, cudaGraphExec_t> graphs;
   std::string err;
-  double *homeX = nullptr;  // x array of the buffer that was current at allocation
+  double *homeX[2] = {};  // x arrays of the buffers that were current and next at allocation
   ladds_object *dObj = nullptr;  // staging of ladds_gpu_functor_pairs (2 x objCap)
   size_t objCap = 0;
   int evalBlocks = 592;     // grid of the candidate-evaluation kernel (4 per SM)
@@ -130,10 +142,14 @@ struct ladds_gpu_ctx {
   uint32_t *denseChunk = nullptr, *denseChunkB = nullptr;  // chunk index of each dense-bin entry
   uint32_t haloStart = 0xffffffffu;  // objects with slot >= haloStart: pair-scan targets only
   uint32_t denseCap = 0;
-  // second set of the sort results: the sort of a step writes one set while the
-  // pair scan of the previous step still reads the other
-  uint32_t *rowStartB = nullptr, *keys1B = nullptr, *vals1B = nullptr, *denseCellsB = nullptr,
-           *denseCountB = nullptr;
+  // second set of the sort's input and results: the propagation and the sort of
+  // a step write one set while the sort and the pair scan of the step before
+  // still read the other
+  uint32_t *rowStartB = nullptr, *sortedKeysB = nullptr, *permB = nullptr, *denseCellsB = nullptr,
+           *denseCountB = nullptr, *grpB = nullptr, *keysB = nullptr, *arrivalB = nullptr, *rowCountsB = nullptr;
+  ScanRec *scanRecsB = nullptr;
+  unsigned long long *dCandCountB = nullptr;
+  float4 *posfB = nullptr, *velfB = nullptr;
   uint16_t *cellOffB = nullptr;
   int sortParity = 0;
   struct Adjoint {          // buffers of the adjoint pair batch (ladds_gpu_adjoint_*)
@@ -162,38 +178,35 @@ int fail(ladds_gpu_ctx *c, int code, const std::string &msg) {
       return fail(c, LADDS_ERR_CUDA, std::string(#call) + ": " + cudaGetErrorString(e_));           \
   } while (0)
 
-// frees a state buffer; the slot-indexed arrays (radius, id, parent) only
-// when withSlotArrays (a context's buffers share them)
-void freeState(DevState &s, bool withSlotArrays) {
-  void *ptrs[] = {s.x, s.y, s.z, s.vx, s.vy, s.vz, s.aom, s.bc, s.tag};
-  for (void *p : ptrs)
+// frees a state buffer; the arrays that a context's buffers share only when
+// withShared
+void freeState(DevState &s, bool withShared) {
+  void *own[] = {s.x, s.y, s.z, s.vx, s.vy, s.vz};
+  for (void *p : own)
     if (p) cudaFree(p);
-  if (withSlotArrays) {
-    void *shared[] = {s.radius, s.id, s.parent};
+  if (withShared) {
+    void *shared[] = {s.aom, s.bc, s.tag, s.radius, s.id, s.parent};
     for (void *p : shared)
       if (p) cudaFree(p);
   }
   s = DevState{};
 }
 
-// allocates a state buffer; the slot-indexed arrays are taken from `shared`
-// (or allocated when it has none)
+// allocates a state buffer; the shared arrays are taken from `shared` (or
+// allocated when it is null)
 cudaError_t allocState(DevState &s, size_t cap, const DevState *shared) {
-  s = DevState{};
-  double **d[] = {&s.x, &s.y, &s.z, &s.vx, &s.vy, &s.vz, &s.aom, &s.bc};
+  s = shared ? *shared : DevState{};
+  double **d[] = {&s.x, &s.y, &s.z, &s.vx, &s.vy, &s.vz};
+  for (double **p : d) *p = nullptr;
   for (double **p : d) {
     cudaError_t e = cudaMalloc(p, cap * sizeof(double));
     if (e != cudaSuccess) return e;
   }
-  cudaError_t e = cudaMalloc(&s.tag, cap * sizeof(uint32_t));
-  if (e != cudaSuccess) return e;
-  if (shared) {
-    s.radius = shared->radius;
-    s.id = shared->id;
-    s.parent = shared->parent;
-    return cudaSuccess;
-  }
-  e = cudaMalloc(&s.radius, cap * sizeof(double));
+  if (shared) return cudaSuccess;
+  cudaError_t e = cudaMalloc(&s.aom, cap * sizeof(double));
+  if (e == cudaSuccess) e = cudaMalloc(&s.bc, cap * sizeof(double));
+  if (e == cudaSuccess) e = cudaMalloc(&s.tag, cap * sizeof(uint32_t));
+  if (e == cudaSuccess) e = cudaMalloc(&s.radius, cap * sizeof(double));
   if (e == cudaSuccess) e = cudaMalloc(&s.id, cap * sizeof(uint64_t));
   if (e == cudaSuccess) e = cudaMalloc(&s.parent, cap * sizeof(uint64_t));
   return e;
@@ -211,21 +224,21 @@ cudaError_t copyDynamic(const DevState &src, const DevState &dst, size_t n, cuda
   return cudaSuccess;
 }
 
-// copies a state buffer (the slot-indexed arrays only when the buffers do not share them)
-cudaError_t copyState(const DevState &src, const DevState &dst, size_t n, cudaStream_t st) {
+// the arrays that a context's buffers share
+cudaError_t copyShared(const DevState &src, const DevState &dst, size_t n, cudaStream_t st) {
   if (n == 0) return cudaSuccess;
-  const double *sd[] = {src.x, src.y, src.z, src.vx, src.vy, src.vz, src.aom, src.bc};
-  double *dd[] = {dst.x, dst.y, dst.z, dst.vx, dst.vy, dst.vz, dst.aom, dst.bc};
-  for (int k = 0; k < 8; ++k) {
-    cudaError_t e = cudaMemcpyAsync(dd[k], sd[k], n * sizeof(double), cudaMemcpyDeviceToDevice, st);
+  const void *sd[] = {src.aom, src.bc, src.radius, src.id, src.parent, src.tag};
+  void *dd[] = {dst.aom, dst.bc, dst.radius, dst.id, dst.parent, dst.tag};
+  for (int k = 0; k < 6; ++k) {
+    cudaError_t e = cudaMemcpyAsync(dd[k], sd[k], n * (k < 5 ? sizeof(double) : sizeof(uint32_t)),
+                                    cudaMemcpyDeviceToDevice, st);
     if (e != cudaSuccess) return e;
   }
-  cudaError_t e = cudaMemcpyAsync(dst.tag, src.tag, n * sizeof(uint32_t), cudaMemcpyDeviceToDevice, st);
-  if (e != cudaSuccess || src.id == dst.id) return e;
-  e = cudaMemcpyAsync(dst.radius, src.radius, n * sizeof(double), cudaMemcpyDeviceToDevice, st);
-  if (e == cudaSuccess) e = cudaMemcpyAsync(dst.id, src.id, n * sizeof(uint64_t), cudaMemcpyDeviceToDevice, st);
-  if (e == cudaSuccess) e = cudaMemcpyAsync(dst.parent, src.parent, n * sizeof(uint64_t), cudaMemcpyDeviceToDevice, st);
-  return e;
+  return cudaSuccess;
+}
+cudaError_t copyState(const DevState &src, const DevState &dst, size_t n, cudaStream_t st) {
+  const cudaError_t e = copyDynamic(src, dst, n, st);
+  return e != cudaSuccess ? e : copyShared(src, dst, n, st);
 }
 
 void dropGraphs(ladds_gpu_ctx *c) {
@@ -238,19 +251,17 @@ int ensureCandCapacity(ladds_gpu_ctx *c, size_t need);
 void freeBuffers(ladds_gpu_ctx *c) {
   freeState(c->cur, true);
   freeState(c->alt, false);
+  freeState(c->alt2, false);
   freeState(c->snap, false);
-  void *ptrs[] = {c->keys0, c->keys1, c->vals0, c->vals1, c->scratchA, c->scratchB, c->scratchC,
-                  c->blockSums, c->posf, c->sortRec, c->scanWs, c->velf, c->keys1B, c->vals1B, c->grp};
-  for (void *p : ptrs)
-    if (p) cudaFree(p);
-  c->posf = nullptr;
-  c->velf = nullptr;
-  c->grp = nullptr;
-  c->sortRec = nullptr;
-  c->scanWs = nullptr;
-  c->keys0 = c->keys1 = c->vals0 = c->vals1 = c->keys1B = c->vals1B = nullptr;
-  c->scratchA = c->scratchB = c->scratchC = c->blockSums = nullptr;
-  c->sortedKeys = c->perm = nullptr;
+  void **ptrs[] = {(void **)&c->keys, (void **)&c->keysB, (void **)&c->arrival, (void **)&c->arrivalB,
+                   (void **)&c->scanRecs, (void **)&c->scanRecsB, (void **)&c->sortRec, (void **)&c->scratchA,
+                   (void **)&c->scratchB, (void **)&c->scratchC, (void **)&c->scanWs, (void **)&c->sortedKeys,
+                   (void **)&c->sortedKeysB, (void **)&c->perm, (void **)&c->permB, (void **)&c->posf,
+                   (void **)&c->posfB, (void **)&c->velf, (void **)&c->velfB, (void **)&c->grp, (void **)&c->grpB};
+  for (void **p : ptrs) {
+    if (*p) cudaFree(*p);
+    *p = nullptr;
+  }
   c->cap = 0;
 }
 
@@ -259,14 +270,13 @@ int ensureCapacity(ladds_gpu_ctx *c, size_t need) {
   if (need > kMaxObjects) return fail(c, LADDS_ERR_INVALID_ARG, "population exceeds 2^28 - 1 objects");
   size_t newCap = std::max<size_t>({need, c->cap + c->cap / 2, 4096});
   newCap = std::min(newCap, kMaxObjects);
-  DevState ncur, nalt, nsnap;
+  DevState ncur, next[3] = {};  // alt, alt2, snap
   cudaError_t e = allocState(ncur, newCap, nullptr);
-  if (e == cudaSuccess) e = allocState(nalt, newCap, &ncur);
-  if (e == cudaSuccess) e = allocState(nsnap, newCap, &ncur);
+  for (DevState &d : next)
+    if (e == cudaSuccess) e = allocState(d, newCap, &ncur);
   if (e != cudaSuccess) {
+    for (DevState &d : next) freeState(d, false);
     freeState(ncur, true);
-    freeState(nalt, false);
-    freeState(nsnap, false);
     cudaGetLastError();
     return fail(c, LADDS_ERR_ALLOC, std::string("device allocation failed: ") + cudaGetErrorString(e));
   }
@@ -275,16 +285,26 @@ int ensureCapacity(ladds_gpu_ctx *c, size_t need) {
     if (e == cudaSuccess) e = cudaStreamSynchronize(c->st);
     if (e != cudaSuccess) return fail(c, LADDS_ERR_CUDA, cudaGetErrorString(e));
   }
-  const size_t n = c->n;
+  const size_t n = c->n, orderN = std::min(c->orderN, c->n);
+  uint32_t *const oldPerm = c->perm;  // the order of the last scan moves to the new buffer below
+  c->perm = nullptr;
+  c->orderN = 0;
+  struct FreeLater {
+    uint32_t *p;
+    ~FreeLater() {
+      if (p) cudaFree(p);
+    }
+  } freeOldPerm{oldPerm};
   freeBuffers(c);
   c->n = n;
   c->cur = ncur;
-  c->alt = nalt;
-  c->snap = nsnap;
-  c->homeX = ncur.x;
-  const size_t scanBlocks = (newCap + 1 + kScanBlock - 1) / kScanBlock;
-  uint32_t **u[] = {&c->keys0,    &c->keys1,    &c->vals0,  &c->vals1, &c->scratchA,
-                    &c->scratchB, &c->scratchC, &c->keys1B, &c->vals1B};
+  c->alt = next[0];
+  c->alt2 = next[1];
+  c->snap = next[2];
+  c->homeX[0] = c->cur.x;
+  c->homeX[1] = c->alt.x;
+  uint32_t **u[] = {&c->keys,     &c->keysB,    &c->arrival,    &c->arrivalB,    &c->scratchA, &c->scratchB,
+                    &c->scratchC, &c->perm,     &c->permB,      &c->sortedKeys,  &c->sortedKeysB};
   for (uint32_t **p : u) {
     if (cudaMalloc(p, (newCap + 1) * sizeof(uint32_t)) != cudaSuccess) {
       cudaGetLastError();
@@ -297,9 +317,13 @@ int ensureCapacity(ladds_gpu_ctx *c, size_t need) {
   if (cudaMalloc(&c->posf, newCap * sizeof(float4)) != cudaSuccess ||
       cudaMalloc(&c->velf, newCap * sizeof(float4)) != cudaSuccess ||
       cudaMalloc(&c->grp, newCap * sizeof(uint32_t)) != cudaSuccess ||
+      cudaMalloc(&c->posfB, newCap * sizeof(float4)) != cudaSuccess ||
+      cudaMalloc(&c->velfB, newCap * sizeof(float4)) != cudaSuccess ||
+      cudaMalloc(&c->grpB, newCap * sizeof(uint32_t)) != cudaSuccess ||
+      cudaMalloc(&c->scanRecs, newCap * sizeof(ScanRec)) != cudaSuccess ||
+      cudaMalloc(&c->scanRecsB, newCap * sizeof(ScanRec)) != cudaSuccess ||
       cudaMalloc(&c->sortRec, newCap * sizeof(unsigned long long)) != cudaSuccess ||
-      cudaMalloc(&c->scanWs, wsWords * sizeof(uint32_t)) != cudaSuccess ||
-      cudaMalloc(&c->blockSums, (scanBlocks + 1) * sizeof(uint32_t)) != cudaSuccess) {
+      cudaMalloc(&c->scanWs, wsWords * sizeof(uint32_t)) != cudaSuccess) {
     cudaGetLastError();
     return fail(c, LADDS_ERR_ALLOC, "device allocation failed (cell-order buffers)");
   }
@@ -320,6 +344,11 @@ int ensureCapacity(ladds_gpu_ctx *c, size_t need) {
       c->denseCap = 0;
       return fail(c, LADDS_ERR_ALLOC, "device allocation failed (dense-cell list)");
     }
+  }
+  if (orderN) {
+    CK(cudaMemcpyAsync(c->perm, oldPerm, orderN * sizeof(uint32_t), cudaMemcpyDeviceToDevice, c->st));
+    CK(cudaStreamSynchronize(c->st));
+    c->orderN = orderN;
   }
   c->cap = newCap;
   c->orderValid = false;
@@ -453,74 +482,77 @@ void collectTimes(ladds_gpu_ctx *c) {
 // ----- pipeline pieces (all enqueue on c->st; no synchronisation) -----
 
 cudaError_t enqueueEphemeris(ladds_gpu_ctx *c, int nSteps) {
-  const int threads = 3 * nSteps, g = blocksFor(threads, 128);
+  const int threads = 3 * nSteps, b = (threads + 31) / 32 * 32;
   const bool split = c->cfg.precision == LADDS_PRECISION_SPLIT;
   if (split)
-    k_ephemeris_dev<<<g, 128, 0, c->st>>>(reinterpret_cast<EphEntryF *>(c->dEph), nSteps, c->dIter, c->dIterBase,
+    k_ephemeris_dev<<<1, b, 0, c->st>>>(reinterpret_cast<EphEntryF *>(c->dEph), nSteps, c->dIter, c->dIterBase,
                                           c->cfg.startTime, c->cfg.deltaT, c->pc.hc1, c->pc.hc2, c->cfg.epochJD,
                                           c->theta0, c->pc.mask);
   else
-    k_ephemeris_dev<<<g, 128, 0, c->st>>>(c->dEph, nSteps, c->dIter, c->dIterBase, c->cfg.startTime, c->cfg.deltaT,
+    k_ephemeris_dev<<<1, b, 0, c->st>>>(c->dEph, nSteps, c->dIter, c->dIterBase, c->cfg.startTime, c->cfg.deltaT,
                                           c->pc.hc1, c->pc.hc2, c->cfg.epochJD, c->theta0, c->pc.mask);
   return cudaMemcpyToSymbolAsync(c_eph, c->dEph, (size_t)threads * (split ? sizeof(EphEntryF) : sizeof(EphEntry)), 0,
                                  cudaMemcpyDeviceToDevice, c->st);
 }
 
-// the bulk copies of k_propagate_staged need 16-byte aligned arrays
-bool stageable(const DevState &s) {
-  const void *p[] = {s.x, s.y, s.z, s.vx, s.vy, s.vz, s.aom, s.bc, s.tag};
-  for (const void *q : p)
-    if (reinterpret_cast<uintptr_t>(q) & 15u) return false;
-  return true;
+ScanInput scanInput(const ladds_gpu_ctx *c) {
+  return ScanInput{c->keys, c->rowCounts, c->arrival, c->scanRecs, c->cur.radius};
 }
 
-// the propagation kernel over objects [0, n) of s on the main stream; with
-// keys, their cell keys and row arrivals go to keyOut / arrOut (indexed as s)
-void launchPropagate(ladds_gpu_ctx *c, const DevState &s, int n, int nSteps, int ephBase, bool keys,
-                     uint32_t *keyOut, uint32_t *arrOut) {
-  const int b = c->cfg.propagateBlock > 0 ? c->cfg.propagateBlock : 256;
-  const int g = blocksFor((size_t)n, b);
-  uint32_t *rc = c->rowCounts;
-  if (keys && stageable(s)) {  // the per-scan propagation: persistent grid, state staged by bulk copies
-    // two CTAs per SM: alone the kernel is faster with four, but it runs beside
-    // the previous iteration's pair scan, which the other slots then serve
-    const int sg = std::max(1, std::min(blocksFor((size_t)n, kStageObjects), c->evalBlocks / 2));
-    if (c->cfg.precision == LADDS_PRECISION_SPLIT)
-      k_propagate_staged<true><<<sg, kStageObjects, 0, c->st>>>(s, n, nSteps, ephBase, c->pc, c->grid, keyOut, rc,
-                                                                arrOut, c->dStatus);
-    else
-      k_propagate_staged<false><<<sg, kStageObjects, 0, c->st>>>(s, n, nSteps, ephBase, c->pc, c->grid, keyOut, rc,
-                                                                 arrOut, c->dStatus);
-    return;
+// nSteps steps of the objects [lo, lo + n), from s to `to`, with the scan
+// input of the end state if a scan follows.  lo is a multiple of 256, so that
+// every array the kernel's bulk copies read starts on a 16-byte boundary.
+void launchPropagate(ladds_gpu_ctx *c, DevState s, DevState to, size_t lo, int n, int nSteps, int ephBase,
+                     bool scan) {
+  ScanInput in = scanInput(c);
+  for (DevState *d : {&s, &to}) {
+    d->x += lo; d->y += lo; d->z += lo; d->vx += lo; d->vy += lo; d->vz += lo;
+    d->aom += lo; d->bc += lo; d->tag += lo;
   }
-  if (c->cfg.precision == LADDS_PRECISION_SPLIT) {
-    if (keys)
-      k_propagate<true, true><<<g, b, 0, c->st>>>(s, n, nSteps, ephBase, c->pc, c->grid, keyOut, rc, arrOut,
-                                                  c->dStatus);
-    else
-      k_propagate<true, false><<<g, b, 0, c->st>>>(s, n, nSteps, ephBase, c->pc, c->grid, nullptr, nullptr, nullptr,
-                                                   c->dStatus);
-  } else {
-    if (keys)
-      k_propagate<false, true><<<g, b, 0, c->st>>>(s, n, nSteps, ephBase, c->pc, c->grid, keyOut, rc, arrOut,
-                                                   c->dStatus);
-    else
-      k_propagate<false, false><<<g, b, 0, c->st>>>(s, n, nSteps, ephBase, c->pc, c->grid, nullptr, nullptr,
-                                                    nullptr, c->dStatus);
-  }
+  in.keys += lo;
+  in.arrival += lo;
+  in.rec += lo;
+  in.radius += lo;
+  // three CTAs per SM: the sort and the scan of the iterations before run
+  // beside the kernel on streams of their own.  Graph step with two / three /
+  // four: 250,000 objects at every fourth iteration 22.5 / 20.7 / 18.9 us, 1e6
+  // 162 / 156 / 150 us, 2e6 391 / 381 / 391 us, 8e6 (40 km) 3331 / 3221 / 3322 us.
+  const int sg = std::max(1, std::min(blocksFor((size_t)n, kStageObjects), c->evalBlocks * 3 / 4));
+  const bool split = c->cfg.precision == LADDS_PRECISION_SPLIT;
+  auto kernel = split ? (scan ? k_propagate_staged<true, true> : k_propagate_staged<true, false>)
+                      : (scan ? k_propagate_staged<false, true> : k_propagate_staged<false, false>);
+  kernel<<<sg, kStageObjects, 0, c->st>>>(s, to, n, nSteps, ephBase, c->pc, c->grid, in, c->dStatus);
 }
 
-// nSteps steps whose stage ephemerides are c_eph[ephBase ...]
-void enqueuePropagate(ladds_gpu_ctx *c, int nSteps, bool keys, int ephBase) {
-  if (c->n == 0) {
-    k_advance<<<1, 32, 0, c->st>>>(c->dIter, nSteps);
-    return;
-  }
-  // with keys: the row counts of the coming sort are accumulated by the kernel
-  if (keys) cudaMemsetAsync(c->rowCounts, 0, ((size_t)c->nRows + 1) * sizeof(uint32_t), c->st);
-  PhaseScope ps(c, kPhProp, c->st, 2);  // propagation + iteration counter
-  launchPropagate(c, c->cur, (int)c->n, nSteps, ephBase, keys, c->keys0, c->scratchC);
-  k_advance<<<1, 32, 0, c->st>>>(c->dIter, nSteps);
+// nSteps steps, in place (stage ephemerides c_eph[ephBase ...])
+void enqueuePropagate(ladds_gpu_ctx *c, int nSteps, int ephBase) {
+  if (!c->n) return;
+  PhaseScope ps(c, kPhProp, c->st);
+  const int b = c->cfg.propagateBlock > 0 ? c->cfg.propagateBlock : 256, g = blocksFor(c->n, b);
+  if (c->cfg.precision == LADDS_PRECISION_SPLIT)
+    k_propagate<true><<<g, b, 0, c->st>>>(c->cur, (int)c->n, nSteps, ephBase, c->pc, c->dStatus);
+  else
+    k_propagate<false><<<g, b, 0, c->st>>>(c->cur, (int)c->n, nSteps, ephBase, c->pc, c->dStatus);
+}
+
+// the next buffer of the ring becomes the current state
+void rotateStates(ladds_gpu_ctx *c) {
+  const DevState old = c->cur;
+  c->cur = c->alt;
+  c->alt = c->alt2;
+  c->alt2 = old;
+}
+// position in the ring and sort set, as captured graphs have them baked in
+int bufferRoles(const ladds_gpu_ctx *c) {
+  return (c->cur.x == c->homeX[0] ? 0 : c->cur.x == c->homeX[1] ? 1 : 2) | 4 * c->sortParity;
+}
+
+// nSteps steps into the next state buffer, which becomes the current one, with
+// the input of the scan that follows them
+void enqueuePropagateStaged(ladds_gpu_ctx *c, int nSteps, int ephBase, bool scan) {
+  PhaseScope ps(c, kPhProp, c->st);
+  launchPropagate(c, c->cur, c->alt, 0, (int)c->n, nSteps, ephBase, scan);
+  rotateStates(c);
 }
 
 // kernels launched by enqueueExclusiveScan for `count` values
@@ -536,24 +568,24 @@ int exclusiveScanKernels(size_t count) {
 // exclusive scan of `count` u32 values (1024-wide block scans; up to 2^20
 // values: block scans, then each block adds the sum of the blocks before it;
 // beyond: three levels, count <= 2^30); block sums live in c->scanWs
-void enqueueExclusiveScan(ladds_gpu_ctx *c, const uint32_t *in, size_t count, uint32_t *out) {
+void enqueueExclusiveScan(ladds_gpu_ctx *c, const uint32_t *in, size_t count, uint32_t *out, cudaStream_t s) {
   const int nb1 = blocksFor(count, kScanBlock);
   uint32_t *s1 = c->scanWs, *s1x = s1 + nb1 + 1;
-  k_scan_blocks<<<nb1, kScanBlock, 0, c->st>>>(in, (int)count, out, s1);
+  k_scan_blocks<<<nb1, kScanBlock, 0, s>>>(in, (int)count, out, s1);
   if (nb1 == 1) return;
   if (kScanFoldSums && nb1 <= kScanBlock) {
-    k_scan_add_prefix<<<nb1, kScanBlock, 0, c->st>>>(out, (int)count, s1);
+    k_scan_add_prefix<<<nb1, kScanBlock, 0, s>>>(out, (int)count, s1);
     return;
   }
   const int nb2 = blocksFor((size_t)nb1, kScanBlock);
   uint32_t *s2 = s1x + nb1 + 1;
-  k_scan_blocks<<<nb2, kScanBlock, 0, c->st>>>(s1, nb1, s1x, s2);
+  k_scan_blocks<<<nb2, kScanBlock, 0, s>>>(s1, nb1, s1x, s2);
   if (nb2 > 1) {
     uint32_t *s2x = s2 + nb2 + 1, *s3 = s2x + nb2 + 1;
-    k_scan_blocks<<<1, kScanBlock, 0, c->st>>>(s2, nb2, s2x, s3);
-    k_scan_add<<<nb2, kScanBlock, 0, c->st>>>(s1x, nb1, s2x);
+    k_scan_blocks<<<1, kScanBlock, 0, s>>>(s2, nb2, s2x, s3);
+    k_scan_add<<<nb2, kScanBlock, 0, s>>>(s1x, nb1, s2x);
   }
-  k_scan_add<<<nb1, kScanBlock, 0, c->st>>>(out, (int)count, s1x);
+  k_scan_add<<<nb1, kScanBlock, 0, s>>>(out, (int)count, s1x);
 }
 
 // the dense bin of the pair scan: on with the counting row sort and the cell tables
@@ -563,67 +595,74 @@ DenseBin denseBin(const ladds_gpu_ctx *c) {
   return DenseBin{on ? c->denseCells : nullptr, c->denseCount, c->denseCap, kDenseCell, c->denseChunk};
 }
 
-// the sort writes the result set that the previous pair scan does not read
+// called before a scan's input is written: the set that neither the sort nor
+// the pair scan before it uses
 void swapSortSets(ladds_gpu_ctx *c) {
+  std::swap(c->keys, c->keysB);
+  std::swap(c->arrival, c->arrivalB);
+  std::swap(c->rowCounts, c->rowCountsB);
+  std::swap(c->scanRecs, c->scanRecsB);
   std::swap(c->rowStart, c->rowStartB);
-  std::swap(c->keys1, c->keys1B);
-  std::swap(c->vals1, c->vals1B);
+  std::swap(c->sortedKeys, c->sortedKeysB);
+  std::swap(c->perm, c->permB);
+  std::swap(c->posf, c->posfB);
+  std::swap(c->velf, c->velfB);
+  std::swap(c->grp, c->grpB);
   std::swap(c->cellOff, c->cellOffB);
   std::swap(c->denseCells, c->denseCellsB);
   std::swap(c->denseChunk, c->denseChunkB);
   std::swap(c->denseCount, c->denseCountB);
+  std::swap(c->dCandCount, c->dCandCountB);
   c->sortParity ^= 1;
 }
 
-// keys0 holds the keys of c->cur in current order, rowCounts their row counts
-// and scratchC their arrival indices (k_propagate<*, true> or k_cell_keys) ->
-// sortedKeys (keys1), perm (vals1) and the row-start table; order = sort by
-// (cell key, slot)
-void enqueueSort(ladds_gpu_ctx *c) {
-  swapSortSets(c);
+// row-start table from the row counts; kernels launched
+int enqueueRowScan(ladds_gpu_ctx *c, cudaStream_t s) {
+  const size_t count = (size_t)c->nRows + 1;
+  const int nb = blocksFor(count, kScanBlock);
+  if (nb <= kRowScanBlocks) {
+    k_row_scan<<<nb, kScanBlock, 0, s>>>(c->rowCounts, (int)count, c->rowStart);
+    return 1;
+  }
+  enqueueExclusiveScan(c, c->rowCounts, count, c->rowStart, s);
+  return exclusiveScanKernels(count);
+}
+
+// keys, arrival, rowCounts and scanRecs hold the scan input of the current
+// state (writeScanInput) -> row-start table, sortedKeys and perm (order = sort
+// by (cell key, slot)) and the scan records in that order.  The placement
+// clears what the next sort and scan on this set count in.
+void enqueueSort(ladds_gpu_ctx *c, cudaStream_t s) {
   const int n = (int)c->n;
   const uint32_t nx = (uint32_t)c->grid.n[0], nRows = c->nRows;
   {
-    PhaseScope ps(c, kPhBucket, c->st, 1 + exclusiveScanKernels((size_t)nRows + 1));
-    cudaMemsetAsync(c->longCount, 0, sizeof(uint32_t), c->st);
-    cudaMemsetAsync(c->denseCount, 0, sizeof(uint32_t), c->st);
-    enqueueExclusiveScan(c, c->rowCounts, (size_t)nRows + 1, c->rowStart);
-    k_bucket_place<<<blocksFor(c->n, kBucketThreads), kBucketThreads, 0, c->st>>>(
-        c->keys0, c->scratchC, c->cur.tag, n, nx, c->rowStart, c->sortRec, c->vals0, c->dStatus);
+    PhaseScope ps(c, kPhBucket, s, 2);
+    const int k = enqueueRowScan(c, s);
+    ps.kernels = 1 + k;
+    k_bucket_place<<<blocksFor(c->n, kBucketThreads), kBucketThreads, 0, s>>>(
+        c->keys, c->arrival, n, nx, c->rowStart, c->sortRec, c->rowCounts, nRows + 1, c->longCount, c->denseCount,
+        c->dCandCount, c->dStatus);
   }
-  PhaseScope ps(c, kPhRowsort, c->st, 2);
+  PhaseScope ps(c, kPhRowsort, s, 2);
   const DenseBin dense = denseBin(c);
+  const CellOrderOut out{c->sortedKeys, c->perm, c->scanRecs, c->posf, c->velf,
+                         c->anyParent ? c->cur.parent : nullptr, c->grp};
   if (nx <= (uint32_t)kRowCountMaxNx) {  // counting sort inside the rows
-    // one resident wave (8 CTAs of 4 warps per SM by shared memory); each warp pipelines its rows
-    const int rowBlocks = std::min(blocksFor((size_t)nRows * 32, kRowSortThreads), 2 * c->evalBlocks);
-    k_bucket_sort_rows<<<rowBlocks, kRowSortThreads, rowSortSmem(nx), c->st>>>(
-        c->rowStart, nRows, nx, c->sortRec, c->vals0, c->keys1, c->vals1, c->longRows, c->longCount, c->cellOff,
-        dense);
+    // one resident wave (10 CTAs of 4 warps per SM); each warp pipelines its rows
+    const int rowBlocks = std::min(blocksFor((size_t)nRows * 32, kRowSortThreads), 5 * c->evalBlocks / 2);
+    k_bucket_sort_rows<<<rowBlocks, kRowSortThreads, rowSortSmem(nx), s>>>(
+        c->rowStart, nRows, nx, c->sortRec, out, c->longRows, c->longCount, c->cellOff, dense);
   } else {
     const int smallBlocks = std::min(blocksFor((size_t)nRows * 32, kBucketThreads), 16 * c->evalBlocks);
-    k_bucket_sort_small<<<smallBlocks, kBucketThreads, 0, c->st>>>(
-        c->rowStart, nRows, nx, c->sortRec, c->vals0, c->keys1, c->vals1, c->longRows, c->longCount, c->cellOff);
+    k_bucket_sort_small<<<smallBlocks, kBucketThreads, 0, s>>>(c->rowStart, nRows, nx, c->sortRec, out, c->longRows,
+                                                               c->longCount, c->cellOff);
   }
-  k_bucket_sort_large<<<c->evalBlocks / 2, kBucketThreads, kLargeRow * 12, c->st>>>(
-      c->rowStart, nx, c->sortRec, c->vals0, c->keys1, c->vals1, c->longRows, c->longCount, c->cellOff, dense);
-  c->sortedKeys = c->keys1;
-  c->perm = c->vals1;
+  k_bucket_sort_large<<<c->evalBlocks / 2, kBucketThreads, kLargeRow * 8, s>>>(
+      c->rowStart, nx, c->sortRec, out, c->longRows, c->longCount, c->cellOff, dense);
 }
 
-// after the gather (enqueueCells) alt holds the state as the scan sees it, perm maps into it
-inline ScanPack scanPack(ladds_gpu_ctx *c) {
-  return ScanPack{c->posf, c->velf, c->alt, c->perm, c->anyParent ? c->grp : nullptr};
-}
-
-// gathers the state into cell order (so that the next propagation, key pass and
-// gather read nearly sequentially: objects move about one cell per step) and
-// writes the packed scan copies
-void enqueueCells(ladds_gpu_ctx *c) {
-  PhaseScope ps(c, kPhPermute, c->st);
-  k_permute<<<blocksFor(c->n, 256), 256, 0, c->st>>>(c->cur, c->alt, c->perm, (int)c->n, scanPack(c),
-                                                      c->dStatus);
-  std::swap(c->cur, c->alt);
-}
+// what the scan of the current state reads
+inline ScanPack scanPack(const ladds_gpu_ctx *c) { return ScanPack{c->posf, c->velf, c->cur, c->perm}; }
 
 // binary32 pre-filter radius of a cutoff: cutoff * (1 + nearRel), rounded up
 inline float prefilterRadius(double cutoff, double nearRel) {
@@ -637,8 +676,6 @@ void enqueueScanWith(ladds_gpu_ctx *c, cudaStream_t s, const ScanConsts &scIn, f
   const DenseBin dense = denseBin(c);
   {
     PhaseScope ps(c, kPhCandidates, s, dense.cells ? 2 : 1);
-    // the two list lengths and the dense bin's next-entry counter
-    cudaMemsetAsync(c->dCandCount, 0, 3 * sizeof(unsigned long long), s);
     const CandSink out{sc,       c->posf,     c->velf,      c->dCand, c->dCandCount, (unsigned long long)c->candCap,
                        c->haloStart, c->anyParent ? c->grp : nullptr};
     const bool buffer = c->cfg.scanScreen == LADDS_SCREEN_BUFFER;
@@ -651,7 +688,7 @@ void enqueueScanWith(ladds_gpu_ctx *c, cudaStream_t s, const ScanConsts &scIn, f
     if (form == LADDS_WALK_ROWS) {
       (buffer ? k_pair_rows<LADDS_SCREEN_BUFFER> : k_pair_rows<LADDS_SCREEN_LISTS>)<<<blocksFor(c->n, kScanCta),
                                                                                        kScanCta, 0, s>>>(
-          c->cur.tag, c->posf, (int)c->n, c->sortedKeys, c->rowStart, c->cellOff, c->grid, cutF, reach * reach,
+          c->perm, c->posf, (int)c->n, c->sortedKeys, c->rowStart, c->cellOff, c->grid, cutF, reach * reach,
           denseMin, c->denseCount, out);
     } else {
       HalfShellRows rows;
@@ -661,14 +698,14 @@ void enqueueScanWith(ladds_gpu_ctx *c, cudaStream_t s, const ScanConsts &scIn, f
                                : k_pair_candidates<LADDS_SCREEN_BUFFER, false>)
                          : (r1 ? k_pair_candidates<LADDS_SCREEN_LISTS, true>
                                : k_pair_candidates<LADDS_SCREEN_LISTS, false>);
-      walk<<<blocksFor(c->n, kScanCta), kScanCta, 0, s>>>(c->cur.tag, c->posf, (int)c->n, c->sortedKeys,
+      walk<<<blocksFor(c->n, kScanCta), kScanCta, 0, s>>>(c->perm, c->posf, (int)c->n, c->sortedKeys,
                                                           c->rowStart, c->cellOff, c->grid, cutF, reach * reach,
                                                           denseMin, c->denseCount, rows, out);
     }
     if (dense.cells)  // the dense bin: grid-stride over the listed cells (count read on the device)
       (buffer ? k_pair_tiles<LADDS_SCREEN_BUFFER>
               : k_pair_tiles<LADDS_SCREEN_LISTS>)<<<4 * c->evalBlocks, kScanCta, 0, s>>>(
-          dense.cells, dense.chunk, dense.count, dense.cap, c->cur.tag, c->posf, c->sortedKeys, c->rowStart,
+          dense.cells, dense.chunk, dense.count, dense.cap, c->perm, c->posf, c->sortedKeys, c->rowStart,
           c->cellOff, c->grid, cutF, reach * reach, out);
   }
   PhaseScope ps(c, kPhEvaluate, s);
@@ -680,56 +717,77 @@ void enqueueScanWith(ladds_gpu_ctx *c, cudaStream_t s, const ScanConsts &scIn, f
                                      (unsigned long long)c->pairCap);
 }
 
-// one iteration; its stage ephemerides are entries 3*slot.. of the chunk table in c_eph
-// `len` iterations starting at iteration itStart (len <= kMaxEphSteps): one
-// ephemeris kernel + one constant-memory copy for the whole chunk.  The pair
-// scan of iteration i (candidates + evaluation) runs on the second stream,
-// concurrently with the propagation and the sort of the next scanned
-// iteration: the scan reads the packed cell-order copies, the pre-gather state,
-// the tags and one set of sort results; the propagation writes none of them and
-// the sort writes the other set.  The next gather, which overwrites the packed
-// copies and the pre-gather state, waits for the scan.  Records carry the
-// chunk's first iteration (stored by the ephemeris kernel) + i.
-void enqueueChunk(ladds_gpu_ctx *c, int64_t itStart, int len, int k) {
-  enqueueEphemeris(c, len);
-  const bool overlap = !c->profiling;
-  bool pending = false;  // a scan on the second stream that the main stream has not joined
-  for (int i = 0; i < len; ++i) {
-    const bool scan = ((itStart + i) % k) == 0 && c->n;
-    enqueuePropagate(c, 1, scan, 3 * i);
-    if (!scan) continue;
-    enqueueSort(c);
-    if (pending) {
-      cudaStreamWaitEvent(c->st, c->evScan, 0);
-      pending = false;
-    }
-    enqueueCells(c);
-    ScanConsts sc = c->sc;
-    sc.dt = c->cfg.deltaT * (double)k;
-    if (overlap) {
-      cudaEventRecord(c->evCells, c->st);
-      cudaStreamWaitEvent(c->st2, c->evCells, 0);
-      enqueueScanWith(c, c->st2, sc, c->cutF, c->dIterBase, i);
-      cudaEventRecord(c->evScan, c->st2);
-      pending = true;
-    } else {
-      enqueueScanWith(c, c->st, sc, c->cutF, c->dIterBase, i);
-    }
-  }
-  if (pending) cudaStreamWaitEvent(c->st, c->evScan, 0);
+// Iterations of a chunk that one propagation launch covers: from iteration i
+// to the next one that is followed by a scan (or to the chunk's end).
+struct StepGroup {
+  int len;
+  bool scan;
+};
+StepGroup nextGroup(int64_t itStart, int i, int len, int k) {
+  int j = i;
+  while (j < len && (itStart + j) % k != 0) ++j;
+  return j < len ? StepGroup{j - i + 1, true} : StepGroup{len - i, false};
 }
 
-// host-side effect of replaying a captured chunk: the buffer swaps of its scans
-void replaySwaps(ladds_gpu_ctx *c, int64_t itStart, int len, int k) {
+// `len` iterations starting at iteration itStart (len <= kMaxEphSteps): one
+// ephemeris kernel + one constant-memory copy for the whole chunk, and one
+// propagation launch per scan (the state stays in registers over the steps
+// since the scan before).  Three streams hand the scanned iterations on:
+// propagation (st), sort (st3), pair scan (st2), so that the scan of an
+// iteration runs beside the sort of the next and the propagation of the one
+// after it.  The state goes round a ring of three buffers and the sort's input
+// and results alternate between two sets, hence, for the i-th scanned iteration:
+//   the propagation waits for sort i - 2 (its input set) and scan i - 3 (its
+//     state buffer),
+//   the sort for its propagation and scan i - 2 (its result set),
+//   the scan for its sort.
+// Records carry the chunk's first iteration (stored by the ephemeris kernel) + i.
+void enqueueChunk(ladds_gpu_ctx *c, int64_t itStart, int len, int k) {
+  enqueueEphemeris(c, len);
+  if (!c->n) return;
+  const bool overlap = !c->profiling;
+  const cudaStream_t sSort = overlap ? c->st3 : c->st, sScan = overlap ? c->st2 : c->st;
   int scans = 0;
-  for (int i = 0; i < len; ++i) scans += ((itStart + i) % k) == 0;
-  if (!scans || !c->n) return;
-  if (scans % 2 == 1) {
-    std::swap(c->cur, c->alt);
-    swapSortSets(c);
+  for (int i = 0; i < len;) {
+    const StepGroup g = nextGroup(itStart, i, len, k);
+    if (overlap && scans >= 2) cudaStreamWaitEvent(c->st, c->evSort[scans % 2], 0);
+    if (overlap && scans >= 3) cudaStreamWaitEvent(c->st, c->evScan[scans % 3], 0);
+    if (g.scan) swapSortSets(c);
+    enqueuePropagateStaged(c, g.len, 3 * i, g.scan);
+    i += g.len;
+    if (!g.scan) break;
+    if (overlap) {
+      cudaEventRecord(c->evProp, c->st);
+      cudaStreamWaitEvent(sSort, c->evProp, 0);
+      if (scans >= 2) cudaStreamWaitEvent(sSort, c->evScan[(scans - 2) % 3], 0);
+    }
+    enqueueSort(c, sSort);
+    if (overlap) {
+      cudaEventRecord(c->evSort[scans % 2], sSort);
+      cudaStreamWaitEvent(sScan, c->evSort[scans % 2], 0);
+    }
+    ScanConsts sc = c->sc;
+    sc.dt = c->cfg.deltaT * (double)k;
+    enqueueScanWith(c, sScan, sc, c->cutF, c->dIterBase, i - 1);
+    if (overlap) cudaEventRecord(c->evScan[scans % 3], sScan);
+    ++scans;
   }
-  c->sortedKeys = c->keys1;
-  c->perm = c->vals1;
+  if (overlap && scans) cudaStreamWaitEvent(c->st, c->evScan[(scans - 1) % 3], 0);
+}
+
+// host-side effect of replaying a captured chunk: the buffer swaps of its
+// propagations and sorts
+void replaySwaps(ladds_gpu_ctx *c, int64_t itStart, int len, int k) {
+  if (!c->n) return;
+  int launches = 0, scans = 0;
+  for (int i = 0; i < len;) {
+    const StepGroup g = nextGroup(itStart, i, len, k);
+    i += g.len;
+    ++launches;
+    scans += g.scan;
+  }
+  for (int r = launches % 3; r > 0; --r) rotateStates(c);
+  if (scans % 2 == 1) swapSortSets(c);
 }
 
 int syncAndStatus(ladds_gpu_ctx *c) {
@@ -851,18 +909,27 @@ int buildGrid(ladds_gpu_ctx *c) {
 }
 
 void freeGridBuffers(ladds_gpu_ctx *c) {
-  void *ptrs[] = {c->rowStart, c->rowStartB, c->rowCounts, c->longRows, c->cellOff, c->cellOffB};
+  void *ptrs[] = {c->rowStart, c->rowStartB, c->rowCounts, c->rowCountsB, c->longRows, c->cellOff, c->cellOffB};
   for (void *p : ptrs)
     if (p) cudaFree(p);
-  c->rowStart = c->rowStartB = c->rowCounts = c->longRows = nullptr;
+  c->rowStart = c->rowStartB = c->rowCounts = c->rowCountsB = c->longRows = nullptr;
   c->cellOff = c->cellOffB = nullptr;
+}
+
+// the row counts of both sets start at zero (every sort leaves them so)
+cudaError_t clearRowCounts(ladds_gpu_ctx *c) {
+  const size_t bytes = ((size_t)c->nRows + 1) * sizeof(uint32_t);
+  const cudaError_t e = cudaMemsetAsync(c->rowCounts, 0, bytes, c->st);
+  return e == cudaSuccess ? cudaMemsetAsync(c->rowCountsB, 0, bytes, c->st) : e;
 }
 
 // row tables of c->grid; the two cell-offset tables when each fits 512 MiB (250^3 cells: 31 MB)
 int allocGridBuffers(ladds_gpu_ctx *c) {
   if (cudaMalloc(&c->rowStart, ((size_t)c->nRows + 1) * sizeof(uint32_t)) != cudaSuccess ||
       cudaMalloc(&c->rowStartB, ((size_t)c->nRows + 1) * sizeof(uint32_t)) != cudaSuccess ||
-      cudaMalloc(&c->rowCounts, 2 * ((size_t)c->nRows + 1) * sizeof(uint32_t)) != cudaSuccess ||
+      cudaMalloc(&c->rowCounts, ((size_t)c->nRows + 1) * sizeof(uint32_t)) != cudaSuccess ||
+      cudaMalloc(&c->rowCountsB, ((size_t)c->nRows + 1) * sizeof(uint32_t)) != cudaSuccess ||
+      clearRowCounts(c) != cudaSuccess ||
       cudaMalloc(&c->longRows, ((size_t)c->nRows + 1) * sizeof(uint32_t)) != cudaSuccess) {
     cudaGetLastError();
     freeGridBuffers(c);
@@ -1012,6 +1079,7 @@ int ladds_gpu_create(const ladds_gpu_config *f, ladds_gpu_ctx **out) {
       cudaMalloc(&c->denseCountB, sizeof(uint32_t)) != cudaSuccess ||
       cudaMalloc(&c->dCount, 3 * sizeof(unsigned long long)) != cudaSuccess ||
       cudaMalloc(&c->dCandCount, 3 * sizeof(unsigned long long)) != cudaSuccess ||
+      cudaMalloc(&c->dCandCountB, 3 * sizeof(unsigned long long)) != cudaSuccess ||
       cudaMalloc(&c->dEph, 3 * kMaxEphSteps * sizeof(EphEntry)) != cudaSuccess ||
       cudaMalloc(&c->dIter, 2 * sizeof(int64_t)) != cudaSuccess ||
       cudaStreamCreateWithFlags(&c->st2, cudaStreamNonBlocking) != cudaSuccess ||
@@ -1028,11 +1096,10 @@ int ladds_gpu_create(const ladds_gpu_config *f, ladds_gpu_ctx **out) {
   cudaMemset(c->dIter, 0, 2 * sizeof(int64_t));
   cudaEventCreate(&c->callStart);
   cudaEventCreate(&c->callEnd);
-  cudaEventCreateWithFlags(&c->evCells, cudaEventDisableTiming);
-  cudaEventCreateWithFlags(&c->evScan, cudaEventDisableTiming);
-  for (auto &e : c->evXfer) cudaEventCreateWithFlags(&e, cudaEventDisableTiming);
+  cudaEventCreateWithFlags(&c->evProp, cudaEventDisableTiming);
+  for (auto &e : c->evSort) cudaEventCreateWithFlags(&e, cudaEventDisableTiming);
+  for (auto &e : c->evScan) cudaEventCreateWithFlags(&e, cudaEventDisableTiming);
   for (auto &e : c->evPipe) cudaEventCreateWithFlags(&e, cudaEventDisableTiming);
-  cudaMemset(c->dCandCount, 0, 3 * sizeof(unsigned long long));
   cudaMemset(c->dCandNeed, 0, sizeof(unsigned long long));
   c->evalBlocks = 4 * std::max(prop.multiProcessorCount, 1);
   // The reach-1 list walk runs beside the propagation and the sort of the next
@@ -1067,7 +1134,7 @@ int ladds_gpu_destroy(ladds_gpu_ctx *c) {
   freeGridBuffers(c);
   void *ptrs[] = {c->longCount, c->denseCount, c->denseCells, c->denseCountB, c->denseCellsB, c->dCount,
                   c->denseChunk, c->denseChunkB, c->dEph,
-                  c->dIter, c->dPairs, c->dCand, c->dCandCount, c->dObj,
+                  c->dIter, c->dPairs, c->dCand, c->dCandCount, c->dCandCountB, c->dObj,
                   c->adj.st, c->adj.bc, c->adj.aom, c->adj.miss, c->adj.grad, c->adj.ckpt, c->adj.rec,
                   c->adj.off, c->adj.arg, c->adj.eph};
   for (void *p : ptrs)
@@ -1079,9 +1146,10 @@ int ladds_gpu_destroy(ladds_gpu_ctx *c) {
   for (auto e : c->eventPool) cudaEventDestroy(e);
   if (c->callStart) cudaEventDestroy(c->callStart);
   if (c->callEnd) cudaEventDestroy(c->callEnd);
-  if (c->evCells) cudaEventDestroy(c->evCells);
-  if (c->evScan) cudaEventDestroy(c->evScan);
-  for (auto e : c->evXfer)
+  if (c->evProp) cudaEventDestroy(c->evProp);
+  for (auto e : c->evSort)
+    if (e) cudaEventDestroy(e);
+  for (auto e : c->evScan)
     if (e) cudaEventDestroy(e);
   for (auto e : c->evPipe)
     if (e) cudaEventDestroy(e);
@@ -1106,6 +1174,7 @@ int ladds_gpu_upload(ladds_gpu_ctx *c, size_t n, const double *x, const double *
   rc = ensureCapacity(c, n);
   if (rc) return rc;
   c->n = 0;
+  c->orderN = 0;
   c->anyParent = false;
   rc = writeArrays(c, 0, n, x, y, z, vx, vy, vz, radius, aom, bcInv, id, parentId, activity);
   if (rc) return rc;
@@ -1218,43 +1287,27 @@ int ladds_gpu_checked_insert(ladds_gpu_ctx *c, size_t n, const double *x, const 
 int ladds_gpu_get_objects(ladds_gpu_ctx *c, const uint32_t *slots, size_t m, ladds_state_record *out) {
   if (!c || (m && (!slots || !out))) return fail(c, LADDS_ERR_INVALID_ARG, "get_objects: bad argument");
   if (!m) return LADDS_OK;
-  std::vector<uint32_t> want(slots, slots + m);
-  std::sort(want.begin(), want.end());
-  want.erase(std::unique(want.begin(), want.end()), want.end());
-  const int mu = (int)want.size();
   std::lock_guard<std::mutex> lk(g_deviceMutex[c->dev & 63]);
+  for (size_t q = 0; q < m; ++q)
+    if (slots[q] >= c->n) return fail(c, LADDS_ERR_INVALID_ARG, "get_objects: no object with slot " + std::to_string(slots[q]));
   CK(cudaSetDevice(c->dev));
   uint32_t *dWant = nullptr;
-  int32_t *dPos = nullptr;
   ladds_state_record *dRec = nullptr;
-  if (cudaMalloc(&dWant, mu * sizeof(uint32_t)) != cudaSuccess || cudaMalloc(&dPos, mu * sizeof(int32_t)) != cudaSuccess ||
-      cudaMalloc(&dRec, mu * sizeof(ladds_state_record)) != cudaSuccess) {
+  if (cudaMalloc(&dWant, m * sizeof(uint32_t)) != cudaSuccess ||
+      cudaMalloc(&dRec, m * sizeof(ladds_state_record)) != cudaSuccess) {
     cudaGetLastError();
     cudaFree(dWant);
-    cudaFree(dPos);
     return fail(c, LADDS_ERR_ALLOC, "get_objects: staging allocation failed");
   }
-  std::vector<int32_t> pos(mu, -1);
-  std::vector<ladds_state_record> rec(mu);
-  cudaError_t e = cudaMemcpyAsync(dWant, want.data(), mu * sizeof(uint32_t), cudaMemcpyHostToDevice, c->st);
-  if (e == cudaSuccess) e = cudaMemsetAsync(dPos, 0xff, mu * sizeof(int32_t), c->st);
-  if (e == cudaSuccess && c->n)
-    k_find_slots<<<blocksFor(c->n, 256), 256, 0, c->st>>>(c->cur.tag, (int)c->n, dWant, mu, dPos);
-  if (e == cudaSuccess) k_gather_records<<<blocksFor((size_t)mu, 128), 128, 0, c->st>>>(c->cur, dPos, mu, dRec);
+  cudaError_t e = cudaMemcpyAsync(dWant, slots, m * sizeof(uint32_t), cudaMemcpyHostToDevice, c->st);
+  if (e == cudaSuccess) k_gather_records<<<blocksFor(m, 128), 128, 0, c->st>>>(c->cur, dWant, (int)m, dRec);
   if (e == cudaSuccess) e = cudaGetLastError();
-  if (e == cudaSuccess) e = cudaMemcpyAsync(pos.data(), dPos, mu * sizeof(int32_t), cudaMemcpyDeviceToHost, c->st);
   if (e == cudaSuccess)
-    e = cudaMemcpyAsync(rec.data(), dRec, mu * sizeof(ladds_state_record), cudaMemcpyDeviceToHost, c->st);
+    e = cudaMemcpyAsync(out, dRec, m * sizeof(ladds_state_record), cudaMemcpyDeviceToHost, c->st);
   if (e == cudaSuccess) e = cudaStreamSynchronize(c->st);
   cudaFree(dWant);
-  cudaFree(dPos);
   cudaFree(dRec);
   if (e != cudaSuccess) return fail(c, LADDS_ERR_CUDA, std::string("get_objects: ") + cudaGetErrorString(e));
-  for (size_t q = 0; q < m; ++q) {
-    const size_t k = std::lower_bound(want.begin(), want.end(), slots[q]) - want.begin();
-    if (pos[k] < 0) return fail(c, LADDS_ERR_INVALID_ARG, "get_objects: no object with slot " + std::to_string(slots[q]));
-    out[q] = rec[k];
-  }
   return LADDS_OK;
 }
 
@@ -1267,26 +1320,20 @@ int ladds_gpu_download(ladds_gpu_ctx *c, size_t cap, size_t *nOut, double *x, do
   if (cap < c->n) return fail(c, LADDS_ERR_CAPACITY, "download buffer smaller than the population");
   if (!c->n) return LADDS_OK;
   CK(cudaSetDevice(c->dev));
-  const int g = blocksFor(c->n, 256);
-  const double *src[] = {c->cur.x, c->cur.y, c->cur.z, c->cur.vx, c->cur.vy, c->cur.vz, c->cur.aom, c->cur.bc};
-  double *dst[] = {x, y, z, vx, vy, vz, aom, bcInv};
-  for (int k = 0; k < 8; ++k) {
-    if (!dst[k]) continue;
-    k_unpermute_f64<<<g, 256, 0, c->st>>>(src[k], c->cur.tag, (int)c->n, c->alt.x);
-    CK(cudaMemcpyAsync(dst[k], c->alt.x, c->n * sizeof(double), cudaMemcpyDeviceToHost, c->st));
-    CK(cudaStreamSynchronize(c->st));
-  }
-  // radius, id and parent are slot-indexed already
-  if (radius) CK(cudaMemcpyAsync(radius, c->cur.radius, c->n * sizeof(double), cudaMemcpyDeviceToHost, c->st));
+  const double *src[] = {c->cur.x,  c->cur.y,   c->cur.z,  c->cur.vx,    c->cur.vy,
+                         c->cur.vz, c->cur.aom, c->cur.bc, c->cur.radius};
+  double *dst[] = {x, y, z, vx, vy, vz, aom, bcInv, radius};
+  for (int k = 0; k < 9; ++k)
+    if (dst[k]) CK(cudaMemcpyAsync(dst[k], src[k], c->n * sizeof(double), cudaMemcpyDeviceToHost, c->st));
   if (id) CK(cudaMemcpyAsync(id, c->cur.id, c->n * sizeof(uint64_t), cudaMemcpyDeviceToHost, c->st));
   if (parentId)
     CK(cudaMemcpyAsync(parentId, c->cur.parent, c->n * sizeof(uint64_t), cudaMemcpyDeviceToHost, c->st));
-  CK(cudaStreamSynchronize(c->st));
   if (activity) {
-    k_unpermute_act<<<g, 256, 0, c->st>>>(c->cur.tag, (int)c->n, (int8_t *)c->alt.tag);
-    CK(cudaMemcpyAsync(activity, c->alt.tag, c->n, cudaMemcpyDeviceToHost, c->st));
-    CK(cudaStreamSynchronize(c->st));
+    int8_t *act = reinterpret_cast<int8_t *>(c->scratchA);
+    k_activity<<<blocksFor(c->n, 256), 256, 0, c->st>>>(c->cur.tag, (int)c->n, act);
+    CK(cudaMemcpyAsync(activity, act, c->n, cudaMemcpyDeviceToHost, c->st));
   }
+  CK(cudaStreamSynchronize(c->st));
   CK(cudaGetLastError());
   return LADDS_OK;
 }
@@ -1302,8 +1349,6 @@ int ladds_gpu_set_state(ladds_gpu_ctx *c, size_t n, const double *x, const doubl
   if (!n) return LADDS_OK;
   CK(cudaSetDevice(c->dev));
   double *dst[] = {c->cur.x, c->cur.y, c->cur.z, c->cur.vx, c->cur.vy, c->cur.vz};
-  double *stage[] = {c->alt.x, c->alt.y, c->alt.z, c->alt.vx, c->alt.vy, c->alt.vz};
-  const int g = blocksFor(n, 256);
   // pageable arrays go through the context's pinned staging, copied on all host
   // threads while the previous array crosses PCIe
   bool pinned[6], staged = false;
@@ -1313,8 +1358,6 @@ int ladds_gpu_set_state(ladds_gpu_ctx *c, size_t n, const double *x, const doubl
   }
   if (staged && !ensurePinStage(c, n))
     for (bool &p : pinned) p = true;  // no pinned memory to spare: the driver stages them
-  // the copies run back to back on the main stream; each array's gather into
-  // cell order runs on the second stream while the next array crosses PCIe
   for (int k = 0; k < 6; ++k) {
     const double *from = src[k];
     if (!pinned[k]) {
@@ -1322,12 +1365,9 @@ int ladds_gpu_set_state(ladds_gpu_ctx *c, size_t n, const double *x, const doubl
       hostCopyOne(pin, src[k], n);
       from = pin;
     }
-    CK(cudaMemcpyAsync(stage[k], from, n * sizeof(double), cudaMemcpyHostToDevice, c->st));
-    CK(cudaEventRecord(c->evXfer[k], c->st));
-    CK(cudaStreamWaitEvent(c->st2, c->evXfer[k], 0));
-    k_permute_from_slots_f64<<<g, 256, 0, c->st2>>>(stage[k], c->cur.tag, (int)n, dst[k]);
+    CK(cudaMemcpyAsync(dst[k], from, n * sizeof(double), cudaMemcpyHostToDevice, c->st));
   }
-  CK(cudaStreamSynchronize(c->st2));
+  CK(cudaStreamSynchronize(c->st));
   CK(cudaGetLastError());
   return LADDS_OK;
 }
@@ -1340,19 +1380,7 @@ int ladds_gpu_get_state(ladds_gpu_ctx *c, size_t n, double *x, double *y, double
   if (!c->n) return LADDS_OK;
   CK(cudaSetDevice(c->dev));
   const double *src[] = {c->cur.x, c->cur.y, c->cur.z, c->cur.vx, c->cur.vy, c->cur.vz};
-  double *stage[] = {c->alt.x, c->alt.y, c->alt.z, c->alt.vx, c->alt.vy, c->alt.vz};
   double *dst[] = {x, y, z, vx, vy, vz};
-  const int g = blocksFor(c->n, 256);
-  // scatters into slot order on the second stream, all launched before the
-  // first copy (a copy into pageable memory blocks the host); each array's
-  // copy waits for its own scatter only
-  CK(cudaEventRecord(c->evXfer[6], c->st));
-  CK(cudaStreamWaitEvent(c->st2, c->evXfer[6], 0));
-  for (int k = 0; k < 6; ++k) {
-    if (!dst[k]) continue;
-    k_unpermute_f64<<<g, 256, 0, c->st2>>>(src[k], c->cur.tag, (int)c->n, stage[k]);
-    CK(cudaEventRecord(c->evXfer[k], c->st2));
-  }
   // pageable arrays come back through the context's pinned staging: each
   // array leaves the pinned buffer on all host threads while the next crosses PCIe
   bool pinned[6], staged = false;
@@ -1364,9 +1392,8 @@ int ladds_gpu_get_state(ladds_gpu_ctx *c, size_t n, double *x, double *y, double
     for (bool &p : pinned) p = true;  // no pinned memory to spare: the driver stages them
   for (int k = 0; k < 6; ++k) {
     if (!dst[k]) continue;
-    CK(cudaStreamWaitEvent(c->st, c->evXfer[k], 0));
     double *to = pinned[k] ? dst[k] : c->pinStage + (size_t)(6 + k) * c->pinCap;
-    CK(cudaMemcpyAsync(to, stage[k], c->n * sizeof(double), cudaMemcpyDeviceToHost, c->st));
+    CK(cudaMemcpyAsync(to, src[k], c->n * sizeof(double), cudaMemcpyDeviceToHost, c->st));
     CK(cudaEventRecord(c->evPipe[k], c->st));
   }
   for (int k = 0; k < 6; ++k) {
@@ -1423,7 +1450,7 @@ int ladds_gpu_integrate(ladds_gpu_ctx *c, int steps) {
   while (left > 0) {
     const int chunk = std::min(left, c->chunkSteps);
     CK(enqueueEphemeris(c, chunk));
-    enqueuePropagate(c, chunk, false, 0);
+    enqueuePropagate(c, chunk, 0);
     left -= chunk;
   }
   const int rc = syncAndStatus(c);
@@ -1436,33 +1463,54 @@ int ladds_gpu_integrate(ladds_gpu_ctx *c, int steps) {
 }  // extern "C"
 
 namespace {
-// Compaction of the objects flagged keep[j] = 1 in scratchA (current order;
-// scratchC holds the same flags in slot order): survivors keep their
-// relative slot order and are renumbered 0..n'-1.  The slot-indexed arrays
-// are compacted through the roll-back buffer's positions and velocities,
-// which hold nothing between calls.
+// The order of the last scan without the objects that a removal takes out
+// (keep[slot] = 0 among n slots; pos = their new slots).  Waits for the stream.
+int compactOrder(ladds_gpu_ctx *c, const uint32_t *keep, const uint32_t *pos, size_t n) {
+  const int m = (int)std::min(c->orderN, n);
+  c->orderN = 0;
+  if (m) {
+    uint32_t *flag = c->keys, *at = c->scratchC, *moved = c->permB;  // free between calls
+    k_order_flags<<<blocksFor(m, 256), 256, 0, c->st>>>(c->perm, keep, m, flag);
+    enqueueExclusiveScan(c, flag, (size_t)m, at, c->st);
+    k_order_compact<<<blocksFor(m, 256), 256, 0, c->st>>>(c->perm, flag, at, pos, m, moved);
+    uint32_t last[2] = {0, 0};
+    CK(cudaMemcpyAsync(&last[0], at + (m - 1), sizeof(uint32_t), cudaMemcpyDeviceToHost, c->st));
+    CK(cudaMemcpyAsync(&last[1], flag + (m - 1), sizeof(uint32_t), cudaMemcpyDeviceToHost, c->st));
+    CK(cudaMemcpyAsync(c->perm, moved, (size_t)m * sizeof(uint32_t), cudaMemcpyDeviceToDevice, c->st));
+    CK(cudaStreamSynchronize(c->st));
+    c->orderN = (size_t)last[0] + last[1];
+  }
+  CK(cudaStreamSynchronize(c->st));
+  CK(cudaGetLastError());
+  return LADDS_OK;
+}
+
+// Compaction of the objects flagged keep[j] = 1 in scratchA: survivors keep
+// their relative slot order and are renumbered 0..n'-1.  The arrays that the
+// state buffers share are compacted through the roll-back buffer's, which
+// hold nothing between calls.
 int compactKept(ladds_gpu_ctx *c) {
   const int n = (int)c->n;
-  uint32_t *keep = c->scratchA, *pos = c->scratchB, *aliveBySlot = c->scratchC, *newSlot = c->keys1;
-  // exclusive scans: positions in the current order, new slot numbers in slot order
-  enqueueExclusiveScan(c, keep, (size_t)n, pos);
-  enqueueExclusiveScan(c, aliveBySlot, (size_t)n, newSlot);
+  uint32_t *keep = c->scratchA, *pos = c->scratchB;
+  enqueueExclusiveScan(c, keep, (size_t)n, pos, c->st);
   CK(cudaGetLastError());
-  double *tRadius = c->snap.x;
-  auto *tId = reinterpret_cast<uint64_t *>(c->snap.y), *tParent = reinterpret_cast<uint64_t *>(c->snap.z);
-  k_compact<<<blocksFor(n, 256), 256, 0, c->st>>>(c->cur, c->alt, keep, pos, newSlot, n, tRadius, tId, tParent);
+  DevState tmp{};
+  tmp.aom = c->snap.x;
+  tmp.bc = c->snap.y;
+  tmp.radius = c->snap.z;
+  tmp.id = reinterpret_cast<uint64_t *>(c->snap.vx);
+  tmp.parent = reinterpret_cast<uint64_t *>(c->snap.vy);
+  tmp.tag = reinterpret_cast<uint32_t *>(c->snap.vz);
+  k_compact<<<blocksFor(n, 256), 256, 0, c->st>>>(c->cur, c->alt, keep, pos, n, tmp);
   uint32_t kept = 0, lastKeep = 0;
   CK(cudaMemcpyAsync(&kept, pos + (n - 1), sizeof(uint32_t), cudaMemcpyDeviceToHost, c->st));
   CK(cudaMemcpyAsync(&lastKeep, keep + (n - 1), sizeof(uint32_t), cudaMemcpyDeviceToHost, c->st));
   CK(cudaStreamSynchronize(c->st));
   CK(cudaGetLastError());
   const size_t m = (size_t)kept + lastKeep;
-  if (m) {  // back into the shared slot-indexed arrays
-    CK(cudaMemcpyAsync(c->cur.radius, tRadius, m * sizeof(double), cudaMemcpyDeviceToDevice, c->st));
-    CK(cudaMemcpyAsync(c->cur.id, tId, m * sizeof(uint64_t), cudaMemcpyDeviceToDevice, c->st));
-    CK(cudaMemcpyAsync(c->cur.parent, tParent, m * sizeof(uint64_t), cudaMemcpyDeviceToDevice, c->st));
-    CK(cudaStreamSynchronize(c->st));
-  }
+  CK(copyShared(tmp, c->cur, m, c->st));
+  const int rc = compactOrder(c, keep, pos, (size_t)n);
+  if (rc) return rc;
   std::swap(c->cur, c->alt);
   c->n = m;
   c->orderValid = false;
@@ -1478,15 +1526,15 @@ int scanState(ladds_gpu_ctx *c, const ScanConsts &sc, float cutF, std::vector<la
   for (int attempt = 0; attempt < 5; ++attempt) {
     CK(cudaMemsetAsync(c->dCount, 0, sizeof(unsigned long long), c->st));
     CK(cudaMemsetAsync(c->dCandNeed, 0, sizeof(unsigned long long), c->st));
-    CK(cudaMemsetAsync(c->rowCounts, 0, ((size_t)c->nRows + 1) * sizeof(uint32_t), c->st));
-    k_cell_keys<<<blocksFor(c->n, 256), 256, 0, c->st>>>(c->cur.x, c->cur.y, c->cur.z, (int)c->n, c->grid,
-                                                          c->keys0, c->rowCounts, c->scratchC);
-    enqueueSort(c);
-    enqueueCells(c);
+    c->orderN = 0;
+    swapSortSets(c);
+    k_scan_input<<<blocksFor(c->n, 256), 256, 0, c->st>>>(c->cur, (int)c->n, c->grid, scanInput(c));
+    enqueueSort(c, c->st);
     enqueueScanWith(c, c->st, sc, cutF, c->dIter, -1);  // records carry the index of the last integrated iteration
     int rc = syncAndStatus(c);
     collectTimes(c);
     if (rc) return rc;
+    c->orderN = c->n;
     unsigned long long cnt = 0;
     bool overflow = false;
     rc = growIfOverflowed(c, &cnt, &overflow);
@@ -1565,27 +1613,20 @@ int ladds_gpu_step(ladds_gpu_ctx *c, int iterations, ladds_pair *out, size_t cap
   const int k = c->cfg.timestepsPerCollisionDetection;
   int scans = 0;
   for (int i = 0; i < iterations; ++i) scans += ((c->hostIter + i) % k) == 0;
-  // snapshot of the call's start state: the call is re-run after a device
-  // pair-buffer overflow and undone when the caller's buffer is too small.  A
-  // one-iteration call changes only the positions and velocities of the
-  // current buffer (its gather writes the other buffer), so they are all it
-  // keeps; undoing it restores them and the buffer roles.
-  const bool light = iterations == 1;
-  const DevState curStart = c->cur, altStart = c->alt;
-  if (light) {
-    CK(copyDynamic(c->cur, c->snap, c->n, c->st));
-  } else {
-    CK(copyState(c->cur, c->snap, c->n, c->st));
-  }
+  // the call's start state: the call is re-run after a device pair-buffer
+  // overflow and undone when the caller's buffer is too small.  A call of one
+  // propagation launch leaves it in its buffer; for longer ones it is copied,
+  // and comes back into the buffer that was current.
+  const DevState ringStart[3] = {c->cur, c->alt, c->alt2};
+  const bool oneLaunch = iterations > 0 && iterations <= c->chunkSteps &&
+                         nextGroup(c->hostIter, 0, iterations, k).len == iterations;
+  if (!oneLaunch) CK(copyDynamic(c->cur, c->snap, c->n, c->st));
   const int64_t startIter = c->hostIter;
   auto rollBack = [&]() -> int {
-    if (light) {
-      c->cur = curStart;
-      c->alt = altStart;
-      CK(copyDynamic(c->snap, c->cur, c->n, c->st));
-    } else {
-      CK(copyState(c->snap, c->cur, c->n, c->st));
-    }
+    c->cur = ringStart[0];
+    c->alt = ringStart[1];
+    c->alt2 = ringStart[2];
+    if (!oneLaunch) CK(copyDynamic(c->snap, c->cur, c->n, c->st));
     CK(cudaMemcpyAsync(c->dIter, &startIter, sizeof(int64_t), cudaMemcpyHostToDevice, c->st));
     CK(cudaStreamSynchronize(c->st));
     c->hostIter = startIter;
@@ -1595,6 +1636,7 @@ int ladds_gpu_step(ladds_gpu_ctx *c, int iterations, ladds_pair *out, size_t cap
   unsigned long long cnt = 0;
   int retries = 0;
   for (;;) {
+    if (scans) c->orderN = 0;
     CK(cudaMemsetAsync(c->dCount, 0, sizeof(unsigned long long), c->st));
     CK(cudaMemsetAsync(c->dCandNeed, 0, sizeof(unsigned long long), c->st));
     const bool graph = c->cfg.useGraphs && !c->profiling && iterations >= 1;
@@ -1603,12 +1645,11 @@ int ladds_gpu_step(ladds_gpu_ctx *c, int iterations, ladds_pair *out, size_t cap
       // pass 1: capture the graphs this call needs (capture performs the host-side
       // buffer swaps; they are undone afterwards), so that no capture happens
       // between the timing events
-      const DevState cur0 = c->cur, alt0 = c->alt;
-      uint32_t *const sk0 = c->sortedKeys, *const pm0 = c->perm;
+      const DevState ring0[3] = {c->cur, c->alt, c->alt2};
       const int par0 = c->sortParity;
       for (int done = 0; done < iterations;) {
         const int len = std::min(iterations - done, c->chunkSteps);
-        const int bufs = (c->cur.x == c->homeX ? 0 : 1) | 2 * c->sortParity;
+        const int bufs = bufferRoles(c);
         const auto key = std::make_tuple(len, (int)((it0 + done) % k), bufs, c->n, c->pairCap);
         if (c->graphs.find(key) == c->graphs.end()) {
           CK(cudaStreamBeginCapture(c->st, cudaStreamCaptureModeThreadLocal));
@@ -1625,16 +1666,15 @@ int ladds_gpu_step(ladds_gpu_ctx *c, int iterations, ladds_pair *out, size_t cap
         }
         done += len;
       }
-      c->cur = cur0;
-      c->alt = alt0;
+      c->cur = ring0[0];
+      c->alt = ring0[1];
+      c->alt2 = ring0[2];
       if (c->sortParity != par0) swapSortSets(c);
-      c->sortedKeys = sk0;
-      c->perm = pm0;
       // pass 2: replay
       CK(cudaEventRecord(c->callStart, c->st));
       for (int done = 0; done < iterations;) {
         const int len = std::min(iterations - done, c->chunkSteps);
-        const int bufs = (c->cur.x == c->homeX ? 0 : 1) | 2 * c->sortParity;
+        const int bufs = bufferRoles(c);
         const auto key = std::make_tuple(len, (int)((it0 + done) % k), bufs, c->n, c->pairCap);
         auto git = c->graphs.find(key);
         if (git == c->graphs.end()) return fail(c, LADDS_ERR_STATE, "graph cache inconsistent");
@@ -1654,6 +1694,7 @@ int ladds_gpu_step(ladds_gpu_ctx *c, int iterations, ladds_pair *out, size_t cap
     bool overflow = false;
     int rc = syncStatusAndGrow(c, &cnt, &overflow);
     collectTimes(c);
+    if (scans && rc != LADDS_ERR_CUDA && rc != LADDS_ERR_DEVICE_CHECK) c->orderN = c->n;
     if (rc) {
       const int rb = rollBack();
       return rb ? rb : rc;
@@ -1715,11 +1756,9 @@ int ladds_gpu_step_host(ladds_gpu_ctx *c, size_t n, const double *const in[6], d
   const int k = c->cfg.timestepsPerCollisionDetection;
   const bool scan = (c->hostIter % k) == 0 && n;
   const int64_t startIter = c->hostIter;
-  // the iteration's source buffer, in slot order: positions and velocities
-  // from the host, the per-object constants and tags scattered out of the
-  // current (cell-ordered) buffer
-  const DevState S = c->snap;
-  const int ni = (int)n;
+  // the host's positions and velocities go to the other buffer, are propagated
+  // there, and make it the current one
+  const DevState S = c->alt;
   // any failure once work is enqueued: nothing of this call may still run when
   // it returns -- its copies into the caller's arrays and its kernels are
   // drained on all three streams -- and the iteration is not counted (the device
@@ -1729,6 +1768,7 @@ int ladds_gpu_step_host(ladds_gpu_ctx *c, size_t n, const double *const in[6], d
     cudaStreamSynchronize(c->st3);
     cudaStreamSynchronize(c->st);
     cudaMemcpyAsync(c->dIter, &startIter, sizeof(int64_t), cudaMemcpyHostToDevice, c->st);
+    clearRowCounts(c);
     cudaStreamSynchronize(c->st);
     c->orderValid = false;
     return rc;
@@ -1741,14 +1781,11 @@ int ladds_gpu_step_host(ladds_gpu_ctx *c, size_t n, const double *const in[6], d
   } while (0)
   CKS(cudaMemsetAsync(c->dCount, 0, 2 * sizeof(unsigned long long), c->st));
   CKS(cudaEventRecord(c->callStart, c->st));
-  if (n) {
-    const int g = blocksFor(n, 256);
-    k_unpermute_f64<<<g, 256, 0, c->st>>>(c->cur.aom, c->cur.tag, ni, S.aom);
-    k_unpermute_f64<<<g, 256, 0, c->st>>>(c->cur.bc, c->cur.tag, ni, S.bc);
-    k_unpermute_tag<<<g, 256, 0, c->st>>>(c->cur.tag, ni, S.tag);
-  }
   CKS(enqueueEphemeris(c, 1));
-  if (scan) CKS(cudaMemsetAsync(c->rowCounts, 0, ((size_t)c->nRows + 1) * sizeof(uint32_t), c->st));
+  if (scan) {
+    c->orderN = 0;
+    swapSortSets(c);
+  }
   // pageable arrays go through pinned staging, copied on all host threads
   // chunk by chunk (the CUDA driver's own staging of pageable copies is slower)
   bool stageIn[6] = {}, stageOut[6] = {}, anyIn = false, anyOut = false;
@@ -1786,10 +1823,7 @@ int ladds_gpu_step_host(ladds_gpu_ctx *c, size_t n, const double *const in[6], d
       CKS(cudaMemcpyAsync(sArr[a] + lo, src[a] + lo, len * sizeof(double), cudaMemcpyHostToDevice, c->st2));
     CKS(cudaEventRecord(c->evPipe[ch], c->st2));
     CKS(cudaStreamWaitEvent(c->st, c->evPipe[ch], 0));
-    DevState Sc = S;
-    Sc.x += lo; Sc.y += lo; Sc.z += lo; Sc.vx += lo; Sc.vy += lo; Sc.vz += lo;
-    Sc.aom += lo; Sc.bc += lo; Sc.tag += lo;
-    launchPropagate(c, Sc, (int)len, 1, 0, scan, c->keys0 + lo, c->scratchC + lo);
+    launchPropagate(c, S, S, lo, (int)len, 1, 0, scan);
     CKS(cudaEventRecord(c->evPipe[kHostChunks + ch], c->st));
     CKS(cudaStreamWaitEvent(c->st3, c->evPipe[kHostChunks + ch], 0));
     for (int a = 0; a < 6; ++a)
@@ -1797,35 +1831,12 @@ int ladds_gpu_step_host(ladds_gpu_ctx *c, size_t n, const double *const in[6], d
     CKS(cudaEventRecord(c->evPipe[2 * kHostChunks + ch], c->st3));
     used = ch + 1;
   }
-  k_advance<<<1, 32, 0, c->st>>>(c->dIter, 1);
-  const DevState curStart = c->cur, altStart = c->alt;
-  // the buffer roles when the call returns (on every path): S is the roll-back
-  // buffer again and (cur, alt) the pair the captured graphs were made with;
-  // the scan reads S as alt until then
-  struct RoleGuard {
-    ladds_gpu_ctx *c;
-    DevState alt;
-    bool on;
-    ~RoleGuard() {
-      if (on) c->alt = alt;
-    }
-  } roles{c, curStart, scan};
   ScanConsts sc = c->sc;
   sc.dt = c->cfg.deltaT * (double)k;
+  if (n) rotateStates(c);
   if (scan) {
-    // sort and gather from the slot-ordered buffer into the other buffer of the
-    // pair, which becomes the current one (as after a scan of ladds_gpu_step)
-    c->cur = S;
-    c->alt = curStart;
-    enqueueSort(c);
-    c->alt = altStart;
-    enqueueCells(c);  // gathers S into altStart, then cur = altStart, alt = S (the scan reads alt)
+    enqueueSort(c, c->st);
     enqueueScanWith(c, c->st, sc, c->cutF, c->dIterBase, 0);
-  } else if (n) {
-    // no scan: the new positions and velocities into the current buffer's order
-    const int g = blocksFor(n, 256);
-    double *const dst[6] = {c->cur.x, c->cur.y, c->cur.z, c->cur.vx, c->cur.vy, c->cur.vz};
-    for (int a = 0; a < 6; ++a) k_permute_from_slots_f64<<<g, 256, 0, c->st>>>(sArr[a], c->cur.tag, ni, dst[a]);
   }
   if (used) {
     CKS(cudaEventRecord(c->evPipe[3 * kHostChunks], c->st3));
@@ -1847,6 +1858,7 @@ int ladds_gpu_step_host(ladds_gpu_ctx *c, size_t n, const double *const in[6], d
   while (overflow) {  // the device buffers have grown: the scan alone runs again on the same state
     if (++retries > 4) return abortCall(fail(c, LADDS_ERR_STATE, "device scan buffers kept overflowing"));
     CKS(cudaMemsetAsync(c->dCount, 0, 2 * sizeof(unsigned long long), c->st));
+    CKS(cudaMemsetAsync(c->dCandCount, 0, 3 * sizeof(unsigned long long), c->st));  // the sort cleared them for one scan
     enqueueScanWith(c, c->st, sc, c->cutF, c->dIterBase, 0);
     rc = syncStatusAndGrow(c, &cnt, &overflow);
     collectTimes(c);
@@ -1859,7 +1871,10 @@ int ladds_gpu_step_host(ladds_gpu_ctx *c, size_t n, const double *const in[6], d
   if (cnt) CKS(cudaMemcpy(recs.data(), c->dPairs, cnt * sizeof(ladds_pair), cudaMemcpyDeviceToHost));
   std::sort(recs.begin(), recs.end(), pairLess);
   c->hostIter += 1;
-  if (scan) c->orderValid = true;
+  if (scan) {
+    c->orderValid = true;
+    c->orderN = n;
+  }
   if (stats) {
     stats->iterations = 1;
     stats->scans = scan ? 1 : 0;
@@ -1902,11 +1917,7 @@ int ladds_gpu_cell_order(ladds_gpu_ctx *c, size_t cap, size_t *n, uint32_t *keys
   if (!c->n) return LADDS_OK;
   CK(cudaSetDevice(c->dev));
   if (keys) CK(cudaMemcpy(keys, c->sortedKeys, c->n * sizeof(uint32_t), cudaMemcpyDeviceToHost));
-  if (slots) {
-    std::vector<uint32_t> tags(c->n);
-    CK(cudaMemcpy(tags.data(), c->cur.tag, c->n * sizeof(uint32_t), cudaMemcpyDeviceToHost));
-    for (size_t i = 0; i < c->n; ++i) slots[i] = tagSlot(tags[i]);
-  }
+  if (slots) CK(cudaMemcpy(slots, c->perm, c->n * sizeof(uint32_t), cudaMemcpyDeviceToHost));
   return LADDS_OK;
 }
 
@@ -1956,17 +1967,17 @@ int removedIdsInSlotOrder(ladds_gpu_ctx *c, uint64_t *removedIds, size_t cap) {
   const int n = (int)c->n;
   unsigned *dCnt = reinterpret_cast<unsigned *>(c->dCandNeed) + 1;  // word 0 holds the removal count
   CK(cudaMemsetAsync(dCnt, 0, sizeof(unsigned), c->st));
-  // keys0 / vals0 / scratchB are free between calls (scratchB is compactKept's output, written later)
-  k_removed_ids<<<blocksFor(n, 256), 256, 0, c->st>>>(c->scratchA, c->cur.tag, c->cur.id, n, c->keys0, c->vals0,
-                                                       c->scratchB, dCnt);
+  // keys / scratchB / scratchC are free between calls (scratchB is compactKept's output, written later)
+  k_removed_ids<<<blocksFor(n, 256), 256, 0, c->st>>>(c->scratchA, c->cur.id, n, c->keys, c->scratchC, c->scratchB,
+                                                       dCnt);
   CK(cudaGetLastError());
   unsigned m = 0;
   CK(cudaMemcpyAsync(&m, dCnt, sizeof(unsigned), cudaMemcpyDeviceToHost, c->st));
   CK(cudaStreamSynchronize(c->st));
   std::vector<uint32_t> sl(m), lo(m), hi(m);
   if (m) {
-    CK(cudaMemcpyAsync(sl.data(), c->keys0, m * sizeof(uint32_t), cudaMemcpyDeviceToHost, c->st));
-    CK(cudaMemcpyAsync(lo.data(), c->vals0, m * sizeof(uint32_t), cudaMemcpyDeviceToHost, c->st));
+    CK(cudaMemcpyAsync(sl.data(), c->keys, m * sizeof(uint32_t), cudaMemcpyDeviceToHost, c->st));
+    CK(cudaMemcpyAsync(lo.data(), c->scratchC, m * sizeof(uint32_t), cudaMemcpyDeviceToHost, c->st));
     CK(cudaMemcpyAsync(hi.data(), c->scratchB, m * sizeof(uint32_t), cudaMemcpyDeviceToHost, c->st));
     CK(cudaStreamSynchronize(c->st));
   }
@@ -1993,8 +2004,8 @@ int ladds_gpu_remove_below(ladds_gpu_ctx *c, double minAltitude, size_t *nRemove
   const double critSq = crit * crit;           // Simulation.cpp:581
   unsigned *dBurnt = reinterpret_cast<unsigned *>(c->dCandNeed);  // scratch word (reset by every scan)
   CK(cudaMemsetAsync(dBurnt, 0, sizeof(unsigned), c->st));
-  k_burnup_flags<<<blocksFor(n, 256), 256, 0, c->st>>>(c->cur.x, c->cur.y, c->cur.z, c->cur.tag, n, critSq,
-                                                        c->scratchA, c->scratchC, dBurnt);
+  k_burnup_flags<<<blocksFor(n, 256), 256, 0, c->st>>>(c->cur.x, c->cur.y, c->cur.z, n, critSq, c->scratchA,
+                                                        dBurnt);
   unsigned burnt = 0;
   CK(cudaMemcpyAsync(&burnt, dBurnt, sizeof(unsigned), cudaMemcpyDeviceToHost, c->st));
   CK(cudaStreamSynchronize(c->st));
@@ -2021,7 +2032,7 @@ int ladds_gpu_remove_escaping(ladds_gpu_ctx *c, size_t *nRemoved, uint64_t *remo
   const double3 hi = make_double3(c->cfg.boxMax[0], c->cfg.boxMax[1], c->cfg.boxMax[2]);
   unsigned *dOut = reinterpret_cast<unsigned *>(c->dCandNeed);  // scratch word (reset by every scan)
   CK(cudaMemsetAsync(dOut, 0, sizeof(unsigned), c->st));
-  k_escape_flags<<<blocksFor(n, 256), 256, 0, c->st>>>(c->cur, n, lo, hi, c->scratchA, c->scratchC, dOut);
+  k_escape_flags<<<blocksFor(n, 256), 256, 0, c->st>>>(c->cur, n, lo, hi, c->scratchA, dOut);
   unsigned escaped = 0;
   CK(cudaMemcpyAsync(&escaped, dOut, sizeof(unsigned), cudaMemcpyDeviceToHost, c->st));
   CK(cudaStreamSynchronize(c->st));
@@ -2054,13 +2065,13 @@ int ladds_gpu_pack_layers(ladds_gpu_ctx *c, int32_t izLo, int32_t izHi, int remo
     }
   }
   const int n = (int)c->n;
-  // keys0 / vals0 are the sort's unsorted-key and source scratch (free between
-  // calls); scratchA / scratchC take the removal flags of compactKept
-  uint32_t *sel = c->keys0, *pos = c->vals0;
-  auto *idx = reinterpret_cast<int32_t *>(c->scratchB);
-  k_layer_flags<<<blocksFor(n, 256), 256, 0, c->st>>>(c->cur.z, c->cur.tag, n, c->grid, izLo, izHi, sel,
-                                                       c->scratchA, c->scratchC);
-  enqueueExclusiveScan(c, sel, (size_t)n, pos);
+  // the sort's keys and arrivals are free between calls; scratchA takes the
+  // removal flags of compactKept
+  uint32_t *sel = c->keys, *pos = c->scratchC, *idx = c->scratchB;
+  const int m = (int)std::min(c->orderN, c->n);  // records leave in the order of the last scan
+  k_layer_flags<<<blocksFor(n, 256), 256, 0, c->st>>>(c->cur.z, c->cur.tag, n, c->perm, m, c->grid, izLo, izHi, sel,
+                                                       c->scratchA);
+  enqueueExclusiveScan(c, sel, (size_t)n, pos, c->st);
   CK(cudaGetLastError());
   uint32_t last[2] = {0, 0};
   CK(cudaMemcpyAsync(&last[0], pos + (n - 1), sizeof(uint32_t), cudaMemcpyDeviceToHost, c->st));
@@ -2071,7 +2082,7 @@ int ladds_gpu_pack_layers(ladds_gpu_ctx *c, int32_t izLo, int32_t izHi, int remo
   if (!count) return LADDS_OK;
   if (remove && !out) return compactKept(c);  // removed without being packed
   if (count > cap) return fail(c, LADDS_ERR_CAPACITY, "pack_layers: more particles than the output holds");
-  k_selected_positions<<<blocksFor(n, 256), 256, 0, c->st>>>(sel, pos, n, idx);
+  k_selected_slots<<<blocksFor(n, 256), 256, 0, c->st>>>(sel, pos, c->perm, m, n, idx);
   k_gather_records<<<blocksFor(count, 128), 128, 0, c->st>>>(c->cur, idx, (int)count, out);
   CK(cudaGetLastError());
   CK(cudaStreamSynchronize(c->st));
@@ -2112,11 +2123,17 @@ int ladds_gpu_truncate(ladds_gpu_ctx *c, size_t n0) {
   if (!c) return LADDS_ERR_INVALID_ARG;
   std::lock_guard<std::mutex> lk(g_deviceMutex[c->dev & 63]);
   if (n0 >= c->n) return LADDS_OK;
-  CK(cudaSetDevice(c->dev));
-  k_truncate_flags<<<blocksFor(c->n, 256), 256, 0, c->st>>>(c->cur.tag, (int)c->n, (uint32_t)n0, c->scratchA,
-                                                             c->scratchC);
-  CK(cudaGetLastError());
-  return compactKept(c);
+  if (c->orderN) {
+    CK(cudaSetDevice(c->dev));
+    k_below_flags<<<blocksFor(c->n, 256), 256, 0, c->st>>>((int)c->n, (uint32_t)n0, c->scratchA, c->scratchB);
+    CK(cudaGetLastError());
+    const int rc = compactOrder(c, c->scratchA, c->scratchB, c->n);
+    if (rc) return rc;
+  }
+  c->n = n0;  // the objects with the last slots
+  c->orderValid = false;
+  dropGraphs(c);
+  return LADDS_OK;
 }
 
 int ladds_gpu_remove_slots(ladds_gpu_ctx *c, const uint32_t *slots, size_t m) {
@@ -2130,8 +2147,7 @@ int ladds_gpu_remove_slots(ladds_gpu_ctx *c, const uint32_t *slots, size_t m) {
   for (size_t i = 0; i < m; ++i) mark[slots[i]] = 1;
   uint8_t *dMark = reinterpret_cast<uint8_t *>(c->scratchB);  // read before compactKept writes scratchB
   CK(cudaMemcpyAsync(dMark, mark.data(), c->n, cudaMemcpyHostToDevice, c->st));
-  k_slot_mark_flags<<<blocksFor(c->n, 256), 256, 0, c->st>>>(c->cur.tag, (int)c->n, dMark, c->scratchA,
-                                                              c->scratchC);
+  k_slot_mark_flags<<<blocksFor(c->n, 256), 256, 0, c->st>>>((int)c->n, dMark, c->scratchA);
   return compactKept(c);
 }
 
@@ -2644,7 +2660,7 @@ int ladds_gpu_adjoint_make_pairs(ladds_gpu_ctx *c, uint64_t seed, size_t nPairs,
 // so that cudaMalloc fails, and callers on a per-iteration latency path that
 // cannot take the implicit device synchronisation of cudaMalloc / cudaFree.
 // All scratch of the sort (row counts and cursors, row-start table, sort
-// records, source indices, long-row list, scan partial sums, status word)
+// records, long-row list, scan partial sums, status word)
 // lives in one file-scope device array of fixed size; the caller supplies the
 // keys and the output buffers.  Every call shares the array and it keeps the
 // last call's contents, so each call clears what must start at zero, and calls
@@ -2658,8 +2674,7 @@ constexpr size_t kNaScanBlocks = (kNaMaxRows + 1 + kScanBlock - 1) / kScanBlock;
 static_assert(kNaScanBlocks <= (size_t)kScanBlock, "two scan levels must cover the row table");
 // byte offsets inside the scratch array
 constexpr size_t kNaRec = 0;                                                   // u64 per object
-constexpr size_t kNaSrc = kNaRec + naRound(8 * kNaMaxObjects);                 // u32 per object
-constexpr size_t kNaCounts = kNaSrc + naRound(4 * kNaMaxObjects);              // counts | cursors
+constexpr size_t kNaCounts = kNaRec + naRound(8 * kNaMaxObjects);              // counts | cursors
 constexpr size_t kNaRowStart = kNaCounts + naRound(8 * (kNaMaxRows + 1));      // u32 per row + 1
 constexpr size_t kNaLong = kNaRowStart + naRound(4 * (kNaMaxRows + 1));        // long-row list
 constexpr size_t kNaMisc = kNaLong + naRound(4 * kNaMaxRows);                  // longCount, status
@@ -2697,12 +2712,11 @@ __global__ void __launch_bounds__(kBucketThreads) k_na_count(const uint32_t *__r
   if (valid && (__ffs(peers) - 1) == (int)(threadIdx.x & 31)) atomicAdd(&rowCount[row], (uint32_t)__popc(peers));
 }
 
-// sort record ix << 32 | j and source j of every object j (the index in keys)
+// sort record ix << 32 | j of every object j (the index in keys)
 __global__ void __launch_bounds__(kBucketThreads) k_na_scatter(const uint32_t *__restrict__ keys, int n, uint32_t nx,
                                                                uint32_t nRows, const uint32_t *__restrict__ rowStart,
                                                                uint32_t *__restrict__ rowCursor,
                                                                unsigned long long *__restrict__ rec,
-                                                               uint32_t *__restrict__ src,
                                                                unsigned *__restrict__ status) {
   const int j = blockIdx.x * blockDim.x + threadIdx.x;
   const int lane = threadIdx.x & 31;
@@ -2722,7 +2736,6 @@ __global__ void __launch_bounds__(kBucketThreads) k_na_scatter(const uint32_t *_
     return;
   }
   rec[pos] = ((unsigned long long)(key - row * nx) << 32) | (uint32_t)j;
-  src[pos] = (uint32_t)j;
 }
 
 struct DeviceGuard {
@@ -2812,7 +2825,6 @@ int ladds_gpu_cell_sort_noalloc(int device, void *stream, const uint32_t *keys, 
   }
   const uint32_t nx = (uint32_t)dims[0], nRows = (uint32_t)nRows64;
   auto *rec = reinterpret_cast<unsigned long long *>(d.scratch + kNaRec);
-  auto *src = reinterpret_cast<uint32_t *>(d.scratch + kNaSrc);
   auto *rowCount = reinterpret_cast<uint32_t *>(d.scratch + kNaCounts);
   uint32_t *rowCursor = rowCount + nRows + 1;
   auto *rowStartS = reinterpret_cast<uint32_t *>(d.scratch + kNaRowStart);
@@ -2821,6 +2833,8 @@ int ladds_gpu_cell_sort_noalloc(int device, void *stream, const uint32_t *keys, 
   auto *status = reinterpret_cast<unsigned *>(d.scratch + kNaMisc + 4);
   auto *s1 = reinterpret_cast<uint32_t *>(d.scratch + kNaScan);
   uint32_t *s1x = s1 + kNaScanBlocks + 1, *s2 = s1x + kNaScanBlocks + 1;
+
+  const CellOrderOut out{sortedKeys, order, nullptr, nullptr, nullptr, nullptr, nullptr};
 
   // every enqueue is checked where it is made; on a failure the stream is
   // drained before returning, so that no copy of this call is still running
@@ -2851,16 +2865,15 @@ int ladds_gpu_cell_sort_noalloc(int device, void *stream, const uint32_t *keys, 
   }
   if (e == cudaSuccess && n) {
     const int gridN = blocksFor(n, kBucketThreads);
-    k_na_scatter<<<gridN, kBucketThreads, 0, s>>>(keys, (int)n, nx, nRows, rowStartS, rowCursor, rec, src, status);
+    k_na_scatter<<<gridN, kBucketThreads, 0, s>>>(keys, (int)n, nx, nRows, rowStartS, rowCursor, rec, status);
     if (ok(cudaGetLastError())) {
       const int smallBlocks = std::min(blocksFor((size_t)nRows * 32, kBucketThreads), 64 * d.sms);
-      k_bucket_sort_small<<<smallBlocks, kBucketThreads, 0, s>>>(rowStartS, nRows, nx, rec, src, sortedKeys, order,
-                                                                 longRows, longCount, nullptr);
+      k_bucket_sort_small<<<smallBlocks, kBucketThreads, 0, s>>>(rowStartS, nRows, nx, rec, out, longRows, longCount,
+                                                                 nullptr);
     }
     if (ok(cudaGetLastError())) {
-      k_bucket_sort_large<<<2 * d.sms, kBucketThreads, kLargeRow * 12, s>>>(
-          rowStartS, nx, rec, src, sortedKeys, order, longRows, longCount, nullptr,
-          DenseBin{nullptr, nullptr, 0, 0, nullptr});
+      k_bucket_sort_large<<<2 * d.sms, kBucketThreads, kLargeRow * 8, s>>>(
+          rowStartS, nx, rec, out, longRows, longCount, nullptr, DenseBin{nullptr, nullptr, 0, 0, nullptr});
       ok(cudaGetLastError());
     }
   }

@@ -251,7 +251,7 @@ __device__ __forceinline__ void warpWindowPairs(uint32_t lo, uint32_t hi, int la
 // output as the grouped walk below; cutF as there.  The loops over the
 // neighbour rows are warp-uniform; inactive lanes contribute empty windows.
 template <int SCREEN>
-__global__ void __launch_bounds__(kScanCta) k_pair_rows(const uint32_t *__restrict__ tags,
+__global__ void __launch_bounds__(kScanCta) k_pair_rows(const uint32_t *__restrict__ perm,
                                                               const float4 *__restrict__ posf, int n,
                                                               const uint32_t *__restrict__ skeys,
                                                               const uint32_t *__restrict__ rowStart,
@@ -265,8 +265,8 @@ __global__ void __launch_bounds__(kScanCta) k_pair_rows(const uint32_t *__restri
   const int warpBase = blockIdx.x * kScanCta + warp * 32;
   const int j = warpBase + lane;
   const bool inRange = j < n;
-  const uint32_t myTag = inRange ? tags[j] : kTagDummy;
-  bool active = inRange && !tagDummy(myTag) && tagSlot(myTag) < out.haloStart;
+  const float4 me = inRange ? __ldg(&posf[j]) : make_float4(0.f, 0.f, 0.f, 0.f);
+  bool active = inRange && !recDeleted(me) && perm[j] < out.haloStart;
   const int32_t nx = g.n[0], ny = g.n[1], nz = g.n[2], R = g.reach;
   int32_t ix = 0, iy = 0, iz = 0;
   if (active) {
@@ -294,7 +294,6 @@ __global__ void __launch_bounds__(kScanCta) k_pair_rows(const uint32_t *__restri
   // cells.  With reach 1, or sparse populations (the list form), the cell
   // windows are kept: trimming them does not pay for its arithmetic.
   const bool perObject = SCREEN == LADDS_SCREEN_BUFFER && R >= 2;  // warp-uniform
-  const float4 me = active && perObject ? __ldg(&posf[j]) : make_float4(0.f, 0.f, 0.f, 0.f);
   const float cf = (float)g.cellSize, invCf = (float)g.invCell;
   const float fy = fminf(fmaxf(me.y - ((float)g.boxMin[1] + (float)iy * cf), 0.f), cf);
   const float fz = fminf(fmaxf(me.z - ((float)g.boxMin[2] + (float)iz * cf), 0.f), cf);
@@ -398,7 +397,7 @@ constexpr uint32_t kDealPass = 1024;  // items of one dealing pass (32 mask word
 // (0, 1), (1, -1), (1, 0), (1, 1), each with x half-width 1, known at compile
 // time (one group of five windows, no row table).
 template <int SCREEN, bool R1>
-__global__ void __launch_bounds__(kScanCta) k_pair_candidates(const uint32_t *__restrict__ tags,
+__global__ void __launch_bounds__(kScanCta) k_pair_candidates(const uint32_t *__restrict__ perm,
                                                               const float4 *__restrict__ posf, int n,
                                                               const uint32_t *__restrict__ skeys,
                                                               const uint32_t *__restrict__ rowStart,
@@ -419,12 +418,12 @@ __global__ void __launch_bounds__(kScanCta) k_pair_candidates(const uint32_t *__
   const int j = warpBase + lane;
   const bool inRange = j < n;
   // the object's own reads, all issued before any of them is used
-  const uint32_t myTag = inRange ? tags[j] : kTagDummy;
+  const uint32_t mySlot = inRange ? perm[j] : 0u;
   const uint32_t key = inRange ? skeys[j] : 0u;
   const float4 me = inRange ? __ldg(&posf[j]) : make_float4(0.f, 0.f, 0.f, 0.f);
   const uint32_t myGrp = out.grp && inRange ? __ldg(&out.grp[j]) : kNoGroup;
   const bool denseOn = cellOff && denseMin != 0xffffffffu && __ldg(denseCount) != 0u;
-  bool active = inRange && !tagDummy(myTag) && tagSlot(myTag) < out.haloStart;
+  bool active = inRange && !recDeleted(me) && mySlot < out.haloStart;
   const int32_t nx = g.n[0], ny = g.n[1], nz = g.n[2], R = g.reach;
   int32_t ix = 0, iy = 0, iz = 0;
   if (active) {
@@ -611,7 +610,7 @@ template <int SCREEN>
 __global__ void __launch_bounds__(kScanCta) k_pair_tiles(const uint32_t *__restrict__ denseCells,
                                                          const uint32_t *__restrict__ denseChunk,
                                                          const uint32_t *__restrict__ denseCount, uint32_t denseCap,
-                                                         const uint32_t *__restrict__ tags,
+                                                         const uint32_t *__restrict__ perm,
                                                          const float4 *__restrict__ posf,
                                                          const uint32_t *__restrict__ skeys,
                                                          const uint32_t *__restrict__ rowStart,
@@ -696,11 +695,11 @@ __global__ void __launch_bounds__(kScanCta) k_pair_tiles(const uint32_t *__restr
       __syncwarp();
       for (uint32_t sBase = s0; sBase < s1; sBase += 32u) {
         const uint32_t si = sBase + (uint32_t)lane;
-        const bool src = si < s1 && !tagDummy(tags[si]) && tagSlot(tags[si]) < out.haloStart;
+        const float4 mf = si < s1 ? __ldg(&posf[si]) : make_float4(0.f, 0.f, 0.f, 0.f);
+        const bool src = si < s1 && !recDeleted(mf) && perm[si] < out.haloStart;
         const uint32_t gs = grp && si < s1 ? __ldg(&grp[si]) : kNoGroup;
         // the batch and the staged block all in the same group: no pair can yield a record
         if (oneGroup && __all_sync(0xffffffffu, !src || gs == g0)) continue;
-        const float4 mf = src ? __ldg(&posf[si]) : make_float4(0.f, 0.f, 0.f, 0.f);
         for (uint32_t u = 0; u < m; ++u) {  // warp-uniform
           const float4 qq = sNb[warp][u];
           const uint32_t k = sK[warp][u];

@@ -1,4 +1,4 @@
-// propagate.cuh -- Yoshida-4 propagation kernel (+ fused cell-key output).
+// propagate.cuh -- Yoshida-4 propagation kernels (+ the input of the scan that follows).
 //
 // Replaces YoshidaIntegrator::integrate(false) (called at Simulation.cpp:297;
 // the integrator itself is in the non-vendored OrbitPropagator).  Form: DKD
@@ -14,6 +14,7 @@
 #pragma once
 #include "bulk_copy.cuh"
 #include "cell_sort.cuh"
+#include "conjunction.cuh"
 #include "forces.cuh"
 #include "state.cuh"
 
@@ -37,19 +38,45 @@ struct PropConsts {
   uint32_t mask;
 };
 
+// floor((v - lo) * inv) with exactly these two roundings; NaN -> 0; clamped to
+// [0, n).  The floor of a value below 2^31 is the low word of its sum with
+// 3 * 2^51 rounded down; larger values, infinities and NaN are told by the high word.
 __device__ __forceinline__ uint32_t cellCoord(double v, double lo, double inv, int32_t n) {
-  // floor((v - lo) * inv) with exactly these two roundings; NaN -> 0; clamped
-  const double u = floor(__dmul_rn(__dsub_rn(v, lo), inv));
-  if (!(u >= 0.0)) return 0u;
-  if (u >= (double)n) return (uint32_t)(n - 1);
-  return (uint32_t)u;
+  const double u = __dmul_rn(__dsub_rn(v, lo), inv);
+  const int hi = __double2hiint(u);
+  if (hi < 0) return 0u;  // negative (or -0)
+  if (hi >= 0x41e00000) return u >= 2147483648.0 ? (uint32_t)(n - 1) : 0u;
+  return (uint32_t)min(__double2loint(__dadd_rd(u, 6755399441055744.0)), n - 1);
 }
 
-__device__ __forceinline__ uint32_t cellKey(double x, double y, double z, const GridDesc &g) {
+struct CellOf {
+  uint32_t row, key;
+};
+__device__ __forceinline__ CellOf cellOf(double x, double y, double z, const GridDesc &g) {
   const uint32_t ix = cellCoord(x, g.boxMin[0], g.invCell, g.n[0]);
   const uint32_t iy = cellCoord(y, g.boxMin[1], g.invCell, g.n[1]);
   const uint32_t iz = cellCoord(z, g.boxMin[2], g.invCell, g.n[2]);
-  return (iz * (uint32_t)g.n[1] + iy) * (uint32_t)g.n[0] + ix;
+  const uint32_t row = iz * (uint32_t)g.n[1] + iy;
+  return {row, row * (uint32_t)g.n[0] + ix};
+}
+
+// What a scan needs of an object that has just been propagated (or is
+// scanned as it is), in slot order: its cell key, its arrival index in its
+// cell row, and its 32-byte scan record (ScanRec).
+struct ScanInput {
+  uint32_t *keys, *rowCount, *arrival;
+  ScanRec *rec;
+  const double *radius;
+};
+// every lane of the warp calls it (inRange = false for lanes without an object)
+__device__ __forceinline__ void writeScanInput(const ScanInput &o, const GridDesc &g, int j, bool inRange,
+                                               const double r[3], const double v[3], uint32_t tag) {
+  const CellOf c = cellOf(r[0], r[1], r[2], g);
+  const uint32_t a = countRowArrival(c.row, inRange, o.rowCount);
+  if (!inRange) return;
+  o.keys[j] = c.key;
+  o.arrival[j] = a;
+  o.rec[j] = scanRec(r, v, o.radius[j], tagDummy(tag));
 }
 
 // nSteps Yoshida-4 steps of one object (stage ephemerides ephBase ... of the
@@ -96,69 +123,48 @@ __device__ __forceinline__ void yoshidaSteps(double r[3], double v[3], double ao
     atomicOr(status, 1u);
 }
 
-// KEYS: also writes the cell key of the end position and counts it into its
-// cell row (rowCount, arrival: see countRowArrival).
-template <bool SPLIT, bool KEYS>
+// Propagation without a scan: nSteps steps in place, one object per thread.
+template <bool SPLIT>
 __global__ void __launch_bounds__(256, 4) k_propagate(DevState s, int n, int nSteps, int ephBase, PropConsts pc,
-                                                   GridDesc g, uint32_t *__restrict__ keys,
-                                                   uint32_t *__restrict__ rowCount, uint32_t *__restrict__ arrival,
                                                    unsigned *__restrict__ status) {
   __shared__ AtmShared<SPLIT> atm;
   loadAtmTable(atm, c_atm);
   __syncthreads();
   const int j = blockIdx.x * blockDim.x + threadIdx.x;
-  if (!KEYS && j >= n) return;
-  const bool inRange = j < n;
-  const uint32_t tag = inRange ? s.tag[j] : kTagDummy;
-  double r[3] = {0.0, 0.0, 0.0};
-  if (inRange) {
-    r[0] = s.x[j];
-    r[1] = s.y[j];
-    r[2] = s.z[j];
-  }
-  if (!tagDummy(tag)) {
-    double v[3] = {s.vx[j], s.vy[j], s.vz[j]};
-    const double aom = s.aom[j], bc = s.bc[j];
-    yoshidaSteps<SPLIT>(r, v, aom, bc, tag, nSteps, ephBase, pc, atm, status);
-    s.x[j] = r[0];
-    s.y[j] = r[1];
-    s.z[j] = r[2];
-    s.vx[j] = v[0];
-    s.vy[j] = v[1];
-    s.vz[j] = v[2];
-  }
-  if (KEYS) {  // every lane of the warp reaches this point
-    const uint32_t key = cellKey(r[0], r[1], r[2], g);
-    const uint32_t a = countRowArrival(key, inRange, (uint32_t)g.n[0], rowCount);
-    if (inRange) {
-      keys[j] = key;
-      arrival[j] = a;
-    }
-  }
+  if (j >= n) return;
+  const uint32_t tag = s.tag[j];
+  if (tagDummy(tag)) return;
+  double r[3] = {s.x[j], s.y[j], s.z[j]}, v[3] = {s.vx[j], s.vy[j], s.vz[j]};
+  yoshidaSteps<SPLIT>(r, v, s.aom[j], s.bc[j], tag, nSteps, ephBase, pc, atm, status);
+  s.x[j] = r[0];
+  s.y[j] = r[1];
+  s.z[j] = r[2];
+  s.vx[j] = v[0];
+  s.vy[j] = v[1];
+  s.vz[j] = v[2];
 }
 
-// The per-scan propagation (with cell keys) over a persistent grid.  CTA b
-// takes the tiles b, b + gridDim.x, ... of kStageObjects consecutive objects.
-// While a tile is propagated, the state of the CTA's next tile is already on
-// its way into shared memory: one thread issues nine bulk copies (x, y, z, vx,
-// vy, vz, aom, bc: 2 KB each; tags: 1 KB) completed on an mbarrier, so no
-// warp stalls on its loads after the first tile, and the atmosphere table is
-// staged once per CTA instead of once per 256 objects.  The partial tile at
-// the end (n % kStageObjects objects) is read directly.  Results are those of
-// k_propagate<SPLIT, true> bit for bit (same per-object arithmetic).  A wait
+// The propagation that ends at a scan (nSteps steps: those since the scan
+// before it), over a persistent grid.  CTA b takes the tiles b, b + gridDim.x,
+// ... of kStageObjects consecutive slots.  While a tile is propagated, the
+// state of the CTA's next tile is already on its way into shared memory: one
+// thread issues nine bulk copies (x, y, z, vx, vy, vz, aom, bc: 2 KB each;
+// tags: 1 KB) completed on an mbarrier, so no warp stalls on its loads after
+// the first tile, and the atmosphere table is staged once per CTA instead of
+// once per 256 objects.  The partial tile at the end (n % kStageObjects
+// objects) is read directly.  The new state goes to `to`, which may be s
+// itself: the state before it stays readable for the pair scan that is still
+// running on it.  Per-object arithmetic and results are k_propagate's.  A wait
 // that runs out (it cannot, unless a copy is lost) sets bit 8 of *status.
 constexpr int kStageObjects = 256;
 constexpr int kStageArrays = 8;
 constexpr uint32_t kStageTxBytes = kStageArrays * kStageObjects * 8 + kStageObjects * 4;
 constexpr uint32_t kStageWaitPolls = 1u << 22;
 
-template <bool SPLIT>
-__global__ void __launch_bounds__(kStageObjects, 4) k_propagate_staged(DevState s, int n, int nSteps, int ephBase,
-                                                                      PropConsts pc, GridDesc g,
-                                                                      uint32_t *__restrict__ keys,
-                                                                      uint32_t *__restrict__ rowCount,
-                                                                      uint32_t *__restrict__ arrival,
-                                                                      unsigned *__restrict__ status) {
+template <bool SPLIT, bool SCAN>
+__global__ void __launch_bounds__(kStageObjects, 4) k_propagate_staged(DevState s, DevState to, int n, int nSteps,
+                                                                      int ephBase, PropConsts pc, GridDesc g,
+                                                                      ScanInput scan, unsigned *__restrict__ status) {
   __shared__ AtmShared<SPLIT> atm;
   __shared__ __align__(16) double sv[kStageArrays][kStageObjects];
   __shared__ __align__(16) uint32_t stag[kStageObjects];
@@ -213,22 +219,17 @@ __global__ void __launch_bounds__(kStageObjects, 4) k_propagate_staged(DevState 
       aom = s.aom[j];
       bc = s.bc[j];
     }
-    if (!tagDummy(tag)) {
-      yoshidaSteps<SPLIT>(r, v, aom, bc, tag, nSteps, ephBase, pc, atm, status);
-      s.x[j] = r[0];
-      s.y[j] = r[1];
-      s.z[j] = r[2];
-      s.vx[j] = v[0];
-      s.vy[j] = v[1];
-      s.vz[j] = v[2];
+    if (!tagDummy(tag)) yoshidaSteps<SPLIT>(r, v, aom, bc, tag, nSteps, ephBase, pc, atm, status);
+    if (inRange) {  // deleted objects too: both buffers hold them
+      to.x[j] = r[0];
+      to.y[j] = r[1];
+      to.z[j] = r[2];
+      to.vx[j] = v[0];
+      to.vy[j] = v[1];
+      to.vz[j] = v[2];
     }
     // every lane of the warp reaches this point
-    const uint32_t key = cellKey(r[0], r[1], r[2], g);
-    const uint32_t a = countRowArrival(key, inRange, (uint32_t)g.n[0], rowCount);
-    if (inRange) {
-      keys[j] = key;
-      arrival[j] = a;
-    }
+    if (SCAN) writeScanInput(scan, g, j, inRange, r, v, tag);
   }
 }
 
@@ -268,18 +269,18 @@ __global__ void k_ephemeris(EphEntry *__restrict__ out, int nSteps, int64_t iter
   ephemerisEntry(jdEpoch, theta0, tau, mask, out[i]);
 }
 
-// cell keys of the current positions + their row counts (as k_propagate<*, true>)
-__global__ void k_cell_keys(const double *__restrict__ x, const double *__restrict__ y, const double *__restrict__ z,
-                            int n, GridDesc g, uint32_t *__restrict__ keys, uint32_t *__restrict__ rowCount,
-                            uint32_t *__restrict__ arrival) {
+// scan input of the current state
+__global__ void k_scan_input(DevState s, int n, GridDesc g, ScanInput scan) {
   const int j = blockIdx.x * blockDim.x + threadIdx.x;
   const bool inRange = j < n;
-  const uint32_t key = inRange ? cellKey(x[j], y[j], z[j], g) : 0u;
-  const uint32_t a = countRowArrival(key, inRange, (uint32_t)g.n[0], rowCount);
+  double r[3] = {0.0, 0.0, 0.0}, v[3] = {0.0, 0.0, 0.0};
+  uint32_t tag = 0;
   if (inRange) {
-    keys[j] = key;
-    arrival[j] = a;
+    r[0] = s.x[j], r[1] = s.y[j], r[2] = s.z[j];
+    v[0] = s.vx[j], v[1] = s.vy[j], v[2] = s.vz[j];
+    tag = s.tag[j];
   }
+  writeScanInput(scan, g, j, inRange, r, v, tag);
 }
 
 }  // namespace ladds

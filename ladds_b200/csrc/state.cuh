@@ -1,12 +1,14 @@
 // state.cuh -- device layout of the particle population.
 //
 // Structure of arrays, one array per attribute of the reference Particle
-// (Particle.h:139-195) that the hot path reads.  Positions and velocities are
-// binary64 (48 B/object), the per-object constants aom / bcInv / radius are
-// binary64, id / parentId are u64 and a u32 tag packs the slot (upload index),
-// the activity state and the dummy ("deleted") flag.  Two copies are kept and
-// swapped: every conjunction scan gathers the population into cell order, so
-// objects stay spatially sorted and the next gather is close to a streaming copy.
+// (Particle.h:139-195) that the hot path reads, indexed by slot (the upload
+// index).  Positions and velocities are binary64 (48 B/object) in two copies:
+// the propagation that ends at a scan reads one and writes the other, so that
+// the scan of the state before it can run beside it and a step can be undone.
+// The per-object constants aom / bcInv / radius (binary64), id / parentId
+// (u64) and a u32 tag (the slot, the activity state and the dummy "deleted"
+// flag) exist once.  Cell order exists only in what the pair scan reads: the
+// row sort gathers 32-byte scan records into it.
 #pragma once
 #include <cstdint>
 
@@ -25,15 +27,21 @@ __host__ __device__ __forceinline__ uint32_t tagSlot(uint32_t t) { return t & kT
 __host__ __device__ __forceinline__ int tagAct(uint32_t t) { return (int)((t >> kTagActShift) & 3u); }
 __host__ __device__ __forceinline__ bool tagDummy(uint32_t t) { return (t & kTagDummy) != 0; }
 
-// One state buffer.  x .. vz, aom, bc and tag are indexed by position (the
-// order the buffer holds the objects in); radius, id and parent are indexed by
-// slot (tagSlot of the tag), do not move when the population is gathered into
-// cell order, and are shared by a context's buffers.
+// One state buffer: x .. vz are its own, the other arrays are shared by a
+// context's buffers.
 struct DevState {
   double *x, *y, *z, *vx, *vy, *vz;
   double *aom, *bc, *radius;
   uint64_t *id, *parent;
   uint32_t *tag;
+};
+
+// What the pair scan reads of an object, written in slot order with its cell
+// key and gathered into cell order by the row sort: one 32-byte sector.
+// Binary32 position with a bound on its rounding error per coordinate (its
+// sign bit marks a deleted object), binary32 velocity, radius rounded up.
+struct __align__(32) ScanRec {
+  float4 pos, vel;
 };
 
 // cell grid: key = (iz * ny + iy) * nx + ix

@@ -1,0 +1,104 @@
+"""The population in slot order on the GPU: the order in which records leave
+(pack_layers) through growth, removal and truncation, the cell order for row
+tables of every scan form, and overlapped iterations against single ones."""
+import numpy as np
+import pytest
+
+pytestmark = pytest.mark.gpu
+
+
+@pytest.fixture(scope="module")
+def capi():
+    import torch
+
+    if not torch.cuda.is_available():
+        pytest.skip("no CUDA device")
+    from ladds_b200 import build, capi
+
+    build.build_gpu()
+    return capi
+
+
+def cloud(n, seed, lo, hi, first_id=0):
+    rng = np.random.default_rng(seed)
+    r = rng.uniform(lo, hi, (n, 3))
+    v = rng.uniform(-2.0, 2.0, (n, 3))
+    one = np.ones(n)
+    return dict(x=r[:, 0], y=r[:, 1], z=r[:, 2], vx=v[:, 0], vy=v[:, 1], vz=v[:, 2], radius=0.1 * one,
+                aom=1e-9 * one, bc_inv=0.01 * one, id=np.arange(first_id, first_id + n, dtype=np.uint64))
+
+
+@pytest.mark.parametrize("scanned", [False, True])
+def test_pack_order_through_growth_removal_truncation(capi, scanned):
+    import torch
+
+    lo, hi = [7000.0, -100.0, -100.0], [7200.0, 100.0, 100.0]
+    a, b = cloud(3000, 1, lo, hi), cloud(6000, 2, lo, hi, 3000)  # the append outgrows the first capacity
+    with capi.Context(capi.default_config(cutoff=10.0, boxMin=lo, boxMax=hi)) as ctx:
+        ctx.upload(a)
+        order = np.arange(3000)
+        if scanned:
+            ctx.conjunctions(1.0)
+            order = ctx.cell_order()[1].astype(np.int64)
+        ctx.append(b)
+        ids = np.concatenate([order, np.arange(3000, 9000)])  # ids in the population's order
+        buf = torch.empty(9000 * 96, dtype=torch.uint8, device="cuda")
+
+        def packed():
+            n = ctx.pack_layers(0, ctx.grid()[0][2], False, buf, 9000)
+            return np.frombuffer(buf.cpu().numpy().tobytes(), dtype=capi.STATE_RECORD_DTYPE)["id"][:n]
+
+        assert np.array_equal(packed(), ids)
+        gone = np.random.default_rng(3).choice(9000, 2500, replace=False)
+        ctx.remove_slots(gone)
+        ids = ids[~np.isin(ids, gone)]
+        assert np.array_equal(packed(), ids)
+        left = np.sort(ids)  # slot order
+        assert np.array_equal(ctx.download()["id"], left)
+        ctx.truncate(4000)
+        ids = ids[np.isin(ids, left[:4000])]
+        assert np.array_equal(packed(), ids)
+        assert np.array_equal(ctx.download()["id"], left[:4000])
+
+
+@pytest.mark.parametrize("ny,nz", [(1, 1), (31, 33), (32, 32), (341, 384), (256, 512), (500, 300), (1100, 1000)])
+def test_cell_order_for_row_tables(capi, ny, nz):
+    """Row counts around one block of the row scan, the last size it takes in one
+    launch (128 blocks), two passes, and three levels (above 2^20 rows)."""
+    n, nx = 20_011, 7
+    lo, hi = np.zeros(3), np.array([nx, ny, nz], dtype=float)
+    pop = cloud(n, ny + nz, lo - 0.5, hi + 0.5)
+    with capi.Context(capi.default_config(cutoff=0.5, cellSize=1.0, boxMin=list(lo), boxMax=list(hi))) as ctx:
+        ctx.upload(pop)
+        for _ in range(2):  # the second sort uses the other set of tables
+            ctx.conjunctions(1.0)
+            keys, slots = ctx.cell_order()
+            assert ctx.grid()[0] == (nx, ny, nz)
+            ix, iy, iz = (np.clip(np.floor(pop[k]), 0, m - 1).astype(np.int64)
+                          for k, m in zip("xyz", (nx, ny, nz)))
+            want = (iz * ny + iy) * nx + ix
+            order = np.argsort(want, kind="stable")
+            assert np.array_equal(slots, order)
+            assert np.array_equal(keys, want[order])
+
+
+@pytest.mark.parametrize("every", [1, 2, 3, 5])
+@pytest.mark.parametrize("precision", [0, 1])
+def test_overlapped_iterations_equal_single_ones(capi, every, precision):
+    """A call of many iterations (ring of three states, two sets of sort tables,
+    one propagation launch per scan) against one call per iteration."""
+    pop = capi.generate_population(0, 5, 3001)
+    pop["activity"][::40] = capi.EVASIVE_PRESERVING
+    kw = dict(componentMask=capi.PROP_ALL, precision=precision, timestepsPerCollisionDetection=every,
+              conjunctionThreshold=70.0)
+    with capi.Context(capi.default_config(**kw)) as a, capi.Context(capi.default_config(**kw)) as b:
+        for ctx in (a, b):
+            ctx.upload(pop)
+            ctx.mark_deleted(np.arange(0, 3001, 37))
+        for calls in (11, 4, 1):
+            many = a.step(calls).records
+            ones = np.concatenate([b.step(1).records for _ in range(calls)])
+            assert len(many) > 0 or calls < every
+            assert many.tobytes() == ones.tobytes()
+            for p, q in zip(a.get_state(), b.get_state()):
+                assert np.array_equal(p, q)
