@@ -145,27 +145,11 @@ __device__ __forceinline__ uint32_t functorPair(const ScanConsts &c, const Obj &
   return flags;
 }
 
-// Binary32 screen of a candidate pair: false only if the pair provably yields
-// no record, i.e. its closest approach over the step exceeds every threshold
-// (collision separation with the radii rounded up, evasion and conjunction
-// cutoffs, their near bands) and d^2 is outside the near band of the cutoff,
-// each by more than the error bound of this computation:
-//   positions: per-coordinate rounding <= posf.w (a 4x bound), velocities
-//   2^-24 |v| per coordinate, times dt; the closest approach over t is
-//   1-Lipschitz in the separation and dt-Lipschitz in the relative velocity;
-//   binary32 arithmetic on separations of size S: 2^-20 S.  FAST: the division
-//   and the square roots are the hardware approximations (relative errors of
-//   a few 2^-23): an error in t moves the distance at second order, and the
-//   distances' own relative error stays far inside the 1e-6 S term.  (FAST
-//   pays where the screen dominates -- dense populations -- and costs where it
-//   does not: its special-function work competes with the propagation that
-//   runs beside the scan.)
-// NaN (identical velocities: the reference's 0/0 path) keeps the pair.
-// the binary32 constants of mayRecord from the scan's parameters (host):
-// dt, factor; rel = 1 + 4 nearRel + 1e-6; thr = max(evasion cutoff, conjunction
-// threshold); cutoff^2, cutoff; nearBand = cutoff^2 nearRel 1.01.  Computed
-// once per scan instead of per screened pair (each was a conversion from
-// binary64 or a square root); the values are those the screen formed itself.
+// The binary32 constants of mayRecord from the scan's parameters (host), formed
+// once per scan: dt, factor; rel = 1 + 4 nearRel + 1e-6; thr = max(evasion
+// cutoff, conjunction threshold); cutoff^2, cutoff; nearBand = cutoff^2 nearRel
+// 1.01; the error bound of the screen, errV vmax + err0 + a multiple of the
+// positions' bounds.
 inline ScanConsts screenConsts(ScanConsts c) {
   c.dtF = (float)c.dt;
   c.factorF = (float)c.factor;
@@ -175,10 +159,26 @@ inline ScanConsts screenConsts(ScanConsts c) {
   c.cut2F = (float)c.cutoffSq;
   c.cutF = std::sqrt(c.cut2F);
   c.nearBandF = c.cut2F * nr * 1.01f;
+  c.errV = (float)((3.5e-7 + 1.7321e-6) * std::fabs(c.dt) * 1.0001);
+  c.err0 = 1e-6f + 1.01e-6f * c.cutF * (1.0f + nr);
   return c;
 }
 
-template <bool FAST = false>
+// Binary32 screen of a pre-filtered pair: false only if the pair provably
+// yields no record, i.e. its closest approach over the step exceeds every
+// threshold (collision separation with the radii rounded up, evasion and
+// conjunction cutoffs, their near bands) and d^2 is outside the near band of
+// the cutoff, each by more than the error bound of this computation:
+//   positions: per-coordinate rounding <= posf.w (a 4x bound), velocities
+//   2^-24 |v| per coordinate, times dt; the closest approach over t is
+//   1-Lipschitz in the separation and dt-Lipschitz in the relative velocity;
+//   binary32 arithmetic on separations of size S: 2^-20 S, with S = |dr| +
+//   |dv| dt bounded by the pre-filter radius and sqrt(3) vmax dt (vmax: the
+//   sum of the two largest velocity components), so that it takes no square
+//   root.  The division is the hardware approximation (relative error of a few
+//   2^-23): an error in t moves the distance at second order.  Distances are
+//   compared as squares; their own relative error stays far inside the S term.
+// NaN (identical velocities: the reference's 0/0 path) keeps the pair.
 __device__ __forceinline__ bool mayRecord(const ScanConsts &c, float4 pa, float4 va, float4 pb, float4 vb) {
   const float dt = c.dtF;
   const float drx = pa.x - pb.x, dry = pa.y - pb.y, drz = pa.z - pb.z;
@@ -186,19 +186,17 @@ __device__ __forceinline__ bool mayRecord(const ScanConsts &c, float4 pa, float4
   const float ox = drx - dvx * dt, oy = dry - dvy * dt, oz = drz - dvz * dt;  // separation at the step start
   const float dv2 = dvx * dvx + dvy * dvy + dvz * dvz;
   const float num = -(ox * dvx + oy * dvy + oz * dvz);
-  float t = FAST ? __fdividef(num, dv2) : num / dv2;  // 0/0: NaN, kept below
+  float t = __fdividef(num, dv2);  // 0/0: NaN, kept below
   t = (t < 0.0f) ? 0.0f : ((dt < t) ? dt : t);
   const float mx = ox + dvx * t, my = oy + dvy * t, mz = oz + dvz * t;
   const float m2 = mx * mx + my * my + mz * mz;
-  const float dl = FAST ? m2 * rsqrtf(m2) : sqrtf(m2);  // FAST: 0 * inf = NaN for m2 = 0, kept
   const float d2 = drx * drx + dry * dry + drz * drz;
   const float vmax = fmaxf(fmaxf(fabsf(va.x), fabsf(va.y)), fabsf(va.z)) +
                      fmaxf(fmaxf(fabsf(vb.x), fabsf(vb.y)), fabsf(vb.z));
-  const float sepScale = FAST ? d2 * rsqrtf(d2) + dv2 * rsqrtf(dv2) * dt : sqrtf(d2) + sqrtf(dv2) * dt;
-  const float err = 3.5f * (pa.w + pb.w) + 3.5e-7f * vmax * dt + 1e-6f * sepScale + 1e-6f;
+  const float err = fmaf(3.51f, pa.w + pb.w, fmaf(c.errV, vmax, c.err0));
   const float sep = (va.w + vb.w) * c.factorF;
-  const float thr = fmaxf(sep, c.thrF) * c.relF;
-  if (!(dl > thr + err)) return true;  // also NaN
+  const float lim = fmaf(fmaxf(sep, c.thrF), c.relF, err);
+  if (!(m2 > lim * lim)) return true;  // also NaN
   // near band of the cutoff gate: |d^2 - cutoff^2| <= nearRel cutoff^2
   const float d2err = 2.0f * c.cutF * err + 1e-5f * c.cut2F;
   return fabsf(d2 - c.cut2F) <= c.nearBandF + d2err;

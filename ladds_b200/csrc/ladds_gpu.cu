@@ -665,8 +665,9 @@ void enqueueSort(ladds_gpu_ctx *c, cudaStream_t s) {
 inline ScanPack scanPack(const ladds_gpu_ctx *c) { return ScanPack{c->posf, c->velf, c->cur, c->perm}; }
 
 // binary32 pre-filter radius of a cutoff: cutoff * (1 + nearRel), rounded up
+// and widened for the test on squares (prefilterPass)
 inline float prefilterRadius(double cutoff, double nearRel) {
-  return (float)(cutoff * (1.0 + nearRel) * (1.0 + 1e-6));
+  return (float)(cutoff * (1.0 + nearRel) * (1.0 + 2e-6));
 }
 
 // candidates + evaluation on stream s; records carry *iterPtr + iterOffset
@@ -682,26 +683,22 @@ void enqueueScanWith(ladds_gpu_ctx *c, cudaStream_t s, const ScanConsts &scIn, f
     // the largest separation a record or a near-band flag can have, with room for rounding
     const double reach = std::sqrt(sc.cutoffSq) * (1.0 + sc.nearRel) * (1.0 + 1e-6);
     const uint32_t denseMin = dense.cells ? dense.minCount : 0xffffffffu;
-    const int form = c->cfg.walkForm != LADDS_WALK_AUTO
-                         ? c->cfg.walkForm
-                         : (!buffer && c->grid.reach == 1 ? LADDS_WALK_GROUPED : LADDS_WALK_ROWS);
-    if (form == LADDS_WALK_ROWS) {
-      (buffer ? k_pair_rows<LADDS_SCREEN_BUFFER> : k_pair_rows<LADDS_SCREEN_LISTS>)<<<blocksFor(c->n, kScanCta),
-                                                                                       kScanCta, 0, s>>>(
-          c->perm, c->posf, (int)c->n, c->sortedKeys, c->rowStart, c->cellOff, c->grid, cutF, reach * reach,
-          denseMin, c->denseCount, out);
-    } else {
-      HalfShellRows rows;
-      buildHalfShellRows(rows, c->grid.reach, c->grid.cellSize, reach * reach);
-      const bool r1 = c->grid.reach == 1 && rows.n == 5;  // the five reach-1 rows, all of half-width 1
-      auto walk = buffer ? (r1 ? k_pair_candidates<LADDS_SCREEN_BUFFER, true>
-                               : k_pair_candidates<LADDS_SCREEN_BUFFER, false>)
-                         : (r1 ? k_pair_candidates<LADDS_SCREEN_LISTS, true>
-                               : k_pair_candidates<LADDS_SCREEN_LISTS, false>);
-      walk<<<blocksFor(c->n, kScanCta), kScanCta, 0, s>>>(c->perm, c->posf, (int)c->n, c->sortedKeys,
-                                                          c->rowStart, c->cellOff, c->grid, cutF, reach * reach,
-                                                          denseMin, c->denseCount, rows, out);
-    }
+    HalfShellRows rows;
+    buildHalfShellRows(rows, c->grid.reach, c->grid.cellSize, reach * reach);
+    // reach 1 and 2 with every row at its full half-width: rows known at compile time
+    const int full = c->grid.reach == 1 ? 5 : c->grid.reach == 2 ? 13 : -1;
+    bool whole = rows.n == full;
+    for (int q = 0; q < rows.n && whole; ++q) whole = (rows.e[q] >> 16) == (uint32_t)c->grid.reach;
+    const int r = whole ? c->grid.reach : 0;
+    auto walk = buffer ? (r == 1   ? k_pair_walk<LADDS_SCREEN_BUFFER, 1>
+                          : r == 2 ? k_pair_walk<LADDS_SCREEN_BUFFER, 2>
+                                   : k_pair_walk<LADDS_SCREEN_BUFFER, 0>)
+                       : (r == 1   ? k_pair_walk<LADDS_SCREEN_LISTS, 1>
+                          : r == 2 ? k_pair_walk<LADDS_SCREEN_LISTS, 2>
+                                   : k_pair_walk<LADDS_SCREEN_LISTS, 0>);
+    walk<<<blocksFor(c->n, kScanCta), kScanCta, 0, s>>>(c->perm, c->posf, (int)c->n, c->sortedKeys, c->rowStart,
+                                                        c->cellOff, c->grid, cutF, reach * reach, denseMin,
+                                                        c->denseCount, rows, out);
     if (dense.cells)  // the dense bin: grid-stride over the listed cells (count read on the device)
       (buffer ? k_pair_tiles<LADDS_SCREEN_BUFFER>
               : k_pair_tiles<LADDS_SCREEN_LISTS>)<<<4 * c->evalBlocks, kScanCta, 0, s>>>(
@@ -1071,7 +1068,7 @@ int ladds_gpu_create(const ladds_gpu_config *f, ladds_gpu_ctx **out) {
   c->sc.evasionSq = f->evasionCutoff * f->evasionCutoff;
   c->sc.conjSq = f->conjunctionThreshold * f->conjunctionThreshold;
   c->sc.nearRel = f->nearThresholdRel;
-  c->cutF = (float)(f->cutoff * (1.0 + f->nearThresholdRel) * (1.0 + 1e-6));
+  c->cutF = prefilterRadius(f->cutoff, f->nearThresholdRel);
   c->theta0 = gmstIAU1982(f->epochJD);
   if (cudaSetDevice(c->dev) != cudaSuccess || cudaStreamCreateWithFlags(&c->st, cudaStreamNonBlocking) != cudaSuccess ||
       allocGridBuffers(c) != LADDS_OK || cudaMalloc(&c->longCount, sizeof(uint32_t)) != cudaSuccess ||
@@ -1102,14 +1099,6 @@ int ladds_gpu_create(const ladds_gpu_config *f, ladds_gpu_ctx **out) {
   for (auto &e : c->evPipe) cudaEventCreateWithFlags(&e, cudaEventDisableTiming);
   cudaMemset(c->dCandNeed, 0, sizeof(unsigned long long));
   c->evalBlocks = 4 * std::max(prop.multiProcessorCount, 1);
-  // The reach-1 list walk runs beside the propagation and the sort of the next
-  // iteration; at its 40 registers twelve of its CTAs fit an SM, and the extra
-  // resident warps slow the iteration beside them more than they speed the
-  // walk.  A shared-memory carveout of 132 KB (57 % of 228 KB) holds it at ten
-  // CTAs per SM: 10 x (12 KB + 1 KB reserved).
-  if (cudaFuncSetAttribute(k_pair_candidates<LADDS_SCREEN_LISTS, true>, cudaFuncAttributePreferredSharedMemoryCarveout,
-                           57) != cudaSuccess)
-    cudaGetLastError();  // a preference only: without it the walk runs with more CTAs per SM
   rc = ensurePairCapacity(c, f->pairCapacity ? (size_t)f->pairCapacity : (size_t)1 << 16);
   if (!rc) rc = ensureCandCapacity(c, (size_t)1 << 16);
   if (rc) {

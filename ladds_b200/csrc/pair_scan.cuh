@@ -1,9 +1,9 @@
 // pair_scan.cuh -- two-phase pair scan over the cell-sorted population.
 //
-// Phase 1, k_pair_candidates: one thread per object of the cell order walks
-// its half-shell like a Newton3 linked-cell traversal -- the rest of its own
-// row window (ix .. ix+R, later objects only) and the rows (dz,dy) > (0,0),
-// each window ix-R .. ix+R.  A window is located with two reads of the row's
+// Phase 1, k_pair_walk: one thread per object of the cell order walks its
+// half-shell like a Newton3 linked-cell traversal -- the rest of its own row
+// window (ix .. ix+R, later objects only) and the rows (dz,dy) > (0,0), each
+// window ix-R .. ix+R.  A window is located with two reads of the row's
 // cell-offset table (written by the cell sort) instead of a search; rows whose
 // offsets do not fit 16 bits, or grids too large for the table, fall back to a
 // binary search on the sorted keys.  A binary32 distance test with a margin
@@ -113,11 +113,13 @@ __host__ __device__ __forceinline__ int rowHalfWidth(int dy, int dz, int R, doub
 // Binary32 pre-filter of one candidate pair with its positions loaded.  The
 // exact binary64 gate is left to the evaluation (functorPair), which loads both
 // records anyway: a gate here would stall the whole warp on two dependent
-// global loads for every pass.
+// global loads for every pass.  cutF carries the pre-filter radius widened by
+// 1e-6 and the bounds are widened with it, so that the square of the sum
+// covers the rounding of d^2.
 __device__ __forceinline__ bool prefilterPass(float4 mf, float4 q, float cutF) {
   const float dx = mf.x - q.x, dy = mf.y - q.y, dz = mf.z - q.z;
-  const float lim = cutF + 2.0f * (mf.w + q.w);
-  return !(dx * dx + dy * dy + dz * dz > lim * lim * 1.000001f);
+  const float lim = fmaf(2.000004f, mf.w + q.w, cutF);
+  return !(dx * dx + dy * dy + dz * dz > lim * lim);
 }
 
 // Where the pre-filtered pairs of a scan go: the screen's constants and
@@ -157,10 +159,9 @@ __device__ __forceinline__ void warpSpill(int lane, uint2 *buf, uint32_t &n, con
 }
 
 // The buffer at the end of the walk (and, LADDS_SCREEN_BUFFER, whenever it is
-// full): screened 32 pairs at a time (all four loads of a lane in flight
-// together); the survivors are appended to the screened list with one global
-// atomic per round that has any.
-template <int SCREEN>
+// full): screened 32 pairs at a time (all loads of a lane in flight together);
+// the survivors are appended to the screened list with one global atomic per
+// round that has any.
 __device__ __forceinline__ void warpFlush(int lane, uint2 *buf, uint32_t &n, const CandSink &out) {
   __syncwarp();
   for (uint32_t b = 0; b < n; b += 32u) {
@@ -169,7 +170,7 @@ __device__ __forceinline__ void warpFlush(int lane, uint2 *buf, uint32_t &n, con
     bool keep = false;
     if (i < n) {
       p = buf[i];
-      keep = mayRecord<SCREEN == LADDS_SCREEN_BUFFER>(out.sc, __ldg(&out.posf[p.x]), __ldg(&out.velf[p.x]), __ldg(&out.posf[p.y]),
+      keep = mayRecord(out.sc, __ldg(&out.posf[p.x]), __ldg(&out.velf[p.x]), __ldg(&out.posf[p.y]),
                        __ldg(&out.velf[p.y]));
     }
     const uint32_t mask = __ballot_sync(0xffffffffu, keep);
@@ -192,7 +193,7 @@ __device__ __forceinline__ void warpAppend(bool pass, uint32_t j, uint32_t k, in
   if (!mask) return;
   if (n + (uint32_t)__popc(mask) > (uint32_t)kWarpCand) {
     if (SCREEN == LADDS_SCREEN_BUFFER)
-      warpFlush<SCREEN>(lane, buf, n, out);
+      warpFlush(lane, buf, n, out);
     else
       warpSpill(lane, buf, n, out);
   }
@@ -210,129 +211,6 @@ __device__ __forceinline__ int windowOwner(uint32_t excl, uint32_t item) {
     if (e <= item) owner += step;
   }
   return owner;
-}
-
-// Warp-balanced walk of one neighbour row: lane l owns the window [lo, hi) of
-// its object; the windows of the warp are concatenated (exclusive prefix
-// `excl`) and dealt out 32 items per round, so every lane tests one pair per
-// round however uneven the windows are.
-template <int SCREEN>
-__device__ __forceinline__ void warpWindowPairs(uint32_t lo, uint32_t hi, int lane, int warpBase,
-                                                const float4 *__restrict__ posf, float cutF, uint2 *sCandW,
-                                                uint32_t &nBuf, const CandSink &out) {
-  const uint32_t cnt = hi - lo;
-  uint32_t incl = cnt;
-#pragma unroll
-  for (int o = 1; o < 32; o <<= 1) {
-    const uint32_t t = __shfl_up_sync(0xffffffffu, incl, o);
-    if (lane >= o) incl += t;
-  }
-  const uint32_t total = __shfl_sync(0xffffffffu, incl, 31);
-  const uint32_t excl = incl - cnt;
-  for (uint32_t base = 0; base < total; base += 32u) {
-    const uint32_t item = base + (uint32_t)lane;
-    const int owner = windowOwner(excl, item);
-    const uint32_t oLo = __shfl_sync(0xffffffffu, lo, owner), oEx = __shfl_sync(0xffffffffu, excl, owner);
-    const uint32_t jj = (uint32_t)(warpBase + owner), k = oLo + (item - oEx);
-    bool pass = item < total && prefilterPass(__ldg(&posf[jj]), __ldg(&posf[k]), cutF);
-    if (pass && out.grp) {  // fragments of one breakup never yield a record
-      const uint32_t g = __ldg(&out.grp[jj]);
-      pass = g == kNoGroup || g != __ldg(&out.grp[k]);
-    }
-    warpAppend<SCREEN>(pass, jj, k, lane, sCandW, nBuf, out);
-  }
-}
-
-// Per-row walk (LADDS_WALK_ROWS): the form for dense populations.  The warp
-// takes the half-shell rows one at a time: every lane locates its window in
-// the row, the windows are concatenated and dealt out 32 items per round with
-// the owner of an item found by a search over the lanes' prefix (few rounds
-// per row: many items per window).  Same pre-filter, screen, group skip and
-// output as the grouped walk below; cutF as there.  The loops over the
-// neighbour rows are warp-uniform; inactive lanes contribute empty windows.
-template <int SCREEN>
-__global__ void __launch_bounds__(kScanCta) k_pair_rows(const uint32_t *__restrict__ perm,
-                                                              const float4 *__restrict__ posf, int n,
-                                                              const uint32_t *__restrict__ skeys,
-                                                              const uint32_t *__restrict__ rowStart,
-                                                              const uint16_t *__restrict__ cellOff, GridDesc g,
-                                                              float cutF, double reachR2, uint32_t denseMin,
-                                                              const uint32_t *__restrict__ denseCount,
-                                                              const CandSink out) {
-  __shared__ uint2 sCand[kScanCta / 32][kWarpCand];
-  const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
-  uint32_t nBuf = 0;  // pairs in this warp's buffer (warp-uniform)
-  const int warpBase = blockIdx.x * kScanCta + warp * 32;
-  const int j = warpBase + lane;
-  const bool inRange = j < n;
-  const float4 me = inRange ? __ldg(&posf[j]) : make_float4(0.f, 0.f, 0.f, 0.f);
-  bool active = inRange && !recDeleted(me) && perm[j] < out.haloStart;
-  const int32_t nx = g.n[0], ny = g.n[1], nz = g.n[2], R = g.reach;
-  int32_t ix = 0, iy = 0, iz = 0;
-  if (active) {
-    const uint32_t key = skeys[j];
-    ix = (int32_t)(key % (uint32_t)nx);
-    const uint32_t row = key / (uint32_t)nx;
-    iy = (int32_t)(row % (uint32_t)ny);
-    iz = (int32_t)(row / (uint32_t)ny);
-    // objects of the dense bin (own cell >= denseMin objects) are scanned by k_pair_tiles
-    if (cellOff && denseMin != 0xffffffffu && __ldg(denseCount) != 0u) {
-      uint32_t a, b;  // the own cell's objects (rows beyond 16-bit offsets: searched)
-      rowWindow(row, (uint32_t)ix, (uint32_t)ix, (uint32_t)nx, rowStart, cellOff, skeys, a, b);
-      if (b - a >= denseMin) active = false;
-    }
-  }
-  const double c2 = g.cellSize * g.cellSize;
-  // Dense populations (the buffer form) with cells below the cutoff (reach >=
-  // 2): the object's own x-window in
-  // each neighbour row: partners lie within reachF of it, and a row whose
-  // (y, z) cell box is dyMin, dzMin away can hold them only within
-  // hw = sqrt(reachF^2 - dyMin^2 - dzMin^2) of its x.  Binary32 geometry with a
-  // 50 m margin over the pre-filter radius (which dwarfs the rounding of
-  // positions and cell edges); offsets inside the own cell are clamped to the
-  // cell, which only widens the windows of objects clamped into boundary
-  // cells.  With reach 1, or sparse populations (the list form), the cell
-  // windows are kept: trimming them does not pay for its arithmetic.
-  const bool perObject = SCREEN == LADDS_SCREEN_BUFFER && R >= 2;  // warp-uniform
-  const float cf = (float)g.cellSize, invCf = (float)g.invCell;
-  const float fy = fminf(fmaxf(me.y - ((float)g.boxMin[1] + (float)iy * cf), 0.f), cf);
-  const float fz = fminf(fmaxf(me.z - ((float)g.boxMin[2] + (float)iz * cf), 0.f), cf);
-  const float xRel = me.x - (float)g.boxMin[0];
-  const float reachF = cutF + 0.05f, reachF2 = reachF * reachF;
-  for (int dz = 0; dz <= R; ++dz) {
-    const float dzMin = dz == 0 ? 0.f : (float)(dz - 1) * cf + (cf - fz);
-    for (int dy = (dz == 0 ? 0 : -R); dy <= R; ++dy) {
-      const int w = rowHalfWidth(dy, dz, R, c2, reachR2);  // warp-uniform
-      if (w < 0) continue;
-      const int32_t jz = iz + dz, jy = iy + dy;
-      int32_t lo32 = dz == 0 && dy == 0 ? ix : max(ix - w, 0), hi32 = min(ix + w, nx - 1);
-      bool inReach = true;
-      if (perObject) {
-        const float dyMin =
-            dy == 0 ? 0.f : dy > 0 ? (float)(dy - 1) * cf + (cf - fy) : (float)(-dy - 1) * cf + fy;
-        const float h2 = reachF2 - dyMin * dyMin - dzMin * dzMin;
-        const float hw = h2 > 0.f ? h2 * rsqrtf(h2) : 0.f;
-        if (!(dz == 0 && dy == 0)) lo32 = max(lo32, (int32_t)floorf((xRel - hw) * invCf));
-        hi32 = min(hi32, (int32_t)floorf((xRel + hw) * invCf));
-        inReach = h2 >= 0.f && hi32 >= lo32;
-      }
-      const bool ok = active && jz < nz && jy >= 0 && jy < ny && inReach;
-      const uint32_t r2 = ok ? (uint32_t)jz * (uint32_t)ny + (uint32_t)jy : 0u;
-      const uint32_t xlo = ok ? (uint32_t)lo32 : 0u;
-      const uint32_t xhi = ok ? (uint32_t)hi32 : 0u;
-      const RowLookup L = rowLoads(r2, xlo, xhi, (uint32_t)nx, rowStart, cellOff);  // four reads in flight
-      uint32_t lo = 0, hi = 0;
-      if (ok) {
-        rowFinish(L, r2, xlo, xhi, (uint32_t)nx, cellOff, skeys, lo, hi);
-        if (dz == 0 && dy == 0) {  // own cell: later objects only
-          lo = (uint32_t)j + 1u;
-          if (hi < lo) hi = lo;
-        }
-      }
-      warpWindowPairs<SCREEN>(lo, hi, lane, warpBase, posf, cutF, sCand[warp], nBuf, out);
-    }
-  }
-  warpFlush<SCREEN>(lane, sCand[warp], nBuf, out);
 }
 
 // Half-shell rows of a scan: (dz, dy, x half-width w) of every neighbour row
@@ -376,39 +254,58 @@ inline void buildHalfShellRows(HalfShellRows &t, int R, double cellSize, double 
   }
 }
 
-constexpr int kWalkGroup = 8;        // neighbour rows whose windows are dealt out together
-constexpr uint32_t kDealPass = 1024;  // items of one dealing pass (32 mask words)
+// neighbour rows whose windows are dealt out together (reach 1: all five; reach 2: the thirteen in two groups)
+constexpr int walkGroup(int reach) { return reach == 1 ? 5 : 7; }
+constexpr uint32_t kDealPass = 1024;  // items of one dealing pass
 
-// cutF: cutoff * (1 + nearRel) rounded up, so that every pair the exact gate or
-// its near band accepts passes the binary32 test.
+// cutF: cutoff * (1 + nearRel) rounded up and widened (prefilterPass), so that
+// every pair the exact gate or its near band accepts passes the binary32 test.
 //
 // One warp walks the half shells of 32 consecutive objects of the cell order.
-// Neighbour rows are taken kWalkGroup at a time: every lane locates its window
-// [lo, hi) in each row of the group (all lookups in flight together), and the
-// non-empty windows of the whole warp -- up to 32 x kWalkGroup -- are listed
-// in shared memory in item order, each with its offset lo - (first item) and
-// its owner lane.  The concatenated items are then dealt out 32 per round:
-// the windows that start inside a round are marked in a bit mask per round
-// (built once per pass with shared atomics), so the window of item i is
-// found as (windows started before the round) + popc(mask & lanes <= i) - 1,
-// one shared load instead of a search.  The objects' own binary32 positions
-// are staged in shared memory once.  Inactive lanes contribute empty windows.
-// R1: reach-1 grids, whose half shell is the five rows (dz, dy) = (0, 0),
-// (0, 1), (1, -1), (1, 0), (1, 1), each with x half-width 1, known at compile
-// time (one group of five windows, no row table).
-template <int SCREEN, bool R1>
-__global__ void __launch_bounds__(kScanCta) k_pair_candidates(const uint32_t *__restrict__ perm,
-                                                              const float4 *__restrict__ posf, int n,
-                                                              const uint32_t *__restrict__ skeys,
-                                                              const uint32_t *__restrict__ rowStart,
-                                                              const uint16_t *__restrict__ cellOff, GridDesc g,
-                                                              float cutF, double reachR2, uint32_t denseMin,
-                                                              const uint32_t *__restrict__ denseCount,
-                                                              const HalfShellRows rows, const CandSink out) {
-  constexpr int W = kScanCta / 32;
-  constexpr int G = R1 ? 5 : kWalkGroup;  // windows per lane and group
+// Neighbour rows are taken walkGroup(REACH) at a time: every lane locates its
+// window [lo, hi) in each row of the group (all lookups in flight together),
+// and the non-empty windows of the whole warp are listed in shared memory in
+// item order, each with its offset lo - (first item) and its owner lane.  The
+// concatenated items are then dealt out 32 per round, so every lane tests one
+// pair per round however uneven the windows are: the windows that start inside
+// a round are marked in a bit mask per round (built once per pass with shared
+// atomics), so the window of item i is found as (windows started before the
+// round) + popc(mask & lanes <= i) - 1, one shared load instead of a search.
+// The objects' own binary32 positions are staged in shared memory once.
+// Inactive lanes contribute empty windows.
+//
+// REACH 1 and 2: the rows (5 and 13, each of half-width REACH) are known at
+// compile time; 0: rows from the table (or computed).  The kernel is bound by
+// instruction issue and by the L1 / shared-memory pipe together (8e6 objects at
+// 40 km: both above 75 %); with the rows at compile time, the bounds of a
+// window formed in cell units and no square root in the screen the candidates
+// take 2.02 ms there, where a per-row walk with a search over the lanes' prefix
+// for every item took 2.32 ms; 1e6 objects at 80 km 64 us either way.  A byte
+// per item written by its owner instead of the masks is slower (2.18 ms: its
+// shared-memory stores), and so are fewer resident CTAs (1e6 graph step 152 us
+// with all that fit, 156 with ten per SM).
+//
+// In the buffer form with cells below the cutoff (reach >= 2) the object's own
+// x-window in each neighbour row is narrowed: partners lie within reachF of it,
+// and a row whose (y, z) cell box is dyMin, dzMin away can hold them only within
+// hw = sqrt(reachF^2 - dyMin^2 - dzMin^2) of its x.  Everything in units of the
+// cell edge, binary32 with a 50 m margin over the pre-filter radius (which
+// dwarfs the rounding of positions and cell edges).  Offsets inside the own
+// cell are clamped to the cell: objects outside the grid count as being on its
+// boundary, where their cells are, and clamping brings no two objects farther
+// apart.
+template <int SCREEN, int REACH>
+__global__ void __launch_bounds__(kScanCta) k_pair_walk(const uint32_t *__restrict__ perm,
+                                                        const float4 *__restrict__ posf, int n,
+                                                        const uint32_t *__restrict__ skeys,
+                                                        const uint32_t *__restrict__ rowStart,
+                                                        const uint16_t *__restrict__ cellOff, GridDesc g, float cutF,
+                                                        double reachR2, uint32_t denseMin,
+                                                        const uint32_t *__restrict__ denseCount,
+                                                        const HalfShellRows rows, const CandSink out) {
+  constexpr int W = kScanCta / 32, G = walkGroup(REACH);
   __shared__ uint2 sCand[W][kWarpCand];
-  __shared__ uint2 sWin[W][32 * G];  // (lo - first item, owner lane) by window rank
+  __shared__ uint2 sWin[W][32 * G];  // (first target - first item, owner lane) by window rank
   __shared__ uint32_t sMask[W][kDealPass / 32];
   __shared__ float4 sOwn[W][32];
   __shared__ uint32_t sGrp[W][32];
@@ -424,85 +321,78 @@ __global__ void __launch_bounds__(kScanCta) k_pair_candidates(const uint32_t *__
   const uint32_t myGrp = out.grp && inRange ? __ldg(&out.grp[j]) : kNoGroup;
   const bool denseOn = cellOff && denseMin != 0xffffffffu && __ldg(denseCount) != 0u;
   bool active = inRange && !recDeleted(me) && mySlot < out.haloStart;
-  const int32_t nx = g.n[0], ny = g.n[1], nz = g.n[2], R = g.reach;
-  int32_t ix = 0, iy = 0, iz = 0;
-  if (active) {
-    ix = (int32_t)(key % (uint32_t)nx);
-    const uint32_t row = key / (uint32_t)nx;
-    iy = (int32_t)(row % (uint32_t)ny);
-    iz = (int32_t)(row / (uint32_t)ny);
-    // objects of the dense bin (own cell >= denseMin objects) are scanned by k_pair_tiles
-    if (denseOn) {
-      uint32_t a, b;  // the own cell's objects (rows beyond 16-bit offsets: searched)
-      rowWindow(row, (uint32_t)ix, (uint32_t)ix, (uint32_t)nx, rowStart, cellOff, skeys, a, b);
-      if (b - a >= denseMin) active = false;
-    }
+  const uint32_t nx = (uint32_t)g.n[0], ny = (uint32_t)g.n[1], nz = (uint32_t)g.n[2];
+  const int R = g.reach;
+  const uint32_t row = key / nx;
+  const int32_t ix = (int32_t)(key - row * nx);
+  const uint32_t iz = row / ny, iy = row - iz * ny;
+  // objects of the dense bin (own cell >= denseMin objects) are scanned by k_pair_tiles
+  if (active && denseOn) {
+    uint32_t a, b;  // the own cell's objects (rows beyond 16-bit offsets: searched)
+    rowWindow(row, (uint32_t)ix, (uint32_t)ix, nx, rowStart, cellOff, skeys, a, b);
+    if (b - a >= denseMin) active = false;
   }
   sOwn[warp][lane] = me;
   if (out.grp) sGrp[warp][lane] = myGrp;
-  const double c2 = g.cellSize * g.cellSize;
-  // Dense populations (the buffer form) with cells below the cutoff (reach >=
-  // 2): the object's own x-window in each neighbour row: partners lie within
-  // reachF of it, and a row whose (y, z) cell box is dyMin, dzMin away can
-  // hold them only within hw = sqrt(reachF^2 - dyMin^2 - dzMin^2) of its x.
-  // Binary32 geometry with a 50 m margin over the pre-filter radius (which
-  // dwarfs the rounding of positions and cell edges); offsets inside the own
-  // cell are clamped to the cell, which only widens the windows of objects
-  // clamped into boundary cells.
-  const bool perObject = !R1 && SCREEN == LADDS_SCREEN_BUFFER && R >= 2;  // warp-uniform
-  const float cf = (float)g.cellSize, invCf = (float)g.invCell;
-  const float fy = fminf(fmaxf(me.y - ((float)g.boxMin[1] + (float)iy * cf), 0.f), cf);
-  const float fz = fminf(fmaxf(me.z - ((float)g.boxMin[2] + (float)iz * cf), 0.f), cf);
-  const float xRel = me.x - (float)g.boxMin[0];
-  const float reachF = cutF + 0.05f, reachF2 = reachF * reachF;
-  const int nq = R1 ? 5 : rows.n >= 0 ? rows.n : (R + 1) + R * (2 * R + 1);
-  const uint32_t pitch = cellOffPitch((uint32_t)nx);
-  __syncwarp();
+  const bool perObject = REACH != 1 && SCREEN == LADDS_SCREEN_BUFFER && R >= 2;  // warp-uniform
+  const float inv = (float)g.invCell;
+  float fx = 0.f, fy = 0.f, fz = 0.f, reach2 = 0.f;
+  if (perObject) {
+    const float cf = (float)g.cellSize, rc = (cutF + 0.05f) * inv;
+    fx = __saturatef((me.x - ((float)g.boxMin[0] + (float)ix * cf)) * inv);
+    fy = __saturatef((me.y - ((float)g.boxMin[1] + (float)iy * cf)) * inv);
+    fz = __saturatef((me.z - ((float)g.boxMin[2] + (float)iz * cf)) * inv);
+    reach2 = rc * rc;
+  }
+  const int nq = REACH == 1 ? 5 : REACH == 2 ? 13 : rows.n >= 0 ? rows.n : (R + 1) + R * (2 * R + 1);
+  const uint32_t pitch = cellOffPitch(nx);
+  const uint16_t *const myOff = cellOff ? cellOff + (size_t)row * pitch : nullptr;
+#pragma unroll
   for (int q0 = 0; q0 < nq; q0 += G) {
-    const int gq = R1 ? G : min(G, nq - q0);  // warp-uniform
     uint32_t lo[G], cnt[G];
 #pragma unroll
     for (int t = 0; t < G; ++t) {
       lo[t] = 0u;
       cnt[t] = 0u;
-      if (t >= gq) continue;
+      if (q0 + t >= nq) continue;  // warp-uniform
       int dz, dy, w;
-      if constexpr (R1) {
-        dz = t >= 2 ? 1 : 0;
-        dy = t == 0 ? 0 : t == 1 ? 1 : t - 3;
-        w = 1;
+      if constexpr (REACH > 0) {
+        halfShellRowOf(q0 + t, REACH, dz, dy);
+        w = REACH;
       } else {
-        halfRow(rows, q0 + t, R, c2, reachR2, dz, dy, w);
+        halfRow(rows, q0 + t, R, g.cellSize * g.cellSize, reachR2, dz, dy, w);
       }
       const bool own = dz == 0 && dy == 0;
-      const int32_t jz = iz + dz, jy = iy + dy;
-      int32_t lo32 = own ? ix : max(ix - w, 0), hi32 = min(ix + w, nx - 1);
-      bool inReach = w >= 0;
+      int32_t lo32 = own ? ix : ix - w, hi32 = ix + w;
+      bool ok = active && w >= 0 && iy + (uint32_t)dy < ny && iz + (uint32_t)dz < nz;
       if (perObject) {
-        const float dzMin = dz == 0 ? 0.f : (float)(dz - 1) * cf + (cf - fz);
-        const float dyMin =
-            dy == 0 ? 0.f : dy > 0 ? (float)(dy - 1) * cf + (cf - fy) : (float)(-dy - 1) * cf + fy;
-        const float h2 = reachF2 - dyMin * dyMin - dzMin * dzMin;
+        const float ez = (float)dz - fz, ey = dy > 0 ? (float)dy - fy : (float)(-dy - 1) + fy;
+        float h2 = reach2;
+        if (dz) h2 -= ez * ez;
+        if (dy) h2 -= ey * ey;
         const float hw = h2 > 0.f ? h2 * rsqrtf(h2) : 0.f;
-        if (!own) lo32 = max(lo32, (int32_t)floorf((xRel - hw) * invCf));
-        hi32 = min(hi32, (int32_t)floorf((xRel + hw) * invCf));
-        inReach = inReach && h2 >= 0.f && hi32 >= lo32;
+        if (!own) lo32 = max(lo32, ix + (int32_t)floorf(fx - hw));
+        hi32 = min(hi32, ix + (int32_t)floorf(fx + hw));
+        ok = ok && h2 >= 0.f;
       }
-      const bool ok = active && jz < nz && jy >= 0 && jy < ny && inReach;
-      const uint32_t r2 = ok ? (uint32_t)jz * (uint32_t)ny + (uint32_t)jy : 0u;
+      lo32 = max(lo32, 0);
+      hi32 = min(hi32, (int32_t)nx - 1);
+      // an inactive lane reads its own row's entries and does not use them
+      const int32_t off = ok ? dz * (int32_t)ny + dy : 0;  // rows ahead
       const uint32_t xlo = ok ? (uint32_t)lo32 : 0u, xhi = ok ? (uint32_t)hi32 : 0u;
+      const uint32_t r2 = row + (uint32_t)off;
       RowLookup L;
       L.rs0 = __ldg(&rowStart[r2]);
       L.rs1 = __ldg(&rowStart[r2 + 1]);
       L.o0 = L.o1 = 0u;
       if (cellOff) {
-        const uint16_t *tp = cellOff + (size_t)r2 * pitch;
+        const uint16_t *tp = myOff + (int64_t)off * (int64_t)pitch;
         L.o0 = __ldg(&tp[xlo]);
         L.o1 = __ldg(&tp[xhi + 1]);
       }
       if (ok) {
         uint32_t a, b;
-        rowFinish(L, r2, xlo, xhi, (uint32_t)nx, cellOff, skeys, a, b);
+        rowFinish(L, r2, xlo, xhi, nx, cellOff, skeys, a, b);
         if (own) {  // own cell: later objects only
           a = (uint32_t)j + 1u;
           if (b < a) b = a;
@@ -529,65 +419,57 @@ __global__ void __launch_bounds__(kScanCta) k_pair_candidates(const uint32_t *__
     }
     const uint32_t total = __shfl_sync(0xffffffffu, inclT, 31);
     if (total == 0u) continue;  // warp-uniform
-    // windows in item order: lane-major, rows in order inside a lane
+    __syncwarp();  // the group before has been read (and the own positions are staged)
     {
       uint32_t item = inclT - tot, rank = inclE - nonEmpty;
 #pragma unroll
       for (int t = 0; t < G; ++t) {
-        if (cnt[t]) {
-          sWin[warp][rank] = make_uint2(lo[t] - item, (uint32_t)lane);
-          ++rank;
-        }
+        if (cnt[t]) sWin[warp][rank++] = make_uint2(lo[t] - item, (uint32_t)lane);
         item += cnt[t];
       }
     }
     for (uint32_t pass = 0; pass < total; pass += kDealPass) {  // warp-uniform
-      __syncwarp();
+      const uint32_t end = min(total - pass, kDealPass);
+      if (pass) __syncwarp();  // the pass before has been read
       sMask[warp][lane] = 0u;
-      // windows started before the pass; marks of the windows starting inside it
+      __syncwarp();
+      // marks of the windows that start inside the pass; windows started before it
       uint32_t before = 0, item = inclT - tot;
 #pragma unroll
       for (int t = 0; t < G; ++t) {
         if (cnt[t]) {
-          if (item < pass) ++before;
+          if (item < pass)
+            ++before;
+          else if (item - pass < kDealPass)
+            atomicOr(&sMask[warp][(item - pass) >> 5], 1u << ((item - pass) & 31u));
         }
         item += cnt[t];
       }
+      uint32_t started = pass ? __reduce_add_sync(0xffffffffu, before) : 0u;
       __syncwarp();
-      item = inclT - tot;
-#pragma unroll
-      for (int t = 0; t < G; ++t) {
-        if (cnt[t] && item >= pass && item - pass < kDealPass)
-          atomicOr(&sMask[warp][(item - pass) >> 5], 1u << ((item - pass) & 31u));
-        item += cnt[t];
-      }
-      uint32_t started = __reduce_add_sync(0xffffffffu, before);
-      __syncwarp();
-      const uint32_t end = min(total - pass, kDealPass);
       for (uint32_t base = 0; base < end; base += 32u) {  // warp-uniform
         const uint32_t mask = sMask[warp][base >> 5];
-        const uint32_t it = pass + base + (uint32_t)lane;
-        const bool valid = base + (uint32_t)lane < end;
+        const uint32_t it = base + (uint32_t)lane;
         const uint32_t rank = started + (uint32_t)__popc(mask & (0xffffffffu >> (31 - lane))) - 1u;
         started += (uint32_t)__popc(mask);
-        bool pass2 = false;
+        bool keep = false;
         uint32_t jj = 0u, k = 0u;
-        if (valid) {
+        if (it < end) {
           const uint2 wv = sWin[warp][rank];
-          k = wv.x + it;
-          jj = (uint32_t)warpBase + wv.y;
-          pass2 = prefilterPass(sOwn[warp][wv.y], __ldg(&posf[k]), cutF);
-          if (pass2 && out.grp) {  // fragments of one breakup never yield a record
-            const uint32_t g = sGrp[warp][wv.y];
-            pass2 = g == kNoGroup || g != __ldg(&out.grp[k]);
+          const uint32_t owner = wv.y;
+          k = pass + it + wv.x;
+          jj = (uint32_t)warpBase + owner;
+          keep = prefilterPass(sOwn[warp][owner], __ldg(&posf[k]), cutF);
+          if (keep && out.grp) {  // fragments of one breakup never yield a record
+            const uint32_t gr = sGrp[warp][owner];
+            keep = gr == kNoGroup || gr != __ldg(&out.grp[k]);
           }
         }
-        warpAppend<SCREEN>(pass2, jj, k, lane, sCand[warp], nBuf, out);
+        warpAppend<SCREEN>(keep, jj, k, lane, sCand[warp], nBuf, out);
       }
     }
-    __syncwarp();
   }
-  warpFlush<SCREEN>(lane, sCand[warp], nBuf, out);
+  warpFlush(lane, sCand[warp], nBuf, out);
 }
 
 // Dense bin of the pair scan (cells with >= kDenseCell objects, listed by the
@@ -602,7 +484,7 @@ __global__ void __launch_bounds__(kScanCta) k_pair_candidates(const uint32_t *__
 // paired with later objects only.  Pairs of one breakup group are skipped: a
 // staged block and a source batch that both belong to one group entirely are
 // not tested at all (a breakup's fragments start at one point, in one cell).
-// Same pre-filter and candidate output as k_pair_candidates, which skips these
+// Same pre-filter and candidate output as k_pair_walk, which skips these
 // objects as sources.
 constexpr uint32_t kTileStage = 256;  // staged neighbour objects per warp and pass
 
@@ -712,7 +594,7 @@ __global__ void __launch_bounds__(kScanCta) k_pair_tiles(const uint32_t *__restr
       __syncwarp();
     }
   }
-  warpFlush<SCREEN>(lane, sCand[warp], nBuf, out);
+  warpFlush(lane, sCand[warp], nBuf, out);
 }
 
 

@@ -63,7 +63,7 @@ struct ScanConsts {
   double nearRel;
   // binary32 forms for the screen of the pair scan (mayRecord), derived from the
   // fields above by screenConsts() before every scan launch
-  float dtF, factorF, relF, thrF, cut2F, cutF, nearBandF;
+  float dtF, factorF, relF, thrF, cut2F, cutF, nearBandF, errV, err0;
 };
 
 }  // namespace ladds

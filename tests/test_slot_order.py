@@ -1,8 +1,11 @@
 """The population in slot order on the GPU: the order in which records leave
 (pack_layers) through growth, removal and truncation, the cell order for row
-tables of every scan form, and overlapped iterations against single ones."""
+tables of every scan form, overlapped iterations against single ones, and the
+pair walk for every reach against the oracle."""
 import numpy as np
 import pytest
+
+from helpers import describe_diff, records_equal, to_oracle
 
 pytestmark = pytest.mark.gpu
 
@@ -102,3 +105,30 @@ def test_overlapped_iterations_equal_single_ones(capi, every, precision):
             assert many.tobytes() == ones.tobytes()
             for p, q in zip(a.get_state(), b.get_state()):
                 assert np.array_equal(p, q)
+
+
+@pytest.mark.parametrize("screen", [0, 1])
+@pytest.mark.parametrize("cell", [20.0, 15.0, 14.0, 10.0, 7.0, 5.0, 2.5])
+def test_pair_walk_for_every_reach(capi, oracle, cell, screen):
+    """Reach 1; reach 2 without and with its corner rows at full width (cells
+    above and below cutoff / sqrt(2) and cutoff / sqrt(3)); 3, 4 and 8 (rows
+    beyond the table).  A third of the objects lie outside the grid box on every
+    side; parents, deleted objects and a halo are among them."""
+    lo, hi = np.array([7000.0, -60.0, -60.0]), np.array([7130.0, 60.0, 70.0])
+    pop = cloud(3000, 17, lo - 35.0, hi + 35.0)
+    pop["parent"] = np.full(3000, np.uint64(0xFFFFFFFFFFFFFFFF))
+    pop["parent"][:300] = np.arange(300) % 3
+    kw = dict(cutoff=20.0, cellSize=cell, boxMin=list(lo), boxMax=list(hi), scanScreen=screen,
+              conjunctionThreshold=15.0, evasionCutoff=3.0)
+    with capi.Context(capi.default_config(**kw)) as ctx:
+        ctx.upload(pop)
+        recs = ctx.conjunctions(1.0)
+        p = oracle.scan_params(cutoff=20.0, dt=1.0, evasion_cutoff=3.0, conjunction_threshold=15.0)
+        ref = oracle.scan_bruteforce(to_oracle(oracle, ctx.download()), p)
+        assert len(ref) > 1000
+        assert records_equal(recs, ref), describe_diff(recs, ref)
+        gone = np.arange(5, 3000, 11)
+        ctx.mark_deleted(gone)
+        left = ctx.conjunctions(1.0)
+        keep = ~np.isin(ref["slotA"], gone) & ~np.isin(ref["slotB"], gone)
+        assert records_equal(left, ref[keep]), describe_diff(left, ref[keep])
