@@ -101,7 +101,7 @@ __device__ __forceinline__ uint32_t countRowArrival(uint32_t row, bool valid, ui
 
 // Scatter with the arrival indices of countRowArrival: no atomics.  Also
 // clears what is counted next: the row counts (nCounts of them), the lengths
-// of the long-row and dense-cell lists, the scan's three list counters.
+// of the long-row and dense-cell lists, the scan's five counters.
 __global__ void __launch_bounds__(kBucketThreads) k_bucket_place(
     const uint32_t *__restrict__ keys, const uint32_t *__restrict__ arrival, int n, uint32_t nx,
     const uint32_t *__restrict__ rowStart, unsigned long long *__restrict__ rec, uint32_t *__restrict__ rowCounts,
@@ -112,7 +112,7 @@ __global__ void __launch_bounds__(kBucketThreads) k_bucket_place(
   if (j == 0) {
     *longCount = 0u;
     *denseCount = 0u;
-    candCount[0] = candCount[1] = candCount[2] = 0ull;
+    for (int q = 0; q < 5; ++q) candCount[q] = 0ull;
   }
   if (j >= n) return;
   const uint32_t key = keys[j], row = key / nx;
@@ -149,13 +149,43 @@ __device__ __forceinline__ void emitCellOrder(const CellOrderOut &o, uint32_t po
 // comparator i of stage (k, jj) of the all-ascending bitonic network
 __device__ __forceinline__ void bitonicPair(uint32_t i, uint32_t k, uint32_t jj, uint32_t &lo, uint32_t &hi) {
   if (jj == k / 2) {  // flip stage
-    const uint32_t g = i / jj, w = i % jj;
-    lo = g * k + w;
-    hi = g * k + k - 1 - w;
+    const uint32_t w = i & (jj - 1u), g = 2u * (i - w);  // jj and k are powers of two
+    lo = g + w;
+    hi = g + k - 1u - w;
   } else {
-    const uint32_t g = i / jj, w = i % jj;
-    lo = g * 2 * jj + w;
+    const uint32_t w = i & (jj - 1u);
+    lo = 2u * (i - w) + w;
     hi = lo + jj;
+  }
+}
+
+// One stage of the network over V[0, L) by the CTA.  Its comparators touch
+// disjoint pairs, so each thread loads U pairs before it compares any: the
+// stage is bound by the latency of its loads (the 256 threads of a CTA, often
+// alone on their SM).
+template <int U>
+__device__ __forceinline__ void bitonicStage(unsigned long long *V, uint32_t L, uint32_t pairs, uint32_t k,
+                                             uint32_t jj) {
+  for (uint32_t i0 = threadIdx.x; i0 < pairs; i0 += (uint32_t)U * blockDim.x) {
+    uint32_t lo[U], hi[U];
+    unsigned long long a[U], b[U];
+#pragma unroll
+    for (int u = 0; u < U; ++u) {
+      bitonicPair(min(i0 + (uint32_t)u * blockDim.x, pairs - 1u), k, jj, lo[u], hi[u]);
+      if (i0 + (uint32_t)u * blockDim.x >= pairs) hi[u] = L;  // past the last comparator
+      a[u] = b[u] = 0ull;
+      if (hi[u] < L) {
+        a[u] = V[lo[u]];
+        b[u] = V[hi[u]];
+      }
+    }
+#pragma unroll
+    for (int u = 0; u < U; ++u) {
+      if (b[u] < a[u]) {
+        V[lo[u]] = b[u];
+        V[hi[u]] = a[u];
+      }
+    }
   }
 }
 
@@ -488,17 +518,7 @@ __global__ void __launch_bounds__(kBucketThreads) k_bucket_sort_large(
     if (inShared) {
       for (uint32_t k = 2; k <= P; k <<= 1) {
         for (uint32_t jj = k / 2; jj > 0; jj >>= 1) {
-          for (uint32_t i = threadIdx.x; i < P / 2; i += blockDim.x) {
-            uint32_t lo, hi;
-            bitonicPair(i, k, jj, lo, hi);
-            if (hi < L) {
-              const unsigned long long a = V[lo], b = V[hi];
-              if (b < a) {
-                V[lo] = b;
-                V[hi] = a;
-              }
-            }
-          }
+          bitonicStage<2>(sv, L, P / 2, k, jj);
           __syncthreads();
         }
       }
@@ -521,17 +541,7 @@ __global__ void __launch_bounds__(kBucketThreads) k_bucket_sort_large(
           __syncthreads();
           for (uint32_t kk = kFirst; kk <= kLast; kk <<= 1) {
             for (uint32_t jj = kk == kFirst ? jjFirst : kk / 2; jj > 0; jj >>= 1) {
-              for (uint32_t i = threadIdx.x; i < (uint32_t)kLargeRow / 2; i += blockDim.x) {
-                uint32_t lo, hi;
-                bitonicPair(i, kk, jj, lo, hi);
-                if (hi < n) {
-                  const unsigned long long x = sv[lo], y = sv[hi];
-                  if (y < x) {
-                    sv[lo] = y;
-                    sv[hi] = x;
-                  }
-                }
-              }
+              bitonicStage<2>(sv, n, (uint32_t)kLargeRow / 2, kk, jj);
               __syncthreads();
             }
           }
@@ -542,33 +552,7 @@ __global__ void __launch_bounds__(kBucketThreads) k_bucket_sort_large(
       blockStages(2u, (uint32_t)kLargeRow, 1u);  // each block sorted
       for (uint32_t k = 2u * (uint32_t)kLargeRow; k <= P; k <<= 1) {
         for (uint32_t jj = k / 2; jj >= (uint32_t)kLargeRow; jj >>= 1) {
-          // the comparators of a stage touch disjoint pairs, so each thread
-          // loads four pairs before it compares any (four loads in flight)
-          for (uint32_t i0 = threadIdx.x; i0 < P / 2; i0 += 4u * blockDim.x) {
-            uint32_t lo[4], hi[4];
-            unsigned long long a[4], b[4];
-            bool ok[4];
-#pragma unroll
-            for (int u = 0; u < 4; ++u) {
-              const uint32_t i = i0 + (uint32_t)u * blockDim.x;
-              ok[u] = false;
-              if (i < P / 2) {
-                bitonicPair(i, k, jj, lo[u], hi[u]);
-                ok[u] = hi[u] < L;
-              }
-              if (ok[u]) {
-                a[u] = V[lo[u]];
-                b[u] = V[hi[u]];
-              }
-            }
-#pragma unroll
-            for (int u = 0; u < 4; ++u) {
-              if (ok[u] && b[u] < a[u]) {
-                V[lo[u]] = b[u];
-                V[hi[u]] = a[u];
-              }
-            }
-          }
+          bitonicStage<2>(rec + s, L, P / 2, k, jj);
           __syncthreads();
         }
         blockStages(k, k, (uint32_t)kLargeRow / 2);
@@ -578,7 +562,15 @@ __global__ void __launch_bounds__(kBucketThreads) k_bucket_sort_large(
       emitCellOrder(out, s + i, r * nx + (uint32_t)(V[i] >> 32), (uint32_t)V[i]);
     if (cellOff && L <= 65535u) {  // offsets are 16-bit; longer rows are searched by the scan
       uint16_t *t = cellOff + (size_t)r * cellOffPitch(nx);
-      fillCellOffsets(t, nx, L, [&](uint32_t i) { return (uint32_t)(V[i] >> 32); }, threadIdx.x, blockDim.x);
+      // the first record of a cell writes its offset and those of the empty cells
+      // before it; a walk along the records was one thread's for a cloud's few
+      // crowded cells (six clouds, rows of up to 3740 objects: kernel 256 -> 73 us,
+      // with the two comparators in flight)
+      for (uint32_t i = threadIdx.x; i <= L; i += blockDim.x) {
+        const uint32_t from = i ? (uint32_t)(V[i - 1] >> 32) + 1u : 0u;
+        const uint32_t to = i < L ? (uint32_t)(V[i] >> 32) : nx;
+        for (uint32_t c = from; c <= to; ++c) t[c] = (uint16_t)i;
+      }
       __syncthreads();
       if (dense.cells)
         for (uint32_t c = threadIdx.x; c < nx; c += blockDim.x) {

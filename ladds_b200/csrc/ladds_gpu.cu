@@ -75,6 +75,9 @@ enum Phase { kPhProp, kPhBucket, kPhRowsort, kPhPermute, kPhCandidates, kPhEvalu
 constexpr int kHostChunks = 4;
 constexpr size_t kHostChunkMin = (size_t)1 << 17;
 
+// dealing passes that a scan's walk can leave to k_pair_tiles (1024 pair tests each)
+constexpr uint32_t kLaterCap = 1u << 17;
+
 }  // namespace
 
 struct ladds_gpu_ctx {
@@ -114,6 +117,7 @@ struct ladds_gpu_ctx {
   size_t pairCap = 0;
   unsigned long long *dCount = nullptr;
   uint2 *dCand = nullptr;  // candidate pairs (sorted indices) of the pair scan
+  uint2 *dLater = nullptr;  // dealing passes left by the walk (kLaterCap)
   size_t candCap = 0;  // entries of each of the two candidate lists
   unsigned long long *dCandCount = nullptr;  // lengths of the candidate lists of the current scan, dense-bin cursor
   unsigned long long *dCandNeed = nullptr;   // largest candidate count of the call
@@ -677,33 +681,34 @@ void enqueueScanWith(ladds_gpu_ctx *c, cudaStream_t s, const ScanConsts &scIn, f
   const DenseBin dense = denseBin(c);
   {
     PhaseScope ps(c, kPhCandidates, s, dense.cells ? 2 : 1);
-    const CandSink out{sc,       c->posf,     c->velf,      c->dCand, c->dCandCount, (unsigned long long)c->candCap,
-                       c->haloStart, c->anyParent ? c->grp : nullptr};
     const bool buffer = c->cfg.scanScreen == LADDS_SCREEN_BUFFER;
     // the largest separation a record or a near-band flag can have, with room for rounding
     const double reach = std::sqrt(sc.cutoffSq) * (1.0 + sc.nearRel) * (1.0 + 1e-6);
-    const uint32_t denseMin = dense.cells ? dense.minCount : 0xffffffffu;
-    HalfShellRows rows;
-    buildHalfShellRows(rows, c->grid.reach, c->grid.cellSize, reach * reach);
+    WalkIn in{c->perm,   c->posf, (int)c->n,     c->sortedKeys, c->rowStart, c->cellOff,
+              c->grid,   cutF,    reach * reach, dense.cells ? dense.minCount : 0xffffffffu,
+              c->denseCount, {},  0};
+    buildHalfShellRows(in.rows, c->grid.reach, c->grid.cellSize, reach * reach);
     // reach 1 and 2 with every row at its full half-width: rows known at compile time
     const int full = c->grid.reach == 1 ? 5 : c->grid.reach == 2 ? 13 : -1;
-    bool whole = rows.n == full;
-    for (int q = 0; q < rows.n && whole; ++q) whole = (rows.e[q] >> 16) == (uint32_t)c->grid.reach;
+    bool whole = in.rows.n == full;
+    for (int q = 0; q < in.rows.n && whole; ++q) whole = (in.rows.e[q] >> 16) == (uint32_t)c->grid.reach;
     const int r = whole ? c->grid.reach : 0;
+    in.groupRows = walkGroup(r);
+    // passes are left for later only where k_pair_tiles follows and the rows are in the table
+    const bool later = dense.cells && in.rows.n > 0 && in.rows.n <= kLaterGroups * in.groupRows;
+    const CandSink out{sc,           c->posf, c->velf, c->dCand, c->dCandCount, (unsigned long long)c->candCap,
+                       c->haloStart, c->anyParent ? c->grp : nullptr, later ? c->dLater : nullptr, kLaterCap};
     auto walk = buffer ? (r == 1   ? k_pair_walk<LADDS_SCREEN_BUFFER, 1>
                           : r == 2 ? k_pair_walk<LADDS_SCREEN_BUFFER, 2>
                                    : k_pair_walk<LADDS_SCREEN_BUFFER, 0>)
                        : (r == 1   ? k_pair_walk<LADDS_SCREEN_LISTS, 1>
                           : r == 2 ? k_pair_walk<LADDS_SCREEN_LISTS, 2>
                                    : k_pair_walk<LADDS_SCREEN_LISTS, 0>);
-    walk<<<blocksFor(c->n, kScanCta), kScanCta, 0, s>>>(c->perm, c->posf, (int)c->n, c->sortedKeys, c->rowStart,
-                                                        c->cellOff, c->grid, cutF, reach * reach, denseMin,
-                                                        c->denseCount, rows, out);
-    if (dense.cells)  // the dense bin: grid-stride over the listed cells (count read on the device)
+    walk<<<blocksFor(c->n, kScanCta), kScanCta, 0, s>>>(in, out);
+    if (dense.cells)  // the dense bin and the passes left by the walk, drawn entry by entry: one resident wave
       (buffer ? k_pair_tiles<LADDS_SCREEN_BUFFER>
-              : k_pair_tiles<LADDS_SCREEN_LISTS>)<<<4 * c->evalBlocks, kScanCta, 0, s>>>(
-          dense.cells, dense.chunk, dense.count, dense.cap, c->perm, c->posf, c->sortedKeys, c->rowStart,
-          c->cellOff, c->grid, cutF, reach * reach, out);
+              : k_pair_tiles<LADDS_SCREEN_LISTS>)<<<kTileCtasPerSm * c->evalBlocks / 4, kScanCta, 0,
+                                                  s>>>(dense.cells, dense.chunk, dense.cap, in, out);
   }
   PhaseScope ps(c, kPhEvaluate, s);
   const int b = c->cfg.scanBlock > 0 ? c->cfg.scanBlock : 256;
@@ -1075,8 +1080,9 @@ int ladds_gpu_create(const ladds_gpu_config *f, ladds_gpu_ctx **out) {
       cudaMalloc(&c->denseCount, sizeof(uint32_t)) != cudaSuccess ||
       cudaMalloc(&c->denseCountB, sizeof(uint32_t)) != cudaSuccess ||
       cudaMalloc(&c->dCount, 3 * sizeof(unsigned long long)) != cudaSuccess ||
-      cudaMalloc(&c->dCandCount, 3 * sizeof(unsigned long long)) != cudaSuccess ||
-      cudaMalloc(&c->dCandCountB, 3 * sizeof(unsigned long long)) != cudaSuccess ||
+      cudaMalloc(&c->dCandCount, kScanCounters * sizeof(unsigned long long)) != cudaSuccess ||
+      cudaMalloc(&c->dCandCountB, kScanCounters * sizeof(unsigned long long)) != cudaSuccess ||
+      cudaMalloc(&c->dLater, kLaterCap * sizeof(uint2)) != cudaSuccess ||
       cudaMalloc(&c->dEph, 3 * kMaxEphSteps * sizeof(EphEntry)) != cudaSuccess ||
       cudaMalloc(&c->dIter, 2 * sizeof(int64_t)) != cudaSuccess ||
       cudaStreamCreateWithFlags(&c->st2, cudaStreamNonBlocking) != cudaSuccess ||
@@ -1123,7 +1129,7 @@ int ladds_gpu_destroy(ladds_gpu_ctx *c) {
   freeGridBuffers(c);
   void *ptrs[] = {c->longCount, c->denseCount, c->denseCells, c->denseCountB, c->denseCellsB, c->dCount,
                   c->denseChunk, c->denseChunkB, c->dEph,
-                  c->dIter, c->dPairs, c->dCand, c->dCandCount, c->dCandCountB, c->dObj,
+                  c->dIter, c->dPairs, c->dCand, c->dCandCount, c->dCandCountB, c->dLater, c->dObj,
                   c->adj.st, c->adj.bc, c->adj.aom, c->adj.miss, c->adj.grad, c->adj.ckpt, c->adj.rec,
                   c->adj.off, c->adj.arg, c->adj.eph};
   for (void *p : ptrs)
@@ -1847,7 +1853,7 @@ int ladds_gpu_step_host(ladds_gpu_ctx *c, size_t n, const double *const in[6], d
   while (overflow) {  // the device buffers have grown: the scan alone runs again on the same state
     if (++retries > 4) return abortCall(fail(c, LADDS_ERR_STATE, "device scan buffers kept overflowing"));
     CKS(cudaMemsetAsync(c->dCount, 0, 2 * sizeof(unsigned long long), c->st));
-    CKS(cudaMemsetAsync(c->dCandCount, 0, 3 * sizeof(unsigned long long), c->st));  // the sort cleared them for one scan
+    CKS(cudaMemsetAsync(c->dCandCount, 0, kScanCounters * sizeof(unsigned long long), c->st));  // the sort cleared them for one scan
     enqueueScanWith(c, c->st, sc, c->cutF, c->dIterBase, 0);
     rc = syncStatusAndGrow(c, &cnt, &overflow);
     collectTimes(c);

@@ -135,7 +135,12 @@ struct CandSink {
   unsigned long long half;
   uint32_t haloStart;  // objects with slot >= haloStart are scan targets only, never sources
   const uint32_t *grp;  // breakup group per cell-order position (null: no object has a parent)
+  // dealing passes that the walk leaves to k_pair_tiles (null: none): their
+  // number in count[3], the next one to be drawn in count[4]
+  uint2 *later;
+  uint32_t laterCap;
 };
+constexpr int kScanCounters = 5;  // the two list lengths, the dense bin's cursor, the passes left and their cursor
 
 // Per-warp candidate buffer in shared memory with its fill count n held in a
 // register (warp-uniform): appends are ballots, no atomics.  Every lane of the
@@ -294,46 +299,85 @@ constexpr uint32_t kDealPass = 1024;  // items of one dealing pass
 // cell are clamped to the cell: objects outside the grid count as being on its
 // boundary, where their cells are, and clamping brings no two objects farther
 // apart.
-template <int SCREEN, int REACH>
-__global__ void __launch_bounds__(kScanCta) k_pair_walk(const uint32_t *__restrict__ perm,
-                                                        const float4 *__restrict__ posf, int n,
-                                                        const uint32_t *__restrict__ skeys,
-                                                        const uint32_t *__restrict__ rowStart,
-                                                        const uint16_t *__restrict__ cellOff, GridDesc g, float cutF,
-                                                        double reachR2, uint32_t denseMin,
-                                                        const uint32_t *__restrict__ denseCount,
-                                                        const HalfShellRows rows, const CandSink out) {
-  constexpr int W = kScanCta / 32, G = walkGroup(REACH);
-  __shared__ uint2 sCand[W][kWarpCand];
-  __shared__ uint2 sWin[W][32 * G];  // (first target - first item, owner lane) by window rank
-  __shared__ uint32_t sMask[W][kDealPass / 32];
-  __shared__ float4 sOwn[W][32];
-  __shared__ uint32_t sGrp[W][32];
-  const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
-  uint32_t nBuf = 0;  // pairs in this warp's buffer (warp-uniform)
-  const int warpBase = blockIdx.x * kScanCta + warp * 32;
+// What the walk of one warp needs besides the lists (see k_pair_walk).
+struct WalkIn {
+  const uint32_t *perm;
+  const float4 *posf;
+  int n;
+  const uint32_t *skeys, *rowStart;
+  const uint16_t *cellOff;
+  GridDesc g;
+  float cutF;
+  double reachR2;
+  uint32_t denseMin;
+  const uint32_t *denseCount;
+  HalfShellRows rows;
+  int groupRows;  // rows that a pass left for later covers
+};
+template <int G>
+struct WalkShared {
+  uint2 win[32 * G];  // (first target - first item, owner lane) by window rank
+  uint32_t mask[kDealPass / 32];
+  float4 own[32];
+  uint32_t grp[32];
+};
+
+// A warp with very many items in one group of rows -- sparse cells beside a
+// fragment cloud's crowded ones -- leaves its passes to k_pair_tiles, whose
+// warps draw them one at a time, instead of holding up the kernel:
+// 590,000 objects with six clouds of 15,000 fragments at 80 km, walk 625 -> 89 us,
+// and tiles 746 -> 139 us with these passes and the group rule below.
+constexpr uint32_t kLaterItems = 4u * kDealPass;
+constexpr uint32_t kLastPass = 1u << 31;  // the last pass of its group: everything from it on
+constexpr uint32_t kNoPass = 0xffffffffu;
+constexpr int kLaterGroups = 32;          // groups of rows that an entry can name (warp base | group, pass)
+
+// false: the list has no room for all of them (its remaining entries are made empty)
+__device__ __forceinline__ bool leaveForLater(const CandSink &out, uint32_t id, uint32_t total, int lane) {
+  if (!out.later) return false;
+  const uint32_t passes = (total + kDealPass - 1) / kDealPass;
+  unsigned long long at = 0;
+  if (lane == 0) at = atomicAdd(&out.count[3], (unsigned long long)passes);
+  at = __shfl_sync(0xffffffffu, at, 0);
+  const bool fits = at + passes <= out.laterCap;
+  for (uint32_t p = (uint32_t)lane; p < passes; p += 32u)
+    if (at + p < out.laterCap) out.later[at + p] = make_uint2(id, !fits ? kNoPass : p + 1 == passes ? p | kLastPass : p);
+  return fits;
+}
+
+// The half-shell rows [qFirst, qEnd) of the 32 objects from warpBase on; all
+// passes, or (ONE) one that was left for later.
+template <int SCREEN, int REACH, int G, bool ONE>
+__device__ __forceinline__ void walkWarp(const WalkIn &in, const CandSink &out, WalkShared<G> &sh, uint2 *sCandW,
+                                         uint32_t &nBuf, int lane, int warpBase, int qFirst, int qEnd,
+                                         uint32_t onlyPass) {
+  const float4 *__restrict__ posf = in.posf;
+  const uint32_t *__restrict__ skeys = in.skeys, *__restrict__ rowStart = in.rowStart;
+  const uint16_t *__restrict__ cellOff = in.cellOff;
+  const GridDesc &g = in.g;
+  const float cutF = in.cutF;
   const int j = warpBase + lane;
-  const bool inRange = j < n;
+  const bool inRange = j < in.n;
   // the object's own reads, all issued before any of them is used
-  const uint32_t mySlot = inRange ? perm[j] : 0u;
+  const uint32_t mySlot = inRange ? in.perm[j] : 0u;
   const uint32_t key = inRange ? skeys[j] : 0u;
   const float4 me = inRange ? __ldg(&posf[j]) : make_float4(0.f, 0.f, 0.f, 0.f);
   const uint32_t myGrp = out.grp && inRange ? __ldg(&out.grp[j]) : kNoGroup;
-  const bool denseOn = cellOff && denseMin != 0xffffffffu && __ldg(denseCount) != 0u;
+  const bool denseOn = cellOff && in.denseMin != 0xffffffffu && __ldg(in.denseCount) != 0u;
   bool active = inRange && !recDeleted(me) && mySlot < out.haloStart;
   const uint32_t nx = (uint32_t)g.n[0], ny = (uint32_t)g.n[1], nz = (uint32_t)g.n[2];
   const int R = g.reach;
   const uint32_t row = key / nx;
   const int32_t ix = (int32_t)(key - row * nx);
   const uint32_t iz = row / ny, iy = row - iz * ny;
-  // objects of the dense bin (own cell >= denseMin objects) are scanned by k_pair_tiles
+  // objects of the dense bin (own cell >= in.denseMin objects) are scanned by k_pair_tiles
   if (active && denseOn) {
     uint32_t a, b;  // the own cell's objects (rows beyond 16-bit offsets: searched)
     rowWindow(row, (uint32_t)ix, (uint32_t)ix, nx, rowStart, cellOff, skeys, a, b);
-    if (b - a >= denseMin) active = false;
+    if (b - a >= in.denseMin) active = false;
   }
-  sOwn[warp][lane] = me;
-  if (out.grp) sGrp[warp][lane] = myGrp;
+  sh.own[lane] = me;
+  if (out.grp) sh.grp[lane] = myGrp;
   const bool perObject = REACH != 1 && SCREEN == LADDS_SCREEN_BUFFER && R >= 2;  // warp-uniform
   const float inv = (float)g.invCell;
   float fx = 0.f, fy = 0.f, fz = 0.f, reach2 = 0.f;
@@ -344,23 +388,22 @@ __global__ void __launch_bounds__(kScanCta) k_pair_walk(const uint32_t *__restri
     fz = __saturatef((me.z - ((float)g.boxMin[2] + (float)iz * cf)) * inv);
     reach2 = rc * rc;
   }
-  const int nq = REACH == 1 ? 5 : REACH == 2 ? 13 : rows.n >= 0 ? rows.n : (R + 1) + R * (2 * R + 1);
   const uint32_t pitch = cellOffPitch(nx);
   const uint16_t *const myOff = cellOff ? cellOff + (size_t)row * pitch : nullptr;
 #pragma unroll
-  for (int q0 = 0; q0 < nq; q0 += G) {
+  for (int q0 = qFirst; q0 < qEnd; q0 += G) {
     uint32_t lo[G], cnt[G];
 #pragma unroll
     for (int t = 0; t < G; ++t) {
       lo[t] = 0u;
       cnt[t] = 0u;
-      if (q0 + t >= nq) continue;  // warp-uniform
+      if (q0 + t >= qEnd) continue;  // warp-uniform
       int dz, dy, w;
       if constexpr (REACH > 0) {
         halfShellRowOf(q0 + t, REACH, dz, dy);
         w = REACH;
       } else {
-        halfRow(rows, q0 + t, R, g.cellSize * g.cellSize, reachR2, dz, dy, w);
+        halfRow(in.rows, q0 + t, R, g.cellSize * g.cellSize, in.reachR2, dz, dy, w);
       }
       const bool own = dz == 0 && dy == 0;
       int32_t lo32 = own ? ix : ix - w, hi32 = ix + w;
@@ -419,19 +462,24 @@ __global__ void __launch_bounds__(kScanCta) k_pair_walk(const uint32_t *__restri
     }
     const uint32_t total = __shfl_sync(0xffffffffu, inclT, 31);
     if (total == 0u) continue;  // warp-uniform
+    if (!ONE && total > kLaterItems && leaveForLater(out, (uint32_t)warpBase | (uint32_t)(q0 / G), total, lane))
+      continue;
+    // ONE: one pass, the last of its group to the end of the items
+    const uint32_t p0 = ONE ? (onlyPass & ~kLastPass) * kDealPass : 0u;
+    const uint32_t p1 = ONE && !(onlyPass & kLastPass) ? min(total, p0 + kDealPass) : total;
     __syncwarp();  // the group before has been read (and the own positions are staged)
     {
       uint32_t item = inclT - tot, rank = inclE - nonEmpty;
 #pragma unroll
       for (int t = 0; t < G; ++t) {
-        if (cnt[t]) sWin[warp][rank++] = make_uint2(lo[t] - item, (uint32_t)lane);
+        if (cnt[t]) sh.win[rank++] = make_uint2(lo[t] - item, (uint32_t)lane);
         item += cnt[t];
       }
     }
-    for (uint32_t pass = 0; pass < total; pass += kDealPass) {  // warp-uniform
+    for (uint32_t pass = p0; pass < p1; pass += kDealPass) {  // warp-uniform
       const uint32_t end = min(total - pass, kDealPass);
-      if (pass) __syncwarp();  // the pass before has been read
-      sMask[warp][lane] = 0u;
+      if (pass != p0) __syncwarp();  // the pass before has been read
+      sh.mask[lane] = 0u;
       __syncwarp();
       // marks of the windows that start inside the pass; windows started before it
       uint32_t before = 0, item = inclT - tot;
@@ -441,34 +489,47 @@ __global__ void __launch_bounds__(kScanCta) k_pair_walk(const uint32_t *__restri
           if (item < pass)
             ++before;
           else if (item - pass < kDealPass)
-            atomicOr(&sMask[warp][(item - pass) >> 5], 1u << ((item - pass) & 31u));
+            atomicOr(&sh.mask[(item - pass) >> 5], 1u << ((item - pass) & 31u));
         }
         item += cnt[t];
       }
       uint32_t started = pass ? __reduce_add_sync(0xffffffffu, before) : 0u;
       __syncwarp();
       for (uint32_t base = 0; base < end; base += 32u) {  // warp-uniform
-        const uint32_t mask = sMask[warp][base >> 5];
+        const uint32_t mask = sh.mask[base >> 5];
         const uint32_t it = base + (uint32_t)lane;
         const uint32_t rank = started + (uint32_t)__popc(mask & (0xffffffffu >> (31 - lane))) - 1u;
         started += (uint32_t)__popc(mask);
         bool keep = false;
         uint32_t jj = 0u, k = 0u;
         if (it < end) {
-          const uint2 wv = sWin[warp][rank];
+          const uint2 wv = sh.win[rank];
           const uint32_t owner = wv.y;
           k = pass + it + wv.x;
           jj = (uint32_t)warpBase + owner;
-          keep = prefilterPass(sOwn[warp][owner], __ldg(&posf[k]), cutF);
+          keep = prefilterPass(sh.own[owner], __ldg(&posf[k]), cutF);
           if (keep && out.grp) {  // fragments of one breakup never yield a record
-            const uint32_t gr = sGrp[warp][owner];
+            const uint32_t gr = sh.grp[owner];
             keep = gr == kNoGroup || gr != __ldg(&out.grp[k]);
           }
         }
-        warpAppend<SCREEN>(keep, jj, k, lane, sCand[warp], nBuf, out);
+        warpAppend<SCREEN>(keep, jj, k, lane, sCandW, nBuf, out);
       }
     }
   }
+}
+
+template <int SCREEN, int REACH>
+__global__ void __launch_bounds__(kScanCta) k_pair_walk(const WalkIn in, const CandSink out) {
+  constexpr int W = kScanCta / 32, G = walkGroup(REACH);
+  __shared__ uint2 sCand[W][kWarpCand];
+  __shared__ WalkShared<G> sh[W];
+  const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+  uint32_t nBuf = 0;  // pairs in this warp's buffer (warp-uniform)
+  const int R = in.g.reach;
+  const int nq = REACH == 1 ? 5 : REACH == 2 ? 13 : in.rows.n >= 0 ? in.rows.n : (R + 1) + R * (2 * R + 1);
+  walkWarp<SCREEN, REACH, G, false>(in, out, sh[warp], sCand[warp], nBuf, lane, blockIdx.x * kScanCta + warp * 32, 0,
+                                    nq, 0u);
   warpFlush(lane, sCand[warp], nBuf, out);
 }
 
@@ -481,49 +542,51 @@ __global__ void __launch_bounds__(kScanCta) k_pair_walk(const uint32_t *__restri
 // source lane (the entry's chunk of the cell's objects, 32 at a time) tests
 // every staged object: no per-pair address work, no divergence but the
 // survivors', no dependent global load inside the loop.  Own-row objects are
-// paired with later objects only.  Pairs of one breakup group are skipped: a
-// staged block and a source batch that both belong to one group entirely are
-// not tested at all (a breakup's fragments start at one point, in one cell).
+// paired with later objects only.  Pairs of one breakup group are skipped: where
+// half of a batch's sources belong to one group, the staged objects of that
+// group are tested against the other sources only (a breakup's fragments start
+// at one point, in one cell, so nearly all pairs of a crowded cell are such).
 // Same pre-filter and candidate output as k_pair_walk, which skips these
-// objects as sources.
+// objects as sources.  Afterwards the warps take the dealing passes that the
+// walk left.
+constexpr int kTileCtasPerSm = 7;     // by its 28 KB of shared memory
 constexpr uint32_t kTileStage = 256;  // staged neighbour objects per warp and pass
 
 template <int SCREEN>
-__global__ void __launch_bounds__(kScanCta) k_pair_tiles(const uint32_t *__restrict__ denseCells,
-                                                         const uint32_t *__restrict__ denseChunk,
-                                                         const uint32_t *__restrict__ denseCount, uint32_t denseCap,
-                                                         const uint32_t *__restrict__ perm,
-                                                         const float4 *__restrict__ posf,
-                                                         const uint32_t *__restrict__ skeys,
-                                                         const uint32_t *__restrict__ rowStart,
-                                                         const uint16_t *__restrict__ cellOff, GridDesc g,
-                                                         float cutF, double reachR2, const CandSink out) {
+__global__ void __launch_bounds__(kScanCta, 8) k_pair_tiles(const uint32_t *__restrict__ denseCells,
+                                                         const uint32_t *__restrict__ denseChunk, uint32_t denseCap,
+                                                         const WalkIn in, const CandSink out) {
   __shared__ uint2 sCand[kScanCta / 32][kWarpCand];
   __shared__ float4 sNb[kScanCta / 32][kTileStage];
   __shared__ uint32_t sK[kScanCta / 32][kTileStage];
   __shared__ uint32_t sG[kScanCta / 32][kTileStage];
   const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+  const float4 *__restrict__ posf = in.posf;
+  const GridDesc &g = in.g;
+  const float cutF = in.cutF;
   uint32_t nBuf = 0;  // pairs in this warp's buffer (warp-uniform)
-  const uint32_t nDense = min(*denseCount, denseCap);
+  const uint32_t nDense = min(*in.denseCount, denseCap);
   const int32_t nx = g.n[0], ny = g.n[1], nz = g.n[2], R = g.reach;
   const int nq = (R + 1) + R * (2 * R + 1);  // half-shell rows (<= 32 for R <= 3)
   const uint32_t *grp = out.grp;
-  // entries are handed out one at a time (out.count[2], zeroed with the list
-  // lengths before the scan), so a warp that drew a long entry -- a crowded
-  // cell's -- does not hold back entries that were dealt to it in advance
-  unsigned long long *next = out.count + 2;
-  for (;;) {
-    if (nDense == 0u) break;  // an empty bin (the common case) costs no atomics
+  // entries are handed out one at a time (cursors zeroed before the scan), so a
+  // warp that drew a long entry -- a crowded cell's -- does not hold back
+  // entries that were dealt to it in advance
+  auto draw = [&](int cursor, uint32_t have) -> uint32_t {
+    if (have == 0u) return 0u;  // nothing listed (the common case) costs no atomics
     uint32_t q = 0;
-    if (lane == 0) q = (uint32_t)min(atomicAdd(next, 1ull), (unsigned long long)nDense);
-    q = __shfl_sync(0xffffffffu, q, 0);
+    if (lane == 0) q = (uint32_t)min(atomicAdd(&out.count[cursor], 1ull), (unsigned long long)have);
+    return __shfl_sync(0xffffffffu, q, 0);
+  };
+  for (;;) {
+    const uint32_t q = draw(2, nDense);
     if (q >= nDense) break;
     const uint32_t key = denseCells[q];
     const uint32_t r = key / (uint32_t)nx;
     const int32_t ix = (int32_t)(key - r * (uint32_t)nx), iy = (int32_t)(r % (uint32_t)ny),
                   iz = (int32_t)(r / (uint32_t)ny);
     uint32_t c0, c1;  // the cell's objects
-    rowWindow(r, (uint32_t)ix, (uint32_t)ix, (uint32_t)nx, rowStart, cellOff, skeys, c0, c1);
+    rowWindow(r, (uint32_t)ix, (uint32_t)ix, (uint32_t)nx, in.rowStart, in.cellOff, in.skeys, c0, c1);
     const uint32_t cw = denseChunk[q];  // chunk | part << 24 | log2(parts) << 28
     const uint32_t part = (cw >> 24) & 15u, partsLog = cw >> 28;
     const uint32_t s0 = c0 + (cw & 0xffffffu) * kTileChunk, s1 = min(c1, s0 + kTileChunk);  // this entry's sources
@@ -533,12 +596,12 @@ __global__ void __launch_bounds__(kScanCta) k_pair_tiles(const uint32_t *__restr
       int dz, dy;
       halfShellRowOf(lane, R, dz, dy);
       const int32_t jz = iz + dz, jy = iy + dy;
-      const int w = rowHalfWidth(dy, dz, R, g.cellSize * g.cellSize, reachR2);
+      const int w = rowHalfWidth(dy, dz, R, g.cellSize * g.cellSize, in.reachR2);
       const uint32_t xlo = lane == 0 ? (uint32_t)ix : (uint32_t)max(ix - w, 0);
       const uint32_t xhi = (uint32_t)min(ix + w, nx - 1);
       if (w >= 0 && jz < nz && jy >= 0 && jy < ny)
-        rowWindow((uint32_t)jz * (uint32_t)ny + (uint32_t)jy, xlo, xhi, (uint32_t)nx, rowStart, cellOff, skeys, lo,
-                  hi);
+        rowWindow((uint32_t)jz * (uint32_t)ny + (uint32_t)jy, xlo, xhi, (uint32_t)nx, in.rowStart, in.cellOff,
+                  in.skeys, lo, hi);
     }
     const uint32_t cnt = hi - lo;
     uint32_t incl = cnt;
@@ -552,46 +615,83 @@ __global__ void __launch_bounds__(kScanCta) k_pair_tiles(const uint32_t *__restr
     const uint32_t ownEnd = __shfl_sync(0xffffffffu, incl, 0);  // staged items [0, ownEnd) are own-row objects
     for (uint32_t stBase = part * kTileStage; stBase < total; stBase += kTileStage << partsLog) {  // this part's blocks
       const uint32_t m = min(kTileStage, total - stBase);
-      bool oneGroup = grp != nullptr;  // every staged object in one breakup group (warp-uniform after the loop)
-      uint32_t g0 = kNoGroup;
       for (uint32_t ib = 0; ib < m; ib += 32u) {  // stage items stBase + i (warp-uniform loop)
         const uint32_t i = ib + (uint32_t)lane, item = stBase + i;
         // row of the item: the last lane whose excl <= item (empty rows share the next excl)
         const int owner = windowOwner(excl, item);
         const uint32_t oLo = __shfl_sync(0xffffffffu, lo, owner), oEx = __shfl_sync(0xffffffffu, excl, owner);
-        uint32_t gi = kNoGroup;
         if (i < m) {
           const uint32_t k = oLo + (item - oEx);
           sNb[warp][i] = __ldg(&posf[k]);
           sK[warp][i] = k;
-          if (grp) {
-            gi = __ldg(&grp[k]);
-            sG[warp][i] = gi;
-          }
-        }
-        if (grp) {
-          if (ib == 0) g0 = __shfl_sync(0xffffffffu, gi, 0);
-          oneGroup = oneGroup && __all_sync(0xffffffffu, i >= m || (gi == g0 && gi != kNoGroup));
+          if (grp) sG[warp][i] = __ldg(&grp[k]);
         }
       }
       __syncwarp();
       for (uint32_t sBase = s0; sBase < s1; sBase += 32u) {
         const uint32_t si = sBase + (uint32_t)lane;
         const float4 mf = si < s1 ? __ldg(&posf[si]) : make_float4(0.f, 0.f, 0.f, 0.f);
-        const bool src = si < s1 && !recDeleted(mf) && perm[si] < out.haloStart;
-        const uint32_t gs = grp && si < s1 ? __ldg(&grp[si]) : kNoGroup;
-        // the batch and the staged block all in the same group: no pair can yield a record
-        if (oneGroup && __all_sync(0xffffffffu, !src || gs == g0)) continue;
-        for (uint32_t u = 0; u < m; ++u) {  // warp-uniform
+        const bool src = si < s1 && !recDeleted(mf) && in.perm[si] < out.haloStart;
+        const uint32_t gs = grp && src ? __ldg(&grp[si]) : kNoGroup;
+        auto test = [&](uint32_t u) {  // every source against staged object u
           const float4 qq = sNb[warp][u];
           const uint32_t k = sK[warp][u];
           const bool sameGroup = grp && gs != kNoGroup && gs == sG[warp][u];
           const bool pass = src && !sameGroup && prefilterPass(mf, qq, cutF) &&
                             !(stBase + u < ownEnd && k <= si);  // own row: later objects only
           warpAppend<SCREEN>(pass, si, k, lane, sCand[warp], nBuf, out);
+        };
+        // the batch's most common breakup group, if half of its sources belong to one
+        uint32_t common = kNoGroup;
+        if (grp) {
+          const uint32_t peers = __match_any_sync(0xffffffffu, gs);
+          const int sources = __popc(__ballot_sync(0xffffffffu, src));
+          const uint32_t half = __ballot_sync(0xffffffffu, gs != kNoGroup && 2 * __popc(peers) >= sources);
+          if (half) common = __shfl_sync(0xffffffffu, gs, __ffs(half) - 1);
+        }
+        if (common == kNoGroup) {
+          for (uint32_t u = 0; u < m; ++u) test(u);  // warp-uniform
+          continue;
+        }
+        // all sources against the staged objects of other groups; the few
+        // sources of other groups, one at a time, against those of this one (32
+        // of them per round): the pairs inside the group are not touched
+        const uint32_t others = __ballot_sync(0xffffffffu, src && gs != common);
+        for (uint32_t ib = 0; ib < m; ib += 32u) {
+          const uint32_t i = ib + (uint32_t)lane;
+          const bool inGroup = i < m && sG[warp][i] == common;
+          for (uint32_t left = __ballot_sync(0xffffffffu, i < m && !inGroup); left; left &= left - 1u)
+            test(ib + (uint32_t)__ffs(left) - 1u);  // warp-uniform
+          if (!others || !__any_sync(0xffffffffu, inGroup)) continue;
+          const float4 qq = i < m ? sNb[warp][i] : make_float4(0.f, 0.f, 0.f, 0.f);
+          const uint32_t k = i < m ? sK[warp][i] : 0u;
+          for (uint32_t left = others; left; left &= left - 1u) {
+            const int o = __ffs(left) - 1;
+            const float4 sf = make_float4(__shfl_sync(0xffffffffu, mf.x, o), __shfl_sync(0xffffffffu, mf.y, o),
+                                          __shfl_sync(0xffffffffu, mf.z, o), __shfl_sync(0xffffffffu, mf.w, o));
+            const uint32_t so = sBase + (uint32_t)o;
+            const bool pass = inGroup && prefilterPass(sf, qq, cutF) && !(stBase + i < ownEnd && k <= so);
+            warpAppend<SCREEN>(pass, so, k, lane, sCand[warp], nBuf, out);
+          }
         }
       }
       __syncwarp();
+    }
+  }
+  // dealing passes of the walk's crowded warps (their lists in the staging area)
+  if (out.later) {
+    static_assert(sizeof(WalkShared<7>) <= sizeof(sNb[0]), "the walk's lists fit the staging area");
+    auto &sh = *reinterpret_cast<WalkShared<7> *>(sNb[warp]);
+    const uint32_t have = (uint32_t)min(out.count[3], (unsigned long long)out.laterCap);
+    for (;;) {
+      const uint32_t q = draw(4, have);
+      if (q >= have) break;
+      const uint2 e = out.later[q];
+      if (e.y == kNoPass) continue;
+      const int q0 = (int)(e.x & 31u) * in.groupRows;
+      __syncwarp();  // the lists of the entry before have been read
+      walkWarp<SCREEN, 0, 7, true>(in, out, sh, sCand[warp], nBuf, lane, (int)(e.x & ~31u), q0,
+                                   min(q0 + in.groupRows, in.rows.n), e.y);
     }
   }
   warpFlush(lane, sCand[warp], nBuf, out);

@@ -132,3 +132,40 @@ def test_pair_walk_for_every_reach(capi, oracle, cell, screen):
         left = ctx.conjunctions(1.0)
         keep = ~np.isin(ref["slotA"], gone) & ~np.isin(ref["slotB"], gone)
         assert records_equal(left, ref[keep]), describe_diff(left, ref[keep])
+
+
+@pytest.mark.parametrize("screen", [0, 1])
+@pytest.mark.parametrize("cell", [20.0, 10.0])
+def test_crowded_cells_beside_sparse_ones(capi, oracle, cell, screen):
+    """Fragment clouds in a few cells: source batches of one group, of two, and
+    of less than half of any; sparse cells beside them whose windows hold enough
+    items for the walk to leave passes to the tiles; rows sorted by a CTA."""
+    rng = np.random.default_rng(23)
+    lo, hi = np.array([7000.0, -50.0, -50.0]), np.array([7100.0, 50.0, 50.0])
+    parts = [(2600, [7030.0, 10.0, 10.0], 3.0, 1), (1500, [7045.0, 10.0, 10.0], 6.0, 2),
+             (400, [7045.0, 12.0, 10.0], 6.0, 3), (30, [7030.0, 10.0, 10.0], 3.0, None)]
+    r = np.concatenate([rng.normal(c, s, (m, 3)) for m, c, s, _ in parts] + [rng.uniform(lo, hi, (900, 3))])
+    n = len(r)
+    pop = cloud(n, 5, lo, hi)
+    pop["x"], pop["y"], pop["z"] = r[:, 0].copy(), r[:, 1].copy(), r[:, 2].copy()
+    none = np.uint64(0xFFFFFFFFFFFFFFFF)
+    pop["parent"] = np.concatenate([np.full(m, none if g is None else np.uint64(g)) for m, _, _, g in parts]
+                                   + [np.full(900, none)])
+    pop["parent"][-60:] = 1  # fragments of the first cloud in sparse cells
+    order = rng.permutation(n)
+    pop = {k: (v if k == "id" else v[order]) for k, v in pop.items()}
+    kw = dict(cutoff=20.0, cellSize=cell, boxMin=list(lo), boxMax=list(hi), scanScreen=screen,
+              conjunctionThreshold=0.5, evasionCutoff=0.1)
+    with capi.Context(capi.default_config(**kw)) as ctx:
+        ctx.upload(pop)
+        recs = ctx.conjunctions(0.2)
+    p = oracle.scan_params(cutoff=20.0, dt=0.2, evasion_cutoff=0.1, conjunction_threshold=0.5)
+    ref = oracle.scan_bruteforce(to_oracle(oracle, capi_pop(pop)), p)
+    assert len(ref) > 200
+    assert records_equal(recs, ref), describe_diff(recs, ref)
+
+
+def capi_pop(pop):
+    from ladds_b200.population import as_population
+
+    return as_population(pop)
