@@ -497,6 +497,99 @@ __global__ void __launch_bounds__(kRowSortThreads) k_bucket_sort_rows(
 }
 
 
+// The same result for short rows: one warp per kBatchRows consecutive rows,
+// whose records are contiguous and staged in shared memory together.  Every
+// lane ranks one object by counting the smaller records of its row, so the
+// batch's objects are ranked side by side however they fall into rows, with no
+// counters to clear, no atomics and two warp barriers; then, row by row, lane l
+// adds up the offsets of its eight cells 8 l .. 8 l + 7 over the row's objects in
+// one 64-bit word of byte counters (rows of up to 255 objects: longer ones are
+// sorted by k_bucket_sort_large) and stores them as one 16-byte piece of the
+// row's cell-offset table.
+constexpr int kBatchRows = 8;
+constexpr uint32_t kBatchObjects = 512;  // staged per warp; batches of more objects go row by row
+__global__ void __launch_bounds__(kRowSortThreads) k_bucket_sort_batches(
+    const uint32_t *__restrict__ rowStart, uint32_t nRows, uint32_t nx, const unsigned long long *__restrict__ rec,
+    const CellOrderOut out, uint32_t *__restrict__ longRows, uint32_t *__restrict__ longCount,
+    uint16_t *__restrict__ cellOff, DenseBin dense) {
+  __shared__ unsigned long long sRec[kRowSortThreads / 32][kBatchObjects];
+  const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+  unsigned long long *sv = sRec[warp];
+  const uint32_t pitch = cellOffPitch(nx);
+  const uint32_t warpId = (blockIdx.x * blockDim.x + threadIdx.x) >> 5;
+  const uint32_t nWarps = (gridDim.x * blockDim.x) >> 5;
+  for (uint32_t r0 = warpId * kBatchRows; r0 < nRows; r0 += nWarps * kBatchRows) {
+    const uint32_t rows = min((uint32_t)kBatchRows, nRows - r0);
+    const uint32_t st = rowStart[min(r0 + min((uint32_t)lane, rows), nRows)];  // lane i: start of row i, lane rows: the end
+    const uint32_t first = __shfl_sync(0xffffffffu, st, 0), end = __shfl_sync(0xffffffffu, st, (int)rows);
+    if (first == end) continue;
+    // whole batch at once, or row by row
+    const uint32_t step = end - first <= kBatchObjects ? rows : 1u;
+    for (uint32_t i0 = 0; i0 < rows; i0 += step) {  // warp-uniform
+      const uint32_t s0 = __shfl_sync(0xffffffffu, st, (int)i0), s1 = __shfl_sync(0xffffffffu, st, (int)(i0 + step));
+      const uint32_t S = s1 - s0;
+      if (S == 0u) continue;
+      if (step == 1u && S > 255u) {
+        if (lane == 0) longRows[atomicAdd(longCount, 1u)] = r0 + i0;
+        continue;
+      }
+      __syncwarp();
+      for (uint32_t e = (uint32_t)lane; e < S; e += 32u) sv[e] = rec[s0 + e];
+      __syncwarp();
+      for (uint32_t eb = 0; eb < S; eb += 32u) {  // warp-uniform
+        const uint32_t e = eb + (uint32_t)lane, at = s0 + min(e, S - 1u);
+        // the object's row: the last of the batch that starts at or before it
+        uint32_t i = i0;
+#pragma unroll
+        for (int q = 1; q < kBatchRows; ++q) {
+          const uint32_t b = __shfl_sync(0xffffffffu, st, q);
+          if ((uint32_t)q < i0 + step && (uint32_t)q > i0 && b <= at) i = (uint32_t)q;
+        }
+        const uint32_t a = __shfl_sync(0xffffffffu, st, (int)i) - s0, b = __shfl_sync(0xffffffffu, st, (int)i + 1) - s0;
+        if (e < S && b - a <= 255u) {
+          const unsigned long long mine = sv[e];
+          uint32_t rank = 0;
+          for (uint32_t q = a; q < b; ++q) rank += sv[q] < mine ? 1u : 0u;
+          emitCellOrder(out, s0 + a + rank, (r0 + i) * nx + (uint32_t)(mine >> 32), (uint32_t)mine);
+        }
+      }
+      for (uint32_t i = i0; i < i0 + step; ++i) {  // warp-uniform
+        const uint32_t a = __shfl_sync(0xffffffffu, st, (int)i) - s0, b = __shfl_sync(0xffffffffu, st, (int)i + 1) - s0;
+        if (a == b) continue;
+        if (b - a > 255u) {
+          if (lane == 0) longRows[atomicAdd(longCount, 1u)] = r0 + i;
+          continue;
+        }
+        if (!cellOff) continue;
+        for (uint32_t c0 = 0; c0 <= nx; c0 += 256u) {
+          const int mineC = (int)c0 + 8 * lane;
+          unsigned long long off = 0ull;  // byte q: objects in cells < mineC + q
+          for (uint32_t q = a; q < b; ++q) {
+            const int d = (int)(uint32_t)(sv[q] >> 32) - mineC;
+            off += d < 0 ? 0x0101010101010101ull : d < 7 ? 0x0101010101010101ull << (8 * (d + 1)) : 0ull;
+          }
+          uint32_t v[9];
+#pragma unroll
+          for (int q = 0; q < 8; ++q) v[q] = (uint32_t)(off >> (8 * q)) & 0xffu;
+          if ((uint32_t)mineC < pitch)
+            *reinterpret_cast<uint4 *>(cellOff + (size_t)(r0 + i) * pitch + mineC) =
+                make_uint4(v[0] | (v[1] << 16), v[2] | (v[3] << 16), v[4] | (v[5] << 16), v[6] | (v[7] << 16));
+          if (dense.cells && b - a >= dense.minCount) {
+            v[8] = __shfl_down_sync(0xffffffffu, v[0], 1);
+            if (lane == 31) {  // objects in cells < mineC + 8
+              v[8] = 0;
+              for (uint32_t q = a; q < b; ++q) v[8] += (int)(uint32_t)(sv[q] >> 32) < mineC + 8 ? 1u : 0u;
+            }
+#pragma unroll
+            for (int q = 0; q < 8; ++q)
+              if (v[q + 1] - v[q] >= dense.minCount) denseAppend(dense, (r0 + i) * nx + (uint32_t)(mineC + q), v[q + 1] - v[q]);
+          }
+        }
+      }
+    }
+  }
+}
+
 __global__ void __launch_bounds__(kBucketThreads) k_bucket_sort_large(
     const uint32_t *__restrict__ rowStart, uint32_t nx, unsigned long long *__restrict__ rec, const CellOrderOut out,
     const uint32_t *__restrict__ longRows, const uint32_t *__restrict__ longCount,

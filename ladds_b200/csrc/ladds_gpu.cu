@@ -651,7 +651,16 @@ void enqueueSort(ladds_gpu_ctx *c, cudaStream_t s) {
   const DenseBin dense = denseBin(c);
   const CellOrderOut out{c->sortedKeys, c->perm, c->scanRecs, c->posf, c->velf,
                          c->anyParent ? c->cur.parent : nullptr, c->grp};
-  if (nx <= (uint32_t)kRowCountMaxNx) {  // counting sort inside the rows
+  // Few objects per row: most rows are empty or hold one or two, and a warp per
+  // row waits out a chain of shared-memory steps for each.  Graph step by
+  // batches / by rows at 62,500 rows: 10,000 objects 16.1 / 22.6 us, 31,000 20.9 /
+  // 27.0, 62,000 26.8 / 30.9, 78,000 30.7 / 32.8, 94,000 34.2 / 33.6, 180,000 56 / 49.
+  if (nx <= (uint32_t)kRowCountMaxNx && 4 * c->n <= 5 * (size_t)nRows) {
+    const int batchBlocks = std::min(blocksFor(((size_t)nRows + kBatchRows - 1) / kBatchRows * 32, kRowSortThreads),
+                                     5 * c->evalBlocks / 2);
+    k_bucket_sort_batches<<<batchBlocks, kRowSortThreads, 0, s>>>(c->rowStart, nRows, nx, c->sortRec, out,
+                                                                  c->longRows, c->longCount, c->cellOff, dense);
+  } else if (nx <= (uint32_t)kRowCountMaxNx) {  // counting sort inside the rows
     // one resident wave (10 CTAs of 4 warps per SM); each warp pipelines its rows
     const int rowBlocks = std::min(blocksFor((size_t)nRows * 32, kRowSortThreads), 5 * c->evalBlocks / 2);
     k_bucket_sort_rows<<<rowBlocks, kRowSortThreads, rowSortSmem(nx), s>>>(

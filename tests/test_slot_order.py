@@ -169,3 +169,37 @@ def capi_pop(pop):
     from ladds_b200.population import as_population
 
     return as_population(pop)
+
+
+@pytest.mark.parametrize("n", [1, 31, 700, 9000])
+def test_sparse_rows_in_batches(capi, oracle, n):
+    """Fewer objects than rows: batches of rows sorted side by side, with rows of
+    254 to 257 objects (byte counters to 255), crowded cells, one batch of more
+    objects than it stages, and an empty last batch (rows not a multiple of 8)."""
+    nx, ny, nz = 300, 101, 99
+    lo, hi = np.zeros(3), np.array([nx, ny, nz], dtype=float)
+    rng = np.random.default_rng(n)
+    pop = cloud(n, 4, lo, hi)
+    if n >= 9000:
+        at = 0
+        for count, (y, z) in ((254, (10, 5)), (255, (30, 5)), (256, (50, 6)), (257, (70, 7)), (250, (2, 50)),
+                              (200, (3, 50)), (180, (4, 50))):
+            s = slice(at, at + count)
+            pop["x"][s] = rng.uniform(0, nx, count) if count != 255 else 40.0 + rng.uniform(0, 5, count)
+            pop["y"][s], pop["z"][s] = y + 0.5, z + rng.uniform(0.0, 1.0, count)
+            at += count
+    order = rng.permutation(n)
+    pop = {k: (v if k == "id" else v[order]) for k, v in pop.items()}
+    kw = dict(cutoff=0.9, cellSize=1.0, boxMin=list(lo), boxMax=list(hi), conjunctionThreshold=0.6, evasionCutoff=0.1)
+    with capi.Context(capi.default_config(**kw)) as ctx:
+        ctx.upload(pop)
+        recs = ctx.conjunctions(0.1)
+        keys, slots = ctx.cell_order()
+    ix, iy, iz = (np.clip(np.floor(pop[k]), 0, m - 1).astype(np.int64) for k, m in zip("xyz", (nx, ny, nz)))
+    want = (iz * ny + iy) * nx + ix
+    order = np.argsort(want, kind="stable")
+    assert np.array_equal(slots, order) and np.array_equal(keys, want[order])
+    p = oracle.scan_params(cutoff=0.9, dt=0.1, evasion_cutoff=0.1, conjunction_threshold=0.6)
+    ref = oracle.scan_bruteforce(to_oracle(oracle, capi_pop(pop)), p)
+    assert n < 9000 or len(ref) > 100
+    assert records_equal(recs, ref), describe_diff(recs, ref)
