@@ -14,6 +14,7 @@
 // Multi-iteration calls are captured once into a CUDA graph per (iterations,
 // iteration % k, current buffers) and replayed.
 #include <cuda_runtime.h>
+#include <omp.h>
 
 #include <algorithm>
 #include <cmath>
@@ -21,8 +22,10 @@
 #include <cstring>
 #include <map>
 #include <mutex>
+#include <set>
 #include <string>
 #include <tuple>
+#include <type_traits>
 #include <vector>
 
 #include "../../include/ladds_gpu.h"
@@ -78,9 +81,77 @@ constexpr size_t kHostChunkMin = (size_t)1 << 17;
 // dealing passes that a scan's walk can leave to k_pair_tiles (1024 pair tests each)
 constexpr uint32_t kLaterCap = 1u << 17;
 
+// results of a call in pinned host memory: enqueued behind the call's work, so
+// that one wait brings them (the words as they lie at dCount, a removal's count,
+// and the first records)
+constexpr size_t kMailRecords = 256;
+struct CallMail {
+  unsigned long long words[4];
+  ladds_pair recs[kMailRecords];
+};
+
+// Everything sized by the population: one allocation, cut up by layoutObjects.
+struct ObjectBuffers {
+  DevState cur{}, alt{}, alt2{}, snap{};  // the current state, the next two buffers of its ring, the roll-back copy
+  uint32_t *keys = nullptr, *arrival = nullptr;  // cell keys and row arrivals of the state to be scanned, slot order
+  ScanRec *scanRecs = nullptr;                   // its scan records, slot order
+  unsigned long long *sortRec = nullptr;         // (ix << 32 | slot) sort records of the bucket sort
+  uint32_t *sortedKeys = nullptr, *perm = nullptr;  // result of the last sort: cell keys, slots
+  float4 *posf = nullptr;                 // binary32 positions + rounding bound, cell order
+  float4 *velf = nullptr;                 // binary32 velocities + radius of the cell order
+  uint32_t *grp = nullptr;                // breakup group of the cell order (parent id, or kNoGroup)
+  uint32_t *scratchA = nullptr, *scratchB = nullptr, *scratchC = nullptr;
+  uint32_t *denseCells = nullptr, *denseChunk = nullptr;  // dense bin of the pair scan: cells, chunk of each entry
+  uint32_t denseCap = 0;
+  // second set of the sort's input and results: the propagation and the sort of
+  // a step write one set while the sort and the pair scan of the step before
+  // still read the other (with the second row tables of the context)
+  uint32_t *keysB = nullptr, *arrivalB = nullptr, *sortedKeysB = nullptr, *permB = nullptr, *grpB = nullptr,
+           *denseCellsB = nullptr, *denseChunkB = nullptr;
+  ScanRec *scanRecsB = nullptr;
+  float4 *posfB = nullptr, *velfB = nullptr;
+  double *homeX[2] = {};  // x arrays of the buffers that were current and next at allocation
+};
+
+// cuts the buffers of `cap` objects out of base (null: only counts); returns the bytes
+size_t layoutObjects(ObjectBuffers &o, size_t cap, char *base) {
+  size_t at = 0;
+  auto take = [&](auto *&p, size_t count) {
+    p = base ? reinterpret_cast<std::remove_reference_t<decltype(p)>>(base + at) : nullptr;
+    at += (count * sizeof(*p) + 255) & ~(size_t)255;
+  };
+  // x .. vz of a state follow one another at one distance: a copy of all six is
+  // one two-dimensional copy
+  DevState shared{};
+  take(shared.aom, cap);
+  take(shared.bc, cap);
+  take(shared.radius, cap);
+  take(shared.id, cap);
+  take(shared.parent, cap);
+  take(shared.tag, cap);
+  for (DevState *d : {&o.cur, &o.alt, &o.alt2, &o.snap}) {
+    *d = shared;
+    for (double **q : {&d->x, &d->y, &d->z, &d->vx, &d->vy, &d->vz}) take(*q, cap);
+  }
+  for (uint32_t **q : {&o.keys, &o.keysB, &o.arrival, &o.arrivalB, &o.scratchA, &o.scratchB, &o.scratchC, &o.perm,
+                       &o.permB, &o.sortedKeys, &o.sortedKeysB, &o.grp, &o.grpB})
+    take(*q, cap + 1);
+  for (float4 **q : {&o.posf, &o.posfB, &o.velf, &o.velfB}) take(*q, cap);
+  take(o.scanRecs, cap);
+  take(o.scanRecsB, cap);
+  take(o.sortRec, cap);
+  // every listed cell holds >= kDenseCell objects and adds one entry per kTileChunk of them and part of
+  // its staged side (up to 2^kTilePartsLogMax parts, for cells of >= 64 * 4^kTilePartsLogMax objects)
+  o.denseCap = (uint32_t)(cap / kDenseCell + cap / kTileChunk * (1u << kTilePartsLogMax) + 1);
+  for (uint32_t **q : {&o.denseCells, &o.denseCellsB, &o.denseChunk, &o.denseChunkB}) take(*q, o.denseCap);
+  o.homeX[0] = o.cur.x;
+  o.homeX[1] = o.alt.x;
+  return at;
+}
+
 }  // namespace
 
-struct ladds_gpu_ctx {
+struct ladds_gpu_ctx : ObjectBuffers {
   ladds_gpu_config cfg{};
   GridDesc grid{};
   PropConsts pc{};
@@ -97,22 +168,18 @@ struct ladds_gpu_ctx {
   std::vector<ladds_pair> pending;  // records of a ladds_gpu_step_host call whose buffer was too small
   int64_t *dIterBase = nullptr;  // first iteration of the chunk being run (device)
   size_t n = 0, cap = 0;
-  DevState cur{}, alt{}, alt2{}, snap{};  // the current state, the next two buffers of its ring, the roll-back copy
-  uint32_t *keys = nullptr, *arrival = nullptr;     // cell keys and row arrivals of the state to be scanned, slot order
-  ScanRec *scanRecs = nullptr;                      // its scan records, slot order
-  unsigned long long *sortRec = nullptr;  // (ix << 32 | slot) sort records of the bucket sort
+  char *objects = nullptr;  // the allocation behind the object buffers
+  char *tables = nullptr;   // the allocation behind the row tables
+  char *words = nullptr;    // the allocation behind the counters and small tables
+  CallMail *mail = nullptr;
   uint32_t *rowCounts = nullptr;          // objects per row; all zero but between a propagation and its sort
   uint32_t *longRows = nullptr, *longCount = nullptr;  // rows with more than 256 objects
   uint16_t *cellOff = nullptr;            // per row: offset of every cell inside the row (cellOffPitch entries)
   uint32_t *scanWs = nullptr;             // block sums of the exclusive scans
-  uint32_t *sortedKeys = nullptr, *perm = nullptr;  // result of the last sort: cell keys, slots
-  float4 *posf = nullptr;                 // binary32 positions + rounding bound, cell order
-  float4 *velf = nullptr;                 // binary32 velocities + radius of the cell order
-  uint32_t *grp = nullptr;                // breakup group of the cell order (parent id, or kNoGroup)
+  size_t scanWsWords = 0;
   bool anyParent = false;                 // some object has a parent id: the scan writes and reads grp
   uint32_t *rowStart = nullptr;
   uint32_t nRows = 0;
-  uint32_t *scratchA = nullptr, *scratchB = nullptr, *scratchC = nullptr;
   ladds_pair *dPairs = nullptr;
   size_t pairCap = 0;
   unsigned long long *dCount = nullptr;
@@ -134,27 +201,21 @@ struct ladds_gpu_ctx {
   std::vector<cudaEvent_t> eventPool;
   ladds_phase_times times{};
   cudaEvent_t callStart = nullptr, callEnd = nullptr;
-  std::map<std::tuple<int, int, int, size_t, size_t>, cudaGraphExec_t> graphs;
+  using GraphKey = std::tuple<int, int, int, size_t, size_t>;
+  std::map<GraphKey, cudaGraphExec_t> graphs;
+  std::set<GraphKey> seenChunks;  // chunks that have run once, without a graph
   std::string err;
-  double *homeX[2] = {};  // x arrays of the buffers that were current and next at allocation
   ladds_object *dObj = nullptr;  // staging of ladds_gpu_functor_pairs (2 x objCap)
   size_t objCap = 0;
   int evalBlocks = 592;     // grid of the candidate-evaluation kernel (4 per SM)
   float cutF = 0.f;         // binary32 pre-filter radius: cutoff * (1 + nearRel), rounded up
   int chunkSteps = kMaxEphSteps;  // iterations per ephemeris chunk / captured graph (autotuned)
-  uint32_t *denseCells = nullptr, *denseCount = nullptr;  // dense bin of the pair scan (cells >= kDenseCell)
-  uint32_t *denseChunk = nullptr, *denseChunkB = nullptr;  // chunk index of each dense-bin entry
+  uint32_t *denseCount = nullptr;  // entries of the dense bin
   uint32_t haloStart = 0xffffffffu;  // objects with slot >= haloStart: pair-scan targets only
-  uint32_t denseCap = 0;
-  // second set of the sort's input and results: the propagation and the sort of
-  // a step write one set while the sort and the pair scan of the step before
-  // still read the other
-  uint32_t *rowStartB = nullptr, *sortedKeysB = nullptr, *permB = nullptr, *denseCellsB = nullptr,
-           *denseCountB = nullptr, *grpB = nullptr, *keysB = nullptr, *arrivalB = nullptr, *rowCountsB = nullptr;
-  ScanRec *scanRecsB = nullptr;
+  // the row tables and counters of the second set
+  uint32_t *rowStartB = nullptr, *rowCountsB = nullptr, *denseCountB = nullptr;
   unsigned long long *dCandCountB = nullptr;
-  float4 *posfB = nullptr, *velfB = nullptr;
-  uint16_t *cellOffB = nullptr;
+  uint16_t *cellOffB = nullptr, *cellOffBase = nullptr;
   int sortParity = 0;
   struct Adjoint {          // buffers of the adjoint pair batch (ladds_gpu_adjoint_*)
     size_t nPairs = 0;
@@ -181,40 +242,6 @@ int fail(ladds_gpu_ctx *c, int code, const std::string &msg) {
     if (e_ != cudaSuccess)                                                                          \
       return fail(c, LADDS_ERR_CUDA, std::string(#call) + ": " + cudaGetErrorString(e_));           \
   } while (0)
-
-// frees a state buffer; the arrays that a context's buffers share only when
-// withShared
-void freeState(DevState &s, bool withShared) {
-  void *own[] = {s.x, s.y, s.z, s.vx, s.vy, s.vz};
-  for (void *p : own)
-    if (p) cudaFree(p);
-  if (withShared) {
-    void *shared[] = {s.aom, s.bc, s.tag, s.radius, s.id, s.parent};
-    for (void *p : shared)
-      if (p) cudaFree(p);
-  }
-  s = DevState{};
-}
-
-// allocates a state buffer; the shared arrays are taken from `shared` (or
-// allocated when it is null)
-cudaError_t allocState(DevState &s, size_t cap, const DevState *shared) {
-  s = shared ? *shared : DevState{};
-  double **d[] = {&s.x, &s.y, &s.z, &s.vx, &s.vy, &s.vz};
-  for (double **p : d) *p = nullptr;
-  for (double **p : d) {
-    cudaError_t e = cudaMalloc(p, cap * sizeof(double));
-    if (e != cudaSuccess) return e;
-  }
-  if (shared) return cudaSuccess;
-  cudaError_t e = cudaMalloc(&s.aom, cap * sizeof(double));
-  if (e == cudaSuccess) e = cudaMalloc(&s.bc, cap * sizeof(double));
-  if (e == cudaSuccess) e = cudaMalloc(&s.tag, cap * sizeof(uint32_t));
-  if (e == cudaSuccess) e = cudaMalloc(&s.radius, cap * sizeof(double));
-  if (e == cudaSuccess) e = cudaMalloc(&s.id, cap * sizeof(uint64_t));
-  if (e == cudaSuccess) e = cudaMalloc(&s.parent, cap * sizeof(uint64_t));
-  return e;
-}
 
 // positions and velocities only
 cudaError_t copyDynamic(const DevState &src, const DevState &dst, size_t n, cudaStream_t st) {
@@ -248,25 +275,25 @@ cudaError_t copyState(const DevState &src, const DevState &dst, size_t n, cudaSt
 void dropGraphs(ladds_gpu_ctx *c) {
   for (auto &kv : c->graphs) cudaGraphExecDestroy(kv.second);
   c->graphs.clear();
+  c->seenChunks.clear();
 }
 
 int ensureCandCapacity(ladds_gpu_ctx *c, size_t need);
 
-void freeBuffers(ladds_gpu_ctx *c) {
-  freeState(c->cur, true);
-  freeState(c->alt, false);
-  freeState(c->alt2, false);
-  freeState(c->snap, false);
-  void **ptrs[] = {(void **)&c->keys, (void **)&c->keysB, (void **)&c->arrival, (void **)&c->arrivalB,
-                   (void **)&c->scanRecs, (void **)&c->scanRecsB, (void **)&c->sortRec, (void **)&c->scratchA,
-                   (void **)&c->scratchB, (void **)&c->scratchC, (void **)&c->scanWs, (void **)&c->sortedKeys,
-                   (void **)&c->sortedKeysB, (void **)&c->perm, (void **)&c->permB, (void **)&c->posf,
-                   (void **)&c->posfB, (void **)&c->velf, (void **)&c->velfB, (void **)&c->grp, (void **)&c->grpB};
-  for (void **p : ptrs) {
-    if (*p) cudaFree(*p);
-    *p = nullptr;
+// block sums of the three-level exclusive scans (objects or rows, whichever is longer)
+bool ensureScanWorkspace(ladds_gpu_ctx *c, size_t objects) {
+  const size_t scanLen = std::max(objects + 1, (size_t)c->nRows + 1);
+  const size_t need = 4 * (scanLen / kScanBlock + 2) + 4 * kScanBlock;
+  if (c->scanWs && need <= c->scanWsWords) return true;
+  if (c->scanWs) cudaFree(c->scanWs);
+  c->scanWs = nullptr;
+  c->scanWsWords = 0;
+  if (cudaMalloc(&c->scanWs, need * sizeof(uint32_t)) != cudaSuccess) {
+    cudaGetLastError();
+    return false;
   }
-  c->cap = 0;
+  c->scanWsWords = need;
+  return true;
 }
 
 int ensureCapacity(ladds_gpu_ctx *c, size_t need) {
@@ -274,86 +301,31 @@ int ensureCapacity(ladds_gpu_ctx *c, size_t need) {
   if (need > kMaxObjects) return fail(c, LADDS_ERR_INVALID_ARG, "population exceeds 2^28 - 1 objects");
   size_t newCap = std::max<size_t>({need, c->cap + c->cap / 2, 4096});
   newCap = std::min(newCap, kMaxObjects);
-  DevState ncur, next[3] = {};  // alt, alt2, snap
-  cudaError_t e = allocState(ncur, newCap, nullptr);
-  for (DevState &d : next)
-    if (e == cudaSuccess) e = allocState(d, newCap, &ncur);
-  if (e != cudaSuccess) {
-    for (DevState &d : next) freeState(d, false);
-    freeState(ncur, true);
+  ObjectBuffers fresh;
+  const size_t bytes = layoutObjects(fresh, newCap, nullptr);
+  char *base = nullptr;
+  const cudaError_t e = cudaMalloc(&base, bytes);
+  if (e != cudaSuccess || !ensureScanWorkspace(c, newCap)) {
     cudaGetLastError();
+    if (base) cudaFree(base);
     return fail(c, LADDS_ERR_ALLOC, std::string("device allocation failed: ") + cudaGetErrorString(e));
   }
-  if (c->n) {
-    e = copyState(c->cur, ncur, c->n, c->st);
-    if (e == cudaSuccess) e = cudaStreamSynchronize(c->st);
-    if (e != cudaSuccess) return fail(c, LADDS_ERR_CUDA, cudaGetErrorString(e));
-  }
-  const size_t n = c->n, orderN = std::min(c->orderN, c->n);
-  uint32_t *const oldPerm = c->perm;  // the order of the last scan moves to the new buffer below
-  c->perm = nullptr;
-  c->orderN = 0;
-  struct FreeLater {
-    uint32_t *p;
-    ~FreeLater() {
-      if (p) cudaFree(p);
-    }
-  } freeOldPerm{oldPerm};
-  freeBuffers(c);
-  c->n = n;
-  c->cur = ncur;
-  c->alt = next[0];
-  c->alt2 = next[1];
-  c->snap = next[2];
-  c->homeX[0] = c->cur.x;
-  c->homeX[1] = c->alt.x;
-  uint32_t **u[] = {&c->keys,     &c->keysB,    &c->arrival,    &c->arrivalB,    &c->scratchA, &c->scratchB,
-                    &c->scratchC, &c->perm,     &c->permB,      &c->sortedKeys,  &c->sortedKeysB};
-  for (uint32_t **p : u) {
-    if (cudaMalloc(p, (newCap + 1) * sizeof(uint32_t)) != cudaSuccess) {
-      cudaGetLastError();
-      return fail(c, LADDS_ERR_ALLOC, "device allocation failed (sort buffers)");
+  layoutObjects(fresh, newCap, base);
+  const size_t orderN = std::min(c->orderN, c->n);
+  if (c->n) {  // the population and the order of the last scan
+    cudaError_t m = copyState(c->cur, fresh.cur, c->n, c->st);
+    if (m == cudaSuccess && orderN)
+      m = cudaMemcpyAsync(fresh.perm, c->perm, orderN * sizeof(uint32_t), cudaMemcpyDeviceToDevice, c->st);
+    if (m == cudaSuccess) m = cudaStreamSynchronize(c->st);
+    if (m != cudaSuccess) {
+      cudaFree(base);
+      return fail(c, LADDS_ERR_CUDA, cudaGetErrorString(m));
     }
   }
-  // block sums of the three-level exclusive scans (objects or rows, whichever is longer)
-  const size_t scanLen = std::max(newCap + 1, (size_t)c->nRows + 1);
-  const size_t wsWords = 4 * (scanLen / kScanBlock + 2) + 4 * kScanBlock;
-  if (cudaMalloc(&c->posf, newCap * sizeof(float4)) != cudaSuccess ||
-      cudaMalloc(&c->velf, newCap * sizeof(float4)) != cudaSuccess ||
-      cudaMalloc(&c->grp, newCap * sizeof(uint32_t)) != cudaSuccess ||
-      cudaMalloc(&c->posfB, newCap * sizeof(float4)) != cudaSuccess ||
-      cudaMalloc(&c->velfB, newCap * sizeof(float4)) != cudaSuccess ||
-      cudaMalloc(&c->grpB, newCap * sizeof(uint32_t)) != cudaSuccess ||
-      cudaMalloc(&c->scanRecs, newCap * sizeof(ScanRec)) != cudaSuccess ||
-      cudaMalloc(&c->scanRecsB, newCap * sizeof(ScanRec)) != cudaSuccess ||
-      cudaMalloc(&c->sortRec, newCap * sizeof(unsigned long long)) != cudaSuccess ||
-      cudaMalloc(&c->scanWs, wsWords * sizeof(uint32_t)) != cudaSuccess) {
-    cudaGetLastError();
-    return fail(c, LADDS_ERR_ALLOC, "device allocation failed (cell-order buffers)");
-  }
-  for (uint32_t **p : {&c->denseCells, &c->denseCellsB, &c->denseChunk, &c->denseChunkB}) {
-    if (*p) cudaFree(*p);
-    *p = nullptr;
-  }
-  // every listed cell holds >= kDenseCell objects and adds one entry per kTileChunk of them and part of
-  // its staged side (up to 2^kTilePartsLogMax parts, for cells of >= 64 * 4^kTilePartsLogMax objects)
-  c->denseCap = (uint32_t)(newCap / kDenseCell + newCap / kTileChunk * (1u << kTilePartsLogMax) + 1);
-  for (uint32_t **p : {&c->denseCells, &c->denseCellsB, &c->denseChunk, &c->denseChunkB}) {
-    if (cudaMalloc(p, (size_t)c->denseCap * sizeof(uint32_t)) != cudaSuccess) {
-      cudaGetLastError();
-      for (uint32_t **q : {&c->denseCells, &c->denseCellsB, &c->denseChunk, &c->denseChunkB}) {
-        if (*q) cudaFree(*q);
-        *q = nullptr;
-      }
-      c->denseCap = 0;
-      return fail(c, LADDS_ERR_ALLOC, "device allocation failed (dense-cell list)");
-    }
-  }
-  if (orderN) {
-    CK(cudaMemcpyAsync(c->perm, oldPerm, orderN * sizeof(uint32_t), cudaMemcpyDeviceToDevice, c->st));
-    CK(cudaStreamSynchronize(c->st));
-    c->orderN = orderN;
-  }
+  if (c->objects) cudaFree(c->objects);
+  c->objects = base;
+  static_cast<ObjectBuffers &>(*c) = fresh;
+  c->orderN = orderN;
   c->cap = newCap;
   c->orderValid = false;
   dropGraphs(c);
@@ -389,25 +361,6 @@ int ensureCandCapacity(ladds_gpu_ctx *c, size_t need) {
   c->dCand = p;
   c->candCap = newCap;
   dropGraphs(c);
-  return LADDS_OK;
-}
-
-// After a scan call: grows the record / candidate buffers that overflowed.
-// *overflow tells whether the call has to be re-run.
-int growIfOverflowed(ladds_gpu_ctx *c, unsigned long long *records, bool *overflow) {
-  unsigned long long words[2] = {0, 0};  // record count, largest candidate count (adjacent)
-  CK(cudaMemcpy(words, c->dCount, sizeof(words), cudaMemcpyDeviceToHost));
-  const unsigned long long cnt = words[0], need = words[1];
-  *records = cnt;
-  *overflow = cnt > c->pairCap || need > c->candCap;
-  if (cnt > c->pairCap) {
-    const int rc = ensurePairCapacity(c, (size_t)cnt);
-    if (rc) return rc;
-  }
-  if (need > c->candCap) {
-    const int rc = ensureCandCapacity(c, (size_t)need);
-    if (rc) return rc;
-  }
   return LADDS_OK;
 }
 
@@ -786,6 +739,13 @@ void enqueueChunk(ladds_gpu_ctx *c, int64_t itStart, int len, int k) {
   if (overlap && scans) cudaStreamWaitEvent(c->st, c->evScan[(scans - 1) % 3], 0);
 }
 
+// A chunk is captured into a graph where the launches bound its iterations
+// (eight kernels of an iteration take about 30 us to launch, and 20 us in a graph
+// at 31,000 objects; 1e6 objects take 152.2 us in a graph and 153.3 us launched one
+// by one), and only once it is known to come again: capturing 128 iterations
+// takes some 10 ms.
+constexpr size_t kGraphObjects = 125000;
+
 // host-side effect of replaying a captured chunk: the buffer swaps of its
 // propagations and sorts
 void replaySwaps(ladds_gpu_ctx *c, int64_t itStart, int len, int k) {
@@ -801,39 +761,87 @@ void replaySwaps(ladds_gpu_ctx *c, int64_t itStart, int len, int k) {
   if (scans % 2 == 1) swapSortSets(c);
 }
 
-int syncAndStatus(ladds_gpu_ctx *c) {
-  CK(cudaStreamSynchronize(c->st));
-  CK(cudaGetLastError());
-  unsigned status = 0;
-  CK(cudaMemcpy(&status, c->dStatus, sizeof(unsigned), cudaMemcpyDeviceToHost));
-  if (status) CK(cudaMemset(c->dStatus, 0, sizeof(unsigned)));
+// whether every chunk of a call has a graph, has run before, or comes twice in
+// the call; notes those that come for the first time
+bool chunksWorthCapturing(ladds_gpu_ctx *c, int64_t it0, int iterations, int k) {
+  const DevState ring0[3] = {c->cur, c->alt, c->alt2};
+  const int par0 = c->sortParity;
+  bool worth = true;
+  std::map<ladds_gpu_ctx::GraphKey, int> times;
+  for (int done = 0; done < iterations;) {
+    const int len = std::min(iterations - done, c->chunkSteps);
+    ++times[std::make_tuple(len, (int)((it0 + done) % k), bufferRoles(c), c->n, c->pairCap)];
+    replaySwaps(c, it0 + done, len, k);
+    done += len;
+  }
+  c->cur = ring0[0];
+  c->alt = ring0[1];
+  c->alt2 = ring0[2];
+  if (c->sortParity != par0) swapSortSets(c);
+  for (const auto &t : times)
+    if (t.second < 2 && !c->graphs.count(t.first) && c->seenChunks.insert(t.first).second) worth = false;
+  return worth;
+}
+
+// what a status word means
+int statusError(ladds_gpu_ctx *c, unsigned status) {
+  if (status) CK(cudaMemsetAsync(c->dStatus, 0, sizeof(unsigned), c->st));
   if (status & 4u) return fail(c, LADDS_ERR_DEVICE_CHECK, "a device-side index check failed (sort / gather)");
   if (status & 8u) return fail(c, LADDS_ERR_DEVICE_CHECK, "a bounded device wait ran out (staged propagation)");
   if (status & 1u) return fail(c, LADDS_ERR_NONFINITE, "a position or velocity became NaN/Inf during propagation");
   return LADDS_OK;
 }
 
-// syncAndStatus + growIfOverflowed with one read of the three words after the sync
-int syncStatusAndGrow(ladds_gpu_ctx *c, unsigned long long *records, bool *overflow) {
+int syncAndStatus(ladds_gpu_ctx *c) {
+  c->mail->words[2] = 0;
+  CK(cudaMemcpyAsync(&c->mail->words[2], c->dStatus, sizeof(unsigned), cudaMemcpyDeviceToHost, c->st));
   CK(cudaStreamSynchronize(c->st));
   CK(cudaGetLastError());
-  unsigned long long w[3] = {0, 0, 0};  // record count, largest candidate count, status
-  CK(cudaMemcpy(w, c->dCount, sizeof(w), cudaMemcpyDeviceToHost));
-  const unsigned status = (unsigned)(w[2] & 0xffffffffull);
-  if (status) CK(cudaMemset(c->dStatus, 0, sizeof(unsigned)));
-  if (status & 4u) return fail(c, LADDS_ERR_DEVICE_CHECK, "a device-side index check failed (sort / gather)");
-  if (status & 8u) return fail(c, LADDS_ERR_DEVICE_CHECK, "a bounded device wait ran out (staged propagation)");
-  if (status & 1u) return fail(c, LADDS_ERR_NONFINITE, "a position or velocity became NaN/Inf during propagation");
+  return statusError(c, (unsigned)(c->mail->words[2] & 0xffffffffull));
+}
+
+// The end of a call with scans: the counts, the status and the first records
+// come with the call's work, so that one wait brings them; grows the buffers
+// that overflowed (*overflow: the scans have to run again).
+int syncStatusAndGrow(ladds_gpu_ctx *c, unsigned long long *records, bool *overflow) {
+  CK(cudaMemcpyAsync(c->mail->words, c->dCount, 3 * sizeof(unsigned long long), cudaMemcpyDeviceToHost, c->st));
+  CK(cudaMemcpyAsync(c->mail->recs, c->dPairs, std::min(c->pairCap, kMailRecords) * sizeof(ladds_pair),
+                     cudaMemcpyDeviceToHost, c->st));
+  CK(cudaStreamSynchronize(c->st));
+  CK(cudaGetLastError());
+  const unsigned long long *w = c->mail->words;  // record count, largest candidate count, status
+  const int rc = statusError(c, (unsigned)(w[2] & 0xffffffffull));
+  if (rc) return rc;
   *records = w[0];
   *overflow = w[0] > c->pairCap || w[1] > c->candCap;
   if (w[0] > c->pairCap) {
-    const int rc = ensurePairCapacity(c, (size_t)w[0]);
-    if (rc) return rc;
+    const int rp = ensurePairCapacity(c, (size_t)w[0]);
+    if (rp) return rp;
   }
   if (w[1] > c->candCap) {
-    const int rc = ensureCandCapacity(c, (size_t)w[1]);
-    if (rc) return rc;
+    const int rp = ensureCandCapacity(c, (size_t)w[1]);
+    if (rp) return rp;
   }
+  return LADDS_OK;
+}
+
+// the cnt records of the scans that syncStatusAndGrow waited for
+cudaError_t fetchRecords(ladds_gpu_ctx *c, size_t cnt, std::vector<ladds_pair> &recs) {
+  recs.resize(cnt);
+  if (!cnt) return cudaSuccess;
+  if (cnt > kMailRecords)
+    return cudaMemcpy(recs.data(), c->dPairs, cnt * sizeof(ladds_pair), cudaMemcpyDeviceToHost);
+  std::memcpy(recs.data(), c->mail->recs, cnt * sizeof(ladds_pair));
+  return cudaSuccess;
+}
+
+// a 32-bit count in device memory, after the work enqueued on the stream
+int fetchCount(ladds_gpu_ctx *c, const unsigned *device, unsigned *count) {
+  c->mail->words[3] = 0;
+  CK(cudaMemcpyAsync(&c->mail->words[3], device, sizeof(unsigned), cudaMemcpyDeviceToHost, c->st));
+  CK(cudaStreamSynchronize(c->st));
+  CK(cudaGetLastError());
+  *count = (unsigned)(c->mail->words[3] & 0xffffffffull);
   return LADDS_OK;
 }
 
@@ -920,9 +928,10 @@ int buildGrid(ladds_gpu_ctx *c) {
 }
 
 void freeGridBuffers(ladds_gpu_ctx *c) {
-  void *ptrs[] = {c->rowStart, c->rowStartB, c->rowCounts, c->rowCountsB, c->longRows, c->cellOff, c->cellOffB};
-  for (void *p : ptrs)
-    if (p) cudaFree(p);
+  if (c->tables) cudaFree(c->tables);
+  if (c->cellOffBase) cudaFree(c->cellOffBase);
+  c->tables = nullptr;
+  c->cellOffBase = nullptr;
   c->rowStart = c->rowStartB = c->rowCounts = c->rowCountsB = c->longRows = nullptr;
   c->cellOff = c->cellOffB = nullptr;
 }
@@ -936,24 +945,56 @@ cudaError_t clearRowCounts(ladds_gpu_ctx *c) {
 
 // row tables of c->grid; the two cell-offset tables when each fits 512 MiB (250^3 cells: 31 MB)
 int allocGridBuffers(ladds_gpu_ctx *c) {
-  if (cudaMalloc(&c->rowStart, ((size_t)c->nRows + 1) * sizeof(uint32_t)) != cudaSuccess ||
-      cudaMalloc(&c->rowStartB, ((size_t)c->nRows + 1) * sizeof(uint32_t)) != cudaSuccess ||
-      cudaMalloc(&c->rowCounts, ((size_t)c->nRows + 1) * sizeof(uint32_t)) != cudaSuccess ||
-      cudaMalloc(&c->rowCountsB, ((size_t)c->nRows + 1) * sizeof(uint32_t)) != cudaSuccess ||
-      clearRowCounts(c) != cudaSuccess ||
-      cudaMalloc(&c->longRows, ((size_t)c->nRows + 1) * sizeof(uint32_t)) != cudaSuccess) {
+  const size_t row = (((size_t)c->nRows + 1) * sizeof(uint32_t) + 255) & ~(size_t)255;
+  if (cudaMalloc(&c->tables, 5 * row) != cudaSuccess) {
     cudaGetLastError();
-    freeGridBuffers(c);
+    c->tables = nullptr;
     return fail(c, LADDS_ERR_ALLOC, "device allocation of the cell-row tables failed");
   }
-  const size_t cellOffBytes = (size_t)c->nRows * cellOffPitch((uint32_t)c->grid.n[0]) * sizeof(uint16_t);
-  if (cellOffBytes <= ((size_t)1 << 29) && (cudaMalloc(&c->cellOff, cellOffBytes) != cudaSuccess ||
-                                               cudaMalloc(&c->cellOffB, cellOffBytes) != cudaSuccess)) {
+  uint32_t **t[] = {&c->rowStart, &c->rowStartB, &c->rowCounts, &c->rowCountsB, &c->longRows};
+  for (int k = 0; k < 5; ++k) *t[k] = reinterpret_cast<uint32_t *>(c->tables + k * row);
+  if (clearRowCounts(c) != cudaSuccess) {
     cudaGetLastError();
-    if (c->cellOff) cudaFree(c->cellOff);
-    c->cellOff = c->cellOffB = nullptr;  // the scan then searches the sorted keys
+    freeGridBuffers(c);
+    return fail(c, LADDS_ERR_CUDA, "the cell-row tables could not be cleared");
+  }
+  const size_t cells = (size_t)c->nRows * cellOffPitch((uint32_t)c->grid.n[0]);
+  if (cells * sizeof(uint16_t) <= ((size_t)1 << 29)) {
+    if (cudaMalloc(&c->cellOffBase, 2 * cells * sizeof(uint16_t)) == cudaSuccess) {
+      c->cellOff = c->cellOffBase;
+      c->cellOffB = c->cellOffBase + cells;
+    } else {
+      cudaGetLastError();
+      c->cellOffBase = nullptr;  // the scan then searches the sorted keys
+    }
   }
   return LADDS_OK;
+}
+
+// the counters and small tables of a context: one allocation, zeroed
+cudaError_t allocWords(ladds_gpu_ctx *c) {
+  constexpr size_t line = 256;
+  const size_t later = kLaterCap * sizeof(uint2), eph = 3 * kMaxEphSteps * sizeof(EphEntry);
+  cudaError_t e = cudaMalloc(&c->words, 8 * line + later + eph);
+  if (e != cudaSuccess) {
+    c->words = nullptr;
+    return e;
+  }
+  auto at = [&](size_t k) { return reinterpret_cast<unsigned long long *>(c->words + k * line); };
+  // record count, largest candidate count and status side by side: one read after a call
+  c->dCount = at(0);
+  c->dCandNeed = c->dCount + 1;
+  c->dStatus = reinterpret_cast<unsigned *>(c->dCount + 2);
+  c->dCandCount = at(1);
+  c->dCandCountB = at(2);
+  c->dIter = reinterpret_cast<int64_t *>(at(3));
+  c->dIterBase = c->dIter + 1;
+  c->longCount = reinterpret_cast<uint32_t *>(at(4));
+  c->denseCount = reinterpret_cast<uint32_t *>(at(5));
+  c->denseCountB = reinterpret_cast<uint32_t *>(at(6));
+  c->dLater = reinterpret_cast<uint2 *>(at(8));
+  c->dEph = reinterpret_cast<EphEntry *>(c->words + 8 * line + later);
+  return cudaMemsetAsync(c->words, 0, 8 * line, c->st);
 }
 
 constexpr size_t kHostCopyBlock = (size_t)1 << 17;  // doubles per task of the staging copies
@@ -970,13 +1011,30 @@ bool isPinned(const void *p) {
 // dst[a][lo, lo + len) = src[a][lo, lo + len) for the arrays with use[a], on all host threads
 void hostCopy(double *const dst[6], const double *const src[6], const bool use[6], size_t lo, size_t len) {
   const long per = (long)((len + kHostCopyBlock - 1) / kHostCopyBlock);
-#pragma omp parallel for schedule(static)
+  // few objects: waking all threads costs more than the copies (a host-owned
+  // iteration of 10,000 objects: 128 us with three threads, 147 with one or all)
+  const int threads = len <= kHostCopyBlock / 4 ? std::min(3, omp_get_max_threads()) : omp_get_max_threads();
+#pragma omp parallel for schedule(static) num_threads(threads)
   for (long t = 0; t < 6 * per; ++t) {
     const int a = (int)(t / per);
     if (!use[a]) continue;
     const size_t b = lo + (size_t)(t % per) * kHostCopyBlock, e = std::min(b + kHostCopyBlock, lo + len);
     std::memcpy(dst[a] + b, src[a] + b, (e - b) * sizeof(double));
   }
+}
+
+// six arrays, elements [lo, lo + len): one two-dimensional copy where both
+// sides hold them at one distance, else a copy each
+cudaError_t copySix(double *const dst[6], const double *const src[6], size_t lo, size_t len, bool together,
+                    size_t srcStride, size_t dstStride, cudaMemcpyKind kind, cudaStream_t st) {
+  if (together)
+    return cudaMemcpy2DAsync(dst[0] + lo, dstStride * sizeof(double), src[0] + lo, srcStride * sizeof(double),
+                             len * sizeof(double), 6, kind, st);
+  for (int a = 0; a < 6; ++a) {
+    const cudaError_t e = cudaMemcpyAsync(dst[a] + lo, src[a] + lo, len * sizeof(double), kind, st);
+    if (e != cudaSuccess) return e;
+  }
+  return cudaSuccess;
 }
 
 // dst[0, n) = src[0, n) on all host threads
@@ -1085,34 +1143,20 @@ int ladds_gpu_create(const ladds_gpu_config *f, ladds_gpu_ctx **out) {
   c->cutF = prefilterRadius(f->cutoff, f->nearThresholdRel);
   c->theta0 = gmstIAU1982(f->epochJD);
   if (cudaSetDevice(c->dev) != cudaSuccess || cudaStreamCreateWithFlags(&c->st, cudaStreamNonBlocking) != cudaSuccess ||
-      allocGridBuffers(c) != LADDS_OK || cudaMalloc(&c->longCount, sizeof(uint32_t)) != cudaSuccess ||
-      cudaMalloc(&c->denseCount, sizeof(uint32_t)) != cudaSuccess ||
-      cudaMalloc(&c->denseCountB, sizeof(uint32_t)) != cudaSuccess ||
-      cudaMalloc(&c->dCount, 3 * sizeof(unsigned long long)) != cudaSuccess ||
-      cudaMalloc(&c->dCandCount, kScanCounters * sizeof(unsigned long long)) != cudaSuccess ||
-      cudaMalloc(&c->dCandCountB, kScanCounters * sizeof(unsigned long long)) != cudaSuccess ||
-      cudaMalloc(&c->dLater, kLaterCap * sizeof(uint2)) != cudaSuccess ||
-      cudaMalloc(&c->dEph, 3 * kMaxEphSteps * sizeof(EphEntry)) != cudaSuccess ||
-      cudaMalloc(&c->dIter, 2 * sizeof(int64_t)) != cudaSuccess ||
+      allocGridBuffers(c) != LADDS_OK || allocWords(c) != cudaSuccess ||
+      cudaHostAlloc(&c->mail, sizeof(CallMail), cudaHostAllocDefault) != cudaSuccess ||
       cudaStreamCreateWithFlags(&c->st2, cudaStreamNonBlocking) != cudaSuccess ||
       cudaStreamCreateWithFlags(&c->st3, cudaStreamNonBlocking) != cudaSuccess) {
     cudaGetLastError();
     ladds_gpu_destroy(c);
     return LADDS_ERR_ALLOC;
   }
-  c->dIterBase = c->dIter + 1;
-  // record count, largest candidate count and status words side by side: one read after a step
-  c->dCandNeed = c->dCount + 1;
-  c->dStatus = reinterpret_cast<unsigned *>(c->dCount + 2);
-  cudaMemset(c->dCount, 0, 3 * sizeof(unsigned long long));
-  cudaMemset(c->dIter, 0, 2 * sizeof(int64_t));
   cudaEventCreate(&c->callStart);
   cudaEventCreate(&c->callEnd);
   cudaEventCreateWithFlags(&c->evProp, cudaEventDisableTiming);
   for (auto &e : c->evSort) cudaEventCreateWithFlags(&e, cudaEventDisableTiming);
   for (auto &e : c->evScan) cudaEventCreateWithFlags(&e, cudaEventDisableTiming);
   for (auto &e : c->evPipe) cudaEventCreateWithFlags(&e, cudaEventDisableTiming);
-  cudaMemset(c->dCandNeed, 0, sizeof(unsigned long long));
   c->evalBlocks = 4 * std::max(prop.multiProcessorCount, 1);
   rc = ensurePairCapacity(c, f->pairCapacity ? (size_t)f->pairCapacity : (size_t)1 << 16);
   if (!rc) rc = ensureCandCapacity(c, (size_t)1 << 16);
@@ -1134,13 +1178,10 @@ int ladds_gpu_destroy(ladds_gpu_ctx *c) {
   cudaSetDevice(c->dev);
   if (c->st) cudaStreamSynchronize(c->st);
   dropGraphs(c);
-  freeBuffers(c);
   freeGridBuffers(c);
-  void *ptrs[] = {c->longCount, c->denseCount, c->denseCells, c->denseCountB, c->denseCellsB, c->dCount,
-                  c->denseChunk, c->denseChunkB, c->dEph,
-                  c->dIter, c->dPairs, c->dCand, c->dCandCount, c->dCandCountB, c->dLater, c->dObj,
-                  c->adj.st, c->adj.bc, c->adj.aom, c->adj.miss, c->adj.grad, c->adj.ckpt, c->adj.rec,
-                  c->adj.off, c->adj.arg, c->adj.eph};
+  void *ptrs[] = {c->objects,  c->words,    c->scanWs,  c->dPairs,   c->dCand,   c->dObj,
+                  c->adj.st,   c->adj.bc,   c->adj.aom, c->adj.miss, c->adj.grad, c->adj.ckpt,
+                  c->adj.rec,  c->adj.off,  c->adj.arg, c->adj.eph};
   for (void *p : ptrs)
     if (p) cudaFree(p);
   for (auto &t : c->events) {
@@ -1158,6 +1199,7 @@ int ladds_gpu_destroy(ladds_gpu_ctx *c) {
   for (auto e : c->evPipe)
     if (e) cudaEventDestroy(e);
   if (c->pinStage) cudaFreeHost(c->pinStage);
+  if (c->mail) cudaFreeHost(c->mail);
   if (c->st3) cudaStreamDestroy(c->st3);
   if (c->st2) cudaStreamDestroy(c->st2);
   if (c->st) cudaStreamDestroy(c->st);
@@ -1528,24 +1570,20 @@ int scanState(ladds_gpu_ctx *c, const ScanConsts &sc, float cutF, std::vector<la
   recs.clear();
   if (!c->n) return LADDS_OK;
   for (int attempt = 0; attempt < 5; ++attempt) {
-    CK(cudaMemsetAsync(c->dCount, 0, sizeof(unsigned long long), c->st));
-    CK(cudaMemsetAsync(c->dCandNeed, 0, sizeof(unsigned long long), c->st));
+    CK(cudaMemsetAsync(c->dCount, 0, 2 * sizeof(unsigned long long), c->st));
     c->orderN = 0;
     swapSortSets(c);
     k_scan_input<<<blocksFor(c->n, 256), 256, 0, c->st>>>(c->cur, (int)c->n, c->grid, scanInput(c));
     enqueueSort(c, c->st);
     enqueueScanWith(c, c->st, sc, cutF, c->dIter, -1);  // records carry the index of the last integrated iteration
-    int rc = syncAndStatus(c);
+    unsigned long long cnt = 0;
+    bool overflow = false;
+    const int rc = syncStatusAndGrow(c, &cnt, &overflow);
     collectTimes(c);
     if (rc) return rc;
     c->orderN = c->n;
-    unsigned long long cnt = 0;
-    bool overflow = false;
-    rc = growIfOverflowed(c, &cnt, &overflow);
-    if (rc) return rc;
     if (!overflow) {
-      recs.resize(cnt);
-      if (cnt) CK(cudaMemcpy(recs.data(), c->dPairs, cnt * sizeof(ladds_pair), cudaMemcpyDeviceToHost));
+      CK(fetchRecords(c, (size_t)cnt, recs));
       c->orderValid = true;
       std::sort(recs.begin(), recs.end(), pairLess);
       return LADDS_OK;
@@ -1641,10 +1679,10 @@ int ladds_gpu_step(ladds_gpu_ctx *c, int iterations, ladds_pair *out, size_t cap
   int retries = 0;
   for (;;) {
     if (scans) c->orderN = 0;
-    CK(cudaMemsetAsync(c->dCount, 0, sizeof(unsigned long long), c->st));
-    CK(cudaMemsetAsync(c->dCandNeed, 0, sizeof(unsigned long long), c->st));
-    const bool graph = c->cfg.useGraphs && !c->profiling && iterations >= 1;
+    CK(cudaMemsetAsync(c->dCount, 0, 2 * sizeof(unsigned long long), c->st));
     const int64_t it0 = c->hostIter;
+    const bool graph = c->cfg.useGraphs && !c->profiling && iterations >= 1 && c->n < kGraphObjects &&
+                       chunksWorthCapturing(c, it0, iterations, k);
     if (graph) {
       // pass 1: capture the graphs this call needs (capture performs the host-side
       // buffer swaps; they are undone afterwards), so that no capture happens
@@ -1714,8 +1752,8 @@ int ladds_gpu_step(ladds_gpu_ctx *c, int iterations, ladds_pair *out, size_t cap
   }
   float ms = 0;
   cudaEventElapsedTime(&ms, c->callStart, c->callEnd);
-  std::vector<ladds_pair> recs(cnt);
-  if (cnt) CK(cudaMemcpy(recs.data(), c->dPairs, cnt * sizeof(ladds_pair), cudaMemcpyDeviceToHost));
+  std::vector<ladds_pair> recs;
+  CK(fetchRecords(c, (size_t)cnt, recs));
   std::sort(recs.begin(), recs.end(), pairLess);
   *nOut = recs.size();
   if (recs.size() > cap || (!out && !recs.empty())) {
@@ -1812,26 +1850,28 @@ int ladds_gpu_step_host(ladds_gpu_ctx *c, size_t n, const double *const in[6], d
     src[a] = stageIn[a] ? pinIn[a] : in[a];
     dstHost[a] = stageOut[a] ? pinOut[a] : outState[a];
   }
+  // all six arrays through the staging buffer: one two-dimensional copy a chunk
+  const bool allIn = anyIn && std::all_of(stageIn, stageIn + 6, [](bool b) { return b; });
+  const bool allOut = anyOut && std::all_of(stageOut, stageOut + 6, [](bool b) { return b; });
   // chunks: host->device on st2, propagation on st, device->host on st3
   const int chunks = (int)std::max<size_t>(1, std::min<size_t>((size_t)kHostChunks, n / kHostChunkMin));
   // chunk starts on multiples of 256 objects keep every chunk's arrays 16-byte aligned (staged propagation)
   const size_t per = ((n + (size_t)chunks - 1) / (size_t)chunks + 255) / 256 * 256;
   double *const sArr[6] = {S.x, S.y, S.z, S.vx, S.vy, S.vz};
+  const size_t devStride = (size_t)(S.y - S.x);
   int used = 0;
   for (int ch = 0; ch < chunks && n; ++ch) {
     const size_t lo = (size_t)ch * per;
     if (lo >= n) break;
     const size_t len = std::min(per, n - lo);
     if (anyIn) hostCopy(pinIn, in, stageIn, lo, len);
-    for (int a = 0; a < 6; ++a)
-      CKS(cudaMemcpyAsync(sArr[a] + lo, src[a] + lo, len * sizeof(double), cudaMemcpyHostToDevice, c->st2));
+    CKS(copySix(sArr, src, lo, len, allIn, c->pinCap, devStride, cudaMemcpyHostToDevice, c->st2));
     CKS(cudaEventRecord(c->evPipe[ch], c->st2));
     CKS(cudaStreamWaitEvent(c->st, c->evPipe[ch], 0));
     launchPropagate(c, S, S, lo, (int)len, 1, 0, scan);
     CKS(cudaEventRecord(c->evPipe[kHostChunks + ch], c->st));
     CKS(cudaStreamWaitEvent(c->st3, c->evPipe[kHostChunks + ch], 0));
-    for (int a = 0; a < 6; ++a)
-      CKS(cudaMemcpyAsync(dstHost[a] + lo, sArr[a] + lo, len * sizeof(double), cudaMemcpyDeviceToHost, c->st3));
+    CKS(copySix(dstHost, sArr, lo, len, allOut, devStride, c->pinCap, cudaMemcpyDeviceToHost, c->st3));
     CKS(cudaEventRecord(c->evPipe[2 * kHostChunks + ch], c->st3));
     used = ch + 1;
   }
@@ -1871,8 +1911,8 @@ int ladds_gpu_step_host(ladds_gpu_ctx *c, size_t n, const double *const in[6], d
   CKS(cudaStreamSynchronize(c->st3));
   float ms = 0;
   cudaEventElapsedTime(&ms, c->callStart, c->callEnd);
-  std::vector<ladds_pair> recs(cnt);
-  if (cnt) CKS(cudaMemcpy(recs.data(), c->dPairs, cnt * sizeof(ladds_pair), cudaMemcpyDeviceToHost));
+  std::vector<ladds_pair> recs;
+  CKS(fetchRecords(c, (size_t)cnt, recs));
   std::sort(recs.begin(), recs.end(), pairLess);
   c->hostIter += 1;
   if (scan) {
@@ -2011,15 +2051,14 @@ int ladds_gpu_remove_below(ladds_gpu_ctx *c, double minAltitude, size_t *nRemove
   k_burnup_flags<<<blocksFor(n, 256), 256, 0, c->st>>>(c->cur.x, c->cur.y, c->cur.z, n, critSq, c->scratchA,
                                                         dBurnt);
   unsigned burnt = 0;
-  CK(cudaMemcpyAsync(&burnt, dBurnt, sizeof(unsigned), cudaMemcpyDeviceToHost, c->st));
-  CK(cudaStreamSynchronize(c->st));
-  CK(cudaGetLastError());
+  int rc = fetchCount(c, dBurnt, &burnt);
+  if (rc) return rc;
   if (!burnt) return LADDS_OK;  // nothing burns up: the state, its order and the captured graphs stay
   if (removedIds) {  // ids of the removed objects, in slot order, before the compaction renumbers them
     const int rid = removedIdsInSlotOrder(c, removedIds, cap);
     if (rid) return rid;
   }
-  int rc = compactKept(c);
+  rc = compactKept(c);
   if (rc) return rc;
   if (nRemoved) *nRemoved = (size_t)n - c->n;
   return LADDS_OK;
@@ -2038,15 +2077,14 @@ int ladds_gpu_remove_escaping(ladds_gpu_ctx *c, size_t *nRemoved, uint64_t *remo
   CK(cudaMemsetAsync(dOut, 0, sizeof(unsigned), c->st));
   k_escape_flags<<<blocksFor(n, 256), 256, 0, c->st>>>(c->cur, n, lo, hi, c->scratchA, dOut);
   unsigned escaped = 0;
-  CK(cudaMemcpyAsync(&escaped, dOut, sizeof(unsigned), cudaMemcpyDeviceToHost, c->st));
-  CK(cudaStreamSynchronize(c->st));
-  CK(cudaGetLastError());
+  int rc = fetchCount(c, dOut, &escaped);
+  if (rc) return rc;
   if (!escaped) return LADDS_OK;  // nobody leaves: the state, its order and the captured graphs stay
   if (removedIds) {  // ids of the removed objects, in slot order, before the compaction renumbers them
     const int rid = removedIdsInSlotOrder(c, removedIds, cap);
     if (rid) return rid;
   }
-  int rc = compactKept(c);
+  rc = compactKept(c);
   if (rc) return rc;
   if (nRemoved) *nRemoved = (size_t)n - c->n;
   return LADDS_OK;
@@ -2420,16 +2458,7 @@ int ladds_gpu_autotune(ladds_gpu_ctx *c, int stepsPerTrial, ladds_tune_trial *tr
     int rc = buildGrid(c);
     if (!rc) rc = allocGridBuffers(c);
     if (rc) return rc;
-    if (c->cap) {  // the row-start scan's partial sums are sized by max(objects, rows)
-      const size_t scanLen = std::max(c->cap + 1, (size_t)c->nRows + 1);
-      const size_t wsWords = 4 * (scanLen / kScanBlock + 2) + 4 * kScanBlock;
-      if (c->scanWs) cudaFree(c->scanWs);
-      c->scanWs = nullptr;
-      if (cudaMalloc(&c->scanWs, wsWords * sizeof(uint32_t)) != cudaSuccess) {
-        cudaGetLastError();
-        return fail(c, LADDS_ERR_ALLOC, "autotune: scan workspace");
-      }
-    }
+    if (c->cap && !ensureScanWorkspace(c, c->cap)) return fail(c, LADDS_ERR_ALLOC, "autotune: scan workspace");
     c->orderValid = false;
   }
   *best = bestT;

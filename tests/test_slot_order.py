@@ -89,16 +89,17 @@ def test_cell_order_for_row_tables(capi, ny, nz):
 @pytest.mark.parametrize("precision", [0, 1])
 def test_overlapped_iterations_equal_single_ones(capi, every, precision):
     """A call of many iterations (ring of three states, two sets of sort tables,
-    one propagation launch per scan) against one call per iteration."""
+    one propagation launch per scan; the repeated calls in graphs) against one
+    call per iteration without graphs."""
     pop = capi.generate_population(0, 5, 3001)
     pop["activity"][::40] = capi.EVASIVE_PRESERVING
     kw = dict(componentMask=capi.PROP_ALL, precision=precision, timestepsPerCollisionDetection=every,
               conjunctionThreshold=70.0)
-    with capi.Context(capi.default_config(**kw)) as a, capi.Context(capi.default_config(**kw)) as b:
+    with capi.Context(capi.default_config(**kw)) as a, capi.Context(capi.default_config(useGraphs=0, **kw)) as b:
         for ctx in (a, b):
             ctx.upload(pop)
             ctx.mark_deleted(np.arange(0, 3001, 37))
-        for calls in (11, 4, 1):
+        for calls in (11, 4, 1) + (30,) * 6:
             many = a.step(calls).records
             ones = np.concatenate([b.step(1).records for _ in range(calls)])
             assert len(many) > 0 or calls < every
