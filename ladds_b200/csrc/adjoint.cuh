@@ -108,7 +108,7 @@ __device__ __forceinline__ void accelConservativeJvp(uint32_t mask, const double
 
 // g^T (da/dr, da/dv, da/dbc) of the full FP64 set at (r, v), accumulated into lr, lv, lbc
 __device__ __forceinline__ void accelVjp(uint32_t mask, const double r[3], const double v[3], double aom,
-                                         double bcInv, const EphEntry &e, const AtmShared<false> &atm, const double g[3],
+                                         double bcInv, const EphEntry &e, const double2 *atm, const double g[3],
                                          double lr[3], double lv[3], double &lbc) {
   if (mask & ~kPropDRAG) {
     double dc[3];
@@ -122,13 +122,11 @@ __device__ __forceinline__ void accelVjp(uint32_t mask, const double r[3], const
     const double r2 = x * x + y * y + z * z, rinv = rsqrt(r2);
     const double wx = v[0] + kOmegaEarth * y, wy = v[1] - kOmegaEarth * x, wz = v[2];
     const double w2 = wx * wx + wy * wy + wz * wz, winv = w2 > 0.0 ? rsqrt(w2) : 0.0, wn = w2 * winv;
-    const double h = r2 * rinv - kREarth;
-    const int b = atmBand(atm, h);
-    const double rho = atm.rho0[b] * exp((atm.h0[b] - h) * atm.invH[b]);
-    const double K = -0.5e3 * rho * bcInv;
+    const double2 air = atmDensity(atm, r2 * rinv - kREarth);
+    const double rho = air.x, K = -0.5e3 * rho * bcInv;
     const double wg = wx * g[0] + wy * g[1] + wz * g[2];
     // formed beside the density's exponential, which they do not depend on
-    const double wgw = wg * winv, kq = wn * wg * (atm.invH[b] * rinv);
+    const double wgw = wg * winv, kq = wn * wg * (air.y * rinv);
     const double c1 = K * wn, c2 = K * wgw;
     const double qx = c1 * g[0] + c2 * wx, qy = c1 * g[1] + c2 * wy, qz = c1 * g[2] + c2 * wz;
     lv[0] += qx;
@@ -146,7 +144,7 @@ __device__ __forceinline__ void accelVjp(uint32_t mask, const double r[3], const
 // One FP64 Yoshida step (the expression forms of k_propagate); the three stage
 // accelerations go to acc if non-null.  e3 = the step's three stage entries.
 __device__ __forceinline__ void adjStep(uint32_t mask, double r[3], double v[3], double aom, double bc,
-                                        const EphEntry *e3, const AtmShared<false> &atm, const PropConsts &pc,
+                                        const EphEntry *e3, const double2 *atm, const PropConsts &pc,
                                         double acc[3][3]) {
   double a[3];
 #pragma unroll
@@ -272,7 +270,7 @@ struct EphStage {
 template <int N>
 __device__ __forceinline__ void adjStepWarps(AdjExchange<N> &ex, int &half, uint32_t mask, double r[3],
                                              double v[3], double aom, double bc, const EphEntry *e3,
-                                             const AtmShared<false> &atm, const PropConsts &pc, double acc[3][3]) {
+                                             const double2 *atm, const PropConsts &pc, double acc[3][3]) {
   const uint32_t mine = mask & adjWarpTerms(threadIdx.x >> 5);
   const double hc[3] = {pc.hc1, pc.hc2, pc.hc2}, hd[3] = {pc.hd1, pc.hd2, pc.hd1};
 #pragma unroll
@@ -295,7 +293,7 @@ __device__ __forceinline__ void adjStepWarps(AdjExchange<N> &ex, int &half, uint
 // accelVjp with the terms shared out over the block's warps, summed into lr, lv, lbc
 __device__ __forceinline__ void accelVjpWarps(AdjExchange<7> &ex, int &half, uint32_t mask, const double r[3],
                                               const double v[3], double aom, double bc, const EphEntry &e,
-                                              const AtmShared<false> &atm, const double g[3], double lr[3],
+                                              const double2 *atm, const double g[3], double lr[3],
                                               double lv[3], double &lbc) {
   double t[7] = {0.0, 0.0, 0.0, 0.0, 0.0, 0.0, 0.0};
   accelVjp(mask & adjWarpTerms(threadIdx.x >> 5), r, v, aom, bc, e, atm, g, t, t + 3, t[6]);
@@ -313,7 +311,7 @@ __device__ __forceinline__ void accelVjpWarps(AdjExchange<7> &ex, int &half, uin
 __device__ __forceinline__ void adjReverseStepWarps(AdjExchange<7> &ex, int &half, uint32_t mask,
                                                     const double r0[3], const double v0[3],
                                                     const double acc[3][3], double aom, double bc,
-                                                    const EphEntry *e3, const AtmShared<false> &atm,
+                                                    const EphEntry *e3, const double2 *atm,
                                                     const PropConsts &pc, double lr[3], double lv[3],
                                                     double &lbc) {
   double r1[3], v1[3], r2[3], v2[3], r3[3];
@@ -362,8 +360,6 @@ __device__ __forceinline__ double pairMiss(const double ri[3], const double vi[3
   return dot3rn(dr, dr);
 }
 
-__device__ __forceinline__ void loadAtm(AtmShared<false> &atm) { loadAtmTable(atm, c_atm); }
-
 __device__ __forceinline__ double shflPartner(unsigned m, double x) { return __shfl_xor_sync(m, x, 1); }
 
 // Object SoA: st[c * nObj + j], c = x, y, z, vx, vy, vz; objects 2p (A) and
@@ -376,11 +372,9 @@ __global__ void __launch_bounds__(kAdjWarps * 32) k_adj_forward(
     const double *__restrict__ st, const double *__restrict__ bc, const double *__restrict__ aom, int nObj,
     int steps, int ck, const EphEntry *__restrict__ eph, PropConsts pc, double dt, double *__restrict__ ckpt,
     double *__restrict__ miss, int *__restrict__ argStep) {
-  __shared__ AtmShared<false> atm;
   __shared__ AdjExchange<3> ex;
   __shared__ uint4 ephBuf[kEphChunkWords];
-  loadAtm(atm);
-  __syncthreads();
+  const double2 *atm = pc.atm;
   const EphEntry *ephS = reinterpret_cast<const EphEntry *>(ephBuf);
   EphStage es;
   es.fetch(eph, steps, 0);
@@ -433,11 +427,9 @@ __global__ void __launch_bounds__(kAdjWarps * 32) k_adj_backward(
     const double *__restrict__ bc, const double *__restrict__ aom, int nObj, int steps, int ck,
     const EphEntry *__restrict__ eph, PropConsts pc, double dt, const double *__restrict__ ckpt,
     const int *__restrict__ argStep, double *__restrict__ rec, double *__restrict__ grad) {
-  __shared__ AtmShared<false> atm;
   __shared__ AdjExchange<7> ex;
   __shared__ uint4 ephBuf[kEphChunkWords];
-  loadAtm(atm);
-  __syncthreads();
+  const double2 *atm = pc.atm;
   const EphEntry *ephS = reinterpret_cast<const EphEntry *>(ephBuf);
   EphStage es;
   const int j0 = blockIdx.x * kAdjObjs + (threadIdx.x & 31);
@@ -567,9 +559,7 @@ __global__ void __launch_bounds__(128) k_adj_make_pairs(double *__restrict__ st,
                                                         const int *__restrict__ tca, const double *__restrict__ off,
                                                         const EphEntry *__restrict__ eph, PropConsts pc,
                                                         PropConsts back) {
-  __shared__ AtmShared<false> atm;
-  loadAtm(atm);
-  __syncthreads();
+  const double2 *atm = pc.atm;
   const int p = blockIdx.x * blockDim.x + threadIdx.x;
   if (p >= nPairs) return;
   const int nObj = 2 * nPairs, a = 2 * p, b = 2 * p + 1;

@@ -19,11 +19,13 @@
 //   - FP64: the indirect third-body accelerations of both bodies are one
 //     vector of the ephemeris entry;
 //   - quotients are products with table reciprocals, square roots x rsqrt(x).
-// Measured (1e6 objects, 128 steps in a launch, per step; before: the terms one
-// by one): full set FP64 47.7 -> 33.5 us, split 33.8 -> 30.2 us; the default
-// set (without the third bodies) 35.0 -> 29.5 and 22.6 -> 20.6 us.  The split
-// form's binary32 terms keep their order of operations: evaluated with fewer
-// operations (23.5 us) they move an object by 1e-8 km in 128 steps.
+// Measured (1e6 objects, full set, 128 steps in a launch, per step; before: the
+// terms one by one): FP64 47.7 -> 33.4 us by the sharing, 30.0 with the density
+// table, 27.4 with the mask known at compile time; split 33.8 -> 30.2 -> 26.9 us
+// (10,000 objects: 3.2 -> 2.2 and 2.4 -> 1.7 us).  The split form's binary32 terms
+// keep their order of operations: evaluated with fewer operations they move an
+// object by 1e-8 km in 128 steps; two objects at a time in paired binary32
+// instructions were no gain (28.7 against 30.2 us before the mask was known).
 #pragma once
 #include "physics.cuh"
 
@@ -34,57 +36,57 @@ constexpr double kJ3Coef = -2.5 * kJ3 * kMuEarth * kREarth * kREarth * kREarth;
 constexpr double kSrpCoef = kCR * kPSrp * kAU * kAU * 1.0e3;
 constexpr uint32_t kPropTesseral = kPropC22 | kPropS22;
 
-// The band is found without a search: every band edge of the table is a
-// multiple of 5 km, so the band of h in [0, 1000) km is a function of
-// floor(h / 5) (a 200-entry table; 1000 km and above: the last band).
-constexpr int kAtmBand5 = 201;
-template <bool SPLIT>
-struct AtmShared;
-template <>
-struct AtmShared<false> {
-  double h0[kAtmBands], rho0[kAtmBands], invH[kAtmBands];
-  uint8_t band5[kAtmBand5 + 3];  // band of the altitudes [5 i, 5 i + 5) km
-};
-// split precision: the band's constants themselves per 5 km,
-// (h0, 1 / H, rho0): one 16-byte read per evaluation
-template <>
-struct AtmShared<true> {
+// Atmosphere tables.  Every band edge of the model is a multiple of 5 km.
+//   FP64: per kilometre of altitude in [0, 2048) km the density at its middle
+//     and 1 / H (one table per context, built by k_atm_table and read through the
+//     L1 cache, which it fits): the exponential's argument is then within
+//     1 / (2 H) <= 0.093 of zero and needs no range reduction.  1e6 objects, full
+//     set, per step: 33.4 -> 30.0 us against a band search and exp((h0 - h) / H).
+//   split: per 5 km (h0, 1 / H, rho0) of the band; 1000 km and above: the last.
+//     In shared memory: a 16-byte read on the force evaluation's chain.
+constexpr int kAtmFine = 2048, kAtmBand5 = 201;
+struct AtmShared {
   float4 row5[kAtmBand5];
 };
+__constant__ AtmRow c_atm[kAtmBands] = LADDS_ATM_TABLE;
 
-__device__ __forceinline__ int atmBandOf5(const AtmRow *rows, int i) {  // largest k with h0[k] <= 5 i
+__device__ __forceinline__ int atmBandOf(double h) {  // largest k with h0[k] <= h (0 below the table, and for NaN)
   int k = 0;
-  while (k + 1 < kAtmBands && rows[k + 1].h0 <= 5.0 * i) ++k;
+  while (k + 1 < kAtmBands && c_atm[k + 1].h0 <= h) ++k;
   return k;
 }
-
-// stages the atmosphere table in shared memory (every thread of the block calls it)
-__device__ __forceinline__ void loadAtmTable(AtmShared<false> &atm, const AtmRow *rows) {
-  for (int i = threadIdx.x; i < kAtmBands; i += blockDim.x) {
-    atm.h0[i] = rows[i].h0;
-    atm.rho0[i] = rows[i].rho0;
-    atm.invH[i] = 1.0 / rows[i].H;
-  }
-  for (int i = threadIdx.x; i < kAtmBand5; i += blockDim.x) atm.band5[i] = (uint8_t)atmBandOf5(rows, i);
+__global__ void k_atm_table(double2 *__restrict__ fine) {
+  const int i = blockIdx.x * blockDim.x + threadIdx.x;
+  if (i >= kAtmFine) return;
+  const AtmRow r = c_atm[atmBandOf((double)i)];
+  fine[i] = make_double2(r.rho0 * exp(-((double)i + 0.5 - r.h0) / r.H), 1.0 / r.H);
 }
-__device__ __forceinline__ void loadAtmTable(AtmShared<true> &atm, const AtmRow *rows) {
+// stages the split form's table in shared memory (every thread of the block calls it)
+__device__ __forceinline__ void loadAtmTable(AtmShared &atm) {
   for (int i = threadIdx.x; i < kAtmBand5; i += blockDim.x) {
-    const AtmRow r = rows[atmBandOf5(rows, i)];
+    const AtmRow r = c_atm[atmBandOf(5.0 * i)];
     atm.row5[i] = make_float4((float)r.h0, 1.0f / (float)r.H, (float)r.rho0, 0.0f);
   }
 }
 
-// band index: largest k with h0[k] <= h (0 below the table).  The 5 km table
-// gives it up to the rounding of h / 5 at a band edge (every band is at least
-// 5 km wide), which one comparison with each neighbouring edge corrects: the
-// result equals a search of h0 for every h (NaN: band 0).
-__device__ __forceinline__ int atmBand(const AtmShared<false> &t, double h) {
-  int k = t.band5[min(max((int)(h * 0.2), 0), kAtmBand5 - 1)];
-  if (h < t.h0[k])
-    k = max(k - 1, 0);
-  else if (k + 1 < kAtmBands && h >= t.h0[k + 1])
-    k = k + 1;
-  return k;
+// altitudes outside the fine table
+__device__ __noinline__ double2 atmOutside(double h) {
+  const AtmRow r = c_atm[atmBandOf(h)];
+  return make_double2(r.rho0 * exp(-(h - r.h0) / r.H), 1.0 / r.H);
+}
+
+// density [kg/m^3] and 1 / H [1/km] at altitude h.  The kilometre is floor(h):
+// the low word of h + 3 * 2^51 rounded down, so a band begins exactly at its
+// edge.  exp of |x| <= 0.093 by its Taylor polynomial of degree 9 (remainder
+// x^10 / 10! < 1.4e-17), even and odd parts side by side.
+__device__ __forceinline__ double2 atmDensity(const double2 *__restrict__ fine, double h) {
+  if ((uint32_t)__double2hiint(h) >= 0x40a00000u) return atmOutside(h);  // negative, >= 2048 km, NaN
+  const double m = __dadd_rd(h, 6755399441055744.0);
+  const double2 t = __ldg(&fine[__double2loint(m)]);
+  const double x = ((m - 6755399441055744.0) + 0.5 - h) * t.y, x2 = x * x;
+  const double even = 1.0 + x2 * (1.0 / 2 + x2 * (1.0 / 24 + x2 * (1.0 / 720 + x2 * (1.0 / 40320))));
+  const double odd = 1.0 + x2 * (1.0 / 6 + x2 * (1.0 / 120 + x2 * (1.0 / 5040 + x2 * (1.0 / 362880))));
+  return make_double2(t.x * (even + x * odd), t.y);
 }
 
 // x sqrt(1 / x), 0 at 0
@@ -122,7 +124,7 @@ __device__ __forceinline__ bool inShadow(double x, double y, double z, double r2
 
 // FP64 acceleration of the terms of the mask
 __device__ __forceinline__ void accel(uint32_t mask, const double r[3], const double v[3], double aom, double bcInv,
-                                      const EphEntry &e, const AtmShared<false> &atm, double a[3]) {
+                                      const EphEntry &e, const double2 *fine, double a[3]) {
   const double x = r[0], y = r[1], z = r[2];
   const double r2 = x * x + y * y + z * z;
   const double rinv = rsqrt(r2);
@@ -152,10 +154,7 @@ __device__ __forceinline__ void accel(uint32_t mask, const double r[3], const do
   if (mask & kPropDRAG) {
     const double wx = v[0] + kOmegaEarth * y, wy = v[1] - kOmegaEarth * x, wz = v[2];
     const double wn = sqrtOf(wx * wx + wy * wy + wz * wz);
-    const double h = r2 * rinv - kREarth;
-    const int b = atmBand(atm, h);
-    const double rho = atm.rho0[b] * exp((atm.h0[b] - h) * atm.invH[b]);
-    const double k = -0.5e3 * rho * bcInv * wn;
+    const double k = -0.5e3 * atmDensity(fine, r2 * rinv - kREarth).x * bcInv * wn;
     c[0] += k * wx;
     c[1] += k * wy;
     c[2] += k * wz;
@@ -171,106 +170,110 @@ __device__ __forceinline__ void accel(uint32_t mask, const double r[3], const do
   a[2] = c[2];
 }
 
+// The binary32 terms of the split form are written with explicitly rounded
+// operations (a product fused into a sum only where it says so): their rounding,
+// not the binary64 part's, decides where an object is after some hundred steps,
+// and it does not depend on which terms a kernel has side by side.
+__device__ __forceinline__ float mulf(float a, float b) { return __fmul_rn(a, b); }
+__device__ __forceinline__ float addf(float a, float b) { return __fadd_rn(a, b); }
+__device__ __forceinline__ float subf(float a, float b) { return __fsub_rn(a, b); }
+__device__ __forceinline__ float fmaf_(float a, float b, float c) { return __fmaf_rn(a, b, c); }
+
 // Battin's f(q) = (1+q)^{3/2} - 1 written without cancellation.  The
 // binary32 terms use the approximate square root (s * rsqrt(s)) and division
 // of the hardware: their few-ulp errors are far below the split form's
 // binary32 rounding of the perturbations themselves.
 __device__ __forceinline__ float battinF(float q) {
-  const float s = 1.0f + q;
-  const float s32 = s * (s * rsqrtf(s));
-  return __fdividef(q * (3.0f + q * (3.0f + q)), 1.0f + s32);
+  const float s = addf(1.0f, q);
+  const float num = mulf(q, fmaf_(q, addf(3.0f, q), 3.0f));
+  return __fdividef(num, fmaf_(s, mulf(s, rsqrtf(s)), 1.0f));
 }
 
-// Split-precision acceleration of the terms of the mask.  The binary32 terms
-// keep one order of operations and of summation: their rounding, not the
-// binary64 part's, decides where an object is after some hundred steps.
+// third body at p: adds -mu / |d|^3 (r + f(q) p) to b, with d = p - r and
+// q = r.(r - 2 p) / |p|^2; di = 1 / |d|
+__device__ __forceinline__ void thirdBody(const float r[3], const float *p, float invP2, float mu, float di,
+                                          float b[3]) {
+  const float q = mulf(fmaf_(r[2], fmaf_(-2.0f, p[2], r[2]),
+                             fmaf_(r[0], fmaf_(-2.0f, p[0], r[0]), mulf(r[1], fmaf_(-2.0f, p[1], r[1])))),
+                       invP2);
+  const float k = mulf(mulf(mulf(-mu, di), di), di);
+  const float f = battinF(q);
+#pragma unroll
+  for (int i = 0; i < 3; ++i) b[i] = fmaf_(k, fmaf_(f, p[i], r[i]), b[i]);
+}
+
+// Split-precision acceleration of the terms of the mask.
 __device__ __forceinline__ void accel(uint32_t mask, const double r[3], const double v[3], float aom, float bcInv,
-                                      const EphEntryF &e, const AtmShared<true> &atm, double a[3]) {
+                                      const EphEntryF &e, const AtmShared &atm, double a[3]) {
   const double x = r[0], y = r[1], z = r[2];
   const double r2 = x * x + y * y + z * z;
   const double rinv = rsqrt(r2);
   const double rinv2 = rinv * rinv;
-  const float xf = (float)x, yf = (float)y, zf = (float)z;
-  float bx = 0.f, by = 0.f, bz = 0.f;
+  const float rf[3] = {(float)x, (float)y, (float)z};
+  float b[3] = {0.f, 0.f, 0.f};
   if (mask & (kPropJ3 | kPropTesseral)) {
     const float rinvf = (float)rinv, rinv2f = (float)rinv2;
     if (mask & kPropJ3) {
-      const float k = (float)kJ3Coef * (rinv2f * rinv2f * rinv2f * rinvf);
-      const float z2 = zf * zf;
-      const float f = 3.0f * zf - 7.0f * z2 * zf * rinv2f;
-      const float z2r2 = z2 * rinv2f;
-      bx += k * xf * f;
-      by += k * yf * f;
+      const float k = mulf((float)kJ3Coef, mulf(mulf(mulf(rinv2f, rinv2f), rinv2f), rinvf));
+      const float z2 = mulf(rf[2], rf[2]);
+      const float f = fmaf_(3.0f, rf[2], -mulf(mulf(mulf(7.0f, z2), rf[2]), rinv2f));
+      b[0] = mulf(mulf(k, rf[0]), f);
+      b[1] = mulf(mulf(k, rf[1]), f);
       // 6 z^2 - 7 z^4 / r^2 - 0.6 r^2 == z^2 (6 - 7 z^2/r^2) - 0.6 r^2
-      bz += k * (z2 * (6.0f - 7.0f * z2r2) - 0.6f * (float)r2);
+      b[2] = mulf(k, fmaf_(z2, fmaf_(-7.0f, mulf(z2, rinv2f), 6.0f), -mulf(0.6f, (float)r2)));
     }
     if (mask & kPropTesseral) {
       const float C = (mask & kPropC22) ? (float)kC22 : 0.0f;
       const float S = (mask & kPropS22) ? (float)kS22 : 0.0f;
       const float c = e.cosT, s = e.sinT;
-      const float xe = c * xf + s * yf, ye = -s * xf + c * yf;
-      const float g = C * (xe * xe - ye * ye) + 2.0f * S * xe * ye;
-      const float k = (float)(3.0 * kMuEarth * kREarth * kREarth) * (rinv2f * rinv2f * rinvf);
-      const float axe = k * (2.0f * (C * xe + S * ye) - 5.0f * g * xe * rinv2f);
-      const float aye = k * (2.0f * (S * xe - C * ye) - 5.0f * g * ye * rinv2f);
-      bx += c * axe - s * aye;
-      by += s * axe + c * aye;
-      bz += k * (-5.0f * g * zf * rinv2f);
+      const float xe = fmaf_(c, rf[0], mulf(s, rf[1])), ye = fmaf_(c, rf[1], -mulf(s, rf[0]));
+      const float g = fmaf_(mulf(2.0f * S, xe), ye, mulf(C, fmaf_(xe, xe, -mulf(ye, ye))));
+      const float k = mulf((float)(3.0 * kMuEarth * kREarth * kREarth), mulf(mulf(rinv2f, rinv2f), rinvf));
+      const float g5 = mulf(5.0f, g);
+      const float axe = mulf(k, fmaf_(-mulf(g5, xe), rinv2f, mulf(2.0f, fmaf_(C, xe, mulf(S, ye)))));
+      const float aye = mulf(k, fmaf_(-mulf(g5, ye), rinv2f, mulf(2.0f, fmaf_(S, xe, -mulf(C, ye)))));
+      b[0] = addf(b[0], fmaf_(c, axe, -mulf(s, aye)));
+      b[1] = addf(b[1], fmaf_(s, axe, mulf(c, aye)));
+      b[2] = fmaf_(k, -mulf(mulf(g5, rf[2]), rinv2f), b[2]);
     }
   }
-  float srp = 0.f, sx = 0.f, sy = 0.f, sz = 0.f;  // radiation pressure: srp (sx, sy, sz) towards the Sun
+  float srp = 0.f, d[3] = {0.f, 0.f, 0.f};  // radiation pressure: -srp d, d towards the Sun
   if (mask & (kPropSOL | kPropSRP)) {
-    const float *sp = e.sun;
-    sx = sp[0] - xf, sy = sp[1] - yf, sz = sp[2] - zf;
-    const float di = rsqrtf(sx * sx + sy * sy + sz * sz);
-    if (mask & kPropSOL) {
-      // q = r.(r - 2s) / |s|^2 ;  a = -mu / |d|^3 (r + f(q) s),  d = s - r
-      const float q = (xf * (xf - 2.0f * sp[0]) + yf * (yf - 2.0f * sp[1]) + zf * (zf - 2.0f * sp[2])) * e.sunInvS2;
-      const float k = -(float)kMuSun * di * di * di;
-      const float f = battinF(q);
-      bx += k * (xf + f * sp[0]);
-      by += k * (yf + f * sp[1]);
-      bz += k * (zf + f * sp[2]);
-    }
+#pragma unroll
+    for (int i = 0; i < 3; ++i) d[i] = subf(e.sun[i], rf[i]);
+    const float di = rsqrtf(fmaf_(d[2], d[2], fmaf_(d[0], d[0], mulf(d[1], d[1]))));
+    if (mask & kPropSOL) thirdBody(rf, e.sun, e.sunInvS2, (float)kMuSun, di, b);
     // the shadow edge in binary64: it switches the whole SRP term, and a
     // binary32 edge (~0.4 m) flips stage evaluations near it, which moved
     // single objects by up to 0.3 m per day against the FP64 path
     if ((mask & kPropSRP) && !inShadow(x, y, z, r2, e.sunHat)) {
       // (AU * di)^2 * di keeps every factor inside binary32 range
-      const float au = (float)kAU * di;
-      srp = (float)(kCR * kPSrp * 1.0e3) * aom * (au * au * di);
+      const float au = mulf((float)kAU, di);
+      srp = mulf(mulf((float)(kCR * kPSrp * 1.0e3), aom), mulf(mulf(au, au), di));
     }
   }
   if (mask & kPropLUN) {
-    const float *sp = e.moon;
-    const float q = (xf * (xf - 2.0f * sp[0]) + yf * (yf - 2.0f * sp[1]) + zf * (zf - 2.0f * sp[2])) * e.moonInvS2;
-    const float dx = sp[0] - xf, dy = sp[1] - yf, dz = sp[2] - zf;
-    const float di = rsqrtf(dx * dx + dy * dy + dz * dz);
-    const float k = -(float)kMuMoon * di * di * di;
-    const float f = battinF(q);
-    bx += k * (xf + f * sp[0]);
-    by += k * (yf + f * sp[1]);
-    bz += k * (zf + f * sp[2]);
+    const float m[3] = {subf(e.moon[0], rf[0]), subf(e.moon[1], rf[1]), subf(e.moon[2], rf[2])};
+    const float di = rsqrtf(fmaf_(m[2], m[2], fmaf_(m[0], m[0], mulf(m[1], m[1]))));
+    thirdBody(rf, e.moon, e.moonInvS2, (float)kMuMoon, di, b);
   }
   if (mask & kPropSRP) {
-    bx -= srp * sx;
-    by -= srp * sy;
-    bz -= srp * sz;
+#pragma unroll
+    for (int i = 0; i < 3; ++i) b[i] = fmaf_(-srp, d[i], b[i]);
   }
   if (mask & kPropDRAG) {
-    const float wx = (float)v[0] + (float)kOmegaEarth * yf, wy = (float)v[1] - (float)kOmegaEarth * xf,
-                wz = (float)v[2];
-    const float w2 = wx * wx + wy * wy + wz * wz;
-    const float wn = w2 > 0.0f ? w2 * rsqrtf(w2) : 0.0f;
+    const float w[3] = {fmaf_((float)kOmegaEarth, rf[1], (float)v[0]), fmaf_(-(float)kOmegaEarth, rf[0], (float)v[1]),
+                        (float)v[2]};
+    const float w2 = fmaf_(w[2], w[2], fmaf_(w[0], w[0], mulf(w[1], w[1])));
+    const float wn = w2 > 0.0f ? mulf(w2, rsqrtf(w2)) : 0.0f;
     // an altitude within binary32 rounding of a band edge may take the
     // neighbouring band, whose density agrees there to the table's continuity
     const float h = (float)(r2 * rinv - kREarth);
-    const float4 row = atm.row5[min(max((int)(h * 0.2f), 0), kAtmBand5 - 1)];
-    const float rho = row.z * __expf(-(h - row.x) * row.y);
-    const float k = -0.5e3f * rho * bcInv * wn;
-    bx += k * wx;
-    by += k * wy;
-    bz += k * wz;
+    const float4 row = atm.row5[min(max((int)mulf(h, 0.2f), 0), kAtmBand5 - 1)];
+    const float rho = mulf(row.z, __expf(mulf(-subf(h, row.x), row.y)));
+    const float k = mulf(mulf(mulf(-0.5e3f, rho), bcInv), wn);
+#pragma unroll
+    for (int i = 0; i < 3; ++i) b[i] = fmaf_(k, w[i], b[i]);
   }
   double sr = 0.0, az = 0.0;
   if (mask & (kPropKEP | kPropJ2)) {
@@ -282,9 +285,9 @@ __device__ __forceinline__ void accel(uint32_t mask, const double r[3], const do
       az = 2.0 * k;
     }
   }
-  a[0] = sr * x + (double)bx;
-  a[1] = sr * y + (double)by;
-  a[2] = (sr + az) * z + (double)bz;
+  a[0] = sr * x + (double)b[0];
+  a[1] = sr * y + (double)b[1];
+  a[2] = (sr + az) * z + (double)b[2];
 }
 
 }  // namespace ladds

@@ -71,6 +71,10 @@ __global__ void __launch_bounds__(3 * kMaxEphSteps) k_ephemeris_dev(Entry *__res
 
 inline int blocksFor(size_t n, int b) { return (int)((n + (size_t)b - 1) / (size_t)b); }
 
+constexpr uint32_t kMaskFull = LADDS_PROP_ALL;
+constexpr uint32_t kMaskDefault =
+    LADDS_PROP_KEP | LADDS_PROP_J2 | LADDS_PROP_C22 | LADDS_PROP_S22 | LADDS_PROP_SRP | LADDS_PROP_DRAG;
+
 enum Phase { kPhProp, kPhBucket, kPhRowsort, kPhPermute, kPhCandidates, kPhEvaluate };
 
 // ladds_gpu_step_host moves the state in at most this many chunks, each at
@@ -452,6 +456,17 @@ cudaError_t enqueueEphemeris(ladds_gpu_ctx *c, int nSteps) {
                                  cudaMemcpyDeviceToDevice, c->st);
 }
 
+// the propagation kernel of a component mask: the full and the default set have
+// kernels of their own, whose terms are not cut off from one another by branches
+// on the mask (a force evaluation is a long chain: 1e6 objects, full set, 30.0 ->
+// 27.4 us per step in FP64 and 30.2 -> 26.9 in the split form)
+template <typename Pick>
+auto forMask(uint32_t mask, Pick pick) {
+  if (mask == kMaskFull) return pick(std::integral_constant<uint32_t, kMaskFull>{});
+  if (mask == kMaskDefault) return pick(std::integral_constant<uint32_t, kMaskDefault>{});
+  return pick(std::integral_constant<uint32_t, 0u>{});
+}
+
 ScanInput scanInput(const ladds_gpu_ctx *c) {
   return ScanInput{c->keys, c->rowCounts, c->arrival, c->scanRecs, c->cur.radius};
 }
@@ -476,8 +491,12 @@ void launchPropagate(ladds_gpu_ctx *c, DevState s, DevState to, size_t lo, int n
   // 162 / 156 / 150 us, 2e6 391 / 381 / 391 us, 8e6 (40 km) 3331 / 3221 / 3322 us.
   const int sg = std::max(1, std::min(blocksFor((size_t)n, kStageObjects), c->evalBlocks * 3 / 4));
   const bool split = c->cfg.precision == LADDS_PRECISION_SPLIT;
-  auto kernel = split ? (scan ? k_propagate_staged<true, true> : k_propagate_staged<true, false>)
-                      : (scan ? k_propagate_staged<false, true> : k_propagate_staged<false, false>);
+  auto pick = [&](auto mask) {
+    constexpr uint32_t M = decltype(mask)::value;
+    return split ? (scan ? k_propagate_staged<true, true, M> : k_propagate_staged<true, false, M>)
+                 : (scan ? k_propagate_staged<false, true, M> : k_propagate_staged<false, false, M>);
+  };
+  auto kernel = forMask(c->pc.mask, pick);
   kernel<<<sg, kStageObjects, 0, c->st>>>(s, to, n, nSteps, ephBase, c->pc, c->grid, in, c->dStatus);
 }
 
@@ -486,10 +505,12 @@ void enqueuePropagate(ladds_gpu_ctx *c, int nSteps, int ephBase) {
   if (!c->n) return;
   PhaseScope ps(c, kPhProp, c->st);
   const int b = c->cfg.propagateBlock > 0 ? c->cfg.propagateBlock : 256, g = blocksFor(c->n, b);
-  if (c->cfg.precision == LADDS_PRECISION_SPLIT)
-    k_propagate<true><<<g, b, 0, c->st>>>(c->cur, (int)c->n, nSteps, ephBase, c->pc, c->dStatus);
-  else
-    k_propagate<false><<<g, b, 0, c->st>>>(c->cur, (int)c->n, nSteps, ephBase, c->pc, c->dStatus);
+  const bool split = c->cfg.precision == LADDS_PRECISION_SPLIT;
+  auto kernel = forMask(c->pc.mask, [&](auto mask) {
+    constexpr uint32_t M = decltype(mask)::value;
+    return split ? k_propagate<true, M> : k_propagate<false, M>;
+  });
+  kernel<<<g, b, 0, c->st>>>(c->cur, (int)c->n, nSteps, ephBase, c->pc, c->dStatus);
 }
 
 // the next buffer of the ring becomes the current state
@@ -975,7 +996,7 @@ int allocGridBuffers(ladds_gpu_ctx *c) {
 cudaError_t allocWords(ladds_gpu_ctx *c) {
   constexpr size_t line = 256;
   const size_t later = kLaterCap * sizeof(uint2), eph = 3 * kMaxEphSteps * sizeof(EphEntry);
-  cudaError_t e = cudaMalloc(&c->words, 8 * line + later + eph);
+  cudaError_t e = cudaMalloc(&c->words, 8 * line + later + eph + kAtmFine * sizeof(double2));
   if (e != cudaSuccess) {
     c->words = nullptr;
     return e;
@@ -994,7 +1015,11 @@ cudaError_t allocWords(ladds_gpu_ctx *c) {
   c->denseCountB = reinterpret_cast<uint32_t *>(at(6));
   c->dLater = reinterpret_cast<uint2 *>(at(8));
   c->dEph = reinterpret_cast<EphEntry *>(c->words + 8 * line + later);
-  return cudaMemsetAsync(c->words, 0, 8 * line, c->st);
+  auto *fineT = reinterpret_cast<double2 *>(c->words + 8 * line + later + eph);
+  k_atm_table<<<blocksFor(kAtmFine, 256), 256, 0, c->st>>>(fineT);
+  c->pc.atm = fineT;
+  e = cudaGetLastError();
+  return e != cudaSuccess ? e : cudaMemsetAsync(c->words, 0, 8 * line, c->st);
 }
 
 constexpr size_t kHostCopyBlock = (size_t)1 << 17;  // doubles per task of the staging copies
@@ -1071,8 +1096,7 @@ void ladds_gpu_config_default(ladds_gpu_config *f) {
   if (!f) return;
   std::memset(f, 0, sizeof(*f));
   f->deltaT = 10.0;
-  f->componentMask =
-      LADDS_PROP_KEP | LADDS_PROP_J2 | LADDS_PROP_C22 | LADDS_PROP_S22 | LADDS_PROP_SRP | LADDS_PROP_DRAG;
+  f->componentMask = kMaskDefault;
   f->epochJD = 2459580.5;  // 2022-01-01 00:00 UTC (cfg/default_cfg.yaml:9)
   f->startTime = 0.0;
   f->cutoff = 80.0;

@@ -9,8 +9,7 @@
 // One thread per object, state held in registers across `nSteps` steps, so
 // a multi-step launch touches HBM once (read 64 B + write 48 B per object).
 // Ephemeris entries of all stages of the launch live in __constant__ memory
-// (uniform across the warp).  The atmosphere table is staged in shared memory
-// (the band index diverges across the warp).
+// (uniform across the warp).
 #pragma once
 #include "bulk_copy.cuh"
 #include "cell_sort.cuh"
@@ -26,16 +25,19 @@ constexpr int kMaxEphSteps = 128;  // 3 * 128 entries * 112 B (FP64) or 88 B (sp
 template <bool SPLIT>
 using EphOf = typename std::conditional<SPLIT, EphEntryF, EphEntry>::type;
 static_assert(sizeof(EphEntryF) <= sizeof(EphEntry), "the stage table holds entries of either form");
-__constant__ __align__(16) unsigned char c_eph[3 * kMaxEphSteps * sizeof(EphEntry)];
+__constant__ __align__(256) unsigned char c_eph[3 * kMaxEphSteps * sizeof(EphEntry)];
 template <bool SPLIT>
 __device__ __forceinline__ const EphOf<SPLIT> *stageTable() {
   return reinterpret_cast<const EphOf<SPLIT> *>(c_eph);
 }
-__constant__ AtmRow c_atm[kAtmBands] = LADDS_ATM_TABLE;
+// the atmosphere table that a force evaluation reads
+template <bool SPLIT>
+using AtmOf = typename std::conditional<SPLIT, AtmShared, const double2 *>::type;
 
 struct PropConsts {
   double hc1, hc2, hd1, hd2;  // Yoshida coefficients * dt
   uint32_t mask;
+  const double2 *atm;  // the fine atmosphere table
 };
 
 // floor((v - lo) * inv) with exactly these two roundings; NaN -> 0; clamped to
@@ -86,7 +88,7 @@ __device__ __forceinline__ void writeScanInput(const ScanInput &o, const GridDes
 template <bool SPLIT>
 __device__ __forceinline__ void yoshidaLoop(uint32_t mask, double r[3], double v[3], double aom, double bc,
                                             int nSteps, int ephBase, const PropConsts &pc,
-                                            const AtmShared<SPLIT> &atm) {
+                                            const AtmOf<SPLIT> &atm) {
   using C = typename std::conditional<SPLIT, float, double>::type;
   const C aomC = (C)aom, bcC = (C)bc;
   const EphOf<SPLIT> *e = stageTable<SPLIT>() + ephBase;
@@ -111,31 +113,40 @@ __device__ __forceinline__ void yoshidaLoop(uint32_t mask, double r[3], double v
     for (int k = 0; k < 3; ++k) r[k] += pc.hc1 * v[k];
   }
 }
-template <bool SPLIT>
+// MASK: the launch's component mask where it is known at compile time, else 0.
+template <bool SPLIT, uint32_t MASK>
 __device__ __forceinline__ void yoshidaSteps(double r[3], double v[3], double aom, double bc, uint32_t tag,
                                              int nSteps, int ephBase, const PropConsts &pc,
-                                             const AtmShared<SPLIT> &atm, unsigned *__restrict__ status) {
+                                             const AtmShared &atmS, unsigned *__restrict__ status) {
+  const AtmOf<SPLIT> &atm = [&]() -> const AtmOf<SPLIT> & {
+    if constexpr (SPLIT)
+      return atmS;
+    else
+      return pc.atm;
+  }();
   if (tagAct(tag) == kEvasivePreserving)
     yoshidaLoop<SPLIT>(pc.mask & kPropKEP, r, v, aom, bc, nSteps, ephBase, pc, atm);
   else
-    yoshidaLoop<SPLIT>(pc.mask, r, v, aom, bc, nSteps, ephBase, pc, atm);
+    yoshidaLoop<SPLIT>(MASK ? MASK : pc.mask, r, v, aom, bc, nSteps, ephBase, pc, atm);
   if (!(isfinite(r[0]) && isfinite(r[1]) && isfinite(r[2]) && isfinite(v[0]) && isfinite(v[1]) && isfinite(v[2])))
     atomicOr(status, 1u);
 }
 
 // Propagation without a scan: nSteps steps in place, one object per thread.
-template <bool SPLIT>
+template <bool SPLIT, uint32_t MASK>
 __global__ void __launch_bounds__(256, 4) k_propagate(DevState s, int n, int nSteps, int ephBase, PropConsts pc,
                                                    unsigned *__restrict__ status) {
-  __shared__ AtmShared<SPLIT> atm;
-  loadAtmTable(atm, c_atm);
-  __syncthreads();
+  __shared__ AtmShared atmS;
+  if (SPLIT) {
+    loadAtmTable(atmS);
+    __syncthreads();
+  }
   const int j = blockIdx.x * blockDim.x + threadIdx.x;
   if (j >= n) return;
   const uint32_t tag = s.tag[j];
   if (tagDummy(tag)) return;
   double r[3] = {s.x[j], s.y[j], s.z[j]}, v[3] = {s.vx[j], s.vy[j], s.vz[j]};
-  yoshidaSteps<SPLIT>(r, v, s.aom[j], s.bc[j], tag, nSteps, ephBase, pc, atm, status);
+  yoshidaSteps<SPLIT, MASK>(r, v, s.aom[j], s.bc[j], tag, nSteps, ephBase, pc, atmS, status);
   s.x[j] = r[0];
   s.y[j] = r[1];
   s.z[j] = r[2];
@@ -150,8 +161,7 @@ __global__ void __launch_bounds__(256, 4) k_propagate(DevState s, int n, int nSt
 // state of the CTA's next tile is already on its way into shared memory: one
 // thread issues nine bulk copies (x, y, z, vx, vy, vz, aom, bc: 2 KB each;
 // tags: 1 KB) completed on an mbarrier, so no warp stalls on its loads after
-// the first tile, and the atmosphere table is staged once per CTA instead of
-// once per 256 objects.  The partial tile at the end (n % kStageObjects
+// the first tile.  The partial tile at the end (n % kStageObjects
 // objects) is read directly.  The new state goes to `to`, which may be s
 // itself: the state before it stays readable for the pair scan that is still
 // running on it.  Per-object arithmetic and results are k_propagate's.  A wait
@@ -161,11 +171,11 @@ constexpr int kStageArrays = 8;
 constexpr uint32_t kStageTxBytes = kStageArrays * kStageObjects * 8 + kStageObjects * 4;
 constexpr uint32_t kStageWaitPolls = 1u << 22;
 
-template <bool SPLIT, bool SCAN>
+template <bool SPLIT, bool SCAN, uint32_t MASK>
 __global__ void __launch_bounds__(kStageObjects, 4) k_propagate_staged(DevState s, DevState to, int n, int nSteps,
                                                                       int ephBase, PropConsts pc, GridDesc g,
                                                                       ScanInput scan, unsigned *__restrict__ status) {
-  __shared__ AtmShared<SPLIT> atm;
+  __shared__ AtmShared atmS;
   __shared__ __align__(16) double sv[kStageArrays][kStageObjects];
   __shared__ __align__(16) uint32_t stag[kStageObjects];
   __shared__ __align__(8) unsigned long long sbar;
@@ -185,7 +195,7 @@ __global__ void __launch_bounds__(kStageObjects, 4) k_propagate_staged(DevState 
     mbarInit(&sbar, 1);
     mbarInitFence();
   }
-  loadAtmTable(atm, c_atm);
+  if (SPLIT) loadAtmTable(atmS);
   __syncthreads();
   int t = blockIdx.x;
   if (tid == 0 && t < nFull) issue(t);
@@ -219,7 +229,7 @@ __global__ void __launch_bounds__(kStageObjects, 4) k_propagate_staged(DevState 
       aom = s.aom[j];
       bc = s.bc[j];
     }
-    if (!tagDummy(tag)) yoshidaSteps<SPLIT>(r, v, aom, bc, tag, nSteps, ephBase, pc, atm, status);
+    if (!tagDummy(tag)) yoshidaSteps<SPLIT, MASK>(r, v, aom, bc, tag, nSteps, ephBase, pc, atmS, status);
     if (inRange) {  // deleted objects too: both buffers hold them
       to.x[j] = r[0];
       to.y[j] = r[1];
