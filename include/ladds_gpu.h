@@ -523,13 +523,14 @@ typedef struct {
 } ladds_adjoint_pair;
 
 /* Forward sweep: the loss, per-pair min dl2 (missSq) and its step (tcaStep,
- * 1-based), both may be NULL; stores the states every checkpointEvery steps on
- * the device for the backward sweep.  deviceMs (may be NULL): kernel time. */
+ * 1-based), both may be NULL; keeps on the device what the backward sweep needs:
+ * 96 bytes per object and step where that is at most 1 GiB, else the states
+ * every checkpointEvery steps.  deviceMs (may be NULL): kernel time. */
 int ladds_gpu_adjoint_forward(ladds_gpu_ctx *ctx, const ladds_adjoint_pair *pairs, size_t nPairs, int steps,
                               int checkpointEvery, double *missSq, int32_t *tcaStep, double *loss,
                               double *deviceMs);
-/* Backward sweep of the last forward sweep (segments recomputed from the
- * checkpoints): dL_dx0[12 p ..] = dL/d(rA, vA, rB, vB), dL_dbc[2 p ..] =
+/* Backward sweep of the last forward sweep (from checkpoints: segment by segment,
+ * each recomputed): dL_dx0[12 p ..] = dL/d(rA, vA, rB, vB), dL_dbc[2 p ..] =
  * dL/d(bcInvA, bcInvB).  LADDS_ERR_STATE without a preceding forward sweep. */
 int ladds_gpu_adjoint_backward(ladds_gpu_ctx *ctx, double *dL_dx0, double *dL_dbc, double *deviceMs);
 /* Synthetic pairs of the differentiation benchmark: A and B from population 0

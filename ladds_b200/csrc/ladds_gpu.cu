@@ -225,7 +225,8 @@ struct ladds_gpu_ctx : ObjectBuffers {
     size_t nPairs = 0;
     int steps = 0, ck = 0;
     bool forwardDone = false;
-    double *st = nullptr, *bc = nullptr, *aom = nullptr, *miss = nullptr, *grad = nullptr;
+    bool whole = false;  // rec holds every step of the forward sweep (else ckpt its checkpoints)
+    double *st = nullptr, *bc = nullptr, *aom = nullptr, *miss = nullptr, *seed = nullptr, *grad = nullptr;
     double *ckpt = nullptr, *rec = nullptr, *off = nullptr;
     int *arg = nullptr;
     EphEntry *eph = nullptr;
@@ -1204,7 +1205,7 @@ int ladds_gpu_destroy(ladds_gpu_ctx *c) {
   dropGraphs(c);
   freeGridBuffers(c);
   void *ptrs[] = {c->objects,  c->words,    c->scanWs,  c->dPairs,   c->dCand,   c->dObj,
-                  c->adj.st,   c->adj.bc,   c->adj.aom, c->adj.miss, c->adj.grad, c->adj.ckpt,
+                  c->adj.st,   c->adj.bc,   c->adj.aom, c->adj.miss, c->adj.seed, c->adj.grad, c->adj.ckpt,
                   c->adj.rec,  c->adj.off,  c->adj.arg, c->adj.eph};
   for (void *p : ptrs)
     if (p) cudaFree(p);
@@ -2512,35 +2513,70 @@ int ensureDev(ladds_gpu_ctx *c, T *&p, size_t &cap, size_t need) {
   return LADDS_OK;
 }
 
-// buffers of nPairs pairs, `steps` steps, checkpoints every ck; ephemeris of the steps
-int adjPrepare(ladds_gpu_ctx *c, size_t nPairs, int steps, int ck, bool backward) {
+// buffers of nPairs pairs and the ephemeris of `steps` steps
+int adjPrepare(ladds_gpu_ctx *c, size_t nPairs, int steps) {
   auto &A = c->adj;
   const size_t nObj = 2 * nPairs;
   size_t objCap = A.objCap;
   int rc;
   if (nObj > A.objCap) {
-    size_t cap0 = 0, cap1 = 0, cap2 = 0, cap3 = 0, cap4 = 0, cap5 = 0, cap6 = 0;
+    size_t cap0 = 0, cap1 = 0, cap2 = 0, cap3 = 0, cap4 = 0, cap5 = 0, cap6 = 0, cap7 = 0;
     if ((rc = ensureDev(c, A.st, cap0, 6 * nObj)) || (rc = ensureDev(c, A.bc, cap1, nObj)) ||
         (rc = ensureDev(c, A.aom, cap2, nObj)) || (rc = ensureDev(c, A.miss, cap3, nPairs)) ||
         (rc = ensureDev(c, A.grad, cap4, 7 * nObj)) || (rc = ensureDev(c, A.arg, cap5, nPairs)) ||
-        (rc = ensureDev(c, A.off, cap6, 6 * nPairs))) {
+        (rc = ensureDev(c, A.off, cap6, 6 * nPairs)) || (rc = ensureDev(c, A.seed, cap7, 6 * nObj))) {
       A.objCap = 0;
       return rc;
     }
     objCap = nObj;
   }
   A.objCap = objCap;
-  const size_t nSeg = (size_t)((steps + ck - 1) / ck);
-  if ((rc = ensureDev(c, A.ckpt, A.ckptCap, nSeg * 6 * nObj))) return rc;
-  if (backward && (rc = ensureDev(c, A.rec, A.recCap, (size_t)ck * 15 * nObj))) return rc;
-  if ((rc = ensureDev(c, A.eph, A.ephCap, (size_t)3 * steps))) return rc;
-  return LADDS_OK;
+  return ensureDev(c, A.eph, A.ephCap, (size_t)3 * steps);
+}
+
+// The forward sweep leaves the reverse sweep's records (12 doubles per object
+// and step) where all of them fit in this many bytes -- 4096 pairs of 1080 steps
+// are 0.85 GB of the device's 180 -- and checkpoints elsewhere, from which the
+// reverse sweep makes the records segment by segment: a second forward sweep,
+// which is the longer part.  4096 pairs, reverse sweep: 0.79 us per step from kept
+// records, 2.23 by segments of 64 steps.
+constexpr size_t kAdjRecordBytes = (size_t)1 << 30;
+constexpr size_t kAdjRecord = 12;
+
+// whole or by segments, with the buffers of either
+int adjStorage(ladds_gpu_ctx *c, size_t nObj, int steps, int ck) {
+  auto &A = c->adj;
+  const size_t all = (size_t)steps * kAdjRecord * nObj;
+  A.whole = all * sizeof(double) <= kAdjRecordBytes && ensureDev(c, A.rec, A.recCap, all) == LADDS_OK;
+  if (A.whole) return LADDS_OK;
+  const size_t nSeg = ((size_t)steps + ck - 1) / ck;
+  return ensureDev(c, A.ckpt, A.ckptCap, nSeg * 6 * nObj);
 }
 
 int adjEphemeris(ladds_gpu_ctx *c, int steps) {
   k_ephemeris<<<blocksFor((size_t)3 * steps, 128), 128, 0, c->st>>>(c->adj.eph, steps, 0, c->cfg.startTime,
                                                                      c->cfg.deltaT, c->pc.hc1, c->pc.hc2,
                                                                      c->cfg.epochJD, c->theta0, c->pc.mask);
+  CK(cudaGetLastError());
+  return LADDS_OK;
+}
+
+// steps s0 + 1 .. s1 from the states st; records from step s0 + 1 on (or null)
+void adjForward(ladds_gpu_ctx *c, const double *st, int nObj, int s0, int s1, bool sweep, double *rec) {
+  auto &A = c->adj;
+  auto kernel = forMask(c->pc.mask, [](auto mask) { return k_adj_forward<decltype(mask)::value>; });
+  kernel<<<blocksFor(nObj, kAdjObjs), kAdjFwdThreads, 0, c->st>>>(
+      st, A.bc, A.aom, nObj, s0, s1, A.eph, c->pc, c->cfg.deltaT, A.ck, sweep && !A.whole ? A.ckpt : nullptr, rec,
+      sweep ? A.miss : nullptr, A.arg, A.seed);
+}
+
+// the reverse of steps s1 .. s0 + 1 from their records
+int adjBackward(ladds_gpu_ctx *c, int nObj, int s0, int s1) {
+  auto &A = c->adj;
+  auto kernel = forMask(c->pc.mask, [](auto mask) { return k_adj_backward<decltype(mask)::value>; });
+  CK(cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)sizeof(AdjBackShared)));
+  kernel<<<blocksFor(nObj, kAdjObjs), kAdjBwdThreads, sizeof(AdjBackShared), c->st>>>(
+      A.bc, A.aom, nObj, s0, s1, A.eph, c->pc, A.rec, A.arg, A.seed, s1 == A.steps, A.grad);
   CK(cudaGetLastError());
   return LADDS_OK;
 }
@@ -2558,9 +2594,12 @@ int ladds_gpu_adjoint_forward(ladds_gpu_ctx *c, const ladds_adjoint_pair *pairs,
   CK(cudaSetDevice(c->dev));
   auto &A = c->adj;
   A.forwardDone = false;
-  int rc = adjPrepare(c, nPairs, steps, checkpointEvery, false);
-  if (rc) return rc;
   const size_t nObj = 2 * nPairs;
+  int rc = adjPrepare(c, nPairs, steps);
+  if (rc || (rc = adjStorage(c, nObj, steps, checkpointEvery))) return rc;
+  A.nPairs = nPairs;
+  A.steps = steps;
+  A.ck = checkpointEvery;
   // pairs (AoS) -> object SoA
   std::vector<double> st(6 * nObj), bc(nObj), aom(nObj);
   for (size_t p = 0; p < nPairs; ++p) {
@@ -2583,9 +2622,7 @@ int ladds_gpu_adjoint_forward(ladds_gpu_ctx *c, const ladds_adjoint_pair *pairs,
   }
   if ((rc = adjEphemeris(c, steps))) return rc;
   CK(cudaEventRecord(c->callStart, c->st));
-  if (nObj)
-    k_adj_forward<<<blocksFor(nObj, kAdjObjs), kAdjWarps * 32, 0, c->st>>>(A.st, A.bc, A.aom, (int)nObj, steps, checkpointEvery,
-                                                           A.eph, c->pc, c->cfg.deltaT, A.ckpt, A.miss, A.arg);
+  if (nObj) adjForward(c, A.st, (int)nObj, 0, steps, true, A.whole ? A.rec : nullptr);
   CK(cudaEventRecord(c->callEnd, c->st));
   CK(cudaGetLastError());
   std::vector<double> miss(nPairs);
@@ -2605,9 +2642,6 @@ int ladds_gpu_adjoint_forward(ladds_gpu_ctx *c, const ladds_adjoint_pair *pairs,
     if (arg[p] > 0) sum += miss[p];
   }
   if (loss) *loss = sum;
-  A.nPairs = nPairs;
-  A.steps = steps;
-  A.ck = checkpointEvery;
   A.forwardDone = true;
   return LADDS_OK;
 }
@@ -2618,13 +2652,17 @@ int ladds_gpu_adjoint_backward(ladds_gpu_ctx *c, double *dL_dx0, double *dL_dbc,
   if (!A.forwardDone) return fail(c, LADDS_ERR_STATE, "adjoint_backward needs a preceding adjoint_forward");
   std::lock_guard<std::mutex> lk(g_deviceMutex[c->dev & 63]);
   CK(cudaSetDevice(c->dev));
-  int rc = adjPrepare(c, A.nPairs, A.steps, A.ck, true);
-  if (rc) return rc;
   const size_t nObj = 2 * A.nPairs;
+  const int segment = A.whole ? A.steps : std::min(A.ck, A.steps);
+  int rc = ensureDev(c, A.rec, A.recCap, (size_t)segment * kAdjRecord * nObj);
+  if (rc) return rc;
   CK(cudaEventRecord(c->callStart, c->st));
-  if (nObj)
-    k_adj_backward<<<blocksFor(nObj, kAdjObjs), kAdjWarps * 32, 0, c->st>>>(A.bc, A.aom, (int)nObj, A.steps, A.ck, A.eph, c->pc,
-                                                            c->cfg.deltaT, A.ckpt, A.arg, A.rec, A.grad);
+  for (int s1 = A.steps; nObj && s1 > 0;) {
+    const int s0 = (s1 - 1) / segment * segment;
+    if (!A.whole) adjForward(c, A.ckpt + (size_t)(s0 / segment) * 6 * nObj, (int)nObj, s0, s1, false, A.rec);
+    if ((rc = adjBackward(c, (int)nObj, s0, s1))) return rc;
+    s1 = s0;
+  }
   CK(cudaEventRecord(c->callEnd, c->st));
   CK(cudaGetLastError());
   std::vector<double> g(7 * nObj);
@@ -2652,7 +2690,7 @@ int ladds_gpu_adjoint_make_pairs(ladds_gpu_ctx *c, uint64_t seed, size_t nPairs,
   CK(cudaSetDevice(c->dev));
   auto &A = c->adj;
   A.forwardDone = false;
-  int rc = adjPrepare(c, nPairs, steps, steps, false);
+  int rc = adjPrepare(c, nPairs, steps);
   if (rc) return rc;
   const size_t nObj = 2 * nPairs;
   std::vector<double> st(6 * nObj), bc(nObj), aom(nObj), off(6 * nPairs);
