@@ -53,7 +53,7 @@ constexpr int kJacWords = 18;
 __device__ __forceinline__ void accelJacobian(uint32_t mask, const double r[3], const double v[3], double aom,
                                               double bcInv, const EphEntry &e, const double2 *atm, double *m) {
   const double x = r[0], y = r[1], z = r[2];
-  const double r2 = x * x + y * y + z * z, rinv = rsqrt(r2);
+  const double r2 = x * x + y * y + z * z, rinv = rsqrtOf(r2);
   double xx = 0.0, xy = 0.0, xz = 0.0, yy = 0.0, yz = 0.0, zz = 0.0;
   if (mask & (kPropKEP | kPropJ2 | kPropJ3 | kPropTesseral)) {
     const double i2 = rinv * rinv, i3 = i2 * rinv, i5 = i3 * i2, i7 = i5 * i2, q = z * z * i2;
@@ -96,7 +96,7 @@ __device__ __forceinline__ void accelJacobian(uint32_t mask, const double r[3], 
   }
   if (mask & (kPropSOL | kPropSRP)) {
     const double dx = e.sun[0] - x, dy = e.sun[1] - y, dz = e.sun[2] - z;
-    const double di = rsqrt(dx * dx + dy * dy + dz * dz), di2 = di * di;
+    const double di = rsqrtOf(dx * dx + dy * dy + dz * dz), di2 = di * di;
     double k = (mask & kPropSOL) ? kMuSun : 0.0;
     if ((mask & kPropSRP) && !inShadow(x, y, z, r2, e.sunHat)) k -= kSrpCoef * aom;
     k *= di2 * di;
@@ -110,7 +110,7 @@ __device__ __forceinline__ void accelJacobian(uint32_t mask, const double r[3], 
   }
   if (mask & kPropLUN) {
     const double dx = e.moon[0] - x, dy = e.moon[1] - y, dz = e.moon[2] - z;
-    const double di = rsqrt(dx * dx + dy * dy + dz * dz), di2 = di * di;
+    const double di = rsqrtOf(dx * dx + dy * dy + dz * dz), di2 = di * di;
     const double k = kMuMoon * (di2 * di);
     const double k3 = 3.0 * k * di2, tx = k3 * dx, ty = k3 * dy, tz = k3 * dz;
     xx += tx * dx - k;
@@ -123,7 +123,7 @@ __device__ __forceinline__ void accelJacobian(uint32_t mask, const double r[3], 
   double yx = xy, zx = xz, zy = yz;
   if (mask & kPropDRAG) {
     const double wx = v[0] + kOmegaEarth * y, wy = v[1] - kOmegaEarth * x, wz = v[2];
-    const double w2 = wx * wx + wy * wy + wz * wz, winv = w2 > 0.0 ? rsqrt(w2) : 0.0, wn = w2 * winv;
+    const double w2 = wx * wx + wy * wy + wz * wz, winv = w2 >= DBL_MIN ? rsqrtOf(w2) : 0.0, wn = w2 * winv;
     const double2 air = atmDensity(atm, r2 * rinv - kREarth);
     const double c4 = -0.5e3 * air.x * wn, c1 = c4 * bcInv, c2 = -0.5e3 * air.x * bcInv * winv;
     const double ex = c2 * wx, ey = c2 * wy;
@@ -260,7 +260,7 @@ struct EphStage {
 // warp still reads for stage n.  Lanes past the last object step a copy of it
 // (every warp reaches every barrier) and write nothing.  4096 pairs, full set, per
 // step: 2.24 us with four warps that share the terms by the runtime mask and
-// all take the miss distance, 1.34 like this.
+// all take the miss distance, 1.29 like this.
 template <uint32_t MASK>
 __global__ void __launch_bounds__(kAdjFwdThreads) k_adj_forward(
     const double *__restrict__ st, const double *__restrict__ bc, const double *__restrict__ aom, int nObj, int s0,
@@ -376,7 +376,7 @@ __global__ void __launch_bounds__(kAdjFwdThreads) k_adj_forward(
 // steps before; one block barrier per three steps, two buffers.  The producers'
 // loads are issued one batch ahead.  4096 pairs, full set, per step: 4.28 us with the
 // products of each kick formed on the chain (and the segments' states again),
-// 0.79 like this, bound by the FP64 pipe; 512 pairs 3.89 -> 0.47, bound by the chain.
+// 0.76 like this, bound by the FP64 pipe; 512 pairs 3.89 -> 0.45, bound by the chain.
 constexpr int kAdjBatchSteps = 3;
 constexpr int kAdjProducers = 3 * kAdjBatchSteps;
 constexpr int kAdjBwdThreads = (kAdjProducers + 1) * 32;

@@ -22,11 +22,14 @@
 // Measured (1e6 objects, full set, 128 steps in a launch, per step; before: the
 // terms one by one): FP64 47.7 -> 33.4 us by the sharing, 30.0 with the density
 // table, 27.4 with the mask known at compile time; split 33.8 -> 30.2 -> 26.9 us
-// (10,000 objects: 3.2 -> 2.2 and 2.4 -> 1.7 us).  The split form's binary32 terms
+// (10,000 objects: 3.2 -> 2.2 and 2.4 -> 1.7 us).  Then rsqrtOf: 200,000 objects x 720
+// steps in FP64 4.99 -> 4.66 ms, 1e6 split 7.35 -> 7.12 ms for the same steps.  The split form's binary32 terms
 // keep their order of operations: evaluated with fewer operations they move an
 // object by 1e-8 km in 128 steps; two objects at a time in paired binary32
 // instructions were no gain (28.7 against 30.2 us before the mask was known).
 #pragma once
+#include <cfloat>
+
 #include "physics.cuh"
 
 namespace ladds {
@@ -89,8 +92,23 @@ __device__ __forceinline__ double2 atmDensity(const double2 *__restrict__ fine, 
   return make_double2(t.x * (even + x * odd), t.y);
 }
 
-// x sqrt(1 / x), 0 at 0
-__device__ __forceinline__ double sqrtOf(double x) { return x > 0.0 ? x * rsqrt(x) : x; }
+// 1 / sqrt(x) of a normal x > 0: the hardware's approximation y (its low word
+// is zero, so y y is exact; relative error below 2^-20) and three terms of the
+// binomial series of (1 - e)^(-1/2), e = 1 - x y^2.  What the series leaves out
+// is below 2^-77; measured within 0.5000 ulp (the library's function: 0.508).
+// Without that function's branch for special arguments the reciprocal roots of a
+// force evaluation run side by side: three of them, one warp, 212 -> 91 cycles; 16
+// warps on one SM 280 -> 201 (one alone 79 -> 68).
+// NaN at 0 and infinity, where an acceleration is NaN either way.
+__device__ __forceinline__ double rsqrtOf(double x) {
+  double y;
+  asm("rsqrt.approx.ftz.f64 %0, %1;" : "=d"(y) : "d"(x));
+  const double e = fma(-x, y * y, 1.0);
+  return fma(fma(fma(5.0 / 16, e, 3.0 / 8), e, 0.5), e * y, y);
+}
+
+// sqrt(x) of a normal x; x itself below, and for NaN
+__device__ __forceinline__ double sqrtOf(double x) { return x >= DBL_MIN ? x * rsqrtOf(x) : x; }
 
 // the Earth's gravity terms of the mask: acceleration sr r + (ax, ay, az),
 // added to sr and a; r2 = |r|^2, rinv = 1 / |r|
@@ -127,7 +145,7 @@ __device__ __forceinline__ void accel(uint32_t mask, const double r[3], const do
                                       const EphEntry &e, const double2 *fine, double a[3]) {
   const double x = r[0], y = r[1], z = r[2];
   const double r2 = x * x + y * y + z * z;
-  const double rinv = rsqrt(r2);
+  const double rinv = rsqrtOf(r2);
   double c[3] = {0.0, 0.0, 0.0}, sr = 0.0;
   if (mask & (kPropSOL | kPropLUN)) {
 #pragma unroll
@@ -135,7 +153,7 @@ __device__ __forceinline__ void accel(uint32_t mask, const double r[3], const do
   }
   if (mask & (kPropSOL | kPropSRP)) {
     const double dx = e.sun[0] - x, dy = e.sun[1] - y, dz = e.sun[2] - z;
-    const double di = rsqrt(dx * dx + dy * dy + dz * dz);
+    const double di = rsqrtOf(dx * dx + dy * dy + dz * dz);
     double k = (mask & kPropSOL) ? kMuSun : 0.0;
     if ((mask & kPropSRP) && !inShadow(x, y, z, r2, e.sunHat)) k -= kSrpCoef * aom;
     k *= di * di * di;
@@ -145,7 +163,7 @@ __device__ __forceinline__ void accel(uint32_t mask, const double r[3], const do
   }
   if (mask & kPropLUN) {
     const double dx = e.moon[0] - x, dy = e.moon[1] - y, dz = e.moon[2] - z;
-    const double di = rsqrt(dx * dx + dy * dy + dz * dz);
+    const double di = rsqrtOf(dx * dx + dy * dy + dz * dz);
     const double k = kMuMoon * di * di * di;
     c[0] += k * dx;
     c[1] += k * dy;
@@ -180,7 +198,7 @@ __device__ __forceinline__ float subf(float a, float b) { return __fsub_rn(a, b)
 __device__ __forceinline__ float fmaf_(float a, float b, float c) { return __fmaf_rn(a, b, c); }
 
 // Battin's f(q) = (1+q)^{3/2} - 1 written without cancellation.  The
-// binary32 terms use the approximate square root (s * rsqrt(s)) and division
+// binary32 terms use the approximate square root (s * rsqrtOf(s)) and division
 // of the hardware: their few-ulp errors are far below the split form's
 // binary32 rounding of the perturbations themselves.
 __device__ __forceinline__ float battinF(float q) {
@@ -207,7 +225,7 @@ __device__ __forceinline__ void accel(uint32_t mask, const double r[3], const do
                                       const EphEntryF &e, const AtmShared &atm, double a[3]) {
   const double x = r[0], y = r[1], z = r[2];
   const double r2 = x * x + y * y + z * z;
-  const double rinv = rsqrt(r2);
+  const double rinv = rsqrtOf(r2);
   const double rinv2 = rinv * rinv;
   const float rf[3] = {(float)x, (float)y, (float)z};
   float b[3] = {0.f, 0.f, 0.f};

@@ -80,3 +80,26 @@ def test_mask_kernels(capi, oracle, mask, precision, n):
     oracle.propagate(ref, m, 10.0, 20)
     for g, r in zip(states[1], (ref.x, ref.y, ref.z)):
         assert np.max(np.abs(g - r)) < (1e-9 if precision == 0 else 1e-6)
+
+
+@pytest.mark.parametrize("mask", ["kepler", "full"])
+def test_reciprocal_roots_over_their_range(capi, oracle, mask):
+    """Distances from 100 km to 1e7 km and air-relative speeds down to a standstill
+    (where the drag's root has no argument): one step of 1 s against the oracle.  1e-9 km and
+    a few units in the last place of the largest positions."""
+    bits = capi.KEP if mask == "kepler" else capi.PROP_ALL
+    radius = np.concatenate([np.geomspace(1e2, 1e7, 241) if mask == "kepler" else np.geomspace(6500.0, 1e7, 241)])
+    n = len(radius)
+    pop = at_altitudes(radius - 6378.137, 0.01)
+    pop["vy"] = np.where(np.arange(n) % 3 == 0, 7.292115146706979e-5 * radius, np.sqrt(398600.4418 / radius))
+    pop["vz"] = 0.0 * radius
+    with capi.Context(capi.default_config(componentMask=bits, deltaT=1.0)) as ctx:
+        ctx.upload(pop)
+        ctx.integrate(1)
+        got = ctx.get_state()
+    from ladds_b200.population import as_population
+
+    ref = to_oracle(oracle, {k: v.copy() for k, v in as_population(pop).items()})
+    oracle.propagate(ref, bits, 1.0, 1)
+    for g, r in zip(got, (ref.x, ref.y, ref.z, ref.vx, ref.vy, ref.vz)):
+        assert np.all(np.abs(g - r) < 1e-9 + 4e-15 * radius)
