@@ -783,6 +783,27 @@ void replaySwaps(ladds_gpu_ctx *c, int64_t itStart, int len, int k) {
   if (scans % 2 == 1) swapSortSets(c);
 }
 
+// The buffers of a call's start state are baked into its graphs, and a call leaves
+// them one or two places on: three captures of the same chunk (six with the sort
+// sets).  Before a call of some length the state goes back to the first buffer
+// and the first sort set instead, so that the second call of a loop finds or makes its last
+// graph: 31,000 objects, 128 iterations a call: the copy is 10 us of 2.8 ms, a
+// capture 13 - 35 ms, which the fourth to the sixth call had each.  Short calls keep
+// their roles: their captures are short too.
+constexpr int kHomeIterations = 32;
+
+int homeBuffers(ladds_gpu_ctx *c, bool scans) {
+  if (c->cur.x != c->homeX[0]) {
+    const DevState from = c->cur;
+    do rotateStates(c);
+    while (c->cur.x != c->homeX[0]);
+    CK(copyDynamic(from, c->cur, c->n, c->st));
+  }
+  // without a scan the call leaves the last scan's cell order, in the set that is current
+  if (scans && c->sortParity) swapSortSets(c);
+  return LADDS_OK;
+}
+
 // whether every chunk of a call has a graph, has run before, or comes twice in
 // the call; notes those that come for the first time
 bool chunksWorthCapturing(ladds_gpu_ctx *c, int64_t it0, int iterations, int k) {
@@ -1680,6 +1701,10 @@ int ladds_gpu_step(ladds_gpu_ctx *c, int iterations, ladds_pair *out, size_t cap
   const int k = c->cfg.timestepsPerCollisionDetection;
   int scans = 0;
   for (int i = 0; i < iterations; ++i) scans += ((c->hostIter + i) % k) == 0;
+  if (c->cfg.useGraphs && !c->profiling && c->n < kGraphObjects && iterations >= kHomeIterations) {
+    const int rc = homeBuffers(c, scans > 0);
+    if (rc) return rc;
+  }
   // the call's start state: the call is re-run after a device pair-buffer
   // overflow and undone when the caller's buffer is too small.  A call of one
   // propagation launch leaves it in its buffer; for longer ones it is copied,

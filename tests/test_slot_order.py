@@ -108,6 +108,30 @@ def test_overlapped_iterations_equal_single_ones(capi, every, precision):
                 assert np.array_equal(p, q)
 
 
+@pytest.mark.parametrize("every", [1, 4, 100])
+def test_graph_calls_from_every_buffer(capi, every):
+    """Calls of the iterations that graphs are kept for, begun in each of the
+    ring's buffers and sort sets (calls of 1 to 5 iterations in between), and
+    calls without a scan after one with: records, states and the order in which
+    records leave equal those of launches one by one."""
+    import torch
+
+    pop = capi.generate_population(0, 5, 3001)
+    kw = dict(componentMask=capi.PROP_ALL, timestepsPerCollisionDetection=every, conjunctionThreshold=70.0)
+    with capi.Context(capi.default_config(**kw)) as a, capi.Context(capi.default_config(useGraphs=0, **kw)) as b:
+        bufs = [torch.zeros(3001 * capi.STATE_RECORD_DTYPE.itemsize, dtype=torch.uint8, device="cuda") for _ in range(2)]
+        for ctx in (a, b):
+            ctx.upload(pop)
+        for steps in (40, 1, 40, 2, 40, 3, 40, 40, 5, 40, 33, 40):
+            got, want = a.step(steps).records, b.step(steps).records
+            assert got.tobytes() == want.tobytes()
+            for p, q in zip(a.get_state(), b.get_state()):
+                assert np.array_equal(p, q)
+            for ctx, buf in zip((a, b), bufs):
+                assert ctx.pack_layers(0, ctx.grid()[0][2], False, buf, 3001) == 3001
+            assert torch.equal(*bufs)
+
+
 @pytest.mark.parametrize("screen", [0, 1])
 @pytest.mark.parametrize("cell", [20.0, 15.0, 14.0, 10.0, 7.0, 5.0, 2.5])
 def test_pair_walk_for_every_reach(capi, oracle, cell, screen):
