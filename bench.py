@@ -145,16 +145,16 @@ def algorithmic_units(n):
     """Per-step algorithmic bytes of each phase: the bytes the phase must move per object
     at the least, from the data each kernel reads and writes (listed per entry)."""
     return {
-        # read r, v, aom, bcInv, tag (68 B), write r, v (48 B), write the cell key (4 B)
-        "propagate": {"bytes": n * 120},
-        # count (key 4), scatter (key + tag 8 in, record + source 12 out)
-        "bucket": {"bytes": n * (4 + 8 + 12)},
-        # row sort: record + source in (12), sorted key + slot out (8)
-        "rowsort": {"bytes": n * (12 + 8)},
-        # gather r, v, aom, bcInv, tag (68 B) + perm 4 into cell order, radius by slot (8 B); write 68 B SoA
-        # + 32 B binary32 position / velocity copies (radius, id, parent stay in slot order)
-        "permute": {"bytes": n * (68 + 4 + 8 + 68 + 32)},
-        # own key, tag, posf (24 B) + the closest-approach screen of the pre-filtered pairs: binary32
+        # read r, v, aom, bcInv, radius, tag (76 B), write r, v (48 B), the cell key, the arrival index
+        # (8 B) and the binary32 scan record (32 B)
+        "propagate": {"bytes": n * (76 + 48 + 8 + 32)},
+        # placement: key, arrival index in (8), record + source out (12)
+        "bucket": {"bytes": n * (8 + 12)},
+        # row sort: record + source in (12), sorted key + slot out (8), scan record in and out (64)
+        "rowsort": {"bytes": n * (12 + 8 + 64)},
+        # the state stays in slot order: no launches
+        "permute": {"bytes": 0},
+        # own key, slot, binary32 position (24 B) + the closest-approach screen of the pre-filtered pairs: binary32
         # position + velocity of both objects (64 B, ~1.5 pairs per object)
         "candidates": {"bytes": n * (24 + 96)},
         # FP64 records of the few screened pairs (a few per thousand objects): no per-object traffic

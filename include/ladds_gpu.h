@@ -111,12 +111,13 @@ typedef struct {
                                      (0: 256); the propagation before a scan runs a
                                      persistent kernel of 256-object tiles */
   int32_t scanBlock;              /* threads per block of the candidate evaluation (0: 256) */
-  int32_t useGraphs;              /* capture multi-iteration calls in CUDA graphs      */
+  int32_t useGraphs;              /* capture multi-iteration calls in CUDA graphs (below
+                                     125,000 objects, for calls that come again)       */
   uint64_t pairCapacity;          /* initial device pair-buffer capacity (0: auto)     */
   int32_t scanScreen;             /* LADDS_SCREEN_*: how the pair scan screens full
                                      candidate buffers (results do not depend on it)   */
-  int32_t walkForm;               /* LADDS_WALK_*: how the candidate walk deals its
-                                     items (results do not depend on it)               */
+  int32_t walkForm;               /* LADDS_WALK_*: accepted, without effect: one form of
+                                     the pair walk is the fastest for every reach      */
 } ladds_gpu_config;
 
 /* The binary32 closest-approach screen of the pre-filtered pairs (a superset
@@ -406,10 +407,10 @@ int ladds_gpu_cell_sort_noalloc(int device, void *stream, const uint32_t *keys, 
  * ladds_gpu_set_profiling(ctx, 1) (CUDA events on the context's stream; calls
  * then run without graphs and without overlapping scans; the per-chunk
  * ephemeris kernel belongs to no phase):
- *   propagate   Yoshida step + cell keys (k_propagate)
- *   bucket      row counting sort: counts, row-start scan, scatter
- *   rowsort     sort inside the rows + cell-offset tables
- *   permute     gather into cell order + packed scan copies
+ *   propagate   Yoshida steps, cell keys, row counts and scan records
+ *   bucket      row-start scan, placement into rows
+ *   rowsort     sort inside the rows, cell-offset tables, scan records into cell order
+ *   permute     (no launches: the state stays in slot order)
  *   candidates  half-shell walk, pre-filter, exact gate, compaction
  *   evaluate    functor on the gated candidates */
 typedef struct {
