@@ -376,7 +376,7 @@ __global__ void __launch_bounds__(kAdjFwdThreads) k_adj_forward(
 // steps before; one block barrier per three steps, two buffers.  The producers'
 // loads are issued one batch ahead.  4096 pairs, full set, per step: 4.28 us with the
 // products of each kick formed on the chain (and the segments' states again),
-// 0.76 like this, bound by the FP64 pipe; 512 pairs 3.89 -> 0.45, bound by the chain.
+// 0.76 like this (FP64 pipe 51 % busy); 512 pairs 3.89 -> 0.45.
 constexpr int kAdjBatchSteps = 3;
 constexpr int kAdjProducers = 3 * kAdjBatchSteps;
 constexpr int kAdjBwdThreads = (kAdjProducers + 1) * 32;

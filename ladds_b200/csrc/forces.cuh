@@ -22,8 +22,8 @@
 // Measured (1e6 objects, full set, 128 steps in a launch, per step; before: the
 // terms one by one): FP64 47.7 -> 33.4 us by the sharing, 30.0 with the density
 // table, 27.4 with the mask known at compile time; split 33.8 -> 30.2 -> 26.9 us
-// (10,000 objects: 3.2 -> 2.2 and 2.4 -> 1.7 us).  Then rsqrtOf: 200,000 objects x 720
-// steps in FP64 4.99 -> 4.66 ms, 1e6 x 240 split 7.35 -> 7.12 ms.  The split form's binary32 terms
+// (10,000 objects: 3.2 -> 2.2 and 2.4 -> 1.7 us).  Then rsqrtOf: 25.8 and 25.7 us
+// (10,000 objects: 1.8 and 1.5 us).  The split form's binary32 terms
 // keep their order of operations: evaluated with fewer operations they move an
 // object by 1e-8 km in 128 steps; two objects at a time in paired binary32
 // instructions were no gain (28.7 against 30.2 us before the mask was known).
