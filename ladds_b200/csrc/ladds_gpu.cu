@@ -2425,22 +2425,22 @@ int ladds_gpu_autotune(ladds_gpu_ctx *c, int stepsPerTrial, ladds_tune_trial *tr
     }
     return LADDS_OK;
   };
-  // 0. where full candidate buffers are screened (the population's density
-  //    decides), at the current cell edge
+  // 0. the current cell edge, with full candidate buffers listed and screened
+  //    in place (the population's density decides)
+  const int screens[] = {LADDS_SCREEN_LISTS, LADDS_SCREEN_BUFFER};
   {
     const ladds_gpu_config base = cfg;
-    for (int screen : {LADDS_SCREEN_LISTS, LADDS_SCREEN_BUFFER})
-      for (int walk : {LADDS_WALK_GROUPED, LADDS_WALK_ROWS}) {
-        ladds_gpu_config k = base;
-        k.scanScreen = screen;
-        k.walkForm = walk;
-        const int rc = run(k, bestChunk);
-        if (rc) return rc;
-      }
+    for (int screen : screens) {
+      ladds_gpu_config k = base;
+      k.scanScreen = screen;
+      const int rc = run(k, bestChunk);
+      if (rc) return rc;
+    }
   }
   // 1. cell edge in [20, 160] km: cutoff / R (neighbour reach R = 1..4) and
-  //    coarser cells 1.5 and 2 cutoffs wide (reach 1); the current edge is
-  //    measured already
+  //    coarser cells 1.5 and 2 cutoffs wide (reach 1), each with both screens,
+  //    whose order differs between edges (8e6 small debris: 80 km 5.6 ms listed, 5.7
+  //    in place; 40 km 4.3 and 3.0); the current edge is measured already
   {
     const ladds_gpu_config base = cfg;
     std::vector<double> cells = {base.cellSize};
@@ -2452,20 +2452,14 @@ int ladds_gpu_autotune(ladds_gpu_ctx *c, int stepsPerTrial, ladds_tune_trial *tr
       if (cs < 20.0 || cs > 160.0) continue;
       if (i == 1 && base.cellSize <= 0) continue;  // the default edge: measured as the current one
       if (i > 1 && cs == base.cellSize) continue;
-      ladds_gpu_config k = base;
-      k.cellSize = cs;
-      const int rc = run(k, bestChunk);
-      if (rc) return rc;
+      for (int screen : screens) {
+        ladds_gpu_config k = base;
+        k.cellSize = cs;
+        k.scanScreen = screen;
+        const int rc = run(k, bestChunk);
+        if (rc) return rc;
+      }
     }
-  }
-  // 1b. the other walk form at the chosen cell edge (the form that suits a
-  //     cell edge depends on the items per window, which the edge sets)
-  {
-    const ladds_gpu_config base = cfg;
-    ladds_gpu_config k = base;
-    k.walkForm = base.walkForm == LADDS_WALK_ROWS ? LADDS_WALK_GROUPED : LADDS_WALK_ROWS;
-    const int rc = run(k, bestChunk);
-    if (rc) return rc;
   }
   // 2. block shapes of the propagation and of the pair evaluation
   {
