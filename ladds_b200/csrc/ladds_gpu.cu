@@ -34,6 +34,7 @@
 #include "pair_scan.cuh"
 #include "propagate.cuh"
 #include "adjoint.cuh"
+#include "device_buffers.h"
 #include "insert.cuh"
 #include "population.h"
 
@@ -153,11 +154,23 @@ size_t layoutObjects(ObjectBuffers &o, size_t cap, char *base) {
   return at;
 }
 
+// The cell grid and the row tables that go with it.
+struct GridTables {
+  GridDesc grid{};
+  uint32_t nRows = 0;
+  char *tables = nullptr;                 // the allocation behind the row tables
+  uint32_t *rowCounts = nullptr;          // objects per row; all zero but between a propagation and its sort
+  uint32_t *longRows = nullptr;           // rows with more than 256 objects
+  uint32_t *rowStart = nullptr;
+  uint16_t *cellOff = nullptr;            // per row: offset of every cell inside the row (cellOffPitch entries)
+  uint32_t *rowStartB = nullptr, *rowCountsB = nullptr;  // those of the second set
+  uint16_t *cellOffB = nullptr, *cellOffBase = nullptr;
+};
+
 }  // namespace
 
-struct ladds_gpu_ctx : ObjectBuffers {
+struct ladds_gpu_ctx : ObjectBuffers, GridTables {
   ladds_gpu_config cfg{};
-  GridDesc grid{};
   PropConsts pc{};
   ScanConsts sc{};
   double theta0 = 0;
@@ -173,17 +186,12 @@ struct ladds_gpu_ctx : ObjectBuffers {
   int64_t *dIterBase = nullptr;  // first iteration of the chunk being run (device)
   size_t n = 0, cap = 0;
   char *objects = nullptr;  // the allocation behind the object buffers
-  char *tables = nullptr;   // the allocation behind the row tables
   char *words = nullptr;    // the allocation behind the counters and small tables
   CallMail *mail = nullptr;
-  uint32_t *rowCounts = nullptr;          // objects per row; all zero but between a propagation and its sort
-  uint32_t *longRows = nullptr, *longCount = nullptr;  // rows with more than 256 objects
-  uint16_t *cellOff = nullptr;            // per row: offset of every cell inside the row (cellOffPitch entries)
+  uint32_t *longCount = nullptr;          // entries of longRows
   uint32_t *scanWs = nullptr;             // block sums of the exclusive scans
   size_t scanWsWords = 0;
   bool anyParent = false;                 // some object has a parent id: the scan writes and reads grp
-  uint32_t *rowStart = nullptr;
-  uint32_t nRows = 0;
   ladds_pair *dPairs = nullptr;
   size_t pairCap = 0;
   unsigned long long *dCount = nullptr;
@@ -216,10 +224,9 @@ struct ladds_gpu_ctx : ObjectBuffers {
   int chunkSteps = kMaxEphSteps;  // iterations per ephemeris chunk / captured graph (autotuned)
   uint32_t *denseCount = nullptr;  // entries of the dense bin
   uint32_t haloStart = 0xffffffffu;  // objects with slot >= haloStart: pair-scan targets only
-  // the row tables and counters of the second set
-  uint32_t *rowStartB = nullptr, *rowCountsB = nullptr, *denseCountB = nullptr;
+  // the counters of the second set
+  uint32_t *denseCountB = nullptr;
   unsigned long long *dCandCountB = nullptr;
-  uint16_t *cellOffB = nullptr, *cellOffBase = nullptr;
   int sortParity = 0;
   struct Adjoint {          // buffers of the adjoint pair batch (ladds_gpu_adjoint_*)
     size_t nPairs = 0;
@@ -285,20 +292,19 @@ void dropGraphs(ladds_gpu_ctx *c) {
 
 int ensureCandCapacity(ladds_gpu_ctx *c, size_t need);
 
+// device memory, or null where there is none
+void *deviceTake(size_t bytes) {
+  void *p = nullptr;
+  if (cudaMalloc(&p, bytes) == cudaSuccess) return p;
+  cudaGetLastError();
+  return nullptr;
+}
+
 // block sums of the three-level exclusive scans (objects or rows, whichever is longer)
 bool ensureScanWorkspace(ladds_gpu_ctx *c, size_t objects) {
   const size_t scanLen = std::max(objects + 1, (size_t)c->nRows + 1);
   const size_t need = 4 * (scanLen / kScanBlock + 2) + 4 * kScanBlock;
-  if (c->scanWs && need <= c->scanWsWords) return true;
-  if (c->scanWs) cudaFree(c->scanWs);
-  c->scanWs = nullptr;
-  c->scanWsWords = 0;
-  if (cudaMalloc(&c->scanWs, need * sizeof(uint32_t)) != cudaSuccess) {
-    cudaGetLastError();
-    return false;
-  }
-  c->scanWsWords = need;
-  return true;
+  return growBuffer(c->scanWs, c->scanWsWords, need, deviceTake, cudaFree);
 }
 
 int ensureCapacity(ladds_gpu_ctx *c, size_t need) {
@@ -308,12 +314,10 @@ int ensureCapacity(ladds_gpu_ctx *c, size_t need) {
   newCap = std::min(newCap, kMaxObjects);
   ObjectBuffers fresh;
   const size_t bytes = layoutObjects(fresh, newCap, nullptr);
-  char *base = nullptr;
-  const cudaError_t e = cudaMalloc(&base, bytes);
-  if (e != cudaSuccess || !ensureScanWorkspace(c, newCap)) {
-    cudaGetLastError();
+  char *base = static_cast<char *>(deviceTake(bytes));
+  if (!base || !ensureScanWorkspace(c, newCap)) {
     if (base) cudaFree(base);
-    return fail(c, LADDS_ERR_ALLOC, std::string("device allocation failed: ") + cudaGetErrorString(e));
+    return fail(c, LADDS_ERR_ALLOC, "device allocation failed: no memory for " + std::to_string(newCap) + " objects");
   }
   layoutObjects(fresh, newCap, base);
   const size_t orderN = std::min(c->orderN, c->n);
@@ -2489,22 +2493,32 @@ int ladds_gpu_autotune(ladds_gpu_ctx *c, int stepsPerTrial, ladds_tune_trial *tr
   std::lock_guard<std::mutex> lk(g_deviceMutex[c->dev & 63]);
   CK(cudaSetDevice(c->dev));
   CK(cudaStreamSynchronize(c->st));
-  const bool regrid = cfg.cellSize != c->cfg.cellSize;
-  c->cfg.cellSize = cfg.cellSize;
+  if (cfg.cellSize != c->cfg.cellSize) {  // new tables beside the old ones: without memory for them, all stays as it was
+    const double edge = c->cfg.cellSize;
+    const GridTables old = *c;
+    static_cast<GridTables &>(*c) = GridTables{};
+    c->cfg.cellSize = cfg.cellSize;
+    int rc = buildGrid(c);
+    if (!rc) rc = allocGridBuffers(c);
+    if (!rc && c->cap && !ensureScanWorkspace(c, c->cap)) rc = fail(c, LADDS_ERR_ALLOC, "autotune: scan workspace");
+    GridTables spare = old;
+    if (rc) {
+      spare = *c;
+      static_cast<GridTables &>(*c) = old;
+      c->cfg.cellSize = edge;
+    }
+    CK(cudaStreamSynchronize(c->st));  // the new tables are cleared
+    if (spare.tables) cudaFree(spare.tables);
+    if (spare.cellOffBase) cudaFree(spare.cellOffBase);
+    if (rc) return rc;
+    c->orderValid = false;
+  }
   c->cfg.propagateBlock = cfg.propagateBlock;
   c->cfg.scanBlock = cfg.scanBlock;
   c->cfg.scanScreen = cfg.scanScreen;
   c->cfg.walkForm = cfg.walkForm;
   c->chunkSteps = bestChunk;
   dropGraphs(c);
-  if (regrid) {
-    freeGridBuffers(c);
-    int rc = buildGrid(c);
-    if (!rc) rc = allocGridBuffers(c);
-    if (rc) return rc;
-    if (c->cap && !ensureScanWorkspace(c, c->cap)) return fail(c, LADDS_ERR_ALLOC, "autotune: scan workspace");
-    c->orderValid = false;
-  }
   *best = bestT;
   if (nTrials) *nTrials = all.size();
   for (size_t i = 0; i < all.size() && i < cap; ++i) trials[i] = all[i];
