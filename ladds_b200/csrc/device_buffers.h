@@ -1,4 +1,4 @@
-// device_buffers.h -- growth of a device buffer, free of CUDA: the allocator is a parameter.
+// device_buffers.h -- growth and layout rules of device buffers, free of CUDA: the allocator is a parameter.
 #pragma once
 #include <cstddef>
 
@@ -19,5 +19,10 @@ bool growBuffer(T *&p, size_t &cap, size_t need, Take take, Give give) {
   cap = need;
   return true;
 }
+
+// whether a two-dimensional copy takes rows this many bytes apart: the driver
+// refuses a pitch above 2^31 - 1 (cudaDeviceProp::memPitch), which arrays of
+// 2^28 - 1 doubles in 256-byte steps exceed
+constexpr bool copyPitchFits(size_t bytes) { return bytes <= ((size_t)1 << 31) - 1; }
 
 }  // namespace ladds

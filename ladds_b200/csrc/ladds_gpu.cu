@@ -1075,10 +1075,10 @@ void hostCopy(double *const dst[6], const double *const src[6], const bool use[6
 }
 
 // six arrays, elements [lo, lo + len): one two-dimensional copy where both
-// sides hold them at one distance, else a copy each
+// sides hold them at one distance that such a copy can take, else a copy each
 cudaError_t copySix(double *const dst[6], const double *const src[6], size_t lo, size_t len, bool together,
                     size_t srcStride, size_t dstStride, cudaMemcpyKind kind, cudaStream_t st) {
-  if (together)
+  if (together && copyPitchFits(srcStride * sizeof(double)) && copyPitchFits(dstStride * sizeof(double)))
     return cudaMemcpy2DAsync(dst[0] + lo, dstStride * sizeof(double), src[0] + lo, srcStride * sizeof(double),
                              len * sizeof(double), 6, kind, st);
   for (int a = 0; a < 6; ++a) {

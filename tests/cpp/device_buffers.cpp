@@ -1,4 +1,5 @@
-// Growth of a device buffer with an allocator that runs out of memory.
+// Growth of a device buffer with an allocator that runs out of memory; the
+// distance of arrays that one two-dimensional copy can take.
 #include "device_buffers.h"
 
 #include <cassert>
@@ -32,6 +33,9 @@ int main() {
   assert(ladds::growBuffer(p, cap, 150, take, give) && p != first && cap == 150 && held == 600);
   give(p);
   assert(held == 0);
+  // arrays of the largest population (28-bit slots), each on a 256-byte boundary
+  const size_t apart = ((((size_t)1 << 28) - 1) * sizeof(double) + 255) / 256 * 256;
+  assert(!ladds::copyPitchFits(apart) && ladds::copyPitchFits(apart - 256) && ladds::copyPitchFits(8));
   std::puts("device_buffers: ok");
   return 0;
 }

@@ -1,4 +1,5 @@
-"""Growth of the device buffers where memory runs out (tests/cpp/device_buffers.cpp, on the CPU)."""
+"""Growth of the device buffers where memory runs out, and the arrays too far apart
+for one two-dimensional copy (tests/cpp/device_buffers.cpp, on the CPU)."""
 import os
 import shutil
 import subprocess
