@@ -1705,17 +1705,24 @@ int ladds_gpu_step(ladds_gpu_ctx *c, int iterations, ladds_pair *out, size_t cap
   const int k = c->cfg.timestepsPerCollisionDetection;
   int scans = 0;
   for (int i = 0; i < iterations; ++i) scans += ((c->hostIter + i) % k) == 0;
-  if (c->cfg.useGraphs && !c->profiling && c->n < kGraphObjects && iterations >= kHomeIterations) {
+  // the call's start state and the order of the last scan: the call is re-run
+  // after a device pair-buffer overflow and undone when the caller's buffer is
+  // too small.  A call of one propagation launch leaves the state in its buffer and
+  // the order in the other sort set; for longer ones both are copied, and come
+  // back into the buffer and the set that were current.
+  const bool home = c->cfg.useGraphs && !c->profiling && c->n < kGraphObjects && iterations >= kHomeIterations;
+  const bool oneLaunch = iterations > 0 && iterations <= c->chunkSteps &&
+                         nextGroup(c->hostIter, 0, iterations, k).len == iterations;
+  const size_t orderStart = c->orderN;
+  const bool copyOrder = scans && orderStart && (home || !oneLaunch);
+  if (copyOrder)
+    CK(cudaMemcpyAsync(c->scratchC, c->perm, orderStart * sizeof(uint32_t), cudaMemcpyDeviceToDevice, c->st));
+  if (home) {
     const int rc = homeBuffers(c, scans > 0);
     if (rc) return rc;
   }
-  // the call's start state: the call is re-run after a device pair-buffer
-  // overflow and undone when the caller's buffer is too small.  A call of one
-  // propagation launch leaves it in its buffer; for longer ones it is copied,
-  // and comes back into the buffer that was current.
   const DevState ringStart[3] = {c->cur, c->alt, c->alt2};
-  const bool oneLaunch = iterations > 0 && iterations <= c->chunkSteps &&
-                         nextGroup(c->hostIter, 0, iterations, k).len == iterations;
+  const int setStart = c->sortParity;
   if (!oneLaunch) CK(copyDynamic(c->cur, c->snap, c->n, c->st));
   const int64_t startIter = c->hostIter;
   auto rollBack = [&]() -> int {
@@ -1723,9 +1730,13 @@ int ladds_gpu_step(ladds_gpu_ctx *c, int iterations, ladds_pair *out, size_t cap
     c->alt = ringStart[1];
     c->alt2 = ringStart[2];
     if (!oneLaunch) CK(copyDynamic(c->snap, c->cur, c->n, c->st));
+    if (c->sortParity != setStart) swapSortSets(c);
+    if (copyOrder)
+      CK(cudaMemcpyAsync(c->perm, c->scratchC, orderStart * sizeof(uint32_t), cudaMemcpyDeviceToDevice, c->st));
     CK(cudaMemcpyAsync(c->dIter, &startIter, sizeof(int64_t), cudaMemcpyHostToDevice, c->st));
     CK(cudaStreamSynchronize(c->st));
     c->hostIter = startIter;
+    c->orderN = orderStart;
     c->orderValid = false;
     return LADDS_OK;
   };
@@ -1790,7 +1801,6 @@ int ladds_gpu_step(ladds_gpu_ctx *c, int iterations, ladds_pair *out, size_t cap
     bool overflow = false;
     int rc = syncStatusAndGrow(c, &cnt, &overflow);
     collectTimes(c);
-    if (scans && rc != LADDS_ERR_CUDA && rc != LADDS_ERR_DEVICE_CHECK) c->orderN = c->n;
     if (rc) {
       const int rb = rollBack();
       return rb ? rb : rc;
@@ -1817,7 +1827,10 @@ int ladds_gpu_step(ladds_gpu_ctx *c, int iterations, ladds_pair *out, size_t cap
   }
   if (!recs.empty()) std::memcpy(out, recs.data(), recs.size() * sizeof(ladds_pair));
   c->hostIter += iterations;
-  if (scans) c->orderValid = true;
+  if (scans) {
+    c->orderValid = true;
+    c->orderN = c->n;
+  }
   if (stats) {
     stats->iterations = (uint64_t)iterations;
     stats->scans = (uint64_t)scans;
