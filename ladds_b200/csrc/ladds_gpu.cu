@@ -2388,6 +2388,8 @@ int tuneTrial(ladds_gpu_ctx *c, const ladds_gpu_config &cfg, int chunk, int step
   if (!rc && cudaStreamSynchronize(c->st) != cudaSuccess) rc = fail(c, LADDS_ERR_CUDA, "autotune: state copy");
   if (!rc) {
     tc->n = c->n;
+    tc->anyParent = c->anyParent;  // the trial's scans skip and walk what the context's do
+    tc->haloStart = c->haloStart;
     rc = ladds_gpu_set_iteration(tc, c->hostIter);
   }
   std::vector<ladds_pair> recs((size_t)1 << 16);
