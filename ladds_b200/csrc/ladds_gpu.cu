@@ -216,6 +216,7 @@ struct ladds_gpu_ctx : ObjectBuffers, GridTables {
   using GraphKey = std::tuple<int, int, int, size_t, size_t>;
   std::map<GraphKey, cudaGraphExec_t> graphs;
   std::set<GraphKey> seenChunks;  // chunks that have run once, without a graph
+  bool captureAll = false;        // capture chunks at their first sight (an autotuner trial)
   std::string err;
   ladds_object *dObj = nullptr;  // staging of ladds_gpu_functor_pairs (2 x objCap)
   size_t objCap = 0;
@@ -1747,7 +1748,7 @@ int ladds_gpu_step(ladds_gpu_ctx *c, int iterations, ladds_pair *out, size_t cap
     CK(cudaMemsetAsync(c->dCount, 0, 2 * sizeof(unsigned long long), c->st));
     const int64_t it0 = c->hostIter;
     const bool graph = c->cfg.useGraphs && !c->profiling && iterations >= 1 && c->n < kGraphObjects &&
-                       chunksWorthCapturing(c, it0, iterations, k);
+                       (c->captureAll || chunksWorthCapturing(c, it0, iterations, k));
     if (graph) {
       // pass 1: capture the graphs this call needs (capture performs the host-side
       // buffer swaps; they are undone afterwards), so that no capture happens
@@ -1768,6 +1769,7 @@ int ladds_gpu_step(ladds_gpu_ctx *c, int iterations, ladds_pair *out, size_t cap
           cudaGraphDestroy(gr);
           CK(ie);
           c->graphs.emplace(key, ex);
+          CK(cudaGraphUpload(ex, c->st));  // else its first launch does, inside the timing events
         } else {
           replaySwaps(c, it0 + done, len, k);
         }
@@ -2380,6 +2382,8 @@ int tuneTrial(ladds_gpu_ctx *c, const ladds_gpu_config &cfg, int chunk, int step
   int rc = ladds_gpu_create(&cfg, &tc);
   if (rc) return fail(c, rc, "autotune: a trial context could not be created");
   tc->chunkSteps = chunk;
+  // a trial's calls come once; where the context's come again and run in graphs, the trial's do too
+  tc->captureAll = true;
   rc = ensureCapacity(tc, c->n);
   if (!rc && c->n) {
     const cudaError_t e = copyState(c->cur, tc->cur, c->n, c->st);
@@ -2394,7 +2398,7 @@ int tuneTrial(ladds_gpu_ctx *c, const ladds_gpu_config &cfg, int chunk, int step
   }
   std::vector<ladds_pair> recs((size_t)1 << 16);
   ladds_step_stats st{};
-  for (int pass = 0; pass < 2 && !rc; ++pass) {  // warm-up (captures the graphs), then the timed run
+  for (int pass = 0; pass < 2 && !rc; ++pass) {  // warm-up, then the timed run (captures come before its timing events)
     const int n = pass == 0 ? std::min(steps, 2 * chunk) : steps;
     size_t got = 0;
     rc = ladds_gpu_step(tc, n, recs.data(), recs.size(), &got, &st);

@@ -1,5 +1,5 @@
 """The autotuner's trials run what the tuned context runs: the scan's breakup groups
-and halo."""
+and halo, and graphs where the context's calls run in graphs."""
 import numpy as np
 import pytest
 
@@ -54,3 +54,25 @@ def test_trials_skip_breakup_groups(capi):
         assert a.records.tobytes() == b.records.tobytes()
         for p, q in zip(tuned.get_state(), plain.get_state()):
             assert np.array_equal(p, q)
+
+
+@pytest.mark.parametrize("steps", [16, 128])
+def test_trials_run_in_graphs(capi, steps):
+    """Below 125,000 objects, where launches bound an iteration: trials at the context's
+    edge take the time of its own calls in graphs (15.5 us an iteration here), whatever
+    their chunk length; launched one by one they take 2.3 times as long."""
+    pop = capi.generate_population(0, 31, 10_000)
+    with capi.Context(capi.default_config(conjunctionThreshold=0.5)) as tuned, \
+            capi.Context(capi.default_config(conjunctionThreshold=0.5)) as plain:
+        tuned.upload(pop)
+        plain.upload(pop)
+        own = min(plain.step(128).stats.deviceMs / 128 for _ in range(6))
+        edge = plain.grid()[2]
+        trials = [t for _ in range(2) for t in tuned.autotune(steps)[1]]
+        for screen in (0, 1):
+            assert min(t["msPerStep"] for t in trials if t["cellSize"] == edge and t["scanScreen"] == screen) < 1.5 * own
+        by_chunk = {t["chunkSteps"]: [] for t in trials}
+        for t in trials:
+            by_chunk[t["chunkSteps"]].append(t["msPerStep"])
+        assert set(by_chunk) == {32, 64, 128}
+        assert max(min(v) for v in by_chunk.values()) < 1.5 * own
