@@ -21,7 +21,9 @@
 #include <cstdio>
 #include <cstring>
 #include <map>
+#include <memory>
 #include <mutex>
+#include <new>
 #include <set>
 #include <string>
 #include <tuple>
@@ -308,35 +310,84 @@ bool ensureScanWorkspace(ladds_gpu_ctx *c, size_t objects) {
   return growBuffer(c->scanWs, c->scanWsWords, need, deviceTake, cudaFree);
 }
 
+// What a growth carries over: the population of n objects, and the cell order
+// and keys of the last scan.
+struct Carried {
+  void *at;
+  size_t bytes;
+};
+constexpr int kCarried = 14;
+void carriedArrays(const ObjectBuffers &o, size_t n, size_t orderN, Carried (&a)[kCarried]) {
+  const DevState &s = o.cur;
+  void *const p[kCarried] = {s.x,  s.y,      s.z,  s.vx,     s.vy,  s.vz,   s.aom,
+                             s.bc, s.radius, s.id, s.parent, s.tag, o.perm, o.sortedKeys};
+  for (int k = 0; k < kCarried; ++k) a[k] = {p[k], k < 11 ? n * 8 : k == 11 ? n * 4 : orderN * 4};
+}
+
+// Room for `need` objects.  The new block is taken beside the old one, so that a
+// growth that fails leaves all as it was.  Where both do not fit the device, the
+// population waits in host memory while the old block makes room for the new one
+// (the growth by half needs 644 bytes per object of the old capacity on the device instead of
+// 1073), or comes back where it was if even that is too little.
 int ensureCapacity(ladds_gpu_ctx *c, size_t need) {
   if (need <= c->cap) return LADDS_OK;
   if (need > kMaxObjects) return fail(c, LADDS_ERR_INVALID_ARG, "population exceeds 2^28 - 1 objects");
   size_t newCap = std::max<size_t>({need, c->cap + c->cap / 2, 4096});
   newCap = std::min(newCap, kMaxObjects);
-  ObjectBuffers fresh;
-  const size_t bytes = layoutObjects(fresh, newCap, nullptr);
-  char *base = static_cast<char *>(deviceTake(bytes));
-  if (!base || !ensureScanWorkspace(c, newCap)) {
-    if (base) cudaFree(base);
-    return fail(c, LADDS_ERR_ALLOC, "device allocation failed: no memory for " + std::to_string(newCap) + " objects");
-  }
-  layoutObjects(fresh, newCap, base);
+  const std::string noMemory = "device allocation failed: no memory for " + std::to_string(newCap) + " objects";
+  if (!ensureScanWorkspace(c, newCap)) return fail(c, LADDS_ERR_ALLOC, noMemory);
   const size_t orderN = std::min(c->orderN, c->n);
-  if (c->n) {  // the population and the order of the last scan
-    cudaError_t m = copyState(c->cur, fresh.cur, c->n, c->st);
-    if (m == cudaSuccess && orderN)
-      m = cudaMemcpyAsync(fresh.perm, c->perm, orderN * sizeof(uint32_t), cudaMemcpyDeviceToDevice, c->st);
-    if (m == cudaSuccess) m = cudaStreamSynchronize(c->st);
-    if (m != cudaSuccess) {
-      cudaFree(base);
-      return fail(c, LADDS_ERR_CUDA, cudaGetErrorString(m));
+  Carried from[kCarried], to[kCarried];
+  carriedArrays(*c, c->n, orderN, from);
+  ObjectBuffers fresh;
+  size_t cap = newCap;
+  char *base = static_cast<char *>(deviceTake(layoutObjects(fresh, cap, nullptr)));
+  std::unique_ptr<char[]> aside;
+  if (!base && c->objects) {
+    size_t total = 0;
+    for (const Carried &a : from) total += a.bytes;
+    aside.reset(new (std::nothrow) char[total]);
+    if (!aside) return fail(c, LADDS_ERR_ALLOC, noMemory);
+    char *at = aside.get();
+    for (Carried &a : from) {
+      if (a.bytes) CK(cudaMemcpyAsync(at, a.at, a.bytes, cudaMemcpyDeviceToHost, c->st));
+      a.at = at;
+      at += a.bytes;
     }
+    CK(cudaStreamSynchronize(c->st));
+    dropGraphs(c);
+    cudaFree(c->objects);
+    c->objects = nullptr;
+    base = static_cast<char *>(deviceTake(layoutObjects(fresh, cap, nullptr)));
+    if (!base) {
+      cap = c->cap;
+      base = static_cast<char *>(deviceTake(layoutObjects(fresh, cap, nullptr)));
+    }
+    if (!base) {  // the memory just given back has gone elsewhere
+      static_cast<ObjectBuffers &>(*c) = ObjectBuffers{};
+      c->n = c->cap = c->orderN = 0;
+      c->orderValid = false;
+      return fail(c, LADDS_ERR_ALLOC, noMemory + "; the population could not be put back");
+    }
+  }
+  if (!base) return fail(c, LADDS_ERR_ALLOC, noMemory);
+  layoutObjects(fresh, cap, base);
+  carriedArrays(fresh, c->n, orderN, to);
+  cudaError_t m = cudaSuccess;
+  for (int k = 0; k < kCarried && m == cudaSuccess; ++k)
+    if (from[k].bytes) m = cudaMemcpyAsync(to[k].at, from[k].at, from[k].bytes, cudaMemcpyDefault, c->st);
+  if (m == cudaSuccess) m = cudaStreamSynchronize(c->st);
+  if (m != cudaSuccess && !aside) {
+    cudaFree(base);
+    return fail(c, LADDS_ERR_CUDA, cudaGetErrorString(m));
   }
   if (c->objects) cudaFree(c->objects);
   c->objects = base;
   static_cast<ObjectBuffers &>(*c) = fresh;
   c->orderN = orderN;
-  c->cap = newCap;
+  c->cap = cap;
+  if (m != cudaSuccess) return fail(c, LADDS_ERR_CUDA, cudaGetErrorString(m));
+  if (cap < need) return fail(c, LADDS_ERR_ALLOC, noMemory);
   c->orderValid = false;
   dropGraphs(c);
   // candidates that pass the closest-approach screen: a few per thousand objects at LEO
