@@ -524,8 +524,9 @@ typedef struct {
 
 /* Forward sweep: the loss, per-pair min dl2 (missSq) and its step (tcaStep,
  * 1-based), both may be NULL; keeps on the device what the backward sweep needs:
- * 96 bytes per object and step where that is at most 1 GiB, else the states
- * every checkpointEvery steps.  deviceMs (may be NULL): kernel time. */
+ * 96 bytes per object and step where that is at most 1 GiB and can be had (given
+ * up again when another call of the context needs the memory: the backward sweep
+ * then repeats the forward one), else the states every checkpointEvery steps.  deviceMs (may be NULL): kernel time. */
 int ladds_gpu_adjoint_forward(ladds_gpu_ctx *ctx, const ladds_adjoint_pair *pairs, size_t nPairs, int steps,
                               int checkpointEvery, double *missSq, int32_t *tcaStep, double *loss,
                               double *deviceMs);

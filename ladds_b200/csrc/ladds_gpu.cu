@@ -235,7 +235,8 @@ struct ladds_gpu_ctx : ObjectBuffers, GridTables {
     size_t nPairs = 0;
     int steps = 0, ck = 0;
     bool forwardDone = false;
-    bool whole = false;  // rec holds every step of the forward sweep (else ckpt its checkpoints)
+    bool whole = false;    // rec holds every step of the forward sweep
+    bool ckptDone = false;  // ckpt holds its checkpoints
     double *st = nullptr, *bc = nullptr, *aom = nullptr, *miss = nullptr, *seed = nullptr, *grad = nullptr;
     double *ckpt = nullptr, *rec = nullptr, *off = nullptr;
     int *arg = nullptr;
@@ -303,11 +304,25 @@ void *deviceTake(size_t bytes) {
   return nullptr;
 }
 
+// device memory for the context.  Where there is none, the records that an
+// adjoint's forward sweep has kept for its reverse sweep give way: that sweep then
+// takes checkpoints (ladds_gpu_adjoint_backward).
+void *contextTake(ladds_gpu_ctx *c, size_t bytes) {
+  void *p = deviceTake(bytes);
+  if (p || !c->adj.rec) return p;
+  cudaFree(c->adj.rec);
+  c->adj.rec = nullptr;
+  c->adj.recCap = 0;
+  c->adj.whole = false;
+  return deviceTake(bytes);
+}
+
 // block sums of the three-level exclusive scans (objects or rows, whichever is longer)
 bool ensureScanWorkspace(ladds_gpu_ctx *c, size_t objects) {
   const size_t scanLen = std::max(objects + 1, (size_t)c->nRows + 1);
   const size_t need = 4 * (scanLen / kScanBlock + 2) + 4 * kScanBlock;
-  return growBuffer(c->scanWs, c->scanWsWords, need, deviceTake, cudaFree);
+  return growBuffer(c->scanWs, c->scanWsWords, need,
+                    [c](size_t bytes) { return contextTake(c, bytes); }, cudaFree);
 }
 
 // What a growth carries over: the population of n objects, and the cell order
@@ -341,7 +356,7 @@ int ensureCapacity(ladds_gpu_ctx *c, size_t need) {
   carriedArrays(*c, c->n, orderN, from);
   ObjectBuffers fresh;
   size_t cap = newCap;
-  char *base = static_cast<char *>(deviceTake(layoutObjects(fresh, cap, nullptr)));
+  char *base = static_cast<char *>(contextTake(c, layoutObjects(fresh, cap, nullptr)));
   std::unique_ptr<char[]> aside;
   if (!base && c->objects) {
     size_t total = 0;
@@ -398,11 +413,8 @@ int ensureCapacity(ladds_gpu_ctx *c, size_t need) {
 int ensurePairCapacity(ladds_gpu_ctx *c, size_t need) {
   if (need <= c->pairCap) return LADDS_OK;
   size_t newCap = std::max<size_t>(need + need / 2, 1);
-  ladds_pair *p = nullptr;
-  if (cudaMalloc(&p, newCap * sizeof(ladds_pair)) != cudaSuccess) {
-    cudaGetLastError();
-    return fail(c, LADDS_ERR_ALLOC, "device allocation failed (pair buffer)");
-  }
+  auto *p = static_cast<ladds_pair *>(contextTake(c, newCap * sizeof(ladds_pair)));
+  if (!p) return fail(c, LADDS_ERR_ALLOC, "device allocation failed (pair buffer)");
   if (c->dPairs) cudaFree(c->dPairs);
   c->dPairs = p;
   c->pairCap = newCap;
@@ -413,11 +425,9 @@ int ensurePairCapacity(ladds_gpu_ctx *c, size_t need) {
 int ensureCandCapacity(ladds_gpu_ctx *c, size_t need) {
   if (need <= c->candCap) return LADDS_OK;
   size_t newCap = std::max<size_t>(need + need / 2, 1);
-  uint2 *p = nullptr;  // the screened and the spilled list, newCap entries each
-  if (cudaMalloc(&p, 2 * newCap * sizeof(uint2)) != cudaSuccess) {
-    cudaGetLastError();
-    return fail(c, LADDS_ERR_ALLOC, "device allocation failed (candidate buffer)");
-  }
+  // the screened and the spilled list, newCap entries each
+  auto *p = static_cast<uint2 *>(contextTake(c, 2 * newCap * sizeof(uint2)));
+  if (!p) return fail(c, LADDS_ERR_ALLOC, "device allocation failed (candidate buffer)");
   if (c->dCand) cudaFree(c->dCand);
   c->dCand = p;
   c->candCap = newCap;
@@ -2607,11 +2617,8 @@ int ensureDev(ladds_gpu_ctx *c, T *&p, size_t &cap, size_t need) {
   if (p) cudaFree(p);
   p = nullptr;
   cap = 0;
-  if (cudaMalloc(&p, need * sizeof(T)) != cudaSuccess) {
-    cudaGetLastError();
-    p = nullptr;
-    return fail(c, LADDS_ERR_ALLOC, "device allocation for the adjoint pair batch failed");
-  }
+  p = static_cast<T *>(contextTake(c, need * sizeof(T)));
+  if (!p && need) return fail(c, LADDS_ERR_ALLOC, "device allocation for the adjoint pair batch failed");
   cap = need;
   return LADDS_OK;
 }
@@ -2646,14 +2653,17 @@ int adjPrepare(ladds_gpu_ctx *c, size_t nPairs, int steps) {
 constexpr size_t kAdjRecordBytes = (size_t)1 << 30;
 constexpr size_t kAdjRecord = 12;
 
+int adjCheckpoints(ladds_gpu_ctx *c, size_t nObj, int steps, int ck) {
+  const size_t nSeg = ((size_t)steps + ck - 1) / ck;
+  return ensureDev(c, c->adj.ckpt, c->adj.ckptCap, nSeg * 6 * nObj);
+}
+
 // whole or by segments, with the buffers of either
 int adjStorage(ladds_gpu_ctx *c, size_t nObj, int steps, int ck) {
   auto &A = c->adj;
   const size_t all = (size_t)steps * kAdjRecord * nObj;
   A.whole = all * sizeof(double) <= kAdjRecordBytes && ensureDev(c, A.rec, A.recCap, all) == LADDS_OK;
-  if (A.whole) return LADDS_OK;
-  const size_t nSeg = ((size_t)steps + ck - 1) / ck;
-  return ensureDev(c, A.ckpt, A.ckptCap, nSeg * 6 * nObj);
+  return A.whole ? LADDS_OK : adjCheckpoints(c, nObj, steps, ck);
 }
 
 int adjEphemeris(ladds_gpu_ctx *c, int steps) {
@@ -2726,6 +2736,7 @@ int ladds_gpu_adjoint_forward(ladds_gpu_ctx *c, const ladds_adjoint_pair *pairs,
   if ((rc = adjEphemeris(c, steps))) return rc;
   CK(cudaEventRecord(c->callStart, c->st));
   if (nObj) adjForward(c, A.st, (int)nObj, 0, steps, true, A.whole ? A.rec : nullptr);
+  A.ckptDone = !A.whole;
   CK(cudaEventRecord(c->callEnd, c->st));
   CK(cudaGetLastError());
   std::vector<double> miss(nPairs);
@@ -2756,10 +2767,14 @@ int ladds_gpu_adjoint_backward(ladds_gpu_ctx *c, double *dL_dx0, double *dL_dbc,
   std::lock_guard<std::mutex> lk(g_deviceMutex[c->dev & 63]);
   CK(cudaSetDevice(c->dev));
   const size_t nObj = 2 * A.nPairs;
-  const int segment = A.whole ? A.steps : std::min(A.ck, A.steps);
-  int rc = ensureDev(c, A.rec, A.recCap, (size_t)segment * kAdjRecord * nObj);
-  if (rc) return rc;
+  int rc = LADDS_OK;
+  const bool again = !A.whole && !A.ckptDone;  // the records have given way: the forward sweep again, for checkpoints
+  if (again && (rc = adjCheckpoints(c, nObj, A.steps, A.ck))) return rc;
+  const int segment = A.whole ? A.steps : std::min(A.ck, A.steps);  // the records last: a buffer taken after them could free them
+  if ((rc = ensureDev(c, A.rec, A.recCap, (size_t)segment * kAdjRecord * nObj))) return rc;
   CK(cudaEventRecord(c->callStart, c->st));
+  if (again && nObj) adjForward(c, A.st, (int)nObj, 0, A.steps, true, nullptr);
+  A.ckptDone = !A.whole;
   for (int s1 = A.steps; nObj && s1 > 0;) {
     const int s0 = (s1 - 1) / segment * segment;
     if (!A.whole) adjForward(c, A.ckpt + (size_t)(s0 / segment) * 6 * nObj, (int)nObj, s0, s1, false, A.rec);

@@ -79,3 +79,33 @@ def test_growth_beside_full_memory(capi, free_mb, grows):
         assert got.records.tobytes() == want.records.tobytes()
         for a, b in zip(ctx.get_state(), roomy.get_state()):
             assert np.array_equal(a, b)
+
+
+def test_adjoint_records_make_room(capi):
+    """The records that an adjoint's forward sweep keeps (0.85 GB here) give way to a
+    growth that needs their memory, and the reverse sweep takes its checkpoints
+    instead: equal to the bit, also when asked for twice."""
+    import torch
+
+    pop = capi.generate_population(0, 9, N + 1000)
+    first = {k: v[:N] for k, v in pop.items()}
+    more = {k: v[N:] for k, v in pop.items()}
+    with capi.Context(capi.default_config(componentMask=capi.PROP_ALL)) as ctx:
+        pairs, _ = ctx.adjoint_make_pairs(3, 4096, 1080)
+        loss, miss, tca, _ = ctx.adjoint_forward(pairs, 1080, 64)
+        dx, dbc, _ = ctx.adjoint_backward()
+    with capi.Context(capi.default_config(componentMask=capi.PROP_ALL)) as ctx:
+        ctx.upload(first)
+        taken = leave_free(1200 << 20)
+        try:
+            got = ctx.adjoint_forward(pairs, 1080, 64)
+            ctx.append(more)
+            grads = [ctx.adjoint_backward()[:2] for _ in range(2)]
+        finally:
+            del taken
+            torch.cuda.empty_cache()
+        assert ctx.size() == N + 1000
+        assert got[0] == loss and np.array_equal(got[1], miss) and np.array_equal(got[2], tca)
+        for gx, gb in grads:
+            assert np.array_equal(gx, dx) and np.array_equal(gb, dbc)
+        assert np.array_equal(ctx.download()["id"], pop["id"])
