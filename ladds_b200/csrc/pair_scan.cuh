@@ -553,9 +553,9 @@ constexpr int kTileCtasPerSm = 7;     // by its 28 KB of shared memory
 constexpr uint32_t kTileStage = 256;  // staged neighbour objects per warp and pass
 
 template <int SCREEN>
-__global__ void __launch_bounds__(kScanCta, 8) k_pair_tiles(const uint32_t *__restrict__ denseCells,
-                                                         const uint32_t *__restrict__ denseChunk, uint32_t denseCap,
-                                                         const WalkIn in, const CandSink out) {
+__device__ __forceinline__ void pairTiles(const uint32_t *__restrict__ denseCells,
+                                          const uint32_t *__restrict__ denseChunk, uint32_t denseCap, const WalkIn &in,
+                                          const CandSink &out) {
   __shared__ uint2 sCand[kScanCta / 32][kWarpCand];
   __shared__ float4 sNb[kScanCta / 32][kTileStage];
   __shared__ uint32_t sK[kScanCta / 32][kTileStage];
@@ -649,6 +649,14 @@ __global__ void __launch_bounds__(kScanCta, 8) k_pair_tiles(const uint32_t *__re
           const uint32_t half = __ballot_sync(0xffffffffu, gs != kNoGroup && 2 * __popc(peers) >= sources);
           if (half) common = __shfl_sync(0xffffffffu, gs, __ffs(half) - 1);
         }
+        if (!grp) {  // no object has a group: the loop of dense populations
+          for (uint32_t u = 0; u < m; ++u) {  // warp-uniform
+            const uint32_t k = sK[warp][u];
+            const bool pass = src && prefilterPass(mf, sNb[warp][u], cutF) && !(stBase + u < ownEnd && k <= si);
+            warpAppend<SCREEN>(pass, si, k, lane, sCand[warp], nBuf, out);
+          }
+          continue;
+        }
         if (common == kNoGroup) {
           for (uint32_t u = 0; u < m; ++u) test(u);  // warp-uniform
           continue;
@@ -697,6 +705,28 @@ __global__ void __launch_bounds__(kScanCta, 8) k_pair_tiles(const uint32_t *__re
   warpFlush(lane, sCand[warp], nBuf, out);
 }
 
+// The screens want different launch bounds.  Listed: 64 registers (a minimum of
+// eight CTAs), which leave the kernels beside an empty bin's CTAs more room (31,000
+// objects, graph step: 2450 us per 128 iterations, 2478 with 70).  Buffer: no minimum -- with it, of
+// any size, the compiler forms addresses and constants of the screen anew inside the pair loop, or
+// takes registers until fewer CTAs fit.  8e6 objects, walk and tiles at 80 and 160 km: 4.23
+// and 13.2 ms with a minimum of eight, 3.92 and 11.9 without (71 registers, seven CTAs
+// as by shared memory), 3.55 and 9.4 with the loop without groups above.
+template <int SCREEN>
+__global__ void k_pair_tiles(const uint32_t *__restrict__ denseCells, const uint32_t *__restrict__ denseChunk,
+                             uint32_t denseCap, const WalkIn in, const CandSink out);
+template <>
+__global__ void __launch_bounds__(kScanCta, 8) k_pair_tiles<LADDS_SCREEN_LISTS>(
+    const uint32_t *__restrict__ denseCells, const uint32_t *__restrict__ denseChunk, uint32_t denseCap,
+    const WalkIn in, const CandSink out) {
+  pairTiles<LADDS_SCREEN_LISTS>(denseCells, denseChunk, denseCap, in, out);
+}
+template <>
+__global__ void __launch_bounds__(kScanCta) k_pair_tiles<LADDS_SCREEN_BUFFER>(
+    const uint32_t *__restrict__ denseCells, const uint32_t *__restrict__ denseChunk, uint32_t denseCap,
+    const WalkIn in, const CandSink out) {
+  pairTiles<LADDS_SCREEN_BUFFER>(denseCells, denseChunk, denseCap, in, out);
+}
 
 // grid-stride over both candidate lists (lengths read on the device; see CandSink)
 __global__ void __launch_bounds__(256) k_pair_eval(ScanPack pk, const uint2 *__restrict__ cand,
