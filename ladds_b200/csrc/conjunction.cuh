@@ -308,12 +308,15 @@ __global__ void k_slot_mark_flags(int n, const uint8_t *__restrict__ slotMark, u
 }
 
 // compaction: dst[pos[j]] = src[j] for kept j, slots renumbered to pos[j]; the
-// arrays that the state buffers share go to separate ones (tmp)
+// arrays that the state buffers share go to separate ones (tmp); *count = the
+// number kept
 __global__ void k_compact(DevState src, DevState dst, const uint32_t *__restrict__ keep,
-                          const uint32_t *__restrict__ pos, int n, DevState tmp) {
+                          const uint32_t *__restrict__ pos, int n, DevState tmp, uint32_t *__restrict__ count) {
   const int j = blockIdx.x * blockDim.x + threadIdx.x;
-  if (j >= n || !keep[j]) return;
+  if (j >= n) return;
   const uint32_t p = pos[j];
+  if (j == n - 1) *count = p + keep[j];
+  if (!keep[j]) return;
   dst.x[p] = src.x[j];
   dst.y[p] = src.y[j];
   dst.z[p] = src.z[j];
@@ -326,6 +329,18 @@ __global__ void k_compact(DevState src, DevState dst, const uint32_t *__restrict
   tmp.radius[p] = src.radius[j];
   tmp.id[p] = src.id[j];
   tmp.parent[p] = src.parent[j];
+}
+
+// the *count compacted ones back into the shared arrays
+__global__ void k_compact_shared(DevState tmp, DevState dst, const uint32_t *__restrict__ count) {
+  const int j = blockIdx.x * blockDim.x + threadIdx.x;
+  if ((uint32_t)j >= *count) return;
+  dst.aom[j] = tmp.aom[j];
+  dst.bc[j] = tmp.bc[j];
+  dst.radius[j] = tmp.radius[j];
+  dst.id[j] = tmp.id[j];
+  dst.parent[j] = tmp.parent[j];
+  dst.tag[j] = tmp.tag[j];
 }
 
 // exclusive scan of u32 flags, three phases (block sums, scan of sums, apply)

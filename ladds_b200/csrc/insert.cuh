@@ -83,19 +83,22 @@ __global__ void k_gather_records(DevState s, const uint32_t *__restrict__ slots,
 }
 
 // Layer selection of the device-resident exchange (ladds_gpu_pack_layers):
-// sel[i] = 1 if the i-th object of the population's order -- perm for the
-// first m, then slot order -- is live and its cell layer lies in [lo, hi);
-// keep[slot] = !sel (for the removal).
-__global__ void k_layer_flags(const double *__restrict__ z, const uint32_t *__restrict__ tag, int n,
-                              const uint32_t *__restrict__ perm, int m, GridDesc g, int32_t lo, int32_t hi,
-                              uint32_t *__restrict__ sel, uint32_t *__restrict__ keep) {
-  const int i = blockIdx.x * blockDim.x + threadIdx.x;
-  if (i >= n) return;
-  const uint32_t j = i < m ? perm[i] : (uint32_t)i;
+// keep[slot] = 0 for the live objects whose cell layer lies in [lo, hi), 1 for
+// the others (the removal's flags); then sel[i] = !keep of the i-th object of the
+// population's order -- perm for the first m, then slot order.  Through perm go four
+// bytes an object, not its position and tag (1e6 objects after a scan, call 78 -> 70 us
+// with its counts fetched by one wait).
+__global__ void k_layer_flags(const double *__restrict__ z, const uint32_t *__restrict__ tag, int n, GridDesc g,
+                              int32_t lo, int32_t hi, uint32_t *__restrict__ keep) {
+  const int j = blockIdx.x * blockDim.x + threadIdx.x;
+  if (j >= n) return;
   const int32_t iz = (int32_t)cellCoord(z[j], g.boxMin[2], g.invCell, g.n[2]);
-  const uint32_t s = (!tagDummy(tag[j]) && iz >= lo && iz < hi) ? 1u : 0u;
-  sel[i] = s;
-  keep[j] = 1u - s;
+  keep[j] = (!tagDummy(tag[j]) && iz >= lo && iz < hi) ? 0u : 1u;
+}
+__global__ void k_order_select(const uint32_t *__restrict__ keep, const uint32_t *__restrict__ perm, int m, int n,
+                               uint32_t *__restrict__ sel) {
+  const int i = blockIdx.x * blockDim.x + threadIdx.x;
+  if (i < n) sel[i] = 1u - keep[i < m ? perm[i] : (uint32_t)i];
 }
 
 // slots of the selected objects in that order
@@ -105,7 +108,7 @@ __global__ void k_selected_slots(const uint32_t *__restrict__ sel, const uint32_
   if (i < n && sel[i]) slots[pos[i]] = i < m ? perm[i] : (uint32_t)i;
 }
 
-// compaction of an order: flag[i] = keep[perm[i]]; then moved[at[i]] = the new slot of a kept one
+// compaction of an order: flag[i] = keep[perm[i]]; then moved[at[i]] = the new slot of a kept one, *count = their number
 __global__ void k_order_flags(const uint32_t *__restrict__ perm, const uint32_t *__restrict__ keep, int m,
                               uint32_t *__restrict__ flag) {
   const int i = blockIdx.x * blockDim.x + threadIdx.x;
@@ -113,9 +116,11 @@ __global__ void k_order_flags(const uint32_t *__restrict__ perm, const uint32_t 
 }
 __global__ void k_order_compact(const uint32_t *__restrict__ perm, const uint32_t *__restrict__ flag,
                                 const uint32_t *__restrict__ at, const uint32_t *__restrict__ pos, int m,
-                                uint32_t *__restrict__ moved) {
+                                uint32_t *__restrict__ moved, uint32_t *__restrict__ count) {
   const int i = blockIdx.x * blockDim.x + threadIdx.x;
-  if (i < m && flag[i]) moved[at[i]] = pos[perm[i]];
+  if (i >= m) return;
+  if (i == m - 1) *count = at[i] + flag[i];
+  if (flag[i]) moved[at[i]] = pos[perm[i]];
 }
 // a truncation's flags and slots
 __global__ void k_below_flags(int n, uint32_t n0, uint32_t *__restrict__ keep, uint32_t *__restrict__ pos) {
