@@ -2241,18 +2241,16 @@ int ladds_gpu_pack_layers(ladds_gpu_ctx *c, int32_t izLo, int32_t izHi, int remo
   k_layer_flags<<<blocksFor(n, 256), 256, 0, c->st>>>(c->cur.z, c->cur.tag, n, c->grid, izLo, izHi, c->scratchA);
   k_order_select<<<blocksFor(n, 256), 256, 0, c->st>>>(c->scratchA, c->perm, m, n, sel);
   enqueueExclusiveScan(c, sel, (size_t)n, pos, c->st);
+  auto *dSelected = reinterpret_cast<uint32_t *>(c->dCandNeed);  // scratch word (reset by every scan)
+  k_selected_slots<<<blocksFor(n, 256), 256, 0, c->st>>>(sel, pos, c->perm, m, n, idx, dSelected);
   CK(cudaGetLastError());
-  unsigned last = 0;
-  c->mail->words[2] = 0;
-  CK(cudaMemcpyAsync(&c->mail->words[2], sel + (n - 1), sizeof(uint32_t), cudaMemcpyDeviceToHost, c->st));
-  const int rl = fetchCount(c, pos + (n - 1), &last);
+  unsigned count = 0;
+  const int rl = fetchCount(c, dSelected, &count);
   if (rl) return rl;
-  const size_t count = (size_t)last + (size_t)(c->mail->words[2] & 0xffffffffull);
   *nOut = count;
   if (!count) return LADDS_OK;
   if (remove && !out) return compactKept(c);  // removed without being packed
   if (count > cap) return fail(c, LADDS_ERR_CAPACITY, "pack_layers: more particles than the output holds");
-  k_selected_slots<<<blocksFor(n, 256), 256, 0, c->st>>>(sel, pos, c->perm, m, n, idx);
   k_gather_records<<<blocksFor(count, 128), 128, 0, c->st>>>(c->cur, idx, (int)count, out);
   CK(cudaGetLastError());
   CK(cudaStreamSynchronize(c->st));
