@@ -259,13 +259,18 @@ int fail(ladds_gpu_ctx *c, int code, const std::string &msg) {
       return fail(c, LADDS_ERR_CUDA, std::string(#call) + ": " + cudaGetErrorString(e_));           \
   } while (0)
 
-// positions and velocities only
+// positions and velocities only; a state's six arrays lie at one distance, and one
+// copy takes them (10,000 objects, call of two iterations with its roll-back copies:
+// 122 us with a copy each, 101 so)
 cudaError_t copyDynamic(const DevState &src, const DevState &dst, size_t n, cudaStream_t st) {
   if (n == 0) return cudaSuccess;
+  const size_t from = (size_t)(src.y - src.x) * sizeof(double), to = (size_t)(dst.y - dst.x) * sizeof(double);
+  if (copyPitchFits(from) && copyPitchFits(to))
+    return cudaMemcpy2DAsync(dst.x, to, src.x, from, n * sizeof(double), 6, cudaMemcpyDeviceToDevice, st);
   const double *sd[] = {src.x, src.y, src.z, src.vx, src.vy, src.vz};
   double *dd[] = {dst.x, dst.y, dst.z, dst.vx, dst.vy, dst.vz};
   for (int k = 0; k < 6; ++k) {
-    cudaError_t e = cudaMemcpyAsync(dd[k], sd[k], n * sizeof(double), cudaMemcpyDeviceToDevice, st);
+    const cudaError_t e = cudaMemcpyAsync(dd[k], sd[k], n * sizeof(double), cudaMemcpyDeviceToDevice, st);
     if (e != cudaSuccess) return e;
   }
   return cudaSuccess;
