@@ -649,7 +649,7 @@ __device__ __forceinline__ void pairTiles(const uint32_t *__restrict__ denseCell
           const uint32_t half = __ballot_sync(0xffffffffu, gs != kNoGroup && 2 * __popc(peers) >= sources);
           if (half) common = __shfl_sync(0xffffffffu, gs, __ffs(half) - 1);
         }
-        if (!grp) {  // no object has a group: the loop of dense populations
+        if (SCREEN == LADDS_SCREEN_BUFFER && !grp) {  // dense populations, no object with a group
           for (uint32_t u = 0; u < m; ++u) {  // warp-uniform
             const uint32_t k = sK[warp][u];
             const bool pass = src && prefilterPass(mf, sNb[warp][u], cutF) && !(stBase + u < ownEnd && k <= si);
@@ -706,8 +706,9 @@ __device__ __forceinline__ void pairTiles(const uint32_t *__restrict__ denseCell
 }
 
 // The screens want different launch bounds.  Listed: 64 registers (a minimum of
-// eight CTAs), which leave the kernels beside an empty bin's CTAs more room (31,000
-// objects, graph step: 2450 us per 128 iterations, 2478 with 70).  Buffer: no minimum -- with it, of
+// eight CTAs) and one loop, which leave the kernels beside the CTAs of an empty or
+// short bin more room (30,011 objects, graph step: 2450 us per 128 iterations, 2478 with 70
+// registers; 600,000 objects 12.95 ms, 13.03 with both loops).  Buffer: no minimum -- with it, of
 // any size, the compiler forms addresses and constants of the screen anew inside the pair loop, or
 // takes registers until fewer CTAs fit.  8e6 objects, walk and tiles at 80 and 160 km: 4.23
 // and 13.2 ms with a minimum of eight, 3.92 and 11.9 without (71 registers, seven CTAs
