@@ -72,10 +72,12 @@ __device__ __forceinline__ void loadAtmTable(AtmShared &atm) {
   }
 }
 
-// Altitudes above the fine table, where the last band's exponential has no search
-// and no division: 200,000 objects at 9000 km, full set, per step 6.5 us (10.1 by the
-// search below; within the table 6.2), 4096 adjoint pairs there 1470 us a forward
-// sweep of 1080 steps (3452; 1536).
+// Altitudes outside the fine table, out of line: inlined, the exponential slows the
+// path within the table (1e6 objects, default set, 128 iterations 19.66 ms, 19.61 so).
+// Above it the last band's exponential has no search and no division: 200,000
+// objects at 9000 km, full set, per step 6.8 us (10.1 by the search below; within
+// the table 6.2), 4096 adjoint pairs there 1583 us a forward sweep of 1080 steps (3452;
+// 1538).
 constexpr AtmRow lastAtmRow() {
   const AtmRow t[kAtmBands] = LADDS_ATM_TABLE;
   return t[kAtmBands - 1];
@@ -86,18 +88,19 @@ __device__ __forceinline__ double2 atmAbove(double h) {
   return make_double2(kAtmTop.rho0 * exp((kAtmTop.h0 - h) * (1.0 / kAtmTop.H)), 1.0 / kAtmTop.H);
 }
 // altitudes below it, and NaN
-__device__ __noinline__ double2 atmBelow(double h) {
+__device__ __forceinline__ double2 atmBelow(double h) {
   const AtmRow r = c_atm[atmBandOf(h)];
   return make_double2(r.rho0 * exp(-(h - r.h0) / r.H), 1.0 / r.H);
 }
+
+__device__ __noinline__ double2 atmOutside(double h) { return h >= (double)kAtmFine ? atmAbove(h) : atmBelow(h); }
 
 // density [kg/m^3] and 1 / H [1/km] at altitude h.  The kilometre is floor(h):
 // the low word of h + 3 * 2^51 rounded down, so a band begins exactly at its
 // edge.  exp of |x| <= 0.093 by its Taylor polynomial of degree 9 (remainder
 // x^10 / 10! < 1.4e-17), even and odd parts side by side.
 __device__ __forceinline__ double2 atmDensity(const double2 *__restrict__ fine, double h) {
-  if ((uint32_t)__double2hiint(h) >= 0x40c00000u)  // >= 8192 km, negative, NaN
-    return h >= (double)kAtmFine ? atmAbove(h) : atmBelow(h);
+  if ((uint32_t)__double2hiint(h) >= 0x40c00000u) return atmOutside(h);  // >= 8192 km, negative, NaN
   const double m = __dadd_rd(h, 6755399441055744.0);
   const double2 t = __ldg(&fine[__double2loint(m)]);
   const double x = ((m - 6755399441055744.0) + 0.5 - h) * t.y, x2 = x * x;

@@ -69,7 +69,7 @@ def test_density_from_the_ground_to_geostationary(capi, oracle):
 
 def test_altitudes_above_the_table_cost_no_more(capi):
     """Adjoint sweeps of 64 pairs lifted above 8192 km against the same pairs low down, best of
-    five: the same work but for the exponential (0.97 of the time here; 2.3 times as long
+    five: the same work but for the exponential (1.02 of the time here; 2.3 times as long
     when each evaluation searched the bands)."""
     with capi.Context(capi.default_config(componentMask=capi.PROP_ALL)) as ctx:
         pairs, _ = ctx.adjoint_make_pairs(3, 64, 360)
