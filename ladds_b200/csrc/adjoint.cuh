@@ -160,36 +160,25 @@ __device__ __forceinline__ void accelJacobian(uint32_t mask, const double r[3], 
   m[8 * 32] = zz;
 }
 
-// One FP64 Yoshida step (the expression forms of k_propagate); the three stage
-// accelerations go to acc if non-null.  e3 = the step's three stage entries.
+// One FP64 Yoshida step (the expression forms of k_propagate).  e3 = the step's three stage entries.
 __device__ __forceinline__ void adjStep(uint32_t mask, double r[3], double v[3], double aom, double bc,
-                                        const EphEntry *e3, const double2 *atm, const PropConsts &pc,
-                                        double acc[3][3]) {
+                                        const EphEntry *e3, const double2 *atm, const PropConsts &pc) {
   double a[3];
 #pragma unroll
   for (int k = 0; k < 3; ++k) r[k] += pc.hc1 * v[k];
   accel(mask, r, v, aom, bc, e3[0], atm, a);
 #pragma unroll
-  for (int k = 0; k < 3; ++k) {
-    acc[0][k] = a[k];
-    v[k] += pc.hd1 * a[k];
-  }
+  for (int k = 0; k < 3; ++k) v[k] += pc.hd1 * a[k];
 #pragma unroll
   for (int k = 0; k < 3; ++k) r[k] += pc.hc2 * v[k];
   accel(mask, r, v, aom, bc, e3[1], atm, a);
 #pragma unroll
-  for (int k = 0; k < 3; ++k) {
-    acc[1][k] = a[k];
-    v[k] += pc.hd2 * a[k];
-  }
+  for (int k = 0; k < 3; ++k) v[k] += pc.hd2 * a[k];
 #pragma unroll
   for (int k = 0; k < 3; ++k) r[k] += pc.hc2 * v[k];
   accel(mask, r, v, aom, bc, e3[2], atm, a);
 #pragma unroll
-  for (int k = 0; k < 3; ++k) {
-    acc[2][k] = a[k];
-    v[k] += pc.hd1 * a[k];
-  }
+  for (int k = 0; k < 3; ++k) v[k] += pc.hd1 * a[k];
 #pragma unroll
   for (int k = 0; k < 3; ++k) r[k] += pc.hc1 * v[k];
 }
@@ -525,9 +514,8 @@ __global__ void __launch_bounds__(128) k_adj_make_pairs(double *__restrict__ st,
   const int nObj = 2 * nPairs, a = 2 * p, b = 2 * p + 1;
   double r[3] = {st[a], st[nObj + a], st[2 * nObj + a]};
   double v[3] = {st[3 * nObj + a], st[4 * nObj + a], st[5 * nObj + a]};
-  double acc[3][3];
   const int n = tca[p];
-  for (int s = 0; s < n; ++s) adjStep(pc.mask, r, v, aom[a], bc[a], eph + 3 * s, atm, pc, acc);
+  for (int s = 0; s < n; ++s) adjStep(pc.mask, r, v, aom[a], bc[a], eph + 3 * s, atm, pc);
 #pragma unroll
   for (int c = 0; c < 3; ++c) {
     r[c] += off[6 * p + c];
@@ -535,7 +523,7 @@ __global__ void __launch_bounds__(128) k_adj_make_pairs(double *__restrict__ st,
   }
   for (int s = n - 1; s >= 0; --s) {
     const EphEntry e3[3] = {eph[3 * s + 2], eph[3 * s + 1], eph[3 * s]};
-    adjStep(back.mask, r, v, aom[b], bc[b], e3, atm, back, acc);
+    adjStep(back.mask, r, v, aom[b], bc[b], e3, atm, back);
   }
 #pragma unroll
   for (int c = 0; c < 3; ++c) {

@@ -78,7 +78,7 @@ constexpr uint32_t kMaskFull = LADDS_PROP_ALL;
 constexpr uint32_t kMaskDefault =
     LADDS_PROP_KEP | LADDS_PROP_J2 | LADDS_PROP_C22 | LADDS_PROP_S22 | LADDS_PROP_SRP | LADDS_PROP_DRAG;
 
-enum Phase { kPhProp, kPhBucket, kPhRowsort, kPhPermute, kPhCandidates, kPhEvaluate };
+enum Phase { kPhProp, kPhBucket, kPhRowsort, kPhCandidates, kPhEvaluate };
 
 // ladds_gpu_step_host moves the state in at most this many chunks, each at
 // least kHostChunkMin objects (smaller copies cost more than they overlap)
@@ -493,10 +493,6 @@ void collectTimes(ladds_gpu_ctx *c) {
         T.rowsortMs += ms;
         T.rowsortLaunches += k;
         break;
-      case kPhPermute:
-        T.permuteMs += ms;
-        T.permuteLaunches += k;
-        break;
       case kPhCandidates:
         T.candidatesMs += ms;
         T.candidatesLaunches += k;
@@ -606,12 +602,10 @@ void enqueuePropagateStaged(ladds_gpu_ctx *c, int nSteps, int ephBase, bool scan
 }
 
 // kernels launched by enqueueExclusiveScan for `count` values
-constexpr bool kScanFoldSums = true;  // two passes up to kScanBlock^2 values (else three)
-
 int exclusiveScanKernels(size_t count) {
   const int nb1 = blocksFor(count, kScanBlock);
   if (nb1 == 1) return 1;
-  if (kScanFoldSums && nb1 <= kScanBlock) return 2;
+  if (nb1 <= kScanBlock) return 2;
   return blocksFor((size_t)nb1, kScanBlock) > 1 ? 5 : 3;
 }
 
@@ -623,7 +617,7 @@ void enqueueExclusiveScan(ladds_gpu_ctx *c, const uint32_t *in, size_t count, ui
   uint32_t *s1 = c->scanWs, *s1x = s1 + nb1 + 1;
   k_scan_blocks<<<nb1, kScanBlock, 0, s>>>(in, (int)count, out, s1);
   if (nb1 == 1) return;
-  if (kScanFoldSums && nb1 <= kScanBlock) {
+  if (nb1 <= kScanBlock) {
     k_scan_add_prefix<<<nb1, kScanBlock, 0, s>>>(out, (int)count, s1);
     return;
   }
