@@ -683,7 +683,11 @@ void enqueueSort(ladds_gpu_ctx *c, cudaStream_t s) {
     PhaseScope ps(c, kPhBucket, s, 2);
     const int k = enqueueRowScan(c, s);
     ps.kernels = 1 + k;
-    k_bucket_place<<<blocksFor(c->n, kBucketThreads), kBucketThreads, 0, s>>>(
+    // blocks for the objects or, on a fine grid with few of them, for the counts that the
+    // kernel clears: 10 objects in 2.56e6 rows, iteration 339 us by their one block, 152 so
+    const int placeBlocks = std::max(blocksFor(c->n, kBucketThreads),
+                                     std::min(blocksFor((size_t)nRows + 1, 4 * kBucketThreads), c->evalBlocks));
+    k_bucket_place<<<placeBlocks, kBucketThreads, 0, s>>>(
         c->keys, c->arrival, n, nx, c->rowStart, c->sortRec, c->rowCounts, nRows + 1, c->longCount, c->denseCount,
         c->dCandCount, c->dStatus);
   }
