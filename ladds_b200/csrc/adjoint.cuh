@@ -248,8 +248,9 @@ struct EphStage {
 // has passed the barrier of stage n + 1 cannot overwrite the half that a slower
 // warp still reads for stage n.  Lanes past the last object step a copy of it
 // (every warp reaches every barrier) and write nothing.  4096 pairs, full set, per
-// step: 2.24 us with four warps that share the terms by the runtime mask and
-// all take the miss distance, 1.29 like this.
+// step: 2.56 us with four warps that share the terms by the runtime mask and
+// all take the miss distance (2.24 of it with the terms of forces.cuh), 1.41 like
+// this; 512 pairs 2.43 -> 1.33.
 template <uint32_t MASK>
 __global__ void __launch_bounds__(kAdjFwdThreads) k_adj_forward(
     const double *__restrict__ st, const double *__restrict__ bc, const double *__restrict__ aom, int nObj, int s0,
@@ -363,9 +364,10 @@ __global__ void __launch_bounds__(kAdjFwdThreads) k_adj_forward(
 // evaluate those of three steps side by side (warp = stage of a step, lane =
 // object) into shared memory, while a tenth takes the adjoint through the three
 // steps before; one block barrier per three steps, two buffers.  The producers'
-// loads are issued one batch ahead.  4096 pairs, full set, per step: 4.28 us with the
-// products of each kick formed on the chain (and the segments' states again),
-// 0.76 like this (FP64 pipe 51 % busy); 512 pairs 3.89 -> 0.45.
+// loads are issued one batch ahead.  4096 pairs, full set, per step: 6.17 us with the
+// products of each kick formed on the chain (and the segments' states again; 4.28
+// with the terms of forces.cuh), 0.79 like this (FP64 pipe 51 % busy); 512 pairs 5.07 ->
+// 0.46.
 constexpr int kAdjBatchSteps = 3;
 constexpr int kAdjProducers = 3 * kAdjBatchSteps;
 constexpr int kAdjBwdThreads = (kAdjProducers + 1) * 32;

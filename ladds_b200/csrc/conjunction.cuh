@@ -1,20 +1,20 @@
-// conjunction.cuh -- cell table and pair scan.
+// conjunction.cuh -- functor of the pair scan, its screen, and passes over the population.
 //
 // Replaces AutoPas::iteratePairwise(&CollisionFunctor) (Simulation.cpp:220,
 // external traversal) together with CollisionFunctor::AoSFunctor
 // (CollisionFunctor.cpp:40-131) and utils::distanceByLinearInterpolation
 // (DistanceApproximation.cpp:13-58).
 //
-// After the radix sort the population is gathered into cell order.  Keys are
-// row-major, (iz*ny + iy)*nx + ix, so the cells (ix-R..ix+R) of one row are a
-// contiguous key window.  rowStart[r] = first sorted index of row r.  One
-// thread per sorted object visits, like a Newton3 linked-cell traversal, each
-// neighbouring pair once: the rest of its own row window (ix..ix+R, later
-// objects only) and the rows (dz,dy) > (0,0) lexicographically, each located by
-// a binary search inside its row.  The candidate test and the functor use
-// explicitly rounded operations (__dmul_rn / __dadd_rn / __dsub_rn /
-// __ddiv_rn) in the reference's evaluation order, so results are bit-identical
-// to a binary64 CPU evaluation without FMA contraction, NaN path included.
+// Cell keys are row-major, (iz*ny + iy)*nx + ix, and the cell order sorts the
+// objects by (key, slot), so the cells (ix-R..ix+R) of one row are a contiguous
+// window of it; rowStart[r] = first position of row r.  Every pair is visited once,
+// like a Newton3 linked-cell traversal: from its earlier object, which takes the
+// rest of its own row window (ix..ix+R, later objects only) and the rows
+// (dz,dy) > (0,0) lexicographically (pair_scan.cuh: windows by the rows' cell-offset
+// tables, binary32 pre-filter and screen).  The functor uses explicitly rounded
+// operations (__dmul_rn / __dadd_rn / __dsub_rn / __ddiv_rn) in the reference's
+// evaluation order, so results are bit-identical to a binary64 CPU evaluation
+// without FMA contraction, NaN path included.
 #pragma once
 #include <algorithm>
 #include <cmath>

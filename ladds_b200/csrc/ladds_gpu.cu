@@ -1,18 +1,20 @@
 // ladds_gpu.cu -- C ABI of the B200 hot path (see include/ladds_gpu.h).
 //
-// One context = one device, one stream, the device-resident population: one
-// array per attribute in slot order, positions and velocities in two copies
-// (the propagation that ends at a scan reads the current one and writes the
-// other, and they change places) and a third that rolls a ladds_gpu_step call
-// of several iterations back when it has to be re-run.
+// One context = one device, three streams (propagation, sort, pair scan), the
+// device-resident population: one array per attribute in slot order, positions
+// and velocities in a ring of three buffers (the propagation that ends at a scan
+// reads the current one and writes the next, while the scans before it still read
+// theirs) and a fourth copy that a ladds_gpu_step call of several propagation
+// launches is undone from.
 //
-// A scan iteration is: ephemeris of the stage times -> constant memory,
-// Yoshida steps with the cell key, row count and scan record of the end state
-// (one kernel), row-start scan, scatter to the cell rows, sort inside the rows
-// with the gather of the scan records, pair scan.  The population itself is
-// never moved.
-// Multi-iteration calls are captured once into a CUDA graph per (iterations,
-// iteration % k, current buffers) and replayed.
+// A scan iteration is: ephemeris of the stage times -> constant memory (once for
+// up to 128 iterations), Yoshida steps with the cell key, row count and scan record
+// of the end state (one kernel), row-start scan, placement into the cell rows, sort
+// inside the rows with the gather of the scan records, pair scan.  The population
+// itself is never moved.
+// Calls of fewer than 125,000 objects, which launches bound, are captured into CUDA
+// graphs once they come again: one per (iterations, iteration % k, buffers and sort
+// set they begin with, objects, record capacity).
 #include <cuda_runtime.h>
 #include <omp.h>
 
@@ -508,7 +510,7 @@ void collectTimes(ladds_gpu_ctx *c) {
   c->events.clear();
 }
 
-// ----- pipeline pieces (all enqueue on c->st; no synchronisation) -----
+// ----- pipeline pieces (enqueue on the stream they are given, else on c->st; no synchronisation) -----
 
 cudaError_t enqueueEphemeris(ladds_gpu_ctx *c, int nSteps) {
   const int threads = 3 * nSteps, b = (threads + 31) / 32 * 32;
@@ -554,9 +556,14 @@ void launchPropagate(ladds_gpu_ctx *c, DevState s, DevState to, size_t lo, int n
   in.rec += lo;
   in.radius += lo;
   // three CTAs per SM: the sort and the scan of the iterations before run
-  // beside the kernel on streams of their own.  Graph step with two / three /
-  // four: 250,000 objects at every fourth iteration 22.5 / 20.7 / 18.9 us, 1e6
-  // 162 / 156 / 150 us, 2e6 391 / 381 / 391 us, 8e6 (40 km) 3331 / 3221 / 3322 us.
+  // beside the kernel on streams of their own, and four fit.  Graph step (or its like,
+  // launched one by one) in us with two / three / four, full set:
+  //   FP64, scan every step: 100,000 objects 33.3 / 32.9 / 32.9, 250,000 54.8 / 53.7 / 55.0,
+  //     500,000 97.9 / 99.7 / 100.2, 1e6 175 / 168 / 173
+  //   FP64, every fourth: 250,000 19.8 / 18.6 / 18.7, 500,000 32.6 / 31.3 / 35.6, 1e6 62.3 / 57.7 / 57.6
+  //   split, scan every step: 500,000 81.1 / 78.3 / 81.5, 1e6 148.9 / 148.4 / 144.2,
+  //     2e6 364 / 353 / 355, 8e6 (40 km) 3003 / 2986 / 2978
+  //   split, every fourth: 500,000 31.5 / 29.7 / 29.3, 1e6 59.6 / 62.2 / 62.7, 2e6 125 / 123 / 126
   const int sg = std::max(1, std::min(blocksFor((size_t)n, kStageObjects), c->evalBlocks * 3 / 4));
   const bool split = c->cfg.precision == LADDS_PRECISION_SPLIT;
   auto pick = [&](auto mask) {
@@ -2651,7 +2658,7 @@ int adjPrepare(ladds_gpu_ctx *c, size_t nPairs, int steps) {
 // are 0.85 GB of the device's 180 -- and checkpoints elsewhere, from which the
 // reverse sweep makes the records segment by segment: a second forward sweep,
 // which is the longer part.  4096 pairs, reverse sweep: 0.79 us per step from kept
-// records, 2.23 by segments of 64 steps.
+// records, 2.40 by segments of 64 steps.
 constexpr size_t kAdjRecordBytes = (size_t)1 << 30;
 constexpr size_t kAdjRecord = 12;
 

@@ -2,13 +2,14 @@
 //
 // Structure of arrays, one array per attribute of the reference Particle
 // (Particle.h:139-195) that the hot path reads, indexed by slot (the upload
-// index).  Positions and velocities are binary64 (48 B/object) in two copies:
-// the propagation that ends at a scan reads one and writes the other, so that
-// the scan of the state before it can run beside it and a step can be undone.
-// The per-object constants aom / bcInv / radius (binary64), id / parentId
-// (u64) and a u32 tag (the slot, the activity state and the dummy "deleted"
-// flag) exist once.  Cell order exists only in what the pair scan reads: the
-// row sort gathers 32-byte scan records into it.
+// index).  Positions and velocities are binary64 (48 B/object) in a ring of three
+// buffers: the propagation that ends at a scan reads one and writes the next, so
+// that it can run beside the sort and the scan of the iterations before it; a
+// fourth copy is what a call of several launches is undone from.  The per-object
+// constants aom / bcInv / radius (binary64), id / parentId (u64) and a u32 tag (the
+// slot, the activity state and the dummy "deleted" flag) exist once.  Cell order
+// exists only in what the pair scan reads: the row sort gathers 32-byte scan
+// records into it.
 #pragma once
 #include <cstdint>
 
