@@ -148,10 +148,10 @@ def algorithmic_units(n):
         # read r, v, aom, bcInv, radius, tag (76 B), write r, v (48 B), the cell key, the arrival index
         # (8 B) and the binary32 scan record (32 B)
         "propagate": {"bytes": n * (76 + 48 + 8 + 32)},
-        # placement: key, arrival index in (8), record + source out (12)
-        "bucket": {"bytes": n * (8 + 12)},
-        # row sort: record + source in (12), sorted key + slot out (8), scan record in and out (64)
-        "rowsort": {"bytes": n * (12 + 8 + 64)},
+        # placement: key, arrival index in (8), sort record out (8)
+        "bucket": {"bytes": n * (8 + 8)},
+        # row sort: sort record in (8), sorted key + slot out (8), scan record in and out (64)
+        "rowsort": {"bytes": n * (8 + 8 + 64)},
         # the state stays in slot order: no launches
         "permute": {"bytes": 0},
         # own key, slot, binary32 position (24 B) + the closest-approach screen of the pre-filtered pairs: binary32
